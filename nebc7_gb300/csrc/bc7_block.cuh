@@ -13,6 +13,8 @@
  */
 #pragma once
 
+#include <stddef.h>
+
 #include "bc7_defs.cuh"
 
 namespace nebc7 {
@@ -48,13 +50,6 @@ __device__ __forceinline__ Ep EpSwapRot(Ep ep, int rotation)
    the subset's selection list (anchor first, then ascending pixel index) with
    the visible pixels first; transparent pixels carry zero data and an
    alpha-only mask. */
-struct Area
-{
-	uint16_t px[16][4];
-	uint16_t mk[16][4];
-	uint8_t idx[16];
-};
-
 struct AreaInfo
 {
 	uint16_t minmax[8];
@@ -63,20 +58,33 @@ struct AreaInfo
 	bool opaque;
 };
 
+struct Area
+{
+	uint16_t px[16][4];
+	uint16_t mk[16][4];
+	uint8_t idx[16];
+	AreaInfo info;
+};
+
+/* The members up to P are the search passes' (kSearchWarpBytes); the rest is
+   for the draft chain, the pack and the self-check. */
 struct __align__(16) WarpState
 {
 	uint8_t img[16][4];    /* source pixels, A,G,R,B */
 	uint8_t msk[16][4];    /* mask bytes, A,G,R,B */
 	uint16_t px[16][4];    /* masked data */
 	uint16_t mk[16][4];    /* masks widened to 0 / 0xFFFF */
-	uint8_t dec[16][4];    /* decoded block */
 	Area area1;
-	Area sub[3];
+	Area sub[2];
+	Params P;              /* the preset of the block's texture */
+	uint8_t dec[16][4];    /* decoded block */
 	int scan[64];
 	int ways[16];
 	int loops[16];
 	int best[16];
 };
+
+constexpr size_t kSearchWarpBytes = (offsetof(WarpState, dec) + 15) & ~size_t(15);
 
 /* Block-wide values shared by the mode encoders (the scalar part of the
    reference's Cell, src/Bc7Core.h:55). */
@@ -439,63 +447,27 @@ __device__ __forceinline__ void SwapPair(uint16_t* b, int lane)
 	b[lane + 1] = t;
 }
 
-/* Bounds, counts and channel orientation of the pixel subset `member`
-   (bit i = pixel i); order-independent, so a lane can evaluate any subset. */
-__device__ inline NEBC7_SHARED AreaInfo AreaStats(const WarpState& st, const CellRegs& R, const Params& P, uint32_t member)
+/* Sums of a subset's visible pixels: per channel, and over the products of
+   two. */
+struct SubsetSums
 {
-	AreaInfo a;
-	const uint32_t vis = member & R.visible;
-	a.count = __popc(member);
-	a.active = __popc(vis);
-	a.zero = 0;  /* the caller knows the subset's anchor */
+	int sum[4];
+	int GR, RB, BG, AG, AR, AB;
+};
 
-	int m0[4] = { 255, 255, 255, 255 }, m1[4] = { 0, 0, 0, 0 };
-	int sum[4] = { 0, 0, 0, 0 };
-	int sGR = 0, sRB = 0, sBG = 0, sAG = 0, sAR = 0, sAB = 0;
-	const bool fast = (R.visible == 0xFFFF) && R.opaque;
-	if (!fast && a.active < a.count)
-		m0[0] = 0;
-	for (int i = 0; i < 16; i++)
-	{
-		if (!((vis >> i) & 1))
-			continue;
-		const int v0 = st.px[i][0], v1 = st.px[i][1], v2 = st.px[i][2], v3 = st.px[i][3];
-		const int v[4] = { v0, v1, v2, v3 };
-		for (int c = 0; c < 4; c++)
-		{
-			m0[c] = min(m0[c], v[c]);
-			m1[c] = max(m1[c], v[c]);
-			sum[c] += v[c];
-		}
-		sGR += v1 * v2;
-		sRB += v2 * v3;
-		sBG += v3 * v1;
-		sAG += v1 * v0;
-		sAR += v2 * v0;
-		sAB += v3 * v0;
-	}
-	if (!fast)
-	{
-		for (int c = 0; c < 4; c++)
-			if (m1[c] < m0[c])
-				m0[c] = 0;
-	}
+/* Orients the bounds mb (min, max per channel; a.bounds on return) by the
+   signs of the channels' covariances (src/Bc7Core.cpp:330-489). */
+static __device__ NEBC7_SHARED void OrientBounds(AreaInfo& a, const SubsetSums& m, const Params& P)
+{
 	uint16_t mb[8];
-	for (int c = 0; c < 4; c++)
-	{
-		mb[2 * c] = uint16_t(m0[c]);
-		mb[2 * c + 1] = uint16_t(m1[c]);
-	}
 	for (int k = 0; k < 8; k++)
-		a.minmax[k] = mb[k];
-
-	a.opaque = fast ? true : (mb[0] == 255);
+		mb[k] = a.minmax[k];
 	const long long n = a.active;
 	if (a.opaque)
 	{
-		long long covGR = (long long)int(unsigned(sGR) * unsigned(n) - unsigned(sum[1]) * unsigned(sum[2]));
-		long long covRB = (long long)int(unsigned(sRB) * unsigned(n) - unsigned(sum[2]) * unsigned(sum[3]));
-		long long covBG = (long long)int(unsigned(sBG) * unsigned(n) - unsigned(sum[3]) * unsigned(sum[1]));
+		long long covGR = (long long)int(unsigned(m.GR) * unsigned(n) - unsigned(m.sum[1]) * unsigned(m.sum[2]));
+		long long covRB = (long long)int(unsigned(m.RB) * unsigned(n) - unsigned(m.sum[2]) * unsigned(m.sum[3]));
+		long long covBG = (long long)int(unsigned(m.BG) * unsigned(n) - unsigned(m.sum[3]) * unsigned(m.sum[1]));
 		if (covGR < 0)
 		{
 			SwapPair(mb, 4);
@@ -538,12 +510,12 @@ __device__ inline NEBC7_SHARED AreaInfo AreaStats(const WarpState& st, const Cel
 	}
 	else
 	{
-		long long covGR = (long long)int(unsigned(sGR) * unsigned(n) - unsigned(sum[1]) * unsigned(sum[2]));
-		long long covRB = (long long)int(unsigned(sRB) * unsigned(n) - unsigned(sum[2]) * unsigned(sum[3]));
-		long long covBG = (long long)int(unsigned(sBG) * unsigned(n) - unsigned(sum[3]) * unsigned(sum[1]));
-		long long covAG = (long long)int(unsigned(sAG) * unsigned(n) - unsigned(sum[1]) * unsigned(sum[0]));
-		long long covAR = (long long)int(unsigned(sAR) * unsigned(n) - unsigned(sum[2]) * unsigned(sum[0]));
-		long long covAB = (long long)int(unsigned(sAB) * unsigned(n) - unsigned(sum[3]) * unsigned(sum[0]));
+		long long covGR = (long long)int(unsigned(m.GR) * unsigned(n) - unsigned(m.sum[1]) * unsigned(m.sum[2]));
+		long long covRB = (long long)int(unsigned(m.RB) * unsigned(n) - unsigned(m.sum[2]) * unsigned(m.sum[3]));
+		long long covBG = (long long)int(unsigned(m.BG) * unsigned(n) - unsigned(m.sum[3]) * unsigned(m.sum[1]));
+		long long covAG = (long long)int(unsigned(m.AG) * unsigned(n) - unsigned(m.sum[1]) * unsigned(m.sum[0]));
+		long long covAR = (long long)int(unsigned(m.AR) * unsigned(n) - unsigned(m.sum[2]) * unsigned(m.sum[0]));
+		long long covAB = (long long)int(unsigned(m.AB) * unsigned(n) - unsigned(m.sum[3]) * unsigned(m.sum[0]));
 		if (covAG < 0)
 		{
 			SwapPair(mb, 2);
@@ -618,13 +590,130 @@ __device__ inline NEBC7_SHARED AreaInfo AreaStats(const WarpState& st, const Cel
 	}
 	for (int k = 0; k < 8; k++)
 		a.bounds[k] = mb[k];
+}
+
+/* Bounds, counts and channel orientation of the pixel subset `member`
+   (bit i = pixel i); order-independent, so a lane can evaluate any subset. */
+static __device__ NEBC7_SHARED AreaInfo AreaStats(const WarpState& st, const CellRegs& R, const Params& P, uint32_t member)
+{
+	AreaInfo a;
+	const uint32_t vis = member & R.visible;
+	a.count = __popc(member);
+	a.active = __popc(vis);
+	a.zero = 0;  /* the caller knows the subset's anchor */
+
+	int m0[4] = { 255, 255, 255, 255 }, m1[4] = { 0, 0, 0, 0 };
+	SubsetSums m = {};
+	const bool fast = (R.visible == 0xFFFF) && R.opaque;
+	if (!fast && a.active < a.count)
+		m0[0] = 0;
+	for (int i = 0; i < 16; i++)
+	{
+		if (!((vis >> i) & 1))
+			continue;
+		const int v0 = st.px[i][0], v1 = st.px[i][1], v2 = st.px[i][2], v3 = st.px[i][3];
+		const int v[4] = { v0, v1, v2, v3 };
+		for (int c = 0; c < 4; c++)
+		{
+			m0[c] = min(m0[c], v[c]);
+			m1[c] = max(m1[c], v[c]);
+			m.sum[c] += v[c];
+		}
+		m.GR += v1 * v2;
+		m.RB += v2 * v3;
+		m.BG += v3 * v1;
+		m.AG += v1 * v0;
+		m.AR += v2 * v0;
+		m.AB += v3 * v0;
+	}
+	if (!fast)
+	{
+		for (int c = 0; c < 4; c++)
+			if (m1[c] < m0[c])
+				m0[c] = 0;
+	}
+	for (int c = 0; c < 4; c++)
+	{
+		a.minmax[2 * c] = uint16_t(m0[c]);
+		a.minmax[2 * c + 1] = uint16_t(m1[c]);
+	}
+	a.opaque = fast ? true : (m0[0] == 255);
+	OrientBounds(a, m, P);
 	return a;
+}
+
+/* The same for the whole warp and one subset, its pixels on the lanes, into
+   shared memory: about 20 warp reductions instead of 16 passes over the
+   pixels.  `orient`: also the bounds' orientation, which only the
+   candidate lists need. */
+static __device__ NEBC7_SHARED void SubsetStats(AreaInfo& out, const WarpState& st, const CellRegs& R, const Params& P, uint32_t member,
+	int anchor, bool orient, int lane)
+{
+	const uint32_t vis = member & R.visible;
+	const bool on = (vis >> lane) & 1;   /* lanes 16..31 have no pixel */
+	const bool fast = (R.visible == 0xFFFF) && R.opaque;
+	unsigned v[4] = { 0, 0, 0, 0 };
+	if (on)
+	{
+		const ushort4 px = *reinterpret_cast<const ushort4*>(st.px[lane]);
+		v[0] = px.x, v[1] = px.y, v[2] = px.z, v[3] = px.w;
+	}
+	AreaInfo a;
+	a.count = __popc(member);
+	a.active = __popc(vis);
+	a.zero = anchor;
+	unsigned m0[4], m1[4];
+#pragma unroll
+	for (int c = 0; c < 4; c++)
+	{
+		/* an opaque block's alpha is 255 throughout */
+		m0[c] = c == 0 && fast ? 255u : __reduce_min_sync(kFull, on ? v[c] : 255u);
+		m1[c] = c == 0 && fast ? 255u : __reduce_max_sync(kFull, v[c]);
+	}
+	if (!fast)
+	{
+		if (a.active < a.count)
+			m0[0] = 0;
+#pragma unroll
+		for (int c = 0; c < 4; c++)
+			if (m1[c] < m0[c])
+				m0[c] = 0;
+	}
+	a.opaque = fast || m0[0] == 255;
+#pragma unroll
+	for (int c = 0; c < 4; c++)
+	{
+		a.bounds[2 * c] = a.minmax[2 * c] = uint16_t(m0[c]);
+		a.bounds[2 * c + 1] = a.minmax[2 * c + 1] = uint16_t(m1[c]);
+	}
+	if (orient)
+	{
+		SubsetSums m = {};
+#pragma unroll
+		for (int c = 1; c < 4; c++)
+			m.sum[c] = int(__reduce_add_sync(kFull, v[c]));
+		m.GR = int(__reduce_add_sync(kFull, v[1] * v[2]));
+		m.RB = int(__reduce_add_sync(kFull, v[2] * v[3]));
+		m.BG = int(__reduce_add_sync(kFull, v[3] * v[1]));
+		if (!a.opaque)
+		{
+			m.sum[0] = int(__reduce_add_sync(kFull, v[0]));
+			m.AG = int(__reduce_add_sync(kFull, v[1] * v[0]));
+			m.AR = int(__reduce_add_sync(kFull, v[2] * v[0]));
+			m.AB = int(__reduce_add_sync(kFull, v[3] * v[0]));
+		}
+		OrientBounds(a, m, P);
+	}
+	__syncwarp();
+	if (lane == 0)
+		out = a;
+	__syncwarp();
 }
 
 /* Writes the ordered pixel list of a subset into `ar` (lanes 0..15).
    `anchor` is the subset's first pixel; members follow in ascending order,
    visible pixels first. */
-__device__ inline NEBC7_SHARED void BuildAreaList(Area& ar, const WarpState& st, const CellRegs& R, uint32_t member, int anchor, int lane)
+static __device__ NEBC7_SHARED void BuildAreaList(Area& ar, const WarpState& st, const CellRegs& R, uint32_t member, int anchor, int lane)
 {
 	uint32_t rest = member & ~(1u << anchor);
 	/* position of every member in the selection order */

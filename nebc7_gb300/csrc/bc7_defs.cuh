@@ -97,6 +97,8 @@ struct LevelTables
 	const uint8_t* d4h;    /* [511][256] nibbles, by differences (HalfAt) */
 	const uint8_t* d2h;    /* [511][256] nibbles, by differences (HalfAt) */
 	const uint8_t* d3v8;   /* [511][512] bytes of 3-bit indices, by differences (DiffAt) */
+	const uint8_t* h4s;    /* [511][512] squares of the d4h entries, a byte each, by differences (DiffAt) */
+	const uint8_t* h2s;    /* [511][512] squares of the d2h entries */
 };
 
 /* Per-launch encoder settings: the reference's InitTables flags

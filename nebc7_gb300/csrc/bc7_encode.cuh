@@ -173,6 +173,14 @@ __device__ __forceinline__ void LoadCell(WarpState& st, const BlockRef& b, CellR
 	R.opaque = __reduce_and_sync(kFull, alphaAnd) == 255;
 }
 
+/* The whole block as an area: st.area1, and its values in R.a1. */
+__device__ __forceinline__ void BuildWholeBlock(WarpState& st, CellRegs& R, const Params& P, int lane)
+{
+	SubsetStats(st.area1.info, st, R, P, 0xFFFF, 0, true, lane);
+	R.a1 = st.area1.info;
+	BuildAreaList(st.area1, st, R, 0xFFFF, 0, lane);
+}
+
 template<int kD, bool NORMAL>
 __device__ void EncodeBlockAt(WarpState& st, SearchState* ss, const BlockRef& b, const LevelTables& T, const Params& P, int lane)
 {
@@ -236,9 +244,7 @@ __device__ void EncodeBlockAt(WarpState& st, SearchState* ss, const BlockRef& b,
 	double qa = 1.0, qc = 1.0;
 	if (R.errTotal > 0)
 	{
-		R.a1 = AreaStats(st, R, P, 0xFFFF);
-		R.a1.zero = 0;
-		BuildAreaList(st.area1, st, R, 0xFFFF, 0, lane);
+		BuildWholeBlock(st, R, P, lane);
 		R.personalMode = -1;
 		R.personalParam = -1;
 
@@ -351,6 +357,28 @@ __device__ __forceinline__ void BlockFinished(const TexDesc& d, int lane)
 	__syncwarp();
 }
 
+/* The texture's preset and the tables in shared memory: the out-of-line
+   passes take them by reference, and a reference to a local copy or a
+   parameter would read the thread's stack. */
+__device__ __forceinline__ const Params& SharedParams(WarpState& st, const TexDesc& d, int lane)
+{
+	__syncwarp();
+	if (lane == 0)
+		st.P = d.P;
+	__syncwarp();
+	return st.P;
+}
+
+__device__ __forceinline__ void ShareTables(LevelTables (&tables)[2], const LevelTables& T0, const LevelTables& T1)
+{
+	if (threadIdx.x == 0)
+	{
+		tables[0] = T0;
+		tables[1] = T1;
+	}
+	__syncthreads();
+}
+
 /* Encodes queue position k of the launch. */
 template<int kD, bool NORMAL>
 __device__ __forceinline__ void EncodeQueued(WarpState& st, SearchState* ss, const Job& job, const LevelTables& T0,
@@ -359,7 +387,7 @@ __device__ __forceinline__ void EncodeQueued(WarpState& st, SearchState* ss, con
 	TexDesc d;
 	BlockRef b;
 	QueuedBlock(job, k, d, b);
-	const Params P = d.P;
+	const Params& P = SharedParams(st, d, lane);
 	if (kD == kAnyDenoise)
 	{
 		if (d.denoise)
@@ -409,6 +437,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, (SHAPE == kShapeOutlined ||
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	WarpState& st = reinterpret_cast<WarpState*>(encodeSmem)[warp];
+	__shared__ LevelTables tables[2];
+	ShareTables(tables, T0, T1);
 	SearchState* ss = NORMAL ? reinterpret_cast<SearchState*>(encodeSmem + kWarpsPerCta * sizeof(WarpState)) + warp : nullptr;
 	for (;;)
 	{
@@ -418,7 +448,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, (SHAPE == kShapeOutlined ||
 		k = __shfl_sync(kFull, k, 0);
 		if (k >= job.total)
 			break;
-		EncodeQueued<kD, NORMAL>(st, ss, job, T0, T1, k, lane);
+		EncodeQueued<kD, NORMAL>(st, ss, job, tables[0], tables[1], k, lane);
 	}
 }
 

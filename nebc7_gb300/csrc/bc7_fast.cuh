@@ -474,9 +474,9 @@ __device__ void FinalPackPartitioned(WarpState& st, CellRegs& R, const Params& P
 	{
 		const uint32_t member = Member(part, s);
 		const int anchor = Anchor(NS, p, s);
-		AreaInfo ai = AreaStats(st, R, P, member);
-		ai.zero = anchor;
+		SubsetStats(st.sub[0].info, st, R, P, member, anchor, false, lane);
 		BuildAreaList(st.sub[0], st, R, member, anchor, lane);
+		const AreaInfo& ai = st.sub[0].info;
 		ep[s] = R.best[s];
 		if (MODE != 7)
 			ep[s] |= 0xFFFF;

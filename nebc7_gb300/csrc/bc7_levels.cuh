@@ -37,16 +37,6 @@ __device__ __forceinline__ int Wadd(int a, int b) { return int(unsigned(a) + uns
 __device__ __forceinline__ int Wsub(int a, int b) { return int(unsigned(a) - unsigned(b)); }
 __device__ __forceinline__ unsigned Shr32(unsigned v, unsigned s) { return v >> (s & 31); }
 
-/* Whether the scans read the reduced tables of 2- and 3-bit indices through
-   the 8-bit difference tables (DiffBase) or in the reference's per-x
-   layout.  The difference tables serve the full searches best; the compact
-   default-preset kernel, whose time goes to the Mode6Index2 refinement,
-   keeps the per-x layout (its translation unit sets 0). */
-#ifndef NEBC7_REDUCED_BY_DIFF
-#define NEBC7_REDUCED_BY_DIFF 1
-#endif
-constexpr bool kReducedByDiff = NEBC7_REDUCED_BY_DIFF != 0;
-
 /* A reduced table's s-bit endpoint expanded to 8 bits by bit replication. */
 __device__ __forceinline__ int ExpandTo8(int v, int s)
 {
@@ -143,9 +133,24 @@ __device__ __forceinline__ unsigned BitonicSort32(unsigned v, int lane)
 	return v;
 }
 
-__device__ __forceinline__ unsigned MergeTop(unsigned list, unsigned batch, int lane, int N)
+/* Folds the lanes' keys (`want`: the lanes with one below the list's last)
+   into the list of the N smallest.  A few keys are inserted one by one (about
+   12 instructions each), more by a bitonic sort and merge (about 90). */
+__device__ __forceinline__ unsigned MergeTop(unsigned list, unsigned key, unsigned want, int lane, int N)
 {
-	const unsigned s = BitonicSort32(batch, lane);
+	if (__popc(want) <= 6)
+	{
+		do
+		{
+			const unsigned k = __shfl_sync(kFull, key, __ffs(want) - 1);
+			want &= want - 1;
+			const int at = __popc(__ballot_sync(kFull, list < k));
+			const unsigned up = __shfl_up_sync(kFull, list, 1);
+			list = lane < at ? list : (lane == at ? k : up);
+		} while (want);
+		return lane < N ? list : 0xFFFFFFFFu;
+	}
+	const unsigned s = BitonicSort32((want >> lane) & 1 ? key : 0xFFFFFFFFu, lane);
 	const unsigned r = __shfl_sync(kFull, s, 31 - lane);
 	unsigned m = min(list, r);
 #pragma unroll
@@ -157,25 +162,80 @@ __device__ __forceinline__ unsigned MergeTop(unsigned list, unsigned batch, int 
 	return lane < N ? m : 0xFFFFFFFFu;
 }
 
-/* The distinct values of channel `offset` among the first `count` pixels,
-   with their multiplicities, into uniq[] (value | count << 16); returns how
-   many.  The scans sum a candidate's error once per distinct value (the
-   integer sums, and so the saturated ones, are the same). */
-__device__ __forceinline__ int UniqueValues(const Area& ar, int count, int offset, int* uniq, int lane)
+/* The distinct values of channel `c` among the first `count` pixels of an
+   area: the table offset x * stride, and the multiplicity with the value
+   above it (count | x << 8).  The scans sum a candidate's error once per
+   distinct value (the integer sums, and so the saturated ones, are the
+   same).  The smallest and the largest value (L, H) come first: they reject
+   most candidates, which the scans test after every fourth value.  Entries
+   of count 0 fill up to a multiple of 4.  Returns how many values. */
+__device__ __forceinline__ int DistinctValues(const Area& ar, int count, int c, int L, int H, int stride, int2* values, int lane)
 {
-	const int x = lane < count ? int(ar.px[lane & 15][offset]) : -1 - lane;
+	const int x = lane < count ? int(ar.px[lane & 15][c]) : -1 - lane;
 	const unsigned peers = __match_any_sync(kFull, x);
 	const bool leader = lane < count && (__ffs(peers) - 1) == lane;
-	const unsigned lm = __ballot_sync(kFull, leader);
-	const int n = __popc(lm);
+	const unsigned all = __ballot_sync(kFull, leader);
+	const unsigned low = __ballot_sync(kFull, leader && x == L);
+	const unsigned high = __ballot_sync(kFull, leader && x == H) & ~low;
+	const unsigned rest = all & ~(low | high);
+	const int n = __popc(all), first = __popc(low | high);
 	if (leader)
-		uniq[__popc(lm & ((1u << lane) - 1))] = x | (__popc(peers) << 16);
-	/* zero entries (value 0, count 0) up to a multiple of 4, so that a scan
-	   can read four at a time */
+	{
+		const int slot = x == L ? 0 : (x == H ? __popc(low) : first + __popc(rest & ((1u << lane) - 1)));
+		values[slot] = make_int2(x * stride, __popc(peers) | (x << 8));
+	}
 	if (lane >= n && lane < ((n + 3) & ~3))
-		uniq[lane] = 0;
+		values[lane] = make_int2(0, 0);
 	__syncwarp();
 	return n;
+}
+
+/* Four distinct values in registers: the first four, which every batch of a
+   scan reads. */
+struct ValueGroup
+{
+	int off[4];
+	unsigned mult[4];
+
+	__device__ __forceinline__ void Load(const int2* values)
+	{
+		const int4 a = reinterpret_cast<const int4*>(values)[0], b = reinterpret_cast<const int4*>(values)[1];
+		off[0] = a.x, off[1] = a.z, off[2] = b.x, off[3] = b.z;
+		mult[0] = a.y & 0xFF, mult[1] = a.w & 0xFF, mult[2] = b.y & 0xFF, mult[3] = b.w & 0xFF;
+	}
+
+	/* sum of mult * D^2; SQUARED: the table holds the squares */
+	template<bool SQUARED>
+	__device__ __forceinline__ unsigned Sum(const uint8_t* row) const
+	{
+		const unsigned v0 = row[off[0]], v1 = row[off[1]], v2 = row[off[2]], v3 = row[off[3]];
+		if (SQUARED)
+			return (mult[0] * v0 + mult[1] * v1) + (mult[2] * v2 + mult[3] * v3);
+		return (mult[0] * v0 * v0 + mult[1] * v1 * v1) + (mult[2] * v2 * v2 + mult[3] * v3 * v3);
+	}
+};
+
+/* Error sum of a lane's candidate (`row`: its place in the table, the values'
+   offsets go from there), given up after a group of four values once no
+   lane's sum is at most `limit`.  Returns whether some lane's is.
+   Warp-collective. */
+template<bool SQUARED>
+__device__ __forceinline__ bool CandidateSum(const uint8_t* row, const ValueGroup& first, const int2* values, int n, bool on, int limit,
+	int& sum)
+{
+	unsigned s = first.Sum<SQUARED>(row);
+	for (int u = 4;; u += 4)
+	{
+		if (!__any_sync(kFull, on && int(s) <= limit))
+			return false;
+		if (u >= n)
+			break;
+		ValueGroup g;
+		g.Load(values + u);
+		s += g.Sum<SQUARED>(row);
+	}
+	sum = int(s);
+	return true;
 }
 
 /* Sets node 0 (a zero-error candidate) of a list. */
@@ -187,12 +247,33 @@ __device__ __forceinline__ ChanList ZeroList(int2* nodes, int color, int lane)
 	return ChanList{ 0, 1 };
 }
 
-/* LevelsBuffer and LevelsBufferHalf: writes up to maxSize nodes (err, color). */
+/* Place of candidate cc in a table: by differences (DiffBase), or the
+   per-x layout of mode 1's shared-p-bit table. */
+__device__ __forceinline__ int CandidateBase(int cc, int shift, bool byDiff)
+{
+	return byDiff ? DiffBase(cc, shift) : cc;
+}
+
+/* Table offset of a value x from a candidate's place: x times this. */
+__device__ __forceinline__ int ValueStride(int shift, bool byDiff)
+{
+	return byDiff ? -513 : 1 << (2 * shift);
+}
+
+/* LevelsBuffer and LevelsBufferHalf: writes up to maxSize nodes (err, color).
+ *
+ * What bounds it: instruction issue, about 1200 candidates a scan in the
+ * default preset.  Every row of the window has the same candidates (low
+ * endpoints up to the window's, rounded up as the reference's 16-wide chunks
+ * do), so rows and columns are taken as one sequence of candidates in
+ * ascending order, 32 a batch with every lane in use, and a batch ends after
+ * the four values that reject most unless a lane can still enter the list. */
 template<int kD, bool HALF>
-__device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& ar, const AreaInfo& ai, int offset, int weight,
-	int water, int bits, int pbits, bool transparent, const uint8_t* table, bool byDiff, int maxSize, int* uniq, int lane)
+__device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
+	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, int lane)
 {
 	ChanList res{ MaxColorError<kD>() * 2, 0 };
+	const AreaInfo& ai = ar.info;
 	const int shift = bits + int(pbits >= 0 || HALF);
 	const int count = transparent ? ai.active : ai.count;
 	if (transparent && !count)
@@ -217,109 +298,63 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	}
 
 	const Window win = MakeWindow(L, H, d, bits, shift);
-	unsigned top16;
-	if (HALF)
-	{
-		top = min(top, 15 * 15 * 16 + 1);
-		top16 = unsigned(top);
-	}
-	else
-	{
-		if (top > 0xFFFF)
-			top = 0xFFFF;
-		top16 = unsigned(top) & 0xFFFF;
-	}
-	const bool topNeg = HALF && top < 0;   /* signed compare rejects everything */
+	/* errors up to `limit` are below the top: the half tables compare signed
+	   (a negative top rejects everything), the byte tables the low 16 bits */
+	int limit = HALF ? min(top, 15 * 15 * 16 + 1) - 1 : (min(top, 0xFFFF) & 0xFFFF) - 1;
 
-	/* byte tables by (x, c); with 8-bit endpoints (shift 8) the byte table
-	   goes by DiffAt and the half tables by HalfAt */
-	const int rowSize = 1 << (2 * shift);
-	const bool diff = shift == 8 || (kReducedByDiff && byDiff);
-	const int nu = UniqueValues(ar, count, offset, uniq, lane);
 	const bool pvar = HALF || pbits >= 0;
 	const int pH = reverse ? (pbits & 1) : (pbits >> 8);
 	const int pL = reverse ? (pbits >> 8) : (pbits & 1);
+	const int step = pvar ? 2 : 1;
+	/* low endpoints of a row: 0 .. LH | 7; a window of a negative top that
+	   wrapped below zero leaves the part of the first chunk that the
+	   reference's shift count (modulo 32) does */
+	const int span = win.LH >= 0 ? (win.LH | 7) : ((win.LH | 7) & (pvar ? 31 : 15));
+	const int rowLen = pvar ? (span >> 1) + 1 : span + 1;
+	const int stepRows = 32 / rowLen, stepCols = 32 - stepRows * rowLen;
+
+	const int n = DistinctValues(ar, count, offset, L, H, ValueStride(shift, byDiff), values, lane);
+	ValueGroup first;
+	first.Load(values);
 
 	/* list: the maxSize smallest keys so far, lane j the j-th; thr: its last
-	   key (all ones until the list is full), which changes only on a merge.
-	   The number of kept candidates matters only up to maxSize, which is the
-	   number of filled list entries, and a list whose last key has error 0
-	   means maxSize zero-error candidates were found. */
+	   key (all ones until the list is full), which changes only on a merge */
 	unsigned list = 0xFFFFFFFFu;
 	unsigned thr = 0xFFFFFFFFu;
-	const int rowStep = pvar ? 2 : 1;
-	/* hL - cH = LH for every row: when LH is below one chunk, only the first
-	   chunk of a row can be on and a batch takes two rows (lanes 16..31 the
-	   second); the candidate set and the kept keys are unchanged */
-	const int W = pvar ? 32 : 16;
-	const bool twoRows = win.LH < W;
-	for (int iH0 = win.HL + (pvar ? pH : 0); iH0 < win.HH; iH0 += twoRows ? 2 * rowStep : rowStep)
+	int row = lane / rowLen, col = lane - row * rowLen;
+	int iH = win.HL + (pvar ? pH : 0);   /* the batch's first row */
+	while (iH < win.HH)
 	{
-		/* candidates in batches of 32: two 16-candidate chunks per batch */
-		for (int b = 0;; b++)
+		const int myH = iH + row * step;
+		const bool on = myH < win.HH;
+		const int cc = on ? (myH << shift) + col * step + (pvar ? pL : 0) : 0;
+		int s;
+		if (CandidateSum<HALF>(table + CandidateBase(cc, shift, byDiff), first, values, n, on, limit, s))
 		{
-			const int half = lane >> 4, j = lane & 15;
-			const int iH = twoRows ? iH0 + half * rowStep : iH0;
-			const int cH = iH << shift;
-			const int hL = win.LH + cH;
-			const int chunk = twoRows ? b : 2 * b + half;
-			int c, cc;
-			unsigned flags;
-			if (pvar)
+			const unsigned key = (unsigned(s) << 16) | unsigned(cc);
+			const unsigned want = __ballot_sync(kFull, on && s <= limit && key < thr);
+			if (want)
 			{
-				c = cH + 32 * chunk;
-				cc = c + pL + 2 * j;
-				flags = Shr32(~0u, unsigned(max(0, Wsub(c | 31, hL | 7))));
-			}
-			else
-			{
-				c = cH + 16 * chunk;
-				cc = c + j;
-				flags = Shr32(~0u, unsigned(max(0, Wsub(c | 15, hL | 7))) << 1);
-			}
-			const bool chunkOn = (iH < win.HH) && ((c == cH) || (c <= hL));
-			const bool on = chunkOn && ((flags >> (2 * j)) & 1);
-			if (!__any_sync(kFull, chunkOn))
-				break;
-			unsigned key = 0xFFFFFFFFu;
-			if (on)
-			{
-				/* the per-x build reads the 8-bit table by DiffAt, as DiffBase with s = 8 */
-				const int dbase = kReducedByDiff ? DiffBase(cc, shift) : 0;
-				/* four distinct values per step, their table reads in flight
-				   together (unsigned sums do not depend on the order) */
-				auto term = [&](int e) {
-					const int x = e & 0xFFFF;
-					unsigned v;
-					if (HALF)
-						v = HalfAt(table, x, cc & 0xFF, cc >> 8);
-					else if (diff)
-						v = kReducedByDiff ? table[dbase - 513 * x] : DiffAt(table, x, cc & 0xFF, cc >> 8);
-					else
-						v = table[size_t(x) * rowSize + cc];
-					return unsigned(e >> 16) * v * v;
-				};
-				unsigned s = 0;
-				for (int u = 0; u < nu; u += 4)
-				{
-					const int4 e4 = *reinterpret_cast<const int4*>(uniq + u);
-					s += (term(e4.x) + term(e4.y)) + (term(e4.z) + term(e4.w));
-				}
-				if (!HALF && s > 0xFFFF)
-					s = 0xFFFF;
-				const bool keep = HALF ? (!topNeg && int(s) < top) : (s < top16);
-				if (keep)
-					key = (s << 16) | unsigned(cc);
-			}
-			if (__any_sync(kFull, key < thr))
-			{
-				list = MergeTop(list, key < thr ? key : 0xFFFFFFFFu, lane, maxSize);
+				list = MergeTop(list, key, want, lane, maxSize);
 				thr = __shfl_sync(kFull, list, maxSize - 1);
+				limit = min(limit, int(thr >> 16));
+				/* maxSize zero-error candidates found: later ones (larger c)
+				   cannot enter */
+				if (thr < 0x10000u)
+					break;
 			}
 		}
-		/* maxSize zero-error candidates found: later ones (larger c) cannot enter */
-		if (thr < 0x10000u)
-			break;
+		/* the next 32 candidates; row stays relative to the batch's first */
+		row += stepRows;
+		col += stepCols;
+		if (col >= rowLen)
+		{
+			col -= rowLen;
+			row++;
+		}
+		const int ahead = __shfl_sync(kFull, row, 0);
+		iH += ahead * step;
+		row -= ahead;
 	}
 	const int stored = __popc(__ballot_sync(kFull, list != 0xFFFFFFFFu));
 	if (stored)
@@ -334,23 +369,23 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	return res;
 }
 
-/* Out-of-line copy of the scan for its many call sites; the Mode6Index2
-   refinement (the common case of the default preset) inlines the scan. */
+/* Out-of-line copy of the scan for its many call sites. */
 template<int kD, bool HALF>
-__device__ NEBC7_SHARED ChanList ChannelLevels(int2* nodes, const Area& ar, const AreaInfo& ai, int offset, int weight, int water,
-	int bits, int pbits, bool transparent, const uint8_t* table, bool byDiff, int maxSize, int* uniq, int lane)
+__device__ NEBC7_SHARED ChanList ChannelLevels(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
+	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, int lane)
 {
-	return ChannelLevelsScan<kD, HALF>(nodes, ar, ai, offset, weight, water, bits, pbits, transparent, table, byDiff, maxSize, uniq,
-		lane);
+	return ChannelLevelsScan<kD, HALF>(nodes, ar, offset, weight, water, bits, pbits, transparent, table, byDiff, maxSize, values, lane);
 }
 
 /* Single best candidate over the narrower window of the alpha slot of modes
-   4 and 5 (src/SnippetLevelsBuffer.h:148-188, 433-490). */
+   4 and 5 (src/SnippetLevelsBuffer.h:148-188, 433-490): a row's low endpoints
+   go up to its high one. */
 template<int kD>
-__device__ NEBC7_SHARED ChanList ChannelLevelsSingle(int2* nodes, const Area& ar, const AreaInfo& ai, int offset, int weight, int water,
-	int bits, bool transparent, const uint8_t* table, bool byDiff, int* uniq, int lane)
+__device__ NEBC7_SHARED ChanList ChannelLevelsSingle(int2* nodes, const Area& ar, int offset, int weight, int water, int bits,
+	bool transparent, const uint8_t* table, int2* values, int lane)
 {
 	ChanList res{ MaxColorError<kD>() * 2, 0 };
+	const AreaInfo& ai = ar.info;
 	const int shift = bits;
 	const int count = transparent ? ai.active : ai.count;
 	if (transparent && !count)
@@ -365,12 +400,10 @@ __device__ NEBC7_SHARED ChanList ChannelLevelsSingle(int2* nodes, const Area& ar
 	if (L == H && ((((L >> shift) ^ L) & ((1 << (8 - shift)) - 1)) == 0))
 		return ZeroList(nodes, (H << 8) + L, lane);
 	const Window win = MakeWindow(L, H, d, bits, shift);
-	if (top > 0xFFFF)
-		top = 0xFFFF;
-	const unsigned top16 = unsigned(top) & 0xFFFF;
-	const int rowSize = 1 << (2 * shift);
-	const bool diff = shift == 8 || (kReducedByDiff && byDiff);   /* DiffBase */
-	const int nu = UniqueValues(ar, count, offset, uniq, lane);
+	int limit = (min(top, 0xFFFF) & 0xFFFF) - 1;
+	const int n = DistinctValues(ar, count, offset, L, H, ValueStride(shift, true), values, lane);
+	ValueGroup first;
+	first.Load(values);
 
 	unsigned best = 0xFFFFFFFFu;
 	/* two rows per batch when only a row's first chunk can be on */
@@ -384,30 +417,19 @@ __device__ NEBC7_SHARED ChanList ChannelLevelsSingle(int2* nodes, const Area& ar
 			const int cH = iH << shift;
 			const int hL = min(win.LH, iH) + cH;
 			const int c = cH + 16 * (twoRows ? b : 2 * b + half);
-			const int cc = c + j;
 			const unsigned mask = Shr32(~0u, unsigned(max(0, Wsub(c | 15, hL | 7))) << 1);
 			const bool chunkOn = (iH < win.HH) && ((c == cH) || (c <= hL));
 			if (!__any_sync(kFull, chunkOn))
 				break;
-			if (chunkOn && ((mask >> (2 * j)) & 1))
+			const bool on = chunkOn && ((mask >> (2 * j)) & 1);
+			const int cc = on ? c + j : 0;
+			int s;
+			if (CandidateSum<false>(table + DiffBase(cc, shift), first, values, n, on, limit, s))
 			{
-				const int dbase = kReducedByDiff ? DiffBase(cc, shift) : 0;
-				auto term = [&](int e) {
-					const int x = e & 0xFFFF;
-					const unsigned v = diff ? (kReducedByDiff ? table[dbase - 513 * x] : DiffAt(table, x, cc & 0xFF, cc >> 8))
-					                        : table[size_t(x) * rowSize + cc];
-					return unsigned(e >> 16) * v * v;
-				};
-				unsigned s = 0;
-				for (int u = 0; u < nu; u += 4)
-				{
-					const int4 e4 = *reinterpret_cast<const int4*>(uniq + u);
-					s += (term(e4.x) + term(e4.y)) + (term(e4.z) + term(e4.w));
-				}
-				if (s > 0xFFFF)
-					s = 0xFFFF;
-				if (s < top16)
-					best = min(best, (s << 16) | unsigned(cc));
+				if (on && s <= limit)
+					best = min(best, (unsigned(s) << 16) | unsigned(cc));
+				/* equal errors keep the earlier candidate */
+				limit = min(limit, int(__reduce_min_sync(kFull, best) >> 16) - 1);
 			}
 		}
 	}
@@ -426,20 +448,20 @@ __device__ NEBC7_SHARED ChanList ChannelLevelsSingle(int2* nodes, const Area& ar
 
 /* LevelsMinimum::EstimateChannelLevelsReduced (src/SnippetLevelsMinimum.h:117-311):
    the smallest e(c) over the window (or top), rows pruned by their cut-table
-   lower bound.  The minimum does not depend on the visiting order, so rows
-   are visited in order with the running best. */
+   lower bound.  The minimum does not depend on the visiting order; a batch
+   ends after the first four values unless a lane is below the running best
+   (of the batches of a precise encode one in six gets further). */
 template<int kD>
-__device__ NEBC7_SHARED int EstimateChannelLevels(const Area& ar, const AreaInfo& ai, int offset, int weight, int water, int bits,
-	bool transparent, const uint8_t* table, bool byDiff, const uint16_t* tower, int* uniq, int lane)
+__device__ NEBC7_SHARED int EstimateChannelLevels(const Area& ar, int offset, int weight, int water, int bits, bool transparent,
+	const uint8_t* table, bool byDiff, const uint16_t* tower, int2* values, int lane)
 {
-	const int shift = bits;
+	const AreaInfo& ai = ar.info;
 	const int count = transparent ? ai.active : ai.count;
 	if (transparent && !count)
 		return 0;
 	int top = (water + weight - 1) / weight;
 	if (!top)
 		return 0;
-	const int d = WindowRadius<kD>(top);
 	const int L = int(int16_t(ai.minmax[2 * offset]));
 	const int H = int(int16_t(ai.minmax[2 * offset + 1]));
 	if (L == H)
@@ -448,63 +470,48 @@ __device__ NEBC7_SHARED int EstimateChannelLevels(const Area& ar, const AreaInfo
 		return 0;
 	if (bits == 8 && H - L <= 3)
 		return 0;
-	const Window win = MakeWindow(L, H, d, bits, shift);
+	const Window win = MakeWindow(L, H, WindowRadius<kD>(top), bits, bits);
 	if (top > 0xFFFF)
 		top = 0xFFFF;
-	const int rowSize = 1 << (2 * bits);
-	const bool diff = bits == 8 || (kReducedByDiff && byDiff);   /* DiffBase */
-	const int towerSize = 1 << bits;
-	const int nu = UniqueValues(ar, count, offset, uniq, lane);
+	const int n = DistinctValues(ar, count, offset, L, H, ValueStride(bits, byDiff), values, lane);
+	ValueGroup first;
+	first.Load(values);
 
 	int best = top;
 	for (int base = win.HL; base < win.HH; base += 32)
 	{
 		/* lane k holds the cut bound of row base + k */
 		const int iHl = base + lane;
-		unsigned rowLb = 0xFFFF;
+		unsigned bound = 0x7FFFFFFF;
 		if (iHl < win.HH)
 		{
-			auto cut = [&](int e) { return unsigned(e >> 16) * tower[size_t(e & 0xFFFF) * towerSize + iHl]; };
-			unsigned s = 0;
-			for (int u = 0; u < nu; u += 4)
+			auto cut = [&](int e) { return unsigned(e & 0xFF) * tower[((e >> 8) << bits) + iHl]; };
+			bound = 0;
+			for (int u = 0; u < n; u += 4)
 			{
-				const int4 e4 = *reinterpret_cast<const int4*>(uniq + u);
-				s += (cut(e4.x) + cut(e4.y)) + (cut(e4.z) + cut(e4.w));
+				const int4 a = *reinterpret_cast<const int4*>(values + u), b = *reinterpret_cast<const int4*>(values + u + 2);
+				bound += (cut(a.y) + cut(a.w)) + (cut(b.y) + cut(b.w));
 			}
-			rowLb = s > 0xFFFF ? 0xFFFF : s;
+			bound = min(bound, 0xFFFFu);
 		}
-		const int nrows = min(32, win.HH - base);
-		for (int r = 0; r < nrows; r++)
+		/* the rows whose bound is below the best, in order */
+		int next = 0;
+		for (;;)
 		{
-			const int lb = int(__shfl_sync(kFull, rowLb, r));
-			if (lb >= best)
-				continue;
+			const unsigned open = __ballot_sync(kFull, lane >= next && int(bound) < best);
+			if (!open)
+				break;
+			const int r = __ffs(open) - 1;
+			next = r + 1;
 			const int iH = base + r;
-			const int cH = iH << shift;
-			unsigned rowBest = 0xFFFF;
+			const int cH = iH << bits;
 			for (int iL = cH, hL = min(win.LH, iH) + cH; iL <= hL; iL += 32)
 			{
-				/* cc = iL + lane stays in row iH (iL <= hL, iL - cH a multiple of 32) */
-				const int cc = iL + lane;
-				const int dbase = kReducedByDiff ? DiffBase(cc, bits) : 0;
-				auto term = [&](int e) {
-					const int x = e & 0xFFFF;
-					const unsigned v = diff ? (kReducedByDiff ? table[dbase - 513 * x] : DiffAt(table, x, cc & 0xFF, cc >> 8))
-					                        : table[size_t(x) * rowSize + cc];
-					return unsigned(e >> 16) * v * v;
-				};
-				unsigned s = 0;
-				for (int u = 0; u < nu; u += 4)
-				{
-					const int4 e4 = *reinterpret_cast<const int4*>(uniq + u);
-					s += (term(e4.x) + term(e4.y)) + (term(e4.z) + term(e4.w));
-				}
-				if (s > 0xFFFF)
-					s = 0xFFFF;
-				rowBest = min(rowBest, s);
+				/* iL + lane stays in row iH (iL <= hL, iL - cH a multiple of 32) */
+				int s;
+				if (CandidateSum<false>(table + CandidateBase(iL + lane, bits, byDiff), first, values, n, true, best - 1, s))
+					best = __reduce_min_sync(kFull, min(s, best));
 			}
-			rowBest = __reduce_min_sync(kFull, rowBest);
-			best = min(best, int(rowBest));
 		}
 	}
 	return best * weight;

@@ -29,14 +29,41 @@ constexpr bool kHasNormalPasses = true;
 
 constexpr int kBig = 0x7FFFFFFF;
 
+/* Above every error (16 pixels of weight 2000 at distance 127: 5.2e8), and
+   still an int after another error is added. */
+constexpr int kFar = 0x3FFFFFFF;
+
+/* int4 entries per pixel of the candidate table: 20 candidates and one of
+   padding, so that the pixels of a column lie in different banks. */
+constexpr int kTableRow = 21;
+
+/* Per-warp search state.  The staged kernels reserve only the bytes up to the
+   last member their pass uses (SearchBytes), so that more of the SM's memory
+   is L1. */
 struct __align__(16) SearchState
 {
+	int2 values[16];         /* distinct channel values of the subset being scanned (DistinctValues) */
+	ChanList chan[4][4];     /* [p-bit variant][channel]: the lists' minima and lengths */
+	int bound[2][4];         /* [subset][channel]: lower-bound estimates of a two-subset search */
+	int4 plane[4 * 16];      /* error planes of the combination search, [pixel][level]: three of
+	                            4 levels or two of 8 */
 	int2 lists[4][4][32];    /* [p-bit variant][channel][entry] = (error, color) */
-	int planes[3][256];      /* partial error planes of the combination search, [pixel][level] */
-	int2 order[64];          /* full searches: (estimate, partition) */
-	int est[64][3][3];       /* per partition, subset, channel (G, R, B) estimates */
-	int lines[64][2];        /* per partition, estimates of subsets 2 and 3 */
-	int uniq[16];            /* distinct channel values of the subset being scanned */
+	union
+	{
+		struct
+		{
+			int2 order[64];      /* (estimate, partition) */
+			int lines[64][2];    /* per partition, estimates of subsets 2 and 3 */
+			int est[64][3][3];   /* per partition, subset, channel (G, R, B) estimates */
+		} three;                 /* the three-subset searches */
+		int4 table[16 * kTableRow];   /* four channels, 2-bit indices: R's terms, [pixel][candidate] */
+		int plane16[3][256];          /* four channels, 4-bit indices: planes of 16 levels */
+	};
+	struct
+	{
+		int2 order[64];
+		int lines[64][2];
+	} pca;                   /* OPTION_PCA: (estimate, partition), the subsets' bounds */
 };
 
 /* ---------------------------------------------------------------------- */
@@ -128,7 +155,7 @@ __device__ NEBC7_PASS int AreaError(const Area& ar, int active, Ep ep, const int
 
 /* Mode 4/5 error on Area1 (see RotErrorExact) with early exit. */
 template<int kD, int CB, int AB, bool MODE4>
-__device__ NEBC7_PASS int RotErrorW(const Area& ar, const AreaInfo& ai, Ep epImg, int rotation, const int w[4], int water)
+__device__ __noinline__ int RotErrorW(const Area& ar, const AreaInfo& ai, Ep epImg, int rotation, const int w[4], int water)
 {
 	const int a = RotChannel(rotation);
 	LevelSet<CB> LC;
@@ -215,152 +242,381 @@ __device__ __forceinline__ int ReplayInner(bool valid, int brk, int skip, int er
 	return taken;
 }
 
-/* ---------------------------------------------------------------------- */
-/* Modes 0-3: three channels G, R, B (src/Bc7CoreMode0.cpp:242-415)        */
-/* ---------------------------------------------------------------------- */
-
-template<int kD, int IB>
-__device__ NEBC7_SHARED int TryVariants3(const Area& ar, const AreaInfo& ai, const Params& P, const int2* L1, ChanList c1,
-	const int2* L2, ChanList c2, const int2* L3, ChanList c3, Ep& best, int water, int* planes, int lane)
+/* The channel weights by value: an argument of the out-of-line searches
+   that stays in registers. */
+struct Weights
 {
-	const int min1 = c1.minErr, min2 = c2.minErr, min3 = c3.minErr;
-	if (min1 + min2 + min3 >= water)
-		return water;
-	const int n2 = c2.count, n3 = c3.count, np = ai.active;
-	int* pG = planes;
-	int* pGR = planes + 256;
-	const int col2l = lane < n2 ? L2[lane].y : 0;
-	const int col3 = lane < n3 ? L3[lane].y : 0;
-	const int e3base = lane < n3 ? L3[lane].x : kBig;
-	for (int i1 = 0; i1 < c1.count; i1++)
-	{
-		const int e1 = L1[i1].x;
-		if (e1 + min2 + min3 >= water)
-			break;
-		const int col1 = L1[i1].y;
-		/* memoised G+B errors (memGB) and G+R pair errors, one list entry per lane */
-		PlaneAdd<kD, IB>(pG, nullptr, ar, np, 1, col1, P.wG, lane);
-		int memGB = kBig, pairGR = kBig;
-		if (lane < n3)
-			memGB = PlaneError<kD, IB>(pG, ar, np, 3, col3, P.wB, water - min2);
-		if (lane < n2)
-			pairGR = PlaneError<kD, IB>(pG, ar, np, 2, col2l, P.wR, water - min3);
-		for (int i2 = 0; i2 < n2; i2++)
-		{
-			const int e2s = L2[i2].x + e1;
-			if (e2s + min3 >= water)
-				break;
-			const int col2 = L2[i2].y;
-			const int e2 = __shfl_sync(kFull, pairGR, i2);
-			if (e2 + min3 >= water)
-				continue;
-			const bool valid = lane < n3;
-			const int brk = valid ? e3base + e2 : kBig;
-			const int skip = valid ? memGB + min2 : kBig;
-			const bool eval = valid && brk < water && skip < water;
-			/* no lane evaluates: the replay accepts nothing, the plane is not needed */
-			if (!__any_sync(kFull, eval))
-				continue;
-			PlaneAdd<kD, IB>(pGR, pG, ar, np, 2, col2, P.wR, lane);
-			int err = kBig;
-			if (eval)
-				err = PlaneError<kD, IB>(pGR, ar, np, 3, col3, P.wB, water);
-			const int jl = ReplayInner(valid, brk, skip, err, water, lane);
-			if (jl >= 0)
-				best = EpSetCh(Ep2(1, col1, 2, col2), 3, __shfl_sync(kFull, col3, jl));
-		}
-	}
-	return water;
+	int a, g, r, b;
+};
+
+__device__ __forceinline__ Weights WeightsOf(const Params& P)
+{
+	return Weights{ P.wA, P.wG, P.wR, P.wB };
 }
 
+/* A search's outcome: the water it leaves and the endpoints that reached it. */
+struct Found
+{
+	int water;
+	Ep best;
+};
+
+/* min over four levels of a plane row plus a candidate's terms; each step is
+   one fused add-and-minimum. */
+__device__ __forceinline__ int RowMin(int4 p, int4 t)
+{
+	return __viaddmin_s32(p.x, t.x, __viaddmin_s32(p.y, t.y, __viaddmin_s32(p.z, t.z, p.w + t.w)));
+}
+
+/* w * q(x - level)^2 at the four levels of the endpoint pair `col`. */
+template<int kD>
+__device__ __forceinline__ int4 LevelTerms(int x, int col, int w)
+{
+	const int e0 = col & 0xFF, e1 = (col >> 8) & 0xFF;
+	const int q0 = Q<kD>(x - e0), q1 = Q<kD>(x - Interp(e0, e1, 21)), q2 = Q<kD>(x - Interp(e0, e1, 43)), q3 = Q<kD>(x - e1);
+	return make_int4(w * q0 * q0, w * q1 * q1, w * q2 * q2, w * q3 * q3);
+}
+
+/* A lane's candidate terms per pixel and level, kept in registers: the
+   weighted squares with four levels, the plain squares two to a register
+   with eight (at most 127^2 each). */
+template<int kD, int IB>
+struct LaneTerms
+{
+	int4 t[16];
+
+	/* x: the pixel values of the searched channel; rows from np on are zero */
+	__device__ __forceinline__ void Init(const Area& ar, int np, int c, int col, int w)
+	{
+		const int e0 = col & 0xFF, e1 = (col >> 8) & 0xFF;
+		int v[8];
+		if (IB == 3)
+		{
+#pragma unroll
+			for (int k = 0; k < 8; k++)
+				v[k] = Interp(e0, e1, c_interp3[k]);
+		}
+#pragma unroll
+		for (int i = 0; i < 16; i++)
+		{
+			t[i] = make_int4(0, 0, 0, 0);
+			if (i < np)
+			{
+				const int x = ar.px[i][c];
+				if (IB == 2)
+					t[i] = LevelTerms<kD>(x, col, w);
+				else
+				{
+					int q[8];
+#pragma unroll
+					for (int k = 0; k < 8; k++)
+						q[k] = Q<kD>(x - v[k]);
+					t[i] = make_int4(q[0] * q[0] + ((q[1] * q[1]) << 16), q[2] * q[2] + ((q[3] * q[3]) << 16),
+						q[4] * q[4] + ((q[5] * q[5]) << 16), q[6] * q[6] + ((q[7] * q[7]) << 16));
+				}
+			}
+		}
+	}
+
+	/* Error of the lane's candidate over a plane of np pixels (rows up to the
+	   next multiple of four are zero).  Ends once no lane is below its limit,
+	   so a lane's value is exact whenever it is below it.  Warp-collective:
+	   every lane calls it. */
+	__device__ __forceinline__ int Error(const int4* plane, int np, int w, int limit) const
+	{
+		int sum = 0;
+#pragma unroll
+		for (int i = 0; i < 16; i += 4)
+		{
+			if (i >= np)
+				break;
+#pragma unroll
+			for (int j = i; j < i + 4; j++)
+			{
+				if (IB == 2)
+					sum += RowMin(plane[j], t[j]);
+				else
+				{
+					const int4 a = plane[2 * j], b = plane[2 * j + 1];
+					auto two = [&](int p0, int p1, int q) { return min(p0 + w * (q & 0xFFFF), p1 + w * int(unsigned(q) >> 16)); };
+					sum += min(min(two(a.x, a.y, t[j].x), two(a.z, a.w, t[j].y)), min(two(b.x, b.y, t[j].z), two(b.z, b.w, t[j].w)));
+				}
+			}
+			if (!__any_sync(kFull, sum < limit))
+				break;
+		}
+		return sum;
+	}
+};
+
+constexpr int kNoLimit = int(0x80000000u);   /* the limit of a lane without a candidate */
+
+/* The entries of a [pixel][level] plane that a lane holds: pixel
+   lane / L + (32 / L) m, level lane % L. */
+template<int kD, int IB>
+struct PlaneLanes
+{
+	static constexpr int L = 1 << IB, N = L / 2;
+	int wk, row, np;
+
+	__device__ __forceinline__ PlaneLanes(int np_, int lane) : wk(InterpWeights(IB)[lane & (L - 1)]), row(lane >> IB), np(np_) {}
+
+	__device__ __forceinline__ void Pixels(const Area& ar, int c, int (&x)[N]) const
+	{
+#pragma unroll
+		for (int m = 0; m < N; m++)
+			x[m] = row + (32 / L) * m < np ? int(ar.px[row + (32 / L) * m][c]) : 0;
+	}
+
+	/* dst = src + the terms of the endpoint pair `col` */
+	__device__ __forceinline__ void Add(int (&dst)[N], const int (&src)[N], const int (&x)[N], int col, int w) const
+	{
+		const int v = Interp(col & 0xFF, (col >> 8) & 0xFF, wk);
+#pragma unroll
+		for (int m = 0; m < N; m++)
+		{
+			const int q = Q<kD>(x[m] - v);
+			dst[m] = row + (32 / L) * m < np ? src[m] + w * q * q : 0;
+		}
+	}
+
+	__device__ __forceinline__ void Store(int4* plane, const int (&e)[N], int lane) const
+	{
+		int* p = reinterpret_cast<int*>(plane);
+#pragma unroll
+		for (int m = 0; m < N; m++)
+			if ((32 / L) * m < np)
+				p[lane + 32 * m] = e[m];
+		__syncwarp();
+	}
+};
+
+/* ---------------------------------------------------------------------- */
+/* Three channels with one index (src/Bc7CoreMode0.cpp:242-415; modes 4, 5) */
+/* ---------------------------------------------------------------------- */
+
+/* One channel's sorted candidate list in a search: its pixels' channel, its
+   weight, and the list. */
+struct SearchChannel
+{
+	int c, w;
+	const int2* list;
+	int n, minErr;
+};
+
+/* A three-channel search's outcome; taken: an improving combination's
+   endpoint colours are in x, y, z. */
+struct Found3
+{
+	int water;
+	int taken, x, y, z;
+};
+
+/* The combination search over three channels that share an index.  As in
+   SearchFour2, every bound is a lower bound, so the sequential search ends
+   with the first combination, in its order, of the smallest error below the
+   water.  z's candidates are the lanes, their terms in registers; y's errors
+   are summed once per x candidate.  hidden: the pixels that count only with
+   their alpha of 0 (x is then the alpha channel). */
+template<int kD, int IB>
+__device__ NEBC7_SHARED Found3 SearchThree(const Area& ar, int np, SearchChannel X, SearchChannel Y, SearchChannel Z, int hidden,
+	int water, int4* planes, int lane)
+{
+	Found3 f{ water, 0, 0, 0, 0 };
+	if (X.minErr + Y.minErr + Z.minErr >= water)
+		return f;
+	const int2 ly = lane < Y.n ? Y.list[lane] : make_int2(kFar, 0);
+	const int2 lz = lane < Z.n ? Z.list[lane] : make_int2(kFar, 0);
+	int4* const pX = planes;
+	int4* const pXY = planes + 4 * (1 << IB);
+	LaneTerms<kD, IB> terms;
+	int sums = 0;   /* error sums of z's candidates so far */
+	using Lanes = PlaneLanes<kD, IB>;
+	const Lanes pl(np, lane);
+	int xx[Lanes::N], xy[Lanes::N], gx[Lanes::N], gy[Lanes::N];
+	pl.Pixels(ar, X.c, xx);
+	pl.Pixels(ar, Y.c, xy);
+	const int none[Lanes::N] = {};
+	for (int ix = 0; ix < X.n; ix++)
+	{
+		const int2 lx = X.list[ix];
+		if (lx.x + Y.minErr + Z.minErr >= water)
+			break;
+		int ea = 0;
+		if (hidden)
+		{
+			const int q = Q<kD>(min(lx.y & 0xFF, (lx.y >> 8) & 0xFF));
+			ea = q * q * (X.w * hidden);
+		}
+		pl.Add(gx, none, xx, lx.y, X.w);
+		__syncwarp();
+		pl.Store(pX, gx, lane);
+		/* joint errors of this x candidate with every y one */
+		int errXY = kFar;
+		if (lane < Y.n)
+			errXY = PlaneError<kD, IB>(reinterpret_cast<const int*>(pX), ar, np, Y.c, ly.y, Y.w, water - ea - Z.minErr) + ea;
+		/* the first pass sums x's plane with every z candidate (errXZ), the
+		   others take the y candidates still open */
+		int errXZ = 0, iy = -1;
+		for (;;)
+		{
+			const unsigned open = __ballot_sync(kFull, lane > iy && ly.x + lx.x + Z.minErr < water && errXY + Z.minErr < water);
+			if (!open)
+				break;
+			const bool first = iy < 0 && errXZ == 0;
+			int2 y = make_int2(0, 0);
+			bool eval = lane < Z.n;
+			const int4* plane = pX;
+			int limit = water - ea - Y.minErr;
+			if (!first)
+			{
+				iy = __ffs(open) - 1;
+				const int eXY = __shfl_sync(kFull, errXY, iy);
+				y = make_int2(__shfl_sync(kFull, ly.x, iy), __shfl_sync(kFull, ly.y, iy));
+				eval = lz.x + eXY < water && errXZ - 1 + y.x < water;
+				if (!__any_sync(kFull, eval))
+					continue;
+				pl.Add(gy, gx, xy, y.y, Y.w);
+				pl.Store(pXY, gy, lane);
+				plane = pXY;
+				limit = water - ea;
+			}
+			/* the terms in registers pay from the third sum on */
+			if (sums == 2)
+				terms.Init(ar, np, Z.c, lz.y, Z.w);
+			int sum = 0;
+			if (sums >= 2)
+				sum = terms.Error(plane, np, Z.w, eval ? limit : kNoLimit);
+			else if (eval)
+				sum = PlaneError<kD, IB>(reinterpret_cast<const int*>(plane), ar, np, Z.c, lz.y, Z.w, limit);
+			sums++;
+			const int err = eval ? sum + ea : kFar;
+			if (first)
+			{
+				/* 1 + the error: never 0, so that the first pass runs once */
+				errXZ = err + 1;
+				continue;
+			}
+			/* the first lane of the smallest error below the water */
+			const int low = __reduce_min_sync(kFull, err);
+			if (low < water)
+			{
+				water = low;
+				f.taken = 1;
+				f.x = lx.y;
+				f.y = y.y;
+				f.z = __shfl_sync(kFull, lz.y, __ffs(__ballot_sync(kFull, err == low)) - 1);
+			}
+		}
+	}
+	f.water = water;
+	return f;
+}
+
+/* Candidate lists and estimates of the opaque modes: table by differences
+   (DiffBase), except mode 1's shared-p-bit table, which marks endpoint pairs
+   of different parity (0xFF; its estimates read them) and stays in the per-x
+   layout. */
 struct Spec3
 {
 	int bits;               /* candidate list bits */
-	const uint8_t* table;   /* by differences (DiffBase) unless it is the shared-p-bit table */
+	const uint8_t* table;
 	bool byDiff;
 	int estBits;
 	const uint16_t* estTower;
+	int variants;           /* p-bit variants */
 };
 
-template<int MODE>
-__device__ __forceinline__ Spec3 GetSpec3(const LevelTables& T)
+__device__ __forceinline__ Spec3 GetSpec3(int mode, const LevelTables& T)
 {
-	/* mode 1's shared p-bit table marks endpoint pairs of different parity
-	   (0xFF), which its estimates read: it stays in the per-x layout */
-	if (MODE == 0)
-		return Spec3{ 4, kReducedByDiff ? T.d3v8 : T.d3v5, kReducedByDiff, 5, T.c3v5 };
-	if (MODE == 1)
-		return Spec3{ 6, T.d3v7s, false, 7, T.c3v7s };
-	if (MODE == 2)
-		return Spec3{ 5, kReducedByDiff ? T.d2v8 : T.d2v5, kReducedByDiff, 5, T.c2v5 };
-	return Spec3{ 7, T.d2v8, true, 8, T.c2v8 };
-}
-
-template<int MODE>
-__device__ __forceinline__ int NumVariants3() { return MODE == 2 ? 1 : (MODE == 1 ? 2 : 4); }
-
-__device__ __forceinline__ int Pbits(int mode, int v)
-{
+	if (mode == 0)
+		return Spec3{ 4, T.d3v8, true, 5, T.c3v5, 4 };
+	if (mode == 1)
+		return Spec3{ 6, T.d3v7s, false, 7, T.c3v7s, 2 };
 	if (mode == 2)
-		return -1;
-	const int pb[4] = { 0x0101, 0, 1, 1 << 8 };
-	return pb[v];
+		return Spec3{ 5, T.d2v8, true, 5, T.c2v5, 1 };
+	return Spec3{ 7, T.d2v8, true, 8, T.c2v8, 4 };
 }
 
-/* Subset::InitLevels (src/Bc7CoreMode0.cpp:249-268) for variant v. */
-template<int kD, int MODE>
-__device__ NEBC7_PASS bool InitLevels3(SearchState& ss, int v, const Area& ar, const AreaInfo& ai, const Params& P, const Spec3& sp,
-	int water, const int est[3], ChanList cl[3], int lane)
+/* p-bit variant v in the reference's order 0x0101, 0, 1, 1 << 8 (low byte:
+   the low endpoint's). */
+__device__ __forceinline__ int VariantPbits(int v)
 {
-	const int pb = Pbits(MODE, v);
-	cl[0] = ChannelLevels<kD, false>(ss.lists[v][0], ar, ai, 1, P.wG, water - est[1] - est[2], sp.bits, pb, false, sp.table, sp.byDiff, 32,
-		ss.uniq, lane);
-	const int min1 = cl[0].minErr;
-	if (min1 >= water)
-		return false;
-	cl[1] = ChannelLevels<kD, false>(ss.lists[v][1], ar, ai, 2, P.wR, water - min1 - est[2], sp.bits, pb, false, sp.table, sp.byDiff, 32,
-		ss.uniq, lane);
-	const int min2 = cl[1].minErr;
-	if (min1 + min2 >= water)
-		return false;
-	cl[2] = ChannelLevels<kD, false>(ss.lists[v][2], ar, ai, 3, P.wB, water - min1 - min2, sp.bits, pb, false, sp.table, sp.byDiff, 32,
-		ss.uniq, lane);
-	return min1 + min2 + cl[2].minErr < water;
+	return v == 0 ? 0x0101 : (v == 1 ? 0 : (v == 2 ? 1 : 1 << 8));
+}
+
+__device__ __forceinline__ int ChannelWeight(const Params& P, int c)
+{
+	return c == 0 ? P.wA : (c == 1 ? P.wG : (c == 2 ? P.wR : P.wB));
+}
+
+/* The passes below keep one call site of each scan, estimate and combination
+   search, in loops over the subsets, variants and channels: inlined, a
+   kernel holds one copy of each and no call saves registers on the thread's
+   stack (a precise mode-2 search spent more loads on its stack than on the
+   tables, with 14 % of them hits). */
+
+/* Subset::InitLevels (src/Bc7CoreMode0.cpp:249-268) for variant v; estR,
+   estB: lower bounds of the later channels' errors. */
+template<int kD>
+__device__ NEBC7_PASS bool InitLevels3(SearchState& ss, int v, const Area& ar, const Params& P, const Spec3& sp, bool pbit, int water,
+	int estR, int estB, int lane)
+{
+	int used = 0;
+#pragma unroll 1
+	for (int c = 1; c < 4; c++)
+	{
+		const int rest = c == 1 ? estR + estB : (c == 2 ? estB : 0);
+		const ChanList cl = ChannelLevels<kD, false>(ss.lists[v][c - 1], ar, c, ChannelWeight(P, c), water - used - rest, sp.bits,
+			pbit ? VariantPbits(v) : -1, false, sp.table, sp.byDiff, 32, ss.values, lane);
+		if (lane == 0)
+			ss.chan[v][c - 1] = cl;
+		used += cl.minErr;
+		if (used >= water)
+			return false;
+	}
+	__syncwarp();
+	return true;
 }
 
 /* Subsets (src/Bc7CoreMode0.cpp:366-415): all variants' lists start from
    the same water, then the variants are searched in order. */
 template<int kD, int MODE>
-__device__ NEBC7_PASS int SearchSubset3(SearchState& ss, const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T,
-	int water, const int est[3], Ep& best, bool& any, int lane)
+__device__ NEBC7_PASS int SearchSubset3(SearchState& ss, const Area& ar, const Params& P, const Spec3& sp, int water, int estR, int estB,
+	Ep& best, bool& any, int lane)
 {
 	constexpr int IB = (MODE == 0 || MODE == 1) ? 3 : 2;
-	const Spec3 sp = GetSpec3<MODE>(T);
-	ChanList cl[4][3];
-	bool valid[4];
-	any = false;
-	for (int v = 0; v < NumVariants3<MODE>(); v++)
+	int valid = 0;
+#pragma unroll 1
+	for (int v = 0; v < sp.variants; v++)
+		valid |= int(InitLevels3<kD>(ss, v, ar, P, sp, MODE != 2, water, estR, estB, lane)) << v;
+	any = valid != 0;
+#pragma unroll 1
+	for (int v = 0; v < sp.variants; v++)
 	{
-		valid[v] = InitLevels3<kD, MODE>(ss, v, ar, ai, P, sp, water, est, cl[v], lane);
-		any |= valid[v];
+		if (!((valid >> v) & 1))
+			continue;
+		auto channel = [&](int c, int w) { return SearchChannel{ c, w, ss.lists[v][c - 1], ss.chan[v][c - 1].count, ss.chan[v][c - 1].minErr }; };
+		const Found3 f = SearchThree<kD, IB>(ar, ar.info.active, channel(1, P.wG), channel(2, P.wR), channel(3, P.wB), 0, water,
+			ss.plane, lane);
+		water = f.water;
+		if (f.taken)
+			best = EpSetCh(Ep2(1, f.x, 2, f.y), 3, f.z);
 	}
-	for (int v = 0; v < NumVariants3<MODE>(); v++)
-		if (valid[v])
-			water = TryVariants3<kD, IB>(ar, ai, P, ss.lists[v][0], cl[v][0], ss.lists[v][1], cl[v][1], ss.lists[v][2], cl[v][2],
-				best, water, &ss.planes[0][0], lane);
 	return water;
 }
 
+/* Subset s of partition p into `ar` (its pixels and ar.info); `orient` as
+   for SubsetStats. */
 template<int kD>
-__device__ NEBC7_PASS AreaInfo BuildSubset(WarpState& st, const CellRegs& R, const Params& P, Area& ar, int ns, int p, int s, int lane)
+__device__ NEBC7_PASS void BuildSubset(WarpState& st, const CellRegs& R, const Params& P, Area& ar, int ns, int p, int s, bool orient,
+	int lane)
 {
 	const uint32_t part = ns == 3 ? c_part3[p] : c_part2[p];
 	const uint32_t member = Member(part, s);
 	const int anchor = Anchor(ns, p, s);
-	AreaInfo ai = AreaStats(st, R, P, member);
-	ai.zero = anchor;
+	SubsetStats(ar.info, st, R, P, member, anchor, orient, lane);
 	BuildAreaList(ar, st, R, member, anchor, lane);
-	return ai;
 }
 
 /* ModeN::CompressBlock for modes 0-3 (src/Bc7CoreMode0.cpp:417-498). */
@@ -369,69 +625,65 @@ __device__ NEBC7_PASS void RefineOpaque(WarpState& st, SearchState& ss, CellRegs
 {
 	constexpr int NS = (MODE == 0 || MODE == 2) ? 3 : 2;
 	constexpr int IB = (MODE == 0 || MODE == 1) ? 3 : 2;
-	const int p = R.bestParam;
-	Ep mc[3] = { R.best[0], R.best[1], R.best[2] };
-	const int est[3] = { 0, 0, 0 };
+	const Spec3 sp = GetSpec3(MODE, T);
 	const int wGRB[4] = { 0, P.wG, P.wR, P.wB };
+	Ep mc0 = R.best[0], mc1 = R.best[1], mc2 = R.best[2];
 	int error = R.opaqueAlphaError;
 	if (error < R.errTotal)
 	{
+#pragma unroll 1
 		for (int s = 0; s < NS; s++)
 		{
-			const AreaInfo ai = BuildSubset<kD>(st, R, P, st.sub[0], NS, p, s, lane);
-			const int water = AreaError<kD, IB>(st.sub[0], ai.active, mc[s], wGRB, MaxColorError<kD>());
+			BuildSubset<kD>(st, R, P, st.sub[0], NS, R.bestParam, s, true, lane);
+			Ep b = s == 0 ? mc0 : (s == 1 ? mc1 : mc2);
+			int water = AreaError<kD, IB>(st.sub[0], st.sub[0].info.active, b, wGRB, MaxColorError<kD>());
 			if (water)
 			{
 				bool any;
-				Ep b = mc[s];
-				const int w2 = SearchSubset3<kD, MODE>(ss, st.sub[0], ai, P, T, water, est, b, any, lane);
+				const int w2 = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, 0, 0, b, any, lane);
 				if (any)
 				{
-					error += w2;
-					mc[s] = b;
+					water = w2;
+					if (s == 0)
+						mc0 = b;
+					else if (s == 1)
+						mc1 = b;
+					else
+						mc2 = b;
 				}
-				else
-					error += water;
+				error += water;
 			}
 		}
 		if (R.errTotal > error)
 		{
 			R.errTotal = error;
-			R.best[0] = mc[0];
-			R.best[1] = mc[1];
+			R.best[0] = mc0;
+			R.best[1] = mc1;
 			if (NS == 3)
-				R.best[2] = mc[2];
+				R.best[2] = mc2;
 		}
 	}
 }
 
-/* EstimateLevels of modes 0-3 (src/Bc7CoreMode0.cpp:500-530). */
+/* EstimateLevels of modes 0-3 (src/Bc7CoreMode0.cpp:500-530): est[0..2] get
+   the estimates of G, R, B. */
 template<int kD>
-__device__ NEBC7_PASS int EstimateLevels3(SearchState& ss, const Area& ar, const AreaInfo& ai, const Params& P, const Spec3& sp, int water,
-	int est[4], int lane)
+__device__ NEBC7_PASS int EstimateLevels3(SearchState& ss, const Area& ar, const Params& P, const Spec3& sp, int water, int* est, int lane)
 {
 	int error = 0;
-	if (error < water)
+#pragma unroll 1
+	for (int c = 1; c < 4; c++)
 	{
-		const int l1 = EstimateChannelLevels<kD>(ar, ai, 1, P.wG, water - error, sp.estBits, false, sp.table, sp.byDiff, sp.estTower, ss.uniq, lane);
-		est[1] = l1;
-		error += l1;
-		if (error < water)
-		{
-			const int l2 = EstimateChannelLevels<kD>(ar, ai, 2, P.wR, water - error, sp.estBits, false, sp.table, sp.byDiff, sp.estTower, ss.uniq, lane);
-			est[2] = l2;
-			error += l2;
-			if (error < water)
-			{
-				const int l3 = EstimateChannelLevels<kD>(ar, ai, 3, P.wB, water - error, sp.estBits, false, sp.table, sp.byDiff, sp.estTower, ss.uniq, lane);
-				est[3] = l3;
-				error += l3;
-				if (error < water)
-					return error;
-			}
-		}
+		if (!(error < water))
+			return water;
+		const int l = EstimateChannelLevels<kD>(ar, c, ChannelWeight(P, c), water - error, sp.estBits, false, sp.table, sp.byDiff,
+			sp.estTower, ss.values, lane);
+		if (lane == 0)
+			est[c - 1] = l;
+		error += l;
 	}
-	return water;
+	__syncwarp();
+	return error < water ? error : water;
 }
 
 __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
@@ -440,10 +692,12 @@ __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 	   rank = number of entries that must precede */
 	int2 mine[2];
 	int rank[2];
+#pragma unroll
 	for (int h = 0; h < 2; h++)
 	{
 		const int i = lane + 32 * h;
 		rank[h] = -1;
+		mine[h] = make_int2(0, 0);
 		if (i < n)
 		{
 			mine[h] = order[i];
@@ -457,10 +711,71 @@ __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 		}
 	}
 	__syncwarp();
+#pragma unroll
 	for (int h = 0; h < 2; h++)
 		if (rank[h] >= 0)
 			order[rank[h]] = mine[h];
 	__syncwarp();
+}
+
+/* The estimates of partition p of a full search of modes 0 and 2 (the first
+   loop of src/Bc7CoreMode0.cpp:532-642): its subsets' estimates to ss.three,
+   and whether they leave room below the error. */
+template<int kD, int MODE>
+__device__ __forceinline__ bool ThreeSubsetsEstimate(WarpState& st, SearchState& ss, const CellRegs& R, const Params& P, const Spec3& sp,
+	int p, int& total, int lane)
+{
+	int water = R.errTotal - R.denoiseStep - R.opaqueAlphaError;
+	total = R.opaqueAlphaError + R.denoiseStep;
+#pragma unroll 1
+	for (int s = 0; s < 3; s++)
+	{
+		BuildSubset<kD>(st, R, P, st.sub[0], 3, p, s, false, lane);
+		const int line = EstimateLevels3<kD>(ss, st.sub[0], P, sp, water, ss.three.est[p][s], lane);
+		if (!(line < water))
+			return false;
+		if (lane == 0 && s)
+			ss.three.lines[p][s - 1] = line;
+		water -= line;
+		total += line;
+	}
+	return true;
+}
+
+/* The search of partition p from its estimates (the second loop); returns
+   whether it ends the full search. */
+template<int kD, int MODE>
+__device__ __forceinline__ bool ThreeSubsetsPartition(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const Spec3& sp, int p,
+	int lane)
+{
+	Ep mc0 = 0, mc1 = 0, mc2 = 0;
+	int error = R.opaqueAlphaError;
+#pragma unroll 1
+	for (int s = 0; s < 3; s++)
+	{
+		const int rest = s == 0 ? ss.three.lines[p][0] + ss.three.lines[p][1] : (s == 1 ? ss.three.lines[p][1] : 0);
+		const int water = R.errTotal - R.denoiseStep - error - rest;
+		BuildSubset<kD>(st, R, P, st.sub[0], 3, p, s, true, lane);
+		bool any;
+		Ep b = 0;
+		const int r = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, ss.three.est[p][s][1], ss.three.est[p][s][2], b, any, lane);
+		if (!any || !(r < water))
+			return false;
+		error += r;
+		if (s == 0)
+			mc0 = b;
+		else if (s == 1)
+			mc1 = b;
+		else
+			mc2 = b;
+	}
+	R.errTotal = error;
+	R.best[0] = mc0;
+	R.best[1] = mc1;
+	R.best[2] = mc2;
+	R.bestParam = p;
+	R.bestMode = MODE;
+	return error <= R.opaqueAlphaError;
 }
 
 /* Full searches of modes 0 and 2 (src/Bc7CoreMode0.cpp:532-642,
@@ -469,208 +784,142 @@ template<int kD, int MODE>
 __device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
 {
 	constexpr int NP = MODE == 0 ? 16 : 64;
-	const Spec3 sp = GetSpec3<MODE>(T);
-	const int step = R.denoiseStep;
+	const Spec3 sp = GetSpec3(MODE, T);
 	int count = 0;
+#pragma unroll 1
 	for (int p = 0; p < NP; p++)
 	{
 		if (R.personalMode == MODE && R.personalParam == p)
 			continue;
-		int e[3][4];
-		const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 0, lane);
-		const int water1 = R.errTotal - step - R.opaqueAlphaError;
-		const int line1 = EstimateLevels3<kD>(ss, st.sub[0], a1, P, sp, water1, e[0], lane);
-		if (line1 < water1)
+		int total;
+		if (ThreeSubsetsEstimate<kD, MODE>(st, ss, R, P, sp, p, total, lane))
 		{
-			const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 1, lane);
-			const int water2 = water1 - line1;
-			const int line2 = EstimateLevels3<kD>(ss, st.sub[0], a2, P, sp, water2, e[1], lane);
-			if (line2 < water2)
-			{
-				const AreaInfo a3 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 2, lane);
-				const int water3 = water2 - line2;
-				const int line3 = EstimateLevels3<kD>(ss, st.sub[0], a3, P, sp, water3, e[2], lane);
-				if (line3 < water3)
-				{
-					if (lane == 0)
-					{
-						ss.lines[p][0] = line2;
-						ss.lines[p][1] = line3;
-						for (int s = 0; s < 3; s++)
-							for (int c = 1; c < 4; c++)
-								ss.est[p][s][c - 1] = e[s][c];
-						ss.order[count] = make_int2(R.opaqueAlphaError + line1 + line2 + line3 + step, p);
-					}
-					count++;
-				}
-			}
+			if (lane == 0)
+				ss.three.order[count] = make_int2(total, p);
+			count++;
 		}
-		__syncwarp();
 	}
 	__syncwarp();
-	StableSortOrder(ss.order, count, lane);
-
+	StableSortOrder(ss.three.order, count, lane);
+#pragma unroll 1
 	for (int i = 0; i < count; i++)
 	{
-		const int2 o = ss.order[i];
-		if (o.x < R.errTotal)
-		{
-			const int p = o.y;
-			Ep mc[3] = { 0, 0, 0 };
-			const int line3 = ss.lines[p][1];
-			int e1[3] = { ss.est[p][0][0], ss.est[p][0][1], ss.est[p][0][2] };
-			const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 0, lane);
-			const int water1 = R.errTotal - step - R.opaqueAlphaError - ss.lines[p][0] - line3;
-			bool any;
-			int error = SearchSubset3<kD, MODE>(ss, st.sub[0], a1, P, T, water1, e1, mc[0], any, lane);
-			if (!any)
-				continue;
-			if (error < water1)
-			{
-				error += R.opaqueAlphaError;
-				int e2[3] = { ss.est[p][1][0], ss.est[p][1][1], ss.est[p][1][2] };
-				const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 1, lane);
-				const int water2 = R.errTotal - step - error - line3;
-				const int r2 = SearchSubset3<kD, MODE>(ss, st.sub[0], a2, P, T, water2, e2, mc[1], any, lane);
-				if (!any)
-					continue;
-				error += r2;
-				if (error < R.errTotal - step - line3)
-				{
-					int e3[3] = { ss.est[p][2][0], ss.est[p][2][1], ss.est[p][2][2] };
-					const AreaInfo a3 = BuildSubset<kD>(st, R, P, st.sub[0], 3, p, 2, lane);
-					const int water3 = R.errTotal - step - error;
-					const int r3 = SearchSubset3<kD, MODE>(ss, st.sub[0], a3, P, T, water3, e3, mc[2], any, lane);
-					if (!any)
-						continue;
-					error += r3;
-					if (R.errTotal > error + step)
-					{
-						R.errTotal = error;
-						R.best[0] = mc[0];
-						R.best[1] = mc[1];
-						R.best[2] = mc[2];
-						R.bestParam = p;
-						R.bestMode = MODE;
-						if (error <= R.opaqueAlphaError)
-							return;
-					}
-				}
-			}
-		}
+		const int2 o = ss.three.order[i];
+		if (o.x < R.errTotal && ThreeSubsetsPartition<kD, MODE>(st, ss, R, P, sp, o.y, lane))
+			return;
 	}
 }
 
 /* The partition search of modes 1 and 3 from its estimates (the second
    loop of src/Bc7CoreMode1.cpp:473-571, src/Bc7CoreMode3.cpp:471-569):
-   partition p with the principal-axis bounds line1, line2 (0 without
+   partition p with the principal-axis bounds line0, line1 (0 without
    OPTION_PCA).  Returns true when the search ends the full pass. */
 template<int kD, int MODE>
-__device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const Spec3& sp,
-	const LevelTables& T, int p, int line1, int line2, int lane)
+__device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const Spec3& sp, int p,
+	int line0, int line1, int lane)
 {
-	const int step = R.denoiseStep;
-	Ep mc[2] = { 0, 0 };
-	int e1[4], e2[4];
-	const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 2, p, 0, lane);
-	const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[1], 2, p, 1, lane);
-	int w1 = R.errTotal - step - R.opaqueAlphaError - line2;
-	line1 = max(line1, EstimateLevels3<kD>(ss, st.sub[0], a1, P, sp, w1, e1, lane));
-	if (line1 < w1)
+	const int room = R.errTotal - R.denoiseStep - R.opaqueAlphaError;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
 	{
-		int w2 = w1 - line1;
-		line2 = max(line2, EstimateLevels3<kD>(ss, st.sub[1], a2, P, sp, w2, e2, lane));
-		if (line2 < w2)
+		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		const int water = room - line1 - (s == 0 ? 0 : line0);
+		const int line = EstimateLevels3<kD>(ss, st.sub[s], P, sp, water, ss.bound[s], lane);
+		if (s == 0)
+			line0 = max(line0, line);
+		else
+			line1 = max(line1, line);
+		if (!((s == 0 ? line0 : line1) < water))
+			return false;
+	}
+	Ep mc0 = 0, mc1 = 0;
+	int error = 0;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		const int water = room - (s == 0 ? line1 : error);
+		bool any;
+		Ep b = 0;
+		const int r = SearchSubset3<kD, MODE>(ss, st.sub[s], P, sp, water, ss.bound[s][1], ss.bound[s][2], b, any, lane);
+		if (!any || !(r < water))
+			return false;
+		error += r;
+		if (s == 0)
+			mc0 = b;
+		else
+			mc1 = b;
+	}
+	R.errTotal = error + R.opaqueAlphaError;
+	R.best[0] = mc0;
+	R.best[1] = mc1;
+	R.bestParam = p;
+	R.bestMode = MODE;
+	return error <= 0;
+}
+
+/* The partitions' principal-axis bounds and their order (AreaGetBestPca3,
+   src/Bc7Core.cpp:494; EstimateBest, src/Bc7CoreMode7.cpp:559-572): ss.pca
+   lists the partitions whose bounds leave room.  OPTION_PCA only. */
+template<int kD, int MODE>
+__device__ __noinline__ int PcaPartitions(WarpState& st, SearchState& ss, const CellRegs& R, const Params& P, int base, int lane)
+{
+	int count = 0;
+#pragma unroll 1
+	for (int p = 0; p < 64; p++)
+	{
+		if (R.personalMode == MODE && R.personalParam == p)
+			continue;
+		int water = R.errTotal - R.denoiseStep - base, total = base + R.denoiseStep;
+		bool room = true;
+#pragma unroll 1
+		for (int s = 0; s < 2 && room; s++)
 		{
-			w1 = R.errTotal - step - R.opaqueAlphaError - line2;
-			const int est1[3] = { e1[1], e1[2], e1[3] };
-			bool any;
-			int error = SearchSubset3<kD, MODE>(ss, st.sub[0], a1, P, T, w1, est1, mc[0], any, lane);
-			if (any && error < w1)
-			{
-				error += R.opaqueAlphaError;
-				w2 = R.errTotal - step - error;
-				const int est2[3] = { e2[1], e2[2], e2[3] };
-				const int r2 = SearchSubset3<kD, MODE>(ss, st.sub[1], a2, P, T, w2, est2, mc[1], any, lane);
-				if (any)
-				{
-					error += r2;
-					if (R.errTotal > error + step)
-					{
-						R.errTotal = error;
-						R.best[0] = mc[0];
-						R.best[1] = mc[1];
-						R.bestParam = p;
-						R.bestMode = MODE;
-						if (error <= R.opaqueAlphaError)
-							return true;
-					}
-				}
-			}
+			BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+			const int line = PcaBound<kD>(st.sub[s], st.sub[s].info, P, MODE == 7 && !st.sub[s].info.opaque ? 4 : 3, lane);
+			room = line < water;
+			water -= line;
+			total += line;
+			if (lane == 0)
+				ss.pca.lines[p][s] = line;
+		}
+		if (room)
+		{
+			if (lane == 0)
+				ss.pca.order[count] = make_int2(total, p);
+			count++;
 		}
 	}
-	return false;
+	__syncwarp();
+	StableSortOrder(ss.pca.order, count, lane);
+	return count;
 }
 
 /* Full searches of modes 1 and 3 (src/Bc7CoreMode1.cpp:473-571,
    src/Bc7CoreMode3.cpp:471-569).  Without OPTION_PCA every partition's
    bound is zero, so every partition enters with estimate OA + step and the
    stable sort keeps index order; with it, the partitions are estimated and
-   sorted first (AreaGetBestPca3, src/Bc7Core.cpp:494).  Without OPTION_PCA
-   the search may resume at partition `from` (the partitions before it
-   searched already, R as they left it). */
+   sorted first.  Without OPTION_PCA the search may resume at partition
+   `from` (the partitions before it searched already, R as they left it). */
 template<int kD, int MODE>
 __device__ NEBC7_PASS void FullTwoSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane,
 	int from = 0)
 {
-	const Spec3 sp = GetSpec3<MODE>(T);
-	const int step = R.denoiseStep;
-	if (!P.pca)
+	const Spec3 sp = GetSpec3(MODE, T);
+	const int count = P.pca ? PcaPartitions<kD, MODE>(st, ss, R, P, R.opaqueAlphaError, lane) : 64;
+#pragma unroll 1
+	for (int i = P.pca ? 0 : from; i < count; i++)
 	{
-		for (int p = from; p < 64; p++)
+		int p = i, line0 = 0, line1 = 0, estimate = R.opaqueAlphaError + R.denoiseStep;
+		if (P.pca)
 		{
-			if (R.personalMode == MODE && R.personalParam == p)
-				continue;
-			if (!(0 < R.errTotal - step - R.opaqueAlphaError))
-				continue;
-			if (!(R.opaqueAlphaError + step < R.errTotal))
-				continue;
-			if (TwoSubsetsPartition<kD, MODE>(st, ss, R, P, sp, T, p, 0, 0, lane))
-				return;
+			estimate = ss.pca.order[i].x;
+			p = ss.pca.order[i].y;
+			line0 = ss.pca.lines[p][0];
+			line1 = ss.pca.lines[p][1];
 		}
-		return;
-	}
-	int count = 0;
-	for (int p = 0; p < 64; p++)
-	{
-		if (R.personalMode == MODE && R.personalParam == p)
+		else if (R.personalMode == MODE && R.personalParam == p)
 			continue;
-		const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 2, p, 0, lane);
-		const int water1 = R.errTotal - step - R.opaqueAlphaError;
-		const int line1 = PcaBound<kD>(st.sub[0], a1, P, 3, lane);
-		if (line1 < water1)
-		{
-			const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[1], 2, p, 1, lane);
-			const int line2 = PcaBound<kD>(st.sub[1], a2, P, 3, lane);
-			if (line2 < water1 - line1)
-			{
-				if (lane == 0)
-				{
-					ss.lines[p][0] = line1;
-					ss.lines[p][1] = line2;
-					ss.order[count] = make_int2(R.opaqueAlphaError + line1 + line2 + step, p);
-				}
-				count++;
-			}
-		}
-		__syncwarp();
-	}
-	__syncwarp();
-	StableSortOrder(ss.order, count, lane);
-	for (int i = 0; i < count; i++)
-	{
-		const int2 o = ss.order[i];
-		if (o.x < R.errTotal && TwoSubsetsPartition<kD, MODE>(st, ss, R, P, sp, T, o.y, ss.lines[o.y][0], ss.lines[o.y][1], lane))
+		if (estimate < R.errTotal && TwoSubsetsPartition<kD, MODE>(st, ss, R, P, sp, p, line0, line1, lane))
 			return;
 	}
 }
@@ -679,192 +928,324 @@ __device__ NEBC7_PASS void FullTwoSubsets(WarpState& st, SearchState& ss, CellRe
 /* Modes 6, 6Index2, 7: four channels with the transparent-alpha term       */
 /* ---------------------------------------------------------------------- */
 
-template<int kD, int IB, bool T4>
-__device__ __forceinline__ int TryVariants4Body(const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T,
-	const int2* const* Ls, const ChanList* cl, Ep& best, int water, int* planes, int lane)
+/* Error of every lane's candidate over a plane of np pixels (rows up to the
+   next multiple of four are zero): terms from the candidate table's column
+   `at`.  Ends once no lane is below its limit, so a lane's value is exact
+   whenever it is below it.  Warp-collective: every lane calls it. */
+__device__ __forceinline__ int TableError(const int4* plane, const int4* table, int at, int np, int limit)
 {
-	const int min0 = cl[0].minErr, min1 = cl[1].minErr, min2 = cl[2].minErr, min3 = cl[3].minErr;
-	if (min0 + min1 + min2 + min3 >= water)
-		return water;
-	const int n1 = cl[1].count, n2 = cl[2].count, n3 = cl[3].count, np = ai.active;
-	const bool opq = ai.opaque;
-	const int2* L0 = Ls[0];
-	const int2* L1 = Ls[1];
-	const int2* L2 = Ls[2];
-	const int2* L3 = Ls[3];
-	/* an opaque area has alpha 255 and the alpha list holds 0xFFFF only, so the
-	   alpha plane is zero and the A-less weights of the reference's opaque
-	   branch give the same sums as the planes below */
-	int* pA = planes;
-	int* pAG = planes + 256;
-	int* pAGR = planes + 512;
-	const int col1l = lane < n1 ? L1[lane].y : 0;
-	const int col2l = lane < n2 ? L2[lane].y : 0;
-	const int col3 = lane < n3 ? L3[lane].y : 0;
-	const int e3base = lane < n3 ? L3[lane].x : kBig;
-	for (int i0 = 0; i0 < cl[0].count; i0++)
+	int sum = 0;
+	for (int i = 0; i < np; i += 4)
 	{
-		const int e0 = L0[i0].x;
+#pragma unroll
+		for (int j = 0; j < 4; j++)
+			sum += RowMin(plane[i + j], table[(i + j) * kTableRow + at]);
+		if (!__any_sync(kFull, sum < limit))
+			break;
+	}
+	return sum;
+}
+
+/* The four-channel combination search with 2-bit indices (modes 7 and
+   6Index2; src/Bc7CoreMode6.cpp:1163-1331).
+ *
+ * Every bound that the reference compares here is a lower bound of the error
+ * it stands for: a channel's list error takes each pixel's nearest level on
+ * its own, over the same pixels and with the same transparent-alpha term as
+ * the joint error, and a joint error over fewer channels drops non-negative
+ * terms.  So the sequential search ends with the first combination, in its
+ * order, of the smallest error below the water, and any lower bound may
+ * skip: besides the reference's, the sums below take the entry's own list
+ * error where the reference takes the list's minimum, and a level's errors
+ * are computed only when some combination under it is still open.
+ *
+ * What bounds it: instruction issue in the error sums.  A candidate's terms
+ * w q^2 per pixel and level do not depend on the outer loops, so B's are kept
+ * in the lane's registers (lane = candidate) and R's in a shared-memory
+ * table, and a pixel costs one broadcast read of the plane and four fused
+ * add-minimum steps instead of four differences, squares and products. */
+template<int kD>
+__device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
+	const uint8_t* alphaTable, Ep best, int water, int lane)
+{
+	const int4 m01 = *reinterpret_cast<const int4*>(&ss.chan[v][0]), m23 = *reinterpret_cast<const int4*>(&ss.chan[v][2]);
+	const int min0 = m01.x, n0 = m01.y, min1 = m01.z, n1 = m01.w;
+	const int min2 = m23.x, n2 = m23.y, min3 = m23.z, n3 = m23.w;
+	if (min0 + min1 + min2 + min3 >= water)
+		return Found{ water, best };
+	const int2 l1 = lane < n1 ? ss.lists[v][1][lane] : make_int2(kFar, 0);
+	const int2 l2 = lane < n2 ? ss.lists[v][2][lane] : make_int2(kFar, 0);
+	const int2 l3 = lane < n3 ? ss.lists[v][3][lane] : make_int2(kFar, 0);
+	int4* const pA = ss.plane;
+	int4* const pAG = (ss.plane + 16);
+	int4* const pAGR = (ss.plane + 32);
+	const int at = lane < kTableRow - 1 ? lane : kTableRow - 1;
+
+	/* R's table, B's registers */
+	LaneTerms<kD, 2> termsB;
+	termsB.Init(ar, np, 3, l3.y, w.b);
+	if (lane < kTableRow)
+		for (int i = 0; i < ((np + 3) & ~3); i++)
+			ss.table[i * kTableRow + lane] = i < np ? LevelTerms<kD>(int(ar.px[i][2]), l2.y, w.r) : make_int4(0, 0, 0, 0);
+	const PlaneLanes<kD, 2> pl(np, lane);
+	int xa[2], xg[2], ga[2], gg[2], gr[2];
+	pl.Pixels(ar, 0, xa);
+	pl.Pixels(ar, 1, xg);
+	const int zero[2] = { 0, 0 };
+
+	for (int i0 = 0; i0 < n0; i0++)
+	{
+		const int2 a = ss.lists[v][0][i0];
+		const int e0 = a.x;
 		if (e0 + min1 + min2 + min3 >= water)
 			break;
-		const int c0 = L0[i0].y;
-		const int ea = T4 ? TransparentError4(T, P, ai.count, ai.active, c0) : TransparentError2(T, P, ai.count, ai.active, c0);
-		PlaneAdd<kD, IB>(pA, nullptr, ar, np, 0, c0, P.wA, lane);
-		int memAR = kBig, pairAG = kBig;
+		int ea = (count - np) * w.a;
+		if (count > np)
+		{
+			const int d = DiffAt(alphaTable, 0, a.y & 0xFF, (a.y >> 8) & 0xFF);
+			ea *= d * d;
+		}
+		pl.Add(ga, zero, xa, a.y, w.a);
+		__syncwarp();
+		pl.Store(pA, ga, lane);
+		/* joint errors of this alpha candidate with every R and every G one
+		   (an opaque area's alpha term is zero: the list errors are they) */
+		int errAR = l2.x + e0, errAG = l1.x + e0;
 		if (!opq)
 		{
-			if (lane < n2)
-				memAR = PlaneError<kD, IB>(pA, ar, np, 2, col2l, P.wR, water - ea - min1 - min3) + ea;
-			if (lane < n1)
-				pairAG = PlaneError<kD, IB>(pA, ar, np, 1, col1l, P.wG, water - ea - min2 - min3) + ea;
-		}
-		for (int i1 = 0; i1 < n1; i1++)
-		{
-			int e1 = L1[i1].x + e0;
-			if (e1 + min2 + min3 >= water)
-				break;
-			const int c1 = L1[i1].y;
-			if (!opq)
+			const int sumR = TableError(pA, ss.table, at, np, lane < n2 ? water - ea - min1 - min3 : kNoLimit);
+			errAR = lane < n2 ? sumR + ea : kFar;
+			int sum = 0;
+			const int limit = lane < n1 ? water - ea - min2 - min3 : kNoLimit;
+			for (int i = 0; i < np; i++)
 			{
-				e1 = __shfl_sync(kFull, pairAG, i1);
-				if (e1 + min2 + min3 >= water)
-					continue;
-			}
-			PlaneAdd<kD, IB>(pAG, pA, ar, np, 1, c1, P.wG, lane);
-			const Ep base01 = Ep2(0, c0, 1, c1);
-			int memAGB = kBig, pairAGR = kBig;
-			if (lane < n3)
-				memAGB = PlaneError<kD, IB>(pAG, ar, np, 3, col3, P.wB, water - ea - min2) + ea;
-			if (lane < n2)
-				pairAGR = PlaneError<kD, IB>(pAG, ar, np, 2, col2l, P.wR, water - ea - min3) + ea;
-			for (int i2 = 0; i2 < n2; i2++)
-			{
-				const int e2s = L2[i2].x + e1;
-				if (e2s + min3 >= water)
+				sum += RowMin(pA[i], LevelTerms<kD>(int(ar.px[i][1]), l1.y, w.g));
+				if (!__any_sync(kFull, sum < limit))
 					break;
-				const int c2 = L2[i2].y;
-				if (!opq)
-				{
-					const int ear = __shfl_sync(kFull, memAR, i2);
-					if (ear + min1 + min3 >= water)
-						continue;
-				}
-				const int e2 = __shfl_sync(kFull, pairAGR, i2);
-				if (e2 + min3 >= water)
-					continue;
-				const bool valid = lane < n3;
-				const int brk = valid ? e3base + e2 : kBig;
-				const int skip = valid ? memAGB + min2 : kBig;
-				const bool eval = valid && brk < water && skip < water;
-				/* no lane evaluates: the replay accepts nothing, the plane is not needed */
+			}
+			errAG = lane < n1 ? sum + ea : kFar;
+		}
+		int i1 = 0;
+		for (;;)
+		{
+			/* the next G candidate still open */
+			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
+			if (!open1)
+				break;
+			i1 = __ffs(open1) - 1;
+			const int eAG = __shfl_sync(kFull, errAG, i1);
+			const int2 g = make_int2(__shfl_sync(kFull, l1.x, i1), __shfl_sync(kFull, l1.y, i1));
+			i1++;
+			const bool openR = l2.x + eAG + min3 < water && errAR + g.x + min3 < water;
+			if (!__any_sync(kFull, openR))
+				continue;
+			pl.Add(gg, ga, xg, g.y, w.g);
+			pl.Store(pAG, gg, lane);
+			const int sumR = TableError(pAG, ss.table, at, np, openR ? water - ea - min3 : kNoLimit);
+			const int errAGR = openR ? sumR + ea : kFar;
+			unsigned open2 = __ballot_sync(kFull, errAGR + min3 < water);
+			if (!open2)
+				continue;
+			const bool openB = l3.x + eAG + min2 < water;
+			const int sumB = termsB.Error(pAG, np, w.b, openB ? water - ea - min2 : kNoLimit);
+			const int errAGB = openB ? sumB + ea : kFar;
+			while (open2)
+			{
+				const int i2 = __ffs(open2) - 1;
+				open2 &= open2 - 1;
+				const int e2 = __shfl_sync(kFull, errAGR, i2);
+				const int2 r = make_int2(__shfl_sync(kFull, l2.x, i2), __shfl_sync(kFull, l2.y, i2));
+				const bool eval = l3.x + e2 < water && errAGB + r.x < water;
 				if (!__any_sync(kFull, eval))
 					continue;
-				PlaneAdd<kD, IB>(pAGR, pAG, ar, np, 2, c2, P.wR, lane);
-				const Ep base012 = EpSetCh(base01, 2, c2);
-				int err = kBig;
-				if (eval)
-					err = PlaneError<kD, IB>(pAGR, ar, np, 3, col3, P.wB, water - ea) + ea;
-				const int jl = ReplayInner(valid, brk, skip, err, water, lane);
-				if (jl >= 0)
-					best = EpSetCh(base012, 3, __shfl_sync(kFull, col3, jl));
+				const int* t = reinterpret_cast<const int*>(ss.table) + (pl.row * kTableRow + i2) * 4 + (lane & 3);
+				gr[0] = pl.row < np ? gg[0] + t[0] : 0;
+				gr[1] = pl.row + 8 < np ? gg[1] + t[8 * kTableRow * 4] : 0;
+				pl.Store(pAGR, gr, lane);
+				const int sum = termsB.Error(pAGR, np, w.b, eval ? water - ea : kNoLimit);
+				const int err = eval ? sum + ea : kFar;
+				/* the first lane of the smallest error below the water */
+				const int low = __reduce_min_sync(kFull, err);
+				if (low < water)
+				{
+					const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
+					water = low;
+					best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+				}
 			}
 		}
 	}
-	return water;
+	return Found{ water, best };
+}
+
+/* The same search with 4-bit indices (mode 6): sixteen levels a pixel do not
+   fit registers or a table, so a candidate's terms are computed per plane. */
+template<int kD>
+__device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
+	const uint8_t* alphaTable, Ep best, int water, int lane)
+{
+	const int4 m01 = *reinterpret_cast<const int4*>(&ss.chan[v][0]), m23 = *reinterpret_cast<const int4*>(&ss.chan[v][2]);
+	const int min0 = m01.x, n0 = m01.y, min1 = m01.z, n1 = m01.w;
+	const int min2 = m23.x, n2 = m23.y, min3 = m23.z, n3 = m23.w;
+	if (min0 + min1 + min2 + min3 >= water)
+		return Found{ water, best };
+	const int2 l1 = lane < n1 ? ss.lists[v][1][lane] : make_int2(kFar, 0);
+	const int2 l2 = lane < n2 ? ss.lists[v][2][lane] : make_int2(kFar, 0);
+	const int2 l3 = lane < n3 ? ss.lists[v][3][lane] : make_int2(kFar, 0);
+	int* const pA = ss.plane16[0];
+	int* const pAG = ss.plane16[1];
+	int* const pAGR = ss.plane16[2];
+	for (int i0 = 0; i0 < n0; i0++)
+	{
+		const int2 a = ss.lists[v][0][i0];
+		const int e0 = a.x;
+		if (e0 + min1 + min2 + min3 >= water)
+			break;
+		int ea = (count - np) * w.a;
+		if (count > np)
+		{
+			const int d = HalfAt(alphaTable, 0, a.y & 0xFF, (a.y >> 8) & 0xFF);
+			ea *= d * d;
+		}
+		PlaneAdd<kD, 4>(pA, nullptr, ar, np, 0, a.y, w.a, lane);
+		int errAR = l2.x + e0, errAG = l1.x + e0;
+		if (!opq)
+		{
+			if (lane < n2)
+				errAR = PlaneError<kD, 4>(pA, ar, np, 2, l2.y, w.r, water - ea - min1 - min3) + ea;
+			if (lane < n1)
+				errAG = PlaneError<kD, 4>(pA, ar, np, 1, l1.y, w.g, water - ea - min2 - min3) + ea;
+		}
+		int i1 = 0;
+		for (;;)
+		{
+			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
+			if (!open1)
+				break;
+			i1 = __ffs(open1) - 1;
+			const int eAG = __shfl_sync(kFull, errAG, i1);
+			const int2 g = make_int2(__shfl_sync(kFull, l1.x, i1), __shfl_sync(kFull, l1.y, i1));
+			i1++;
+			const bool openR = l2.x + eAG + min3 < water && errAR + g.x + min3 < water;
+			if (!__any_sync(kFull, openR))
+				continue;
+			PlaneAdd<kD, 4>(pAG, pA, ar, np, 1, g.y, w.g, lane);
+			int errAGR = kFar, errAGB = kFar;
+			if (openR)
+				errAGR = PlaneError<kD, 4>(pAG, ar, np, 2, l2.y, w.r, water - ea - min3) + ea;
+			unsigned open2 = __ballot_sync(kFull, errAGR + min3 < water);
+			if (!open2)
+				continue;
+			if (l3.x + eAG + min2 < water)
+				errAGB = PlaneError<kD, 4>(pAG, ar, np, 3, l3.y, w.b, water - ea - min2) + ea;
+			while (open2)
+			{
+				const int i2 = __ffs(open2) - 1;
+				open2 &= open2 - 1;
+				const int e2 = __shfl_sync(kFull, errAGR, i2);
+				const int2 r = make_int2(__shfl_sync(kFull, l2.x, i2), __shfl_sync(kFull, l2.y, i2));
+				const bool eval = l3.x + e2 < water && errAGB + r.x < water;
+				if (!__any_sync(kFull, eval))
+					continue;
+				PlaneAdd<kD, 4>(pAGR, pAG, ar, np, 2, r.y, w.r, lane);
+				int err = kFar;
+				if (eval)
+					err = PlaneError<kD, 4>(pAGR, ar, np, 3, l3.y, w.b, water - ea) + ea;
+				const int low = __reduce_min_sync(kFull, err);
+				if (low < water)
+				{
+					const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
+					water = low;
+					best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+				}
+			}
+		}
+	}
+	return Found{ water, best };
 }
 
 /* Out-of-line copy for modes 6 and 7; the Mode6Index2 refinement (the
    common case of the default preset) inlines the body. */
-template<int kD, int IB, bool T4>
-__device__ NEBC7_SHARED int TryVariants4(const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T, const int2* const* Ls,
-	const ChanList* cl, Ep& best, int water, int* planes, int lane)
+template<int kD, int IB>
+__device__ NEBC7_SHARED Found SearchFour(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
+	const uint8_t* alphaTable, Ep best, int water, int lane)
 {
-	return TryVariants4Body<kD, IB, T4>(ar, ai, P, T, Ls, cl, best, water, planes, lane);
+	if constexpr (IB == 4)
+		return SearchFour4<kD>(ss, v, ar, count, np, opq, w, alphaTable, best, water, lane);
+	else
+		return SearchFour2<kD>(ss, v, ar, count, np, opq, w, alphaTable, best, water, lane);
 }
 
-/* Subset::InitLevels of modes 6 / 6Index2 / 7 (src/Bc7CoreMode6.cpp:1130-1161,
-   src/Bc7CoreMode7.cpp:237-268). */
+/* Subset::InitLevels of modes 6 / 6Index2 (9) / 7 (src/Bc7CoreMode6.cpp:
+   1130-1161, src/Bc7CoreMode7.cpp:237-268) for the p-bits of variant pv into
+   the lists of slot v; est: lower bounds of the channels' errors, or null. */
 template<int kD, int MODE>
-__device__ NEBC7_PASS bool InitLevels4(SearchState& ss, int v, int pbits, const Area& ar, const AreaInfo& ai, const Params& P,
-	const LevelTables& T, int water, const int est[4], ChanList cl[4], int lane)
+__device__ NEBC7_PASS bool InitLevels4(SearchState& ss, int v, int pv, const Area& ar, const Params& P, const LevelTables& T, int water,
+	const int* est, int lane)
 {
-	const int wts[4] = { P.wA, P.wG, P.wR, P.wB };
 	int used = 0;
+	int rest = est ? est[1] + est[2] + est[3] : 0;
+#pragma unroll 1
 	for (int c = 0; c < 4; c++)
 	{
-		int rest = 0;
-		for (int k = c + 1; k < 4; k++)
-			rest += est[k];
-		if (c == 0 && ai.opaque)
-		{
-			cl[0] = ZeroList(ss.lists[v][0], 0xFFFF, lane);
-		}
-		else if (MODE == 6)
-		{
-			cl[c] = ChannelLevels<kD, true>(ss.lists[v][c], ar, ai, c, wts[c], water - used - rest, 7, pbits, c != 0, T.d4h, true, 20, ss.uniq,
-				lane);
-		}
-		else if (MODE == 9)
-		{
-			cl[c] = ChannelLevelsScan<kD, true>(ss.lists[v][c], ar, ai, c, wts[c], water - used - rest, 7, pbits, c != 0, T.d2h, true, 20,
-				ss.uniq, lane);
-		}
+		ChanList cl;
+		if (c == 0 && ar.info.opaque)
+			cl = ZeroList(ss.lists[v][0], 0xFFFF, lane);
 		else
-		{
-			cl[c] = ChannelLevels<kD, false>(ss.lists[v][c], ar, ai, c, wts[c], water - used - rest, 5, pbits, c != 0, kReducedByDiff ? T.d2v8 : T.d2v6,
-				kReducedByDiff, 20,
-				ss.uniq, lane);
-		}
-		used += cl[c].minErr;
+			cl = ChannelLevels<kD, MODE != 7>(ss.lists[v][c], ar, c, ChannelWeight(P, c), water - used - rest, MODE == 7 ? 5 : 7,
+				VariantPbits(pv), c != 0, MODE == 6 ? T.h4s : (MODE == 9 ? T.h2s : T.d2v8), true, 20, ss.values, lane);
+		if (lane == 0)
+			ss.chan[v][c] = cl;
+		used += cl.minErr;
 		if (used >= water)
 			return false;
+		if (est && c < 3)
+			rest -= est[c + 1];
 	}
+	__syncwarp();
 	return true;
 }
 
 template<int kD, int MODE>
-__device__ int TryV4(SearchState& ss, int v, const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T,
-	const ChanList cl[4], Ep& best, int water, int lane)
+__device__ __forceinline__ int TryV4(SearchState& ss, int v, const Area& ar, const Params& P, const LevelTables& T, Ep& best, int water,
+	int lane)
 {
-	const int2* Ls[4] = { ss.lists[v][0], ss.lists[v][1], ss.lists[v][2], ss.lists[v][3] };
-	if (MODE == 6)
-		return TryVariants4<kD, 4, true>(ar, ai, P, T, Ls, cl, best, water, &ss.planes[0][0], lane);
-	if (MODE == 9)
-		return TryVariants4Body<kD, 2, false>(ar, ai, P, T, Ls, cl, best, water, &ss.planes[0][0], lane);
-	return TryVariants4<kD, 2, false>(ar, ai, P, T, Ls, cl, best, water, &ss.planes[0][0], lane);
+	const AreaInfo& ai = ar.info;
+	const Found f = SearchFour<kD, MODE == 6 ? 4 : 2>(ss, v, ar, ai.count, ai.active, ai.opaque, WeightsOf(P), MODE == 6 ? T.d4h : T.d2v8, best,
+		water, lane);
+	best = f.best;
+	return f.water;
 }
 
 /* Mode 6 / 6Index2 CompressSubset (src/Bc7CoreMode6.cpp:1334-1364): each
    later p-bit variant starts from the water left by the earlier ones. */
 template<int kD, int MODE>
-__device__ NEBC7_PASS int CompressSubsetSingle(SearchState& ss, const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T,
-	Ep& mc, int water, int lane)
+__device__ NEBC7_PASS int CompressSubsetSingle(SearchState& ss, const Area& ar, const Params& P, const LevelTables& T, Ep& mc, int water,
+	int lane)
 {
-	const int est[4] = { 0, 0, 0, 0 };
-	const int pb[4] = { 0x0101, 0, 1, 1 << 8 };
-	for (int v = 0; v < (ai.opaque ? 1 : 4); v++)
-	{
-		ChanList cl[4];
-		if (InitLevels4<kD, MODE>(ss, 0, pb[v], ar, ai, P, T, water, est, cl, lane))
-			water = TryV4<kD, MODE>(ss, 0, ar, ai, P, T, cl, mc, water, lane);
-	}
+#pragma unroll 1
+	for (int v = 0; v < (ar.info.opaque ? 1 : 4); v++)
+		if (InitLevels4<kD, MODE>(ss, 0, v, ar, P, T, water, nullptr, lane))
+			water = TryV4<kD, MODE>(ss, 0, ar, P, T, mc, water, lane);
 	return water;
 }
 
-/* Mode 7 Subsets (src/Bc7CoreMode7.cpp:441-494). */
+/* Mode 7 Subsets (src/Bc7CoreMode7.cpp:441-494): all variants' lists start
+   from the same water. */
 template<int kD>
-__device__ NEBC7_PASS int SearchSubset7(SearchState& ss, const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T,
-	int water, const int est[4], Ep& best, bool& any, int lane)
+__device__ NEBC7_PASS int SearchSubset7(SearchState& ss, const Area& ar, const Params& P, const LevelTables& T, int water, const int* est,
+	Ep& best, bool& any, int lane)
 {
-	const int pb[4] = { 0x0101, 0, 1, 1 << 8 };
-	ChanList cl[4][4];
-	bool valid[4] = { false, false, false, false };
-	for (int v = 0; v < (ai.opaque ? 1 : 4); v++)
-		valid[v] = InitLevels4<kD, 7>(ss, v, pb[v], ar, ai, P, T, water, est, cl[v], lane);
-	any = valid[0] || valid[1] || valid[2] || valid[3];
-	for (int v = 0; v < 4; v++)
-		if (valid[v])
-			water = TryV4<kD, 7>(ss, v, ar, ai, P, T, cl[v], best, water, lane);
+	int valid = 0;
+	const int nv = ar.info.opaque ? 1 : 4;
+#pragma unroll 1
+	for (int v = 0; v < nv; v++)
+		valid |= int(InitLevels4<kD, 7>(ss, v, v, ar, P, T, water, est, lane)) << v;
+	any = valid != 0;
+#pragma unroll 1
+	for (int v = 0; v < nv; v++)
+		if ((valid >> v) & 1)
+			water = TryV4<kD, 7>(ss, v, ar, P, T, best, water, lane);
 	return water;
 }
 
@@ -873,7 +1254,7 @@ __device__ NEBC7_PASS void RefineMode6(WarpState& st, SearchState& ss, CellRegs&
 {
 	/* src/Bc7CoreMode6.cpp:1366-1381 */
 	Ep mc = R.best[0];
-	const int error = CompressSubsetSingle<kD, MODE>(ss, st.area1, R.a1, P, T, mc, R.errTotal, lane);
+	const int error = CompressSubsetSingle<kD, MODE>(ss, st.area1, P, T, mc, R.errTotal, lane);
 	if (R.errTotal > error)
 	{
 		R.errTotal = error;
@@ -893,7 +1274,7 @@ __device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R
 	if (line < R.errTotal - step)
 	{
 		Ep mc = 0;
-		const int error = CompressSubsetSingle<kD, 6>(ss, st.area1, R.a1, P, T, mc, R.errTotal - step, lane);
+		const int error = CompressSubsetSingle<kD, 6>(ss, st.area1, P, T, mc, R.errTotal - step, lane);
 		if (R.errTotal > error + step)
 		{
 			R.errTotal = error;
@@ -907,130 +1288,118 @@ template<int kD>
 __device__ NEBC7_PASS void RefineMode7(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
 {
 	/* src/Bc7CoreMode7.cpp:496-557 */
-	const int p = R.bestParam;
-	Ep mc[2] = { R.best[0], R.best[1] };
-	const int est[4] = { 0, 0, 0, 0 };
+	Ep mc0 = R.best[0], mc1 = R.best[1];
 	const int w[4] = { P.wA, P.wG, P.wR, P.wB };
 	int error = 0;
+#pragma unroll 1
 	for (int s = 0; s < 2; s++)
 	{
-		const AreaInfo ai = BuildSubset<kD>(st, R, P, st.sub[0], 2, p, s, lane);
-		int water = AreaError<kD, 2>(st.sub[0], ai.active, mc[s], w, 2 * MaxColorError<kD>());
-		water += TransparentError2(T, P, ai.count, ai.active, int(mc[s] & 0xFFFF));
+		Area& ar = st.sub[0];
+		BuildSubset<kD>(st, R, P, ar, 2, R.bestParam, s, true, lane);
+		Ep b = s == 0 ? mc0 : mc1;
+		int water = AreaError<kD, 2>(ar, ar.info.active, b, w, 2 * MaxColorError<kD>());
+		water += TransparentError2(T, P, ar.info.count, ar.info.active, int(b & 0xFFFF));
 		if (water)
 		{
 			bool any;
-			Ep b = mc[s];
-			const int r = SearchSubset7<kD>(ss, st.sub[0], ai, P, T, water, est, b, any, lane);
+			const int r = SearchSubset7<kD>(ss, ar, P, T, water, nullptr, b, any, lane);
 			if (any)
 			{
-				error += r;
-				mc[s] = b;
+				water = r;
+				if (s == 0)
+					mc0 = b;
+				else
+					mc1 = b;
 			}
-			else
-				error += water;
+			error += water;
 		}
 	}
 	if (R.errTotal > error)
 	{
 		R.errTotal = error;
-		R.best[0] = mc[0];
-		R.best[1] = mc[1];
+		R.best[0] = mc0;
+		R.best[1] = mc1;
 	}
 }
 
-/* EstimateLevels of mode 7 (src/Bc7CoreMode7.cpp:574-627). */
+/* EstimateLevels of mode 7 (src/Bc7CoreMode7.cpp:574-627): est[0..3] get the
+   estimates of A, G, R, B. */
 template<int kD>
-__device__ NEBC7_PASS int EstimateLevels7(SearchState& ss, const Area& ar, const AreaInfo& ai, const Params& P, const LevelTables& T, int water,
-	int est[4], int lane)
+__device__ NEBC7_PASS int EstimateLevels7(SearchState& ss, const Area& ar, const Params& P, const LevelTables& T, int water, int* est,
+	int lane)
 {
-	int error = 0;
-	if (error < water)
+	if (!(0 < water))
+		return water;
+	if (!ar.info.active)
 	{
-		if (!ai.active)
-		{
-			est[0] = est[1] = est[2] = est[3] = 0;
-			return 0;
-		}
-		if (!ai.opaque)
-		{
-			const int l0 = EstimateChannelLevels<kD>(ar, ai, 0, P.wA, water - error, 6, false, kReducedByDiff ? T.d2v8 : T.d2v6, kReducedByDiff,
-				T.c2v6, ss.uniq, lane);
-			est[0] = l0;
-			error += l0;
-		}
-		else
-			est[0] = 0;
-		const int wts[4] = { P.wA, P.wG, P.wR, P.wB };
-		for (int c = 1; c < 4; c++)
-		{
-			if (!(error < water))
-				return water;
-			const int l = EstimateChannelLevels<kD>(ar, ai, c, wts[c], water - error, 6, true, kReducedByDiff ? T.d2v8 : T.d2v6, kReducedByDiff,
-				T.c2v6, ss.uniq, lane);
-			est[c] = l;
-			error += l;
-		}
-		if (error < water)
-			return error;
+		__syncwarp();
+		if (lane < 4)
+			est[lane] = 0;
+		__syncwarp();
+		return 0;
 	}
-	return water;
+	int error = 0;
+#pragma unroll 1
+	for (int c = 0; c < 4; c++)
+	{
+		if (!(error < water))
+			return water;
+		int l = 0;
+		if (c || !ar.info.opaque)
+			l = EstimateChannelLevels<kD>(ar, c, ChannelWeight(P, c), water - error, 6, c != 0, T.d2v8, true, T.c2v6, ss.values, lane);
+		if (lane == 0)
+			est[c] = l;
+		error += l;
+	}
+	__syncwarp();
+	return error < water ? error : water;
 }
 
 /* The partition search of mode 7 from its estimates (the second loop of
    src/Bc7CoreMode7.cpp:629-725): partition p with the principal-axis bounds
-   line1, line2 (0 without OPTION_PCA).  Returns true when the search ends
+   line0, line1 (0 without OPTION_PCA).  Returns true when the search ends
    the full pass. */
 template<int kD>
 __device__ __forceinline__ bool Mode7Partition(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T,
-	int p, int line1, int line2, int lane)
+	int p, int line0, int line1, int lane)
 {
-	const int step = R.denoiseStep;
-	Ep mc[2] = { 0, 0 };
-	int e1[4], e2[4];
-	const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 2, p, 0, lane);
-	const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[1], 2, p, 1, lane);
-	int w1 = R.errTotal - step - line2;
-	line1 = max(line1, EstimateLevels7<kD>(ss, st.sub[0], a1, P, T, w1, e1, lane));
-	if (line1 < w1)
+	const int room = R.errTotal - R.denoiseStep;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
 	{
-		int w2 = w1 - line1;
-		line2 = max(line2, EstimateLevels7<kD>(ss, st.sub[1], a2, P, T, w2, e2, lane));
-		if (line2 < w2)
-		{
-			w1 = R.errTotal - step - line2;
-			bool any;
-			int error = SearchSubset7<kD>(ss, st.sub[0], a1, P, T, w1, e1, mc[0], any, lane);
-			if (any && error < w1)
-			{
-				w2 = R.errTotal - step - error;
-				const int r2 = SearchSubset7<kD>(ss, st.sub[1], a2, P, T, w2, e2, mc[1], any, lane);
-				if (any)
-				{
-					error += r2;
-					if (R.errTotal > error + step)
-					{
-						R.errTotal = error;
-						R.best[0] = mc[0];
-						R.best[1] = mc[1];
-						R.bestParam = p;
-						R.bestMode = 7;
-						if (error <= 0)
-							return true;
-					}
-				}
-			}
-		}
+		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		const int water = room - line1 - (s == 0 ? 0 : line0);
+		const int line = EstimateLevels7<kD>(ss, st.sub[s], P, T, water, ss.bound[s], lane);
+		if (s == 0)
+			line0 = max(line0, line);
+		else
+			line1 = max(line1, line);
+		if (!((s == 0 ? line0 : line1) < water))
+			return false;
 	}
-	return false;
-}
-
-/* EstimateBest of mode 7 (src/Bc7CoreMode7.cpp:559-572): the principal-axis
-   bound over G, R, B for an opaque area, over A, G, R, B otherwise. */
-template<int kD>
-__device__ __forceinline__ int EstimateBest(const Area& ar, const AreaInfo& ai, const Params& P, int lane)
-{
-	return PcaBound<kD>(ar, ai, P, ai.opaque ? 3 : 4, lane);
+	Ep mc0 = 0, mc1 = 0;
+	int error = 0;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		const int water = room - (s == 0 ? line1 : error);
+		bool any;
+		Ep b = 0;
+		const int r = SearchSubset7<kD>(ss, st.sub[s], P, T, water, ss.bound[s], b, any, lane);
+		if (!any || !(r < water))
+			return false;
+		error += r;
+		if (s == 0)
+			mc0 = b;
+		else
+			mc1 = b;
+	}
+	R.errTotal = error;
+	R.best[0] = mc0;
+	R.best[1] = mc1;
+	R.bestParam = p;
+	R.bestMode = 7;
+	return error <= 0;
 }
 
 template<int kD>
@@ -1040,53 +1409,21 @@ __device__ NEBC7_PASS void FullMode7(WarpState& st, SearchState& ss, CellRegs& R
 	/* src/Bc7CoreMode7.cpp:629-725; without OPTION_PCA every partition enters
 	   with estimate step (ties keep index order), and the search may resume
 	   at partition `from` */
-	const int step = R.denoiseStep;
-	if (!P.pca)
+	const int count = P.pca ? PcaPartitions<kD, 7>(st, ss, R, P, 0, lane) : 64;
+#pragma unroll 1
+	for (int i = P.pca ? 0 : from; i < count; i++)
 	{
-		for (int p = from; p < 64; p++)
+		int p = i, line0 = 0, line1 = 0, estimate = R.denoiseStep;
+		if (P.pca)
 		{
-			if (R.personalMode == 7 && R.personalParam == p)
-				continue;
-			if (!(0 < R.errTotal - step))
-				continue;
-			if (!(step < R.errTotal))
-				continue;
-			if (Mode7Partition<kD>(st, ss, R, P, T, p, 0, 0, lane))
-				return;
+			estimate = ss.pca.order[i].x;
+			p = ss.pca.order[i].y;
+			line0 = ss.pca.lines[p][0];
+			line1 = ss.pca.lines[p][1];
 		}
-		return;
-	}
-	int count = 0;
-	for (int p = 0; p < 64; p++)
-	{
-		if (R.personalMode == 7 && R.personalParam == p)
+		else if (R.personalMode == 7 && R.personalParam == p)
 			continue;
-		const AreaInfo a1 = BuildSubset<kD>(st, R, P, st.sub[0], 2, p, 0, lane);
-		const int water1 = R.errTotal - step;
-		const int line1 = EstimateBest<kD>(st.sub[0], a1, P, lane);
-		if (line1 < water1)
-		{
-			const AreaInfo a2 = BuildSubset<kD>(st, R, P, st.sub[1], 2, p, 1, lane);
-			const int line2 = EstimateBest<kD>(st.sub[1], a2, P, lane);
-			if (line2 < water1 - line1)
-			{
-				if (lane == 0)
-				{
-					ss.lines[p][0] = line1;
-					ss.lines[p][1] = line2;
-					ss.order[count] = make_int2(line1 + line2 + step, p);
-				}
-				count++;
-			}
-		}
-		__syncwarp();
-	}
-	__syncwarp();
-	StableSortOrder(ss.order, count, lane);
-	for (int i = 0; i < count; i++)
-	{
-		const int2 o = ss.order[i];
-		if (o.x < R.errTotal && Mode7Partition<kD>(st, ss, R, P, T, o.y, ss.lines[o.y][0], ss.lines[o.y][1], lane))
+		if (estimate < R.errTotal && Mode7Partition<kD>(st, ss, R, P, T, p, line0, line1, lane))
 			return;
 	}
 }
@@ -1096,9 +1433,10 @@ __device__ NEBC7_PASS void FullMode7(WarpState& st, SearchState& ss, CellRegs& R
 /* ---------------------------------------------------------------------- */
 
 template<int kD, int MODE, int CB, int AB>
-__device__ NEBC7_SHARED int TryVariantsRot(const Area& ar, const AreaInfo& ai, const Params& P, const int2* const* Ls, const ChanList* cl,
-	Ep& bestStorage, int water, int rot, int lane)
+__device__ __noinline__ int TryVariantsRot(const Area& ar, const AreaInfo& ai, const Params& P, const SearchState& ss, Ep& bestStorage,
+	int water, int rot, int lane)
 {
+	const ChanList (&cl)[4] = ss.chan[0];
 	const int minA = cl[0].minErr, minG = cl[1].minErr, minR = cl[2].minErr, minB = cl[3].minErr;
 	if (minA + minG + minR + minB >= water)
 		return water;
@@ -1111,10 +1449,10 @@ __device__ NEBC7_SHARED int TryVariantsRot(const Area& ar, const AreaInfo& ai, c
 	const int wAGR[4] = { P.wA, P.wG, P.wR, 0 };
 	const int wAGB[4] = { P.wA, P.wG, 0, P.wB };
 	const int wAGRB[4] = { P.wA, P.wG, P.wR, P.wB };
-	const int2* LA = Ls[0];
-	const int2* LG = Ls[1];
-	const int2* LR = Ls[2];
-	const int2* LB = Ls[3];
+	const int2* LA = ss.lists[0][0];
+	const int2* LG = ss.lists[0][1];
+	const int2* LR = ss.lists[0][2];
+	const int2* LB = ss.lists[0][3];
 	const int colB = lane < nB ? LB[lane].y : 0;
 	const int eBbase = lane < nB ? LB[lane].x : kBig;
 	for (int iA = 0; iA < nA; iA++)
@@ -1196,7 +1534,7 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 	Ep& mcStorage, int water, int rotation, int lane)
 {
 	const Area& ar = st.area1;
-	const AreaInfo& ai = R.a1;
+	const AreaInfo& ai = ar.info;
 	const bool idx32 = MODE == 4 && (rotation & 4);
 	const int a = RotChannel(rotation);
 	int cbits, abits;
@@ -1205,40 +1543,67 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 	{
 		cbits = 5;
 		abits = 6;
-		ctab = kReducedByDiff ? (idx32 ? T.d3v8 : T.d2v8) : (idx32 ? T.d3v5 : T.d2v5);
-		atab = kReducedByDiff ? (idx32 ? T.d2v8 : T.d3v8) : (idx32 ? T.d2v6 : T.d3v6);
+		ctab = idx32 ? T.d3v8 : T.d2v8;
+		atab = idx32 ? T.d2v8 : T.d3v8;
 	}
 	else
 	{
 		cbits = 7;
 		abits = 8;
-		ctab = kReducedByDiff ? T.d2v8 : T.d2v7;
+		ctab = T.d2v8;
 		atab = T.d2v8;
 	}
-	const int wts[4] = { P.wA, P.wG, P.wR, P.wB };
-	ChanList cl[4];
 	int used = 0;
+#pragma unroll 1
 	for (int c = 0; c < 4; c++)
 	{
+		const int w = ChannelWeight(P, c);
+		ChanList cl;
 		if (c == 0 && ai.opaque)
-			cl[0] = ZeroList(ss.lists[0][0], 0xFFFF, lane);
+			cl = ZeroList(ss.lists[0][0], 0xFFFF, lane);
 		else if (c == a)
-			cl[c] = ChannelLevelsSingle<kD>(ss.lists[0][c], ar, ai, c, wts[c], water - used, abits, c != 0, atab, kReducedByDiff || abits == 8,
-				ss.uniq, lane);
+			cl = ChannelLevelsSingle<kD>(ss.lists[0][c], ar, c, w, water - used, abits, c != 0, atab, ss.values, lane);
 		else
-			cl[c] = ChannelLevels<kD, false>(ss.lists[0][c], ar, ai, c, wts[c], water - used, cbits, -1, c != 0, ctab, kReducedByDiff, 32,
-				ss.uniq, lane);
-		used += cl[c].minErr;
+			cl = ChannelLevels<kD, false>(ss.lists[0][c], ar, c, w, water - used, cbits, -1, c != 0, ctab, true, 32, ss.values, lane);
+		if (lane == 0)
+			ss.chan[0][c] = cl;
+		used += cl.minErr;
 		if (used >= water)
 			return water;
 	}
-	const int2* Ls[4] = { ss.lists[0][0], ss.lists[0][1], ss.lists[0][2], ss.lists[0][3] };
+	__syncwarp();
 	const int rot = rotation & 3;
+	/* With every visible pixel's masks full the bounds are lower bounds (the
+	   slot channel's list error is its exact error, and a hidden pixel counts
+	   with its alpha of 0 alone): the three channels that share the colour
+	   index are searched by SearchThree, the slot channel's one candidate a
+	   constant.  Other masks can make a bound exceed the error, and the
+	   reference's order of tests decides: TryVariantsRot. */
+	bool full = true;
+	if (lane < ai.active)
+		full = (ar.mk[lane][0] & ar.mk[lane][1] & ar.mk[lane][2] & ar.mk[lane][3]) == 0xFFFF;
+	if (__all_sync(kFull, full))
+	{
+		const int x = a == 0 ? 1 : 0, y = a <= 1 ? 2 : 1, z = a == 3 ? 2 : 3;
+		auto channel = [&](int c) {
+			return SearchChannel{ c, ChannelWeight(P, c), ss.lists[0][c], ss.chan[0][c].count, ss.chan[0][c].minErr };
+		};
+		const int slot = ss.chan[0][a].minErr;   /* its only candidate's error */
+		const int hidden = a != 0 ? 16 - ai.active : 0;
+		Found3 f;
+		if (idx32)
+			f = SearchThree<kD, 3>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, lane);
+		else
+			f = SearchThree<kD, 2>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, lane);
+		if (f.taken)
+			mcStorage = EpSwapRot(EpSetCh(EpSetCh(Ep2(x, f.x, y, f.y), z, f.z), a, ss.lists[0][a][0].y), rot);
+		return f.water + slot;
+	}
 	if (MODE == 5)
-		return TryVariantsRot<kD, 5, 2, 2>(ar, ai, P, Ls, cl, mcStorage, water, rot, lane);
+		return TryVariantsRot<kD, 5, 2, 2>(ar, ai, P, ss, mcStorage, water, rot, lane);
 	if (idx32)
-		return TryVariantsRot<kD, 4, 3, 2>(ar, ai, P, Ls, cl, mcStorage, water, rot, lane);
-	return TryVariantsRot<kD, 4, 2, 3>(ar, ai, P, Ls, cl, mcStorage, water, rot, lane);
+		return TryVariantsRot<kD, 4, 3, 2>(ar, ai, P, ss, mcStorage, water, rot, lane);
+	return TryVariantsRot<kD, 4, 2, 3>(ar, ai, P, ss, mcStorage, water, rot, lane);
 }
 
 template<int kD>
@@ -1246,6 +1611,7 @@ __device__ NEBC7_PASS void RefineMode4(WarpState& st, SearchState& ss, CellRegs&
 {
 	/* src/Bc7CoreMode4.cpp:1795-1822 */
 	int rotation = R.bestParam;
+#pragma unroll 1
 	for (int i = 0; i < 2; i++, rotation ^= 4)
 	{
 		Ep mc = 0;
@@ -1282,6 +1648,7 @@ __device__ NEBC7_PASS void FullRot(WarpState& st, SearchState& ss, CellRegs& R, 
 	   search may resume at choice `from` */
 	const int step = R.denoiseStep;
 	constexpr int NR = MODE == 4 ? 8 : 4;
+#pragma unroll 1
 	for (int ri = from; ri < NR; ri++)
 	{
 		const int rotation = MODE == 4 ? c_rot4[ri] : c_rot5[ri];

@@ -51,7 +51,10 @@ enum StageStep
 	kStepDraftMode7,       /* fast pass of mode 7 */
 	kStepDraftOpaque31,    /* fast passes of the opaque modes 3 and 1 */
 	kStepDraftOpaque20,    /* fast passes of the opaque modes 2 and 0 */
-	kStepRefine,
+	kStepRefineOpaque,     /* refinement of modes 0-3 */
+	kStepRefineRot,        /* of modes 4 and 5 */
+	kStepRefine6,          /* of modes 6 and 6Index2 */
+	kStepRefine7,          /* of mode 7 */
 	kStepFull3Mode2,
 	kStepFull3Mode0,
 	kStepFull2Mode1,
@@ -188,9 +191,7 @@ __device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const B
 	R.personalParam = r.personalParam;
 	R.personalMode = r.personalMode;
 	R.denoiseStep = r.denoiseStep;
-	R.a1 = AreaStats(st, R, P, 0xFFFF);
-	R.a1.zero = 0;
-	BuildAreaList(st.area1, st, R, 0xFFFF, 0, lane);
+	BuildWholeBlock(st, R, P, lane);
 }
 
 /* One stage: passes of the draft chain after the mode 6 fast pass
@@ -221,20 +222,36 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 		if (R.errTotal > R.opaqueAlphaError + R.denoiseStep)
 			FastOpaque<kD, 0>(st, R, P, lane);
 	}
-	else if constexpr (S == kStepRefine)
+	else if constexpr (S >= kStepRefineOpaque && S <= kStepRefine7)
 	{
-		const int OA = R.opaqueAlphaError;
-		switch (R.bestMode)
+		if (R.errTotal > (S == kStepRefineOpaque ? R.opaqueAlphaError : 0))
 		{
-		case 0: if (R.errTotal > OA) RefineOpaque<kD, 0>(st, ss, R, P, T, lane); break;
-		case 1: if (R.errTotal > OA) RefineOpaque<kD, 1>(st, ss, R, P, T, lane); break;
-		case 2: if (R.errTotal > OA) RefineOpaque<kD, 2>(st, ss, R, P, T, lane); break;
-		case 3: if (R.errTotal > OA) RefineOpaque<kD, 3>(st, ss, R, P, T, lane); break;
-		case 4: if (R.errTotal > 0) RefineMode4<kD>(st, ss, R, P, T, lane); break;
-		case 5: if (R.errTotal > 0) RefineMode5<kD>(st, ss, R, P, T, lane); break;
-		case 6: if (R.errTotal > 0) RefineMode6<kD, 6>(st, ss, R, P, T, lane); break;
-		case 7: if (R.errTotal > 0) RefineMode7<kD>(st, ss, R, P, T, lane); break;
-		case 9: if (R.errTotal > 0) RefineMode6<kD, 9>(st, ss, R, P, T, lane); break;
+			if constexpr (S == kStepRefineOpaque)
+			{
+				switch (R.bestMode)
+				{
+				case 0: RefineOpaque<kD, 0>(st, ss, R, P, T, lane); break;
+				case 1: RefineOpaque<kD, 1>(st, ss, R, P, T, lane); break;
+				case 2: RefineOpaque<kD, 2>(st, ss, R, P, T, lane); break;
+				default: RefineOpaque<kD, 3>(st, ss, R, P, T, lane); break;
+				}
+			}
+			else if constexpr (S == kStepRefineRot)
+			{
+				if (R.bestMode == 4)
+					RefineMode4<kD>(st, ss, R, P, T, lane);
+				else
+					RefineMode5<kD>(st, ss, R, P, T, lane);
+			}
+			else if constexpr (S == kStepRefine6)
+			{
+				if (R.bestMode == 6)
+					RefineMode6<kD, 6>(st, ss, R, P, T, lane);
+				else
+					RefineMode6<kD, 9>(st, ss, R, P, T, lane);
+			}
+			else
+				RefineMode7<kD>(st, ss, R, P, T, lane);
 		}
 		R.personalParam = R.bestParam;
 		R.personalMode = R.bestMode;
@@ -257,6 +274,14 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 		FullMode6<kD>(st, ss, R, P, T, lane);
 }
 
+/* The refinement pass of the block's mode, or the pack. */
+__device__ __forceinline__ int AfterDraft(const CellRegs& R, const Params& P)
+{
+	if (!P.doNormal || P.doDraft == 2)
+		return kStepFinish;
+	return R.bestMode < 4 ? kStepRefineOpaque : (R.bestMode < 6 ? kStepRefineRot : (R.bestMode == 7 ? kStepRefine7 : kStepRefine6));
+}
+
 /* The draft chain's opaque passes run for blocks whose alpha stays above
    239 (src/Bc7Core.cpp:1577), after the transparent chain however far it
    went; then the normal passes, or the pack. */
@@ -264,7 +289,7 @@ __device__ __forceinline__ int AfterTransparentChain(const CellRegs& R, const Pa
 {
 	if (int(int16_t(R.a1.minmax[0])) > 255 - 16 && R.errTotal > R.opaqueAlphaError + R.denoiseStep)
 		return kStepDraftOpaque31;
-	return (P.doNormal && P.doDraft != 2) ? kStepRefine : kStepFinish;
+	return AfterDraft(R, P);
 }
 
 /* The pass after S: the nesting of the draft chain (src/Bc7Core.cpp:
@@ -274,20 +299,22 @@ __device__ __forceinline__ int AfterTransparentChain(const CellRegs& R, const Pa
 __device__ __forceinline__ int NextStep(int S, const CellRegs& R, const Params& P)
 {
 	const int OA = R.opaqueAlphaError, step = R.denoiseStep, e = R.errTotal;
-	const int afterDraft = (P.doNormal && P.doDraft != 2) ? kStepRefine : kStepFinish;
 	switch (S)
 	{
 	case kStepDraftRot: return e > step ? kStepDraftMode7 : AfterTransparentChain(R, P);
 	case kStepDraftMode7: return AfterTransparentChain(R, P);
-	case kStepDraftOpaque31: return e > OA + step ? kStepDraftOpaque20 : afterDraft;
-	case kStepDraftOpaque20: return afterDraft;
+	case kStepDraftOpaque31: return e > OA + step ? kStepDraftOpaque20 : AfterDraft(R, P);
+	case kStepDraftOpaque20: return AfterDraft(R, P);
 	default: break;
 	}
 	if (R.a1.opaque)
 	{
 		switch (S)
 		{
-		case kStepRefine: return e > OA + step ? kStepFull3Mode2 : kStepFinish;
+		case kStepRefineOpaque:
+		case kStepRefineRot:
+		case kStepRefine6:
+		case kStepRefine7: return e > OA + step ? kStepFull3Mode2 : kStepFinish;
 		case kStepFull3Mode2: return e > OA + step ? kStepFull3Mode0 : kStepFinish;
 		case kStepFull3Mode0: return (P.doSlow && e > OA + step) ? kStepFull2Mode1 : kStepFinish;
 		case kStepFull2Mode1: return e > OA + step ? kStepFull2Mode3 : kStepFinish;
@@ -300,7 +327,10 @@ __device__ __forceinline__ int NextStep(int S, const CellRegs& R, const Params& 
 	}
 	switch (S)
 	{
-	case kStepRefine: return e > step ? kStepRot5 : kStepFinish;
+	case kStepRefineOpaque:
+	case kStepRefineRot:
+	case kStepRefine6:
+	case kStepRefine7: return e > step ? kStepRot5 : kStepFinish;
 	case kStepRot5: return e > step ? kStepRot4 : kStepFinish;
 	case kStepRot4: return e > step ? kStepMode7 : kStepFinish;
 	case kStepMode7: return (P.doSlow && e > step) ? kStepMode6 : kStepFinish;
@@ -382,9 +412,7 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 			next = kStepNone;
 		return true;
 	}
-	R.a1 = AreaStats(st, R, P, 0xFFFF);
-	R.a1.zero = 0;
-	BuildAreaList(st.area1, st, R, 0xFFFF, 0, lane);
+	BuildWholeBlock(st, R, P, lane);
 	R.personalMode = -1;
 	R.personalParam = -1;
 	const int water = R.errTotal;
@@ -492,6 +520,28 @@ __device__ __forceinline__ bool StageBlock(WarpState& st, SearchState& ss, const
 	}
 }
 
+/* Shared memory of a warp of stage STAGE: the block state, and the search
+   state as far as the pass uses it (SearchState).  One CTA of the precise
+   mode-2 search took 53 KB with the whole of both, which left 37 KB of L1 for
+   16 warps (18 % hits on the level tables). */
+__host__ __device__ constexpr size_t StageWarpBytes(int stage, bool split)
+{
+	if (stage < kStepRefineOpaque || stage == kStepFinish)
+		return sizeof(WarpState);
+	const bool pca = !split && (stage == kStepFull2Mode1 || stage == kStepFull2Mode3 || stage == kStepMode7);
+	const size_t search = pca ? sizeof(SearchState)
+		: (stage == kStepRefine6 || stage == kStepRefine7 || stage == kStepMode7) ? offsetof(SearchState, table) + sizeof(SearchState::table)
+		: stage == kStepMode6 ? offsetof(SearchState, plane16) + sizeof(SearchState::plane16)
+		: (stage == kStepFull3Mode2 || stage == kStepFull3Mode0) ? offsetof(SearchState, three) + sizeof(SearchState::three)
+		: offsetof(SearchState, three);
+	return kSearchWarpBytes + ((search + 15) & ~size_t(15));
+}
+
+__host__ __device__ constexpr size_t StageSharedBytes(int stage, bool split)
+{
+	return kWarpsPerCta * StageWarpBytes(stage, split);
+}
+
 /* One stage of a staged encode over a list of queue positions (`list`,
    *count entries, taken through *head): the draft kernel takes every
    position (no list); a pass or the finish kernel takes the positions
@@ -503,8 +553,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
-	WarpState& st = reinterpret_cast<WarpState*>(encodeSmem)[warp];
-	SearchState& ss = reinterpret_cast<SearchState*>(encodeSmem + kWarpsPerCta * sizeof(WarpState))[warp];
+	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(STAGE, false));
+	SearchState& ss = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&st) + kSearchWarpBytes);
+	__shared__ LevelTables tables[2];
+	ShareTables(tables, T0, T1);
 	const int n = list ? *count : job.total;
 	for (;;)
 	{
@@ -518,17 +570,17 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 		TexDesc d;
 		BlockRef b;
 		QueuedBlock(job, k, d, b);
-		const Params P = d.P;
+		const Params& P = SharedParams(st, d, lane);
 		bool finished;
 		if constexpr (kD == kAnyDenoise)
 		{
 			if (d.denoise)
-				finished = StageBlock<1, STAGE>(st, ss, b, T1, P, sg, k, lane);
+				finished = StageBlock<1, STAGE>(st, ss, b, tables[1], P, sg, k, lane);
 			else
-				finished = StageBlock<0, STAGE>(st, ss, b, T0, P, sg, k, lane);
+				finished = StageBlock<0, STAGE>(st, ss, b, tables[0], P, sg, k, lane);
 		}
 		else
-			finished = StageBlock<kD, STAGE>(st, ss, b, kD ? T1 : T0, P, sg, k, lane);
+			finished = StageBlock<kD, STAGE>(st, ss, b, tables[kD], P, sg, k, lane);
 		if (finished)
 			BlockFinished(d, lane);
 	}
@@ -590,7 +642,7 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const Block
 			const int OA = R.opaqueAlphaError;
 			if (!(0 < E - step - OA) || !(OA + step < E))
 				return;
-			end = TwoSubsetsPartition<kD, MODE>(st, ss, R, P, GetSpec3<MODE>(T), T, p, 0, 0, lane);
+			end = TwoSubsetsPartition<kD, MODE>(st, ss, R, P, GetSpec3(MODE, T), p, 0, 0, lane);
 		}
 		if (R.errTotal == E)
 			return;
@@ -614,51 +666,31 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const Block
 	atomicMin(sg.firstImp + k, (p << 24) | slot);
 }
 
-/* A round of split pass S over the blocks list[i], i < *count: the first
-   nSplit blocks as tasks (block, candidate p) for p from the block's start
+/* A round of split pass S over the blocks list[i], i < *count (at most
+   kSplitMaxBlocks): tasks (block, candidate p) for p from the block's start
    candidate, taken through *head block by block, so that the candidates of
-   a block go to as many warps; the blocks after them (with more blocks than
-   the task count can number) as one task each, the whole pass in one warp
-   (PassStage). */
+   a block go to as many warps. */
 template<int kD, int S>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, Stages sg, const int* list, const int* count, int* head,
-	int* impCount, int nSplit, LevelTables T0, LevelTables T1)
+	int* impCount, LevelTables T0, LevelTables T1)
 {
 	constexpr int NT = SplitTasks(S);
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
-	WarpState& st = reinterpret_cast<WarpState*>(encodeSmem)[warp];
-	SearchState& ss = reinterpret_cast<SearchState*>(encodeSmem + kWarpsPerCta * sizeof(WarpState))[warp];
-	const int n = *count;
-	const int heavy = n < nSplit ? n : nSplit;
+	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(S, true));
+	SearchState& ss = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&st) + kSearchWarpBytes);
+	__shared__ LevelTables tables[2];
+	ShareTables(tables, T0, T1);
+	const int n = min(*count, kSplitMaxBlocks);
 	for (;;)
 	{
 		int t = 0;
 		if (lane == 0)
 			t = atomicAdd(head, 1);
 		t = __shfl_sync(kFull, t, 0);
-		if (t >= heavy * NT)
-		{
-			const int i = heavy + (t - heavy * NT);
-			if (i >= n)
-				break;
-			const int k = list[i];
-			TexDesc d;
-			BlockRef b;
-			QueuedBlock(job, k, d, b);
-			const Params P = d.P;
-			if constexpr (kD == kAnyDenoise)
-			{
-				if (d.denoise)
-					PassStage<1, S>(st, ss, b, T1, P, sg.rec[k], sg.next[k], sg.start[k], lane);
-				else
-					PassStage<0, S>(st, ss, b, T0, P, sg.rec[k], sg.next[k], sg.start[k], lane);
-			}
-			else
-				PassStage<kD, S>(st, ss, b, kD ? T1 : T0, P, sg.rec[k], sg.next[k], sg.start[k], lane);
-			continue;
-		}
+		if (t >= n * NT)
+			break;
 		const int i = t / NT, p = t % NT;
 		const int k = list[i];
 		if (p < sg.start[k])
@@ -666,7 +698,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		TexDesc d;
 		BlockRef b;
 		QueuedBlock(job, k, d, b);
-		const Params P = d.P;
+		const Params& P = SharedParams(st, d, lane);
 		if (P.pca && SplitMode(S) != 4 && SplitMode(S) != 5)
 		{
 			/* OPTION_PCA orders the partitions by their bounds first: the
@@ -679,18 +711,19 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		if constexpr (kD == kAnyDenoise)
 		{
 			if (d.denoise)
-				SplitTask<1, S>(st, ss, b, T1, P, sg, impCount, k, p, lane);
+				SplitTask<1, S>(st, ss, b, tables[1], P, sg, impCount, k, p, lane);
 			else
-				SplitTask<0, S>(st, ss, b, T0, P, sg, impCount, k, p, lane);
+				SplitTask<0, S>(st, ss, b, tables[0], P, sg, impCount, k, p, lane);
 		}
 		else
-			SplitTask<kD, S>(st, ss, b, kD ? T1 : T0, P, sg, impCount, k, p, lane);
+			SplitTask<kD, S>(st, ss, b, tables[kD], P, sg, impCount, k, p, lane);
 	}
 }
 
 /* Before the first round of a split pass: every block starts at candidate 0
-   with no improvement. */
-static __global__ void __launch_bounds__(256) KSplitPrepare(Stages sg, const int* list, const int* count)
+   with no improvement; blocks past kSplitMaxBlocks (more than the task count
+   can number) go to the one-warp remainder at once. */
+static __global__ void __launch_bounds__(256) KSplitPrepare(Stages sg, const int* list, const int* count, int* restList, int* restCount)
 {
 	const int n = *count;
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -698,6 +731,8 @@ static __global__ void __launch_bounds__(256) KSplitPrepare(Stages sg, const int
 		const int k = list[i];
 		sg.start[k] = 0;
 		sg.firstImp[k] = kSplitNone;
+		if (i >= kSplitMaxBlocks)
+			restList[atomicAdd(restCount, 1)] = k;
 	}
 }
 
@@ -707,12 +742,11 @@ static __global__ void __launch_bounds__(256) KSplitPrepare(Stages sg, const int
    round, in the one-warp remainder's list); a block without an improvement
    has finished the pass and gets its next one (NextStep). */
 template<int S>
-__global__ void __launch_bounds__(256) KSplitCommit(Job job, Stages sg, const int* list, const int* count, int nSplit, int* nextList,
+__global__ void __launch_bounds__(256) KSplitCommit(Job job, Stages sg, const int* list, const int* count, int* nextList,
 	int* nextCount, int* restList, int* restCount, int lastRound)
 {
 	constexpr int MODE = SplitMode(S);
-	/* the blocks after the first nSplit ran their whole pass in one task */
-	const int n = *count < nSplit ? *count : nSplit;
+	const int n = min(*count, kSplitMaxBlocks);
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		const int k = list[i];

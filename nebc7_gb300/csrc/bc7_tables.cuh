@@ -102,6 +102,20 @@ __global__ void KBuildHalfDiff(uint8_t* out, int levels, int denoise)
 	out[t] = uint8_t(res[0] | (res[1] << 4));
 }
 
+/* The squares of a half table's entries (at most 15^2, a byte each), laid
+   out like the byte tables: the candidate lists of modes 6 and 6Index2 read
+   them with one address addition and one load where a nibble takes four
+   instructions more and its square another. */
+__global__ void KBuildHalfSquares(const uint8_t* half, uint8_t* out)
+{
+	const int t = blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= 511 * 512)
+		return;
+	const int a = t >> 9, b = t & 511;
+	const int v = (half[a * 256 + (b >> 1)] >> ((b & 1) << 2)) & 0xF;
+	out[t] = uint8_t(v * v);
+}
+
 /* Byte table by differences (DiffAt): byte (a << 9) + b holds the entry of
    a = cH - x + 255, b = cL - x + 255, quantised like KBuildFull; column 511
    is padding. */

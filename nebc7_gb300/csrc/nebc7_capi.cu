@@ -37,7 +37,7 @@ struct DeviceTables
 {
 	bool built = false;
 	LevelTables t{};
-	void* mem[15] = {};
+	void* mem[17] = {};   /* the level tables of nebc7_table_read, then the two tables of squares */
 };
 
 std::mutex gMutex;
@@ -93,9 +93,9 @@ int BuildTables(int dev, int denoise, const LevelTables** out)
 			cudaFree(d3v8);
 			cudaFree(d2v8);
 		};
-		for (int i = 0; i < kNumLevelTables; i++)
+		for (int i = 0; i < kNumLevelTables + 2; i++)
 		{
-			if (cudaMalloc(&D.mem[i], sizes[i]) != cudaSuccess)
+			if (cudaMalloc(&D.mem[i], i < kNumLevelTables ? sizes[i] : size_t(511) * 512) != cudaSuccess)
 			{
 				release();
 				return SetError(NEBC7_ENOMEM);
@@ -129,6 +129,8 @@ int BuildTables(int dev, int denoise, const LevelTables** out)
 		KBuildHalfDiff<<<grid(511 * 256), tb>>>((uint8_t*)D.mem[13], 4, denoise);
 		KBuildByteDiff<<<grid(511 * 512), tb>>>((uint8_t*)D.mem[0], 4, denoise);
 		KBuildByteDiff<<<grid(511 * 512), tb>>>((uint8_t*)D.mem[14], 8, denoise);
+		KBuildHalfSquares<<<grid(511 * 512), tb>>>((const uint8_t*)D.mem[12], (uint8_t*)D.mem[15]);
+		KBuildHalfSquares<<<grid(511 * 512), tb>>>((const uint8_t*)D.mem[13], (uint8_t*)D.mem[16]);
 		const cudaError_t e = cudaDeviceSynchronize();
 		cudaFree(d3v8);
 		cudaFree(d2v8);
@@ -154,6 +156,8 @@ int BuildTables(int dev, int denoise, const LevelTables** out)
 		t.d4h = (const uint8_t*)D.mem[12];
 		t.d2h = (const uint8_t*)D.mem[13];
 		t.d3v8 = (const uint8_t*)D.mem[14];
+		t.h4s = (const uint8_t*)D.mem[15];
+		t.h2s = (const uint8_t*)D.mem[16];
 		D.built = true;
 	}
 	*out = &D.t;
