@@ -430,7 +430,7 @@ def run_ours(args, rank, world, local):
     value = px * world / (step_ms / 1e3) / 1e6
     # kernels of this library per encode call: the refining variants order the
     # blocks first (bucket and scatter kernels), then KEncode or its staged form
-    launches_per_encode = lib.nebc7_encode_launches(ctypes.byref(st))
+    launches_per_encode = lib.nebc7_encode_kernels(ctypes.byref(st))
 
     # end to end through the C ABI host entry (pinned host buffers, copies inside)
     h_img = torch.from_numpy(padded).pin_memory()

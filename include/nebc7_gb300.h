@@ -155,13 +155,16 @@ int nebc7_decode_blocks_host(const uint8_t* blocks, uint8_t* bgra, int n);
    build of the reference (they are tested against the CPU restatement). */
 int nebc7_set_pca(int on);
 
-/* How many kernels one nebc7_encode_device call with these settings
-   launches (the block order, then the encode: one persistent kernel, or
-   for the presets whose time goes to the full searches the staged form of
-   a kernel per pass and a list kernel before each, the split passes with a
-   task and a commit kernel per round), not counting the sums' reduction;
-   a negative error code for invalid settings. */
+/* The steps of an encode with these settings as its pass structure counts
+   them (the block order's two, then one, or for the full-search presets a
+   list and a step per pass and two per round of a split pass): a fixed
+   number per preset.  The kernels that run them, which is what is launched,
+   are nebc7_encode_kernels'.  A negative error code for invalid settings. */
 int nebc7_encode_launches(const nebc7_settings* settings);
+
+/* How many kernels an encode with these settings launches, not counting the
+   sums' reduction; a negative error code for invalid settings. */
+int nebc7_encode_kernels(const nebc7_settings* settings);
 
 /* Builds the level tables of `denoise` on the current device ahead of use. */
 int nebc7_init_device(int denoise);
