@@ -247,6 +247,54 @@ __device__ __forceinline__ ChanList ZeroList(int2* nodes, int color, int lane)
 	return ChanList{ 0, 1 };
 }
 
+/* The warps that search a block together: the CTA's four, or one alone
+   (size 1).  They exchange candidate lists through shared memory. */
+struct TeamExchange
+{
+	unsigned list[2][4][32];   /* two buffers, taken in turn: one barrier a scan */
+};
+
+struct Team
+{
+	int size, rank;
+	TeamExchange* exchange;
+	int turn;                  /* buffer of the next scan */
+
+	__device__ __forceinline__ void Sync() const
+	{
+		if (size > 1)
+			__syncthreads();
+		else
+			__syncwarp();
+	}
+};
+
+__device__ __forceinline__ Team SingleWarp() { return Team{ 1, 0, nullptr, 0 }; }
+
+/* The N smallest keys of the team's lists (each sorted over the lanes), in
+   every warp. */
+__device__ __forceinline__ unsigned TeamMerge(unsigned list, Team& team, int lane, int N)
+{
+	TeamExchange& x = *team.exchange;
+	x.list[team.turn][team.rank][lane] = list;
+	__syncthreads();
+#pragma unroll 1
+	for (int w = 1; w < 4; w++)
+	{
+		/* the smaller half of two sorted lists is bitonic */
+		unsigned m = min(list, x.list[team.turn][(team.rank + w) & 3][31 - lane]);
+#pragma unroll
+		for (int j = 16; j > 0; j >>= 1)
+		{
+			const unsigned o = __shfl_xor_sync(kFull, m, j);
+			m = ((lane & j) == 0) ? min(m, o) : max(m, o);
+		}
+		list = m;
+	}
+	team.turn ^= 1;
+	return lane < N ? list : 0xFFFFFFFFu;
+}
+
 /* Place of candidate cc in a table: by differences (DiffBase), or the
    per-x layout of mode 1's shared-p-bit table. */
 __device__ __forceinline__ int CandidateBase(int cc, int shift, bool byDiff)
@@ -270,7 +318,7 @@ __device__ __forceinline__ int ValueStride(int shift, bool byDiff)
  * the four values that reject most unless a lane can still enter the list. */
 template<int kD, bool HALF>
 __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
-	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, int lane)
+	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, Team& team, int lane)
 {
 	ChanList res{ MaxColorError<kD>() * 2, 0 };
 	const AreaInfo& ai = ar.info;
@@ -311,7 +359,9 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	   reference's shift count (modulo 32) does */
 	const int span = win.LH >= 0 ? (win.LH | 7) : ((win.LH | 7) & (pvar ? 31 : 15));
 	const int rowLen = pvar ? (span >> 1) + 1 : span + 1;
-	const int stepRows = 32 / rowLen, stepCols = 32 - stepRows * rowLen;
+	/* a team's warps take every fourth batch */
+	const int stride = 32 * team.size, start = 32 * team.rank + lane;
+	const int stepRows = stride / rowLen, stepCols = stride - stepRows * rowLen;
 
 	const int n = DistinctValues(ar, count, offset, L, H, ValueStride(shift, byDiff), values, lane);
 	ValueGroup first;
@@ -321,7 +371,7 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	   key (all ones until the list is full), which changes only on a merge */
 	unsigned list = 0xFFFFFFFFu;
 	unsigned thr = 0xFFFFFFFFu;
-	int row = lane / rowLen, col = lane - row * rowLen;
+	int row = start / rowLen, col = start - row * rowLen;
 	int iH = win.HL + (pvar ? pH : 0);   /* the batch's first row */
 	while (iH < win.HH)
 	{
@@ -344,7 +394,7 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 					break;
 			}
 		}
-		/* the next 32 candidates; row stays relative to the batch's first */
+		/* the next candidates; row stays relative to the batch's first */
 		row += stepRows;
 		col += stepCols;
 		if (col >= rowLen)
@@ -356,6 +406,8 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 		iH += ahead * step;
 		row -= ahead;
 	}
+	if (team.size > 1)
+		list = TeamMerge(list, team, lane, maxSize);
 	const int stored = __popc(__ballot_sync(kFull, list != 0xFFFFFFFFu));
 	if (stored)
 	{
@@ -372,9 +424,9 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 /* Out-of-line copy of the scan for its many call sites. */
 template<int kD, bool HALF>
 __device__ NEBC7_SHARED ChanList ChannelLevels(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
-	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, int lane)
+	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, Team& team, int lane)
 {
-	return ChannelLevelsScan<kD, HALF>(nodes, ar, offset, weight, water, bits, pbits, transparent, table, byDiff, maxSize, values, lane);
+	return ChannelLevelsScan<kD, HALF>(nodes, ar, offset, weight, water, bits, pbits, transparent, table, byDiff, maxSize, values, team, lane);
 }
 
 /* Single best candidate over the narrower window of the alpha slot of modes

@@ -55,6 +55,7 @@ struct __align__(16) SearchState
 			int2 order[64];      /* (estimate, partition) */
 			int lines[64][2];    /* per partition, estimates of subsets 2 and 3 */
 			int est[64][3][3];   /* per partition, subset, channel (G, R, B) estimates */
+			int count;
 		} three;                 /* the three-subset searches */
 		int4 table[16 * kTableRow];   /* four channels, 2-bit indices: R's terms, [pixel][candidate] */
 		int plane16[3][256];          /* four channels, 4-bit indices: planes of 16 levels */
@@ -562,13 +563,14 @@ template<int kD>
 __device__ NEBC7_PASS bool InitLevels3(SearchState& ss, int v, const Area& ar, const Params& P, const Spec3& sp, bool pbit, int water,
 	int estR, int estB, int lane)
 {
+	Team one = SingleWarp();
 	int used = 0;
 #pragma unroll 1
 	for (int c = 1; c < 4; c++)
 	{
 		const int rest = c == 1 ? estR + estB : (c == 2 ? estB : 0);
 		const ChanList cl = ChannelLevels<kD, false>(ss.lists[v][c - 1], ar, c, ChannelWeight(P, c), water - used - rest, sp.bits,
-			pbit ? VariantPbits(v) : -1, false, sp.table, sp.byDiff, 32, ss.values, lane);
+			pbit ? VariantPbits(v) : -1, false, sp.table, sp.byDiff, 32, ss.values, one, lane);
 		if (lane == 0)
 			ss.chan[v][c - 1] = cl;
 		used += cl.minErr;
@@ -688,7 +690,8 @@ __device__ NEBC7_PASS int EstimateLevels3(SearchState& ss, const Area& ar, const
 
 __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 {
-	/* stable sort by unsigned error (src/Bc7Core.cpp:564 radix_sort_partitions):
+	/* stable sort by unsigned error (src/Bc7Core.cpp:564 radix_sort_partitions)
+	   of entries that the reference lists in ascending partition order:
 	   rank = number of entries that must precede */
 	int2 mine[2];
 	int rank[2];
@@ -704,8 +707,8 @@ __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 			int r = 0;
 			for (int k = 0; k < n; k++)
 			{
-				const unsigned ek = unsigned(order[k].x), ei = unsigned(mine[h].x);
-				r += (ek < ei) || (ek == ei && k < i);
+				const int2 o = order[k];
+				r += (unsigned(o.x) < unsigned(mine[h].x)) || (o.x == mine[h].x && o.y < mine[h].y);
 			}
 			rank[h] = r;
 		}
@@ -719,11 +722,11 @@ __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 }
 
 /* The estimates of partition p of a full search of modes 0 and 2 (the first
-   loop of src/Bc7CoreMode0.cpp:532-642): its subsets' estimates to ss.three,
+   loop of src/Bc7CoreMode0.cpp:532-642): its subsets' estimates to out.three,
    and whether they leave room below the error. */
 template<int kD, int MODE>
-__device__ __forceinline__ bool ThreeSubsetsEstimate(WarpState& st, SearchState& ss, const CellRegs& R, const Params& P, const Spec3& sp,
-	int p, int& total, int lane)
+__device__ __forceinline__ bool ThreeSubsetsEstimate(WarpState& st, SearchState& ss, SearchState& out, const CellRegs& R, const Params& P,
+	const Spec3& sp, int p, int& total, int lane)
 {
 	int water = R.errTotal - R.denoiseStep - R.opaqueAlphaError;
 	total = R.opaqueAlphaError + R.denoiseStep;
@@ -731,11 +734,11 @@ __device__ __forceinline__ bool ThreeSubsetsEstimate(WarpState& st, SearchState&
 	for (int s = 0; s < 3; s++)
 	{
 		BuildSubset<kD>(st, R, P, st.sub[0], 3, p, s, false, lane);
-		const int line = EstimateLevels3<kD>(ss, st.sub[0], P, sp, water, ss.three.est[p][s], lane);
+		const int line = EstimateLevels3<kD>(ss, st.sub[0], P, sp, water, out.three.est[p][s], lane);
 		if (!(line < water))
 			return false;
 		if (lane == 0 && s)
-			ss.three.lines[p][s - 1] = line;
+			out.three.lines[p][s - 1] = line;
 		water -= line;
 		total += line;
 	}
@@ -779,27 +782,41 @@ __device__ __forceinline__ bool ThreeSubsetsPartition(WarpState& st, SearchState
 }
 
 /* Full searches of modes 0 and 2 (src/Bc7CoreMode0.cpp:532-642,
-   src/Bc7CoreMode2.cpp:456-566). */
+   src/Bc7CoreMode2.cpp:456-566).  With size > 1 the CTA's warps take every
+   size-th partition's estimates (all from the block's error, whatever the
+   order) into the first warp's state, `stateStride` bytes before each next,
+   and the first warp searches. */
 template<int kD, int MODE>
-__device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane,
+	int size = 1, int rank = 0, size_t stateStride = 0)
 {
 	constexpr int NP = MODE == 0 ? 16 : 64;
 	const Spec3 sp = GetSpec3(MODE, T);
-	int count = 0;
+	SearchState& s0 = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&ss) - rank * stateStride);
+	if (rank == 0 && lane == 0)
+		s0.three.count = 0;
+	if (size > 1)
+		__syncthreads();
+	else
+		__syncwarp();
 #pragma unroll 1
-	for (int p = 0; p < NP; p++)
+	for (int p = rank; p < NP; p += size)
 	{
 		if (R.personalMode == MODE && R.personalParam == p)
 			continue;
 		int total;
-		if (ThreeSubsetsEstimate<kD, MODE>(st, ss, R, P, sp, p, total, lane))
-		{
-			if (lane == 0)
-				ss.three.order[count] = make_int2(total, p);
-			count++;
-		}
+		if (ThreeSubsetsEstimate<kD, MODE>(st, ss, s0, R, P, sp, p, total, lane) && lane == 0)
+			s0.three.order[atomicAdd(&s0.three.count, 1)] = make_int2(total, p);
 	}
-	__syncwarp();
+	if (size > 1)
+	{
+		__syncthreads();
+		if (rank)
+			return;
+	}
+	else
+		__syncwarp();
+	const int count = ss.three.count;
 	StableSortOrder(ss.three.order, count, lane);
 #pragma unroll 1
 	for (int i = 0; i < count; i++)
@@ -946,8 +963,23 @@ __device__ __forceinline__ int TableError(const int4* plane, const int4* table, 
 	return sum;
 }
 
+/* What the warps of a team share of one four-channel search: the smallest
+   error found so far with its place in the search's order (error << 32 |
+   variant, four list indices), and the next unit of each variant. */
+struct TeamSearch
+{
+	unsigned long long key;
+	int next[4];
+};
+
+/* Place of a combination in the search's order. */
+__device__ __forceinline__ unsigned SearchPlace(int v, int i0, int i1, int i2, int i3)
+{
+	return unsigned(((((v << 5 | i0) << 5 | i1) << 5 | i2) << 5) | i3);
+}
+
 /* The four-channel combination search with 2-bit indices (modes 7 and
-   6Index2; src/Bc7CoreMode6.cpp:1163-1331).
+   6Index2; src/Bc7CoreMode6.cpp:1163-1331) over the lists of variant v.
  *
  * Every bound that the reference compares here is a lower bound of the error
  * it stands for: a channel's list error takes each pixel's nearest level on
@@ -957,7 +989,11 @@ __device__ __forceinline__ int TableError(const int4* plane, const int4* table, 
  * order, of the smallest error below the water, and any lower bound may
  * skip: besides the reference's, the sums below take the entry's own list
  * error where the reference takes the list's minimum, and a level's errors
- * are computed only when some combination under it is still open.
+ * are computed only when some combination under it is still open.  For the
+ * same reason the warps of a team may take the alpha candidates (an opaque
+ * area's single one: every fourth G candidate) in any order: the smallest
+ * (error, place) wins, and a warp keeps a combination of the team's error
+ * that lies before the team's.
  *
  * What bounds it: instruction issue in the error sums.  A candidate's terms
  * w q^2 per pixel and level do not depend on the outer loops, so B's are kept
@@ -965,17 +1001,17 @@ __device__ __forceinline__ int TableError(const int4* plane, const int4* table, 
  * table, and a pixel costs one broadcast read of the plane and four fused
  * add-minimum steps instead of four differences, squares and products. */
 template<int kD>
-__device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
-	const uint8_t* alphaTable, Ep best, int water, int lane)
+__device__ __forceinline__ Found SearchFour2(SearchState& ss, const ChanList (&chan)[4], const int2 (*lists)[32], int v, const Area& ar, int count,
+	int np, bool opq, Weights w, const uint8_t* alphaTable, Ep best, int water, TeamSearch* team, int lane)
 {
-	const int4 m01 = *reinterpret_cast<const int4*>(&ss.chan[v][0]), m23 = *reinterpret_cast<const int4*>(&ss.chan[v][2]);
+	const int4 m01 = *reinterpret_cast<const int4*>(&chan[0]), m23 = *reinterpret_cast<const int4*>(&chan[2]);
 	const int min0 = m01.x, n0 = m01.y, min1 = m01.z, n1 = m01.w;
 	const int min2 = m23.x, n2 = m23.y, min3 = m23.z, n3 = m23.w;
 	if (min0 + min1 + min2 + min3 >= water)
 		return Found{ water, best };
-	const int2 l1 = lane < n1 ? ss.lists[v][1][lane] : make_int2(kFar, 0);
-	const int2 l2 = lane < n2 ? ss.lists[v][2][lane] : make_int2(kFar, 0);
-	const int2 l3 = lane < n3 ? ss.lists[v][3][lane] : make_int2(kFar, 0);
+	const int2 l1 = lane < n1 ? lists[1][lane] : make_int2(kFar, 0);
+	const int2 l2 = lane < n2 ? lists[2][lane] : make_int2(kFar, 0);
+	const int2 l3 = lane < n3 ? lists[3][lane] : make_int2(kFar, 0);
 	int4* const pA = ss.plane;
 	int4* const pAG = (ss.plane + 16);
 	int4* const pAGR = (ss.plane + 32);
@@ -992,10 +1028,34 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area&
 	pl.Pixels(ar, 0, xa);
 	pl.Pixels(ar, 1, xg);
 	const int zero[2] = { 0, 0 };
+	/* a team's units: the alpha candidates, or the four stripes of an opaque
+	   area's G candidates */
+	const int stripes = team && opq ? 4 : 1;
 
-	for (int i0 = 0; i0 < n0; i0++)
+	/* the error that a combination at (i0, i1) has to be below: one above the
+	   team's where the team's combination lies behind it */
+	auto refresh = [&](int i0, int i1) {
+		if (team)
+		{
+			const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&team->key);
+			water = int(k >> 32) + int(unsigned(k) > SearchPlace(v, i0, i1, 31, 31));
+		}
+	};
+
+	for (int unit = 0;; unit++)
 	{
-		const int2 a = ss.lists[v][0][i0];
+		if (team)
+		{
+			int u = 0;
+			if (lane == 0)
+				u = atomicAdd(&team->next[v], 1);
+			unit = __shfl_sync(kFull, u, 0);
+		}
+		if (unit >= n0 * stripes)
+			break;
+		const int i0 = team && opq ? 0 : unit;
+		refresh(i0, 0);
+		const int2 a = lists[0][i0];
 		const int e0 = a.x;
 		if (e0 + min1 + min2 + min3 >= water)
 			break;
@@ -1025,14 +1085,17 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area&
 			}
 			errAG = lane < n1 ? sum + ea : kFar;
 		}
+		const bool mine = stripes == 1 || (lane & 3) == unit;
 		int i1 = 0;
 		for (;;)
 		{
 			/* the next G candidate still open */
-			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
+			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && mine && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
 			if (!open1)
 				break;
 			i1 = __ffs(open1) - 1;
+			refresh(i0, i1);
+			const int place1 = i1;
 			const int eAG = __shfl_sync(kFull, errAG, i1);
 			const int2 g = make_int2(__shfl_sync(kFull, l1.x, i1), __shfl_sync(kFull, l1.y, i1));
 			i1++;
@@ -1070,7 +1133,10 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area&
 				{
 					const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
 					water = low;
-					best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+					if (!team)
+						best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+					else if (lane == 0)
+						atomicMin(&team->key, (unsigned long long)(unsigned(low)) << 32 | SearchPlace(v, i0, place1, i2, j));
 				}
 			}
 		}
@@ -1082,7 +1148,7 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, int v, const Area&
    fit registers or a table, so a candidate's terms are computed per plane. */
 template<int kD>
 __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
-	const uint8_t* alphaTable, Ep best, int water, int lane)
+	const uint8_t* alphaTable, Ep best, int water, TeamSearch* team, int lane)
 {
 	const int4 m01 = *reinterpret_cast<const int4*>(&ss.chan[v][0]), m23 = *reinterpret_cast<const int4*>(&ss.chan[v][2]);
 	const int min0 = m01.x, n0 = m01.y, min1 = m01.z, n1 = m01.w;
@@ -1095,8 +1161,27 @@ __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area&
 	int* const pA = ss.plane16[0];
 	int* const pAG = ss.plane16[1];
 	int* const pAGR = ss.plane16[2];
-	for (int i0 = 0; i0 < n0; i0++)
+	const int stripes = team && opq ? 4 : 1;
+	auto refresh = [&](int i0, int i1) {
+		if (team)
+		{
+			const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&team->key);
+			water = int(k >> 32) + int(unsigned(k) > SearchPlace(0, i0, i1, 31, 31));
+		}
+	};
+	for (int unit = 0;; unit++)
 	{
+		if (team)
+		{
+			int u = 0;
+			if (lane == 0)
+				u = atomicAdd(&team->next[0], 1);
+			unit = __shfl_sync(kFull, u, 0);
+		}
+		if (unit >= n0 * stripes)
+			break;
+		const int i0 = team && opq ? 0 : unit;
+		refresh(i0, 0);
 		const int2 a = ss.lists[v][0][i0];
 		const int e0 = a.x;
 		if (e0 + min1 + min2 + min3 >= water)
@@ -1116,13 +1201,16 @@ __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area&
 			if (lane < n1)
 				errAG = PlaneError<kD, 4>(pA, ar, np, 1, l1.y, w.g, water - ea - min2 - min3) + ea;
 		}
+		const bool mine = stripes == 1 || (lane & 3) == unit;
 		int i1 = 0;
 		for (;;)
 		{
-			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
+			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && mine && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
 			if (!open1)
 				break;
 			i1 = __ffs(open1) - 1;
+			refresh(i0, i1);
+			const int place1 = i1;
 			const int eAG = __shfl_sync(kFull, errAG, i1);
 			const int2 g = make_int2(__shfl_sync(kFull, l1.x, i1), __shfl_sync(kFull, l1.y, i1));
 			i1++;
@@ -1156,7 +1244,10 @@ __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area&
 				{
 					const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
 					water = low;
-					best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+					if (!team)
+						best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+					else if (lane == 0)
+						atomicMin(&team->key, (unsigned long long)(unsigned(low)) << 32 | SearchPlace(0, i0, place1, i2, j));
 				}
 			}
 		}
@@ -1167,21 +1258,54 @@ __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area&
 /* Out-of-line copy for modes 6 and 7; the Mode6Index2 refinement (the
    common case of the default preset) inlines the body. */
 template<int kD, int IB>
-__device__ NEBC7_SHARED Found SearchFour(SearchState& ss, int v, const Area& ar, int count, int np, bool opq, Weights w,
-	const uint8_t* alphaTable, Ep best, int water, int lane)
+__device__ NEBC7_SHARED Found SearchFour(SearchState& ss, const SearchState& from, int slot, int v, const Area& ar, Weights w, const uint8_t* alphaTable,
+	Ep best, int water, TeamSearch* team, int lane)
 {
+	const AreaInfo& ai = ar.info;
 	if constexpr (IB == 4)
-		return SearchFour4<kD>(ss, v, ar, count, np, opq, w, alphaTable, best, water, lane);
+		return SearchFour4<kD>(ss, slot, ar, ai.count, ai.active, ai.opaque, w, alphaTable, best, water, team, lane);
 	else
-		return SearchFour2<kD>(ss, v, ar, count, np, opq, w, alphaTable, best, water, lane);
+		return SearchFour2<kD>(ss, from.chan[slot], from.lists[slot], v, ar, ai.count, ai.active, ai.opaque, w, alphaTable, best, water, team,
+			lane);
+}
+
+/* What a team shares of a block's search. */
+struct TeamState
+{
+	TeamSearch search;
+	TeamExchange exchange;
+	int bound[2][4];       /* [subset][channel] estimates */
+	int valid;             /* variants whose lists leave room */
+	int task[3];           /* the CTA's task: queue position, candidate, first improvement */
+};
+
+/* Starts a team's search from `water`; the last one's outcome is read. */
+__device__ __forceinline__ void StartTeamSearch(TeamState& ts, int water)
+{
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		ts.search.key = (unsigned long long)(unsigned(water)) << 32;
+		ts.search.next[0] = ts.search.next[1] = ts.search.next[2] = ts.search.next[3] = 0;
+		ts.valid = 0;
+	}
+	__syncthreads();
+}
+
+/* The endpoints of a team's outcome in the lists it was found in. */
+__device__ __forceinline__ Ep PlaceEndpoints(const int2 (*lists)[32], unsigned place)
+{
+	return EpSetCh(EpSetCh(Ep2(0, lists[0][(place >> 15) & 31].y, 1, lists[1][(place >> 10) & 31].y), 2, lists[2][(place >> 5) & 31].y), 3,
+		lists[3][place & 31].y);
 }
 
 /* Subset::InitLevels of modes 6 / 6Index2 (9) / 7 (src/Bc7CoreMode6.cpp:
    1130-1161, src/Bc7CoreMode7.cpp:237-268) for the p-bits of variant pv into
-   the lists of slot v; est: lower bounds of the channels' errors, or null. */
+   the lists of slot v; est: lower bounds of the channels' errors, or null.
+   Every warp of a team gets the whole lists. */
 template<int kD, int MODE>
 __device__ NEBC7_PASS bool InitLevels4(SearchState& ss, int v, int pv, const Area& ar, const Params& P, const LevelTables& T, int water,
-	const int* est, int lane)
+	const int* est, Team& team, int lane)
 {
 	int used = 0;
 	int rest = est ? est[1] + est[2] + est[3] : 0;
@@ -1193,7 +1317,7 @@ __device__ NEBC7_PASS bool InitLevels4(SearchState& ss, int v, int pv, const Are
 			cl = ZeroList(ss.lists[v][0], 0xFFFF, lane);
 		else
 			cl = ChannelLevels<kD, MODE != 7>(ss.lists[v][c], ar, c, ChannelWeight(P, c), water - used - rest, MODE == 7 ? 5 : 7,
-				VariantPbits(pv), c != 0, MODE == 6 ? T.h4s : (MODE == 9 ? T.h2s : T.d2v8), true, 20, ss.values, lane);
+				VariantPbits(pv), c != 0, MODE == 6 ? T.h4s : (MODE == 9 ? T.h2s : T.d2v8), true, 20, ss.values, team, lane);
 		if (lane == 0)
 			ss.chan[v][c] = cl;
 		used += cl.minErr;
@@ -1206,55 +1330,111 @@ __device__ NEBC7_PASS bool InitLevels4(SearchState& ss, int v, int pv, const Are
 	return true;
 }
 
-template<int kD, int MODE>
-__device__ __forceinline__ int TryV4(SearchState& ss, int v, const Area& ar, const Params& P, const LevelTables& T, Ep& best, int water,
-	int lane)
-{
-	const AreaInfo& ai = ar.info;
-	const Found f = SearchFour<kD, MODE == 6 ? 4 : 2>(ss, v, ar, ai.count, ai.active, ai.opaque, WeightsOf(P), MODE == 6 ? T.d4h : T.d2v8, best,
-		water, lane);
-	best = f.best;
-	return f.water;
-}
-
 /* Mode 6 / 6Index2 CompressSubset (src/Bc7CoreMode6.cpp:1334-1364): each
    later p-bit variant starts from the water left by the earlier ones. */
 template<int kD, int MODE>
 __device__ NEBC7_PASS int CompressSubsetSingle(SearchState& ss, const Area& ar, const Params& P, const LevelTables& T, Ep& mc, int water,
-	int lane)
+	Team& team, TeamState* ts, int lane)
 {
 #pragma unroll 1
 	for (int v = 0; v < (ar.info.opaque ? 1 : 4); v++)
-		if (InitLevels4<kD, MODE>(ss, 0, v, ar, P, T, water, nullptr, lane))
-			water = TryV4<kD, MODE>(ss, 0, ar, P, T, mc, water, lane);
+	{
+		if (!InitLevels4<kD, MODE>(ss, 0, v, ar, P, T, water, nullptr, team, lane))
+			continue;
+		if (team.size > 1)
+			StartTeamSearch(*ts, water);
+		const Found f = SearchFour<kD, MODE == 6 ? 4 : 2>(ss, ss, 0, 0, ar, WeightsOf(P), MODE == 6 ? T.d4h : T.d2v8, mc,
+			team.size > 1 ? water + 1 : water, team.size > 1 ? &ts->search : nullptr, lane);
+		if (team.size > 1)
+		{
+			__syncthreads();
+			const unsigned long long k = ts->search.key;
+			if (int(k >> 32) < water)
+			{
+				water = int(k >> 32);
+				mc = PlaceEndpoints(ss.lists[0], unsigned(k));
+			}
+		}
+		else
+		{
+			water = f.water;
+			mc = f.best;
+		}
+	}
 	return water;
 }
 
 /* Mode 7 Subsets (src/Bc7CoreMode7.cpp:441-494): all variants' lists start
-   from the same water. */
+   from the same water.  A team's warps make a variant's lists each, in slot 0
+   of their own state (`stateStride` bytes apart), then take each other's alpha
+   candidates. */
 template<int kD>
 __device__ NEBC7_PASS int SearchSubset7(SearchState& ss, const Area& ar, const Params& P, const LevelTables& T, int water, const int* est,
-	Ep& best, bool& any, int lane)
+	Ep& best, bool& any, Team& team, TeamState* ts, size_t stateStride, int lane)
 {
-	int valid = 0;
 	const int nv = ar.info.opaque ? 1 : 4;
+	const bool shared = team.size > 1;
+	if (shared)
+		StartTeamSearch(*ts, water);
+	Team one = SingleWarp();
+	int valid = 0;
 #pragma unroll 1
-	for (int v = 0; v < nv; v++)
-		valid |= int(InitLevels4<kD, 7>(ss, v, v, ar, P, T, water, est, lane)) << v;
+	for (int v = team.rank; v < nv; v += team.size)
+		valid |= int(InitLevels4<kD, 7>(ss, shared ? 0 : v, v, ar, P, T, water, est, one, lane)) << v;
+	if (shared)
+	{
+		if (lane == 0 && valid)
+			atomicOr(&ts->valid, valid);
+		__syncthreads();
+		valid = ts->valid;
+	}
 	any = valid != 0;
+	if (!any)
+		return water;
+	const unsigned char* const first = reinterpret_cast<const unsigned char*>(&ss) - team.rank * stateStride;
 #pragma unroll 1
-	for (int v = 0; v < nv; v++)
-		if ((valid >> v) & 1)
-			water = TryV4<kD, 7>(ss, v, ar, P, T, best, water, lane);
+	for (int dv = 0; dv < nv; dv++)
+	{
+		/* a team's warp takes its own variant first, then the others' units */
+		const int v = (team.rank + dv) & (nv - 1);
+		if (!((valid >> v) & 1))
+			continue;
+		const SearchState& sv = shared ? *reinterpret_cast<const SearchState*>(first + v * stateStride) : ss;
+		const int slot = shared ? 0 : v;
+		int limit = water;
+		if (shared)
+		{
+			if (*reinterpret_cast<volatile int*>(&ts->search.next[v]) >= sv.chan[0][0].count * (ar.info.opaque ? 4 : 1))
+				continue;
+			limit = int(*reinterpret_cast<volatile unsigned long long*>(&ts->search.key) >> 32) + 1;
+		}
+		const Found f = SearchFour<kD, 2>(ss, sv, slot, v, ar, WeightsOf(P), T.d2v8, best, limit, shared ? &ts->search : nullptr, lane);
+		if (!shared)
+		{
+			water = f.water;
+			best = f.best;
+		}
+	}
+	if (shared)
+	{
+		__syncthreads();
+		const unsigned long long k = ts->search.key;
+		if (int(k >> 32) < water)
+		{
+			water = int(k >> 32);
+			best = PlaceEndpoints(reinterpret_cast<const SearchState*>(first + (unsigned(k) >> 20) * stateStride)->lists[0], unsigned(k));
+		}
+	}
 	return water;
 }
 
 template<int kD, int MODE>
-__device__ NEBC7_PASS void RefineMode6(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void RefineMode6(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team,
+	TeamState* ts, int lane)
 {
 	/* src/Bc7CoreMode6.cpp:1366-1381 */
 	Ep mc = R.best[0];
-	const int error = CompressSubsetSingle<kD, MODE>(ss, st.area1, P, T, mc, R.errTotal, lane);
+	const int error = CompressSubsetSingle<kD, MODE>(ss, st.area1, P, T, mc, R.errTotal, team, ts, lane);
 	if (R.errTotal > error)
 	{
 		R.errTotal = error;
@@ -1263,7 +1443,8 @@ __device__ NEBC7_PASS void RefineMode6(WarpState& st, SearchState& ss, CellRegs&
 }
 
 template<int kD>
-__device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team,
+	TeamState* ts, int lane)
 {
 	/* src/Bc7CoreMode6.cpp:1398-1422 */
 	if (R.personalMode == 6)
@@ -1274,7 +1455,7 @@ __device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R
 	if (line < R.errTotal - step)
 	{
 		Ep mc = 0;
-		const int error = CompressSubsetSingle<kD, 6>(ss, st.area1, P, T, mc, R.errTotal - step, lane);
+		const int error = CompressSubsetSingle<kD, 6>(ss, st.area1, P, T, mc, R.errTotal - step, team, ts, lane);
 		if (R.errTotal > error + step)
 		{
 			R.errTotal = error;
@@ -1285,7 +1466,8 @@ __device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R
 }
 
 template<int kD>
-__device__ NEBC7_PASS void RefineMode7(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void RefineMode7(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team,
+	TeamState* ts, size_t stateStride, int lane)
 {
 	/* src/Bc7CoreMode7.cpp:496-557 */
 	Ep mc0 = R.best[0], mc1 = R.best[1];
@@ -1302,7 +1484,7 @@ __device__ NEBC7_PASS void RefineMode7(WarpState& st, SearchState& ss, CellRegs&
 		if (water)
 		{
 			bool any;
-			const int r = SearchSubset7<kD>(ss, ar, P, T, water, nullptr, b, any, lane);
+			const int r = SearchSubset7<kD>(ss, ar, P, T, water, nullptr, b, any, team, ts, stateStride, lane);
 			if (any)
 			{
 				water = r;
@@ -1379,13 +1561,75 @@ __device__ __forceinline__ bool Mode7Partition(WarpState& st, SearchState& ss, C
 	}
 	Ep mc0 = 0, mc1 = 0;
 	int error = 0;
+	Team one = SingleWarp();
 #pragma unroll 1
 	for (int s = 0; s < 2; s++)
 	{
 		const int water = room - (s == 0 ? line1 : error);
 		bool any;
 		Ep b = 0;
-		const int r = SearchSubset7<kD>(ss, st.sub[s], P, T, water, ss.bound[s], b, any, lane);
+		const int r = SearchSubset7<kD>(ss, st.sub[s], P, T, water, ss.bound[s], b, any, one, nullptr, 0, lane);
+		if (!any || !(r < water))
+			return false;
+		error += r;
+		if (s == 0)
+			mc0 = b;
+		else
+			mc1 = b;
+	}
+	R.errTotal = error;
+	R.best[0] = mc0;
+	R.best[1] = mc1;
+	R.bestParam = p;
+	R.bestMode = 7;
+	return error <= 0;
+}
+
+/* Mode7Partition by the CTA's four warps: the four channels' estimates, the
+   four p-bit variants' lists and the alpha candidates of the searches are
+   theirs; each warp keeps the block and its subsets in its own state.
+   The estimates take the subset's whole water where the reference takes what
+   the earlier channels leave: an estimate below that rest is the same (a
+   candidate below it lies in both windows), and one that is not ends the
+   subset either way.  A hard partition of an alpha block takes 2 ms in a
+   team where one warp took 8. */
+template<int kD>
+__device__ __forceinline__ bool Mode7PartitionTeam(WarpState& st, SearchState& ss, TeamState& ts, size_t stateStride, CellRegs& R, const Params& P,
+	const LevelTables& T, int p, int rank, int lane)
+{
+	Team team{ 4, rank, &ts.exchange, 0 };
+	const int room = R.errTotal - R.denoiseStep;
+	int line1 = 0, used = 0;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		const Area& ar = st.sub[s];
+		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		const int water = room - used;
+		int l = 0;
+		if (ar.info.active && (rank || !ar.info.opaque) && water > 0)
+			l = EstimateChannelLevels<kD>(ar, rank, ChannelWeight(P, rank), water, 6, rank != 0, T.d2v8, true, T.c2v6, ss.values, lane);
+		if (lane == 0)
+			ts.bound[s][rank] = l;
+		team.Sync();
+		int error = 0;
+#pragma unroll
+		for (int c = 0; c < 4; c++)
+			error = error < water ? error + ts.bound[s][c] : error;
+		if (!(error < water))
+			return false;
+		used += error;
+		line1 = error;
+	}
+	Ep mc0 = 0, mc1 = 0;
+	int error = 0;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		const int water = room - (s == 0 ? line1 : error);
+		bool any;
+		Ep b = 0;
+		const int r = SearchSubset7<kD>(ss, st.sub[s], P, T, water, ts.bound[s], b, any, team, &ts, stateStride, lane);
 		if (!any || !(r < water))
 			return false;
 		error += r;
@@ -1553,6 +1797,7 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		ctab = T.d2v8;
 		atab = T.d2v8;
 	}
+	Team one = SingleWarp();
 	int used = 0;
 #pragma unroll 1
 	for (int c = 0; c < 4; c++)
@@ -1564,7 +1809,7 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		else if (c == a)
 			cl = ChannelLevelsSingle<kD>(ss.lists[0][c], ar, c, w, water - used, abits, c != 0, atab, ss.values, lane);
 		else
-			cl = ChannelLevels<kD, false>(ss.lists[0][c], ar, c, w, water - used, cbits, -1, c != 0, ctab, true, 32, ss.values, lane);
+			cl = ChannelLevels<kD, false>(ss.lists[0][c], ar, c, w, water - used, cbits, -1, c != 0, ctab, true, 32, ss.values, one, lane);
 		if (lane == 0)
 			ss.chan[0][c] = cl;
 		used += cl.minErr;
@@ -1679,6 +1924,7 @@ __device__ NEBC7_PASS void FullRot(WarpState& st, SearchState& ss, CellRegs& R, 
 template<int kD>
 __device__ void NormalPasses(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
 {
+	Team one = SingleWarp();
 	const int OA = R.opaqueAlphaError;
 	const int step = R.denoiseStep;
 
@@ -1690,9 +1936,9 @@ __device__ void NormalPasses(WarpState& st, SearchState& ss, CellRegs& R, const 
 	case 3: if (R.errTotal > OA) RefineOpaque<kD, 3>(st, ss, R, P, T, lane); break;
 	case 4: if (R.errTotal > 0) RefineMode4<kD>(st, ss, R, P, T, lane); break;
 	case 5: if (R.errTotal > 0) RefineMode5<kD>(st, ss, R, P, T, lane); break;
-	case 6: if (R.errTotal > 0) RefineMode6<kD, 6>(st, ss, R, P, T, lane); break;
-	case 7: if (R.errTotal > 0) RefineMode7<kD>(st, ss, R, P, T, lane); break;
-	case 9: if (R.errTotal > 0) RefineMode6<kD, 9>(st, ss, R, P, T, lane); break;
+	case 6: if (R.errTotal > 0) RefineMode6<kD, 6>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 7: if (R.errTotal > 0) RefineMode7<kD>(st, ss, R, P, T, one, nullptr, 0, lane); break;
+	case 9: if (R.errTotal > 0) RefineMode6<kD, 9>(st, ss, R, P, T, one, nullptr, lane); break;
 	}
 
 	R.personalParam = R.bestParam;
@@ -1722,7 +1968,7 @@ __device__ void NormalPasses(WarpState& st, SearchState& ss, CellRegs& R, const 
 								{
 									FullMode7<kD>(st, ss, R, P, T, lane);
 									if (R.errTotal > step)
-										FullMode6<kD>(st, ss, R, P, T, lane);
+										FullMode6<kD>(st, ss, R, P, T, one, nullptr, lane);
 								}
 							}
 						}
@@ -1743,7 +1989,7 @@ __device__ void NormalPasses(WarpState& st, SearchState& ss, CellRegs& R, const 
 				{
 					FullMode7<kD>(st, ss, R, P, T, lane);
 					if (P.doSlow && R.errTotal > step)
-						FullMode6<kD>(st, ss, R, P, T, lane);
+						FullMode6<kD>(st, ss, R, P, T, one, nullptr, lane);
 				}
 			}
 		}

@@ -93,11 +93,13 @@ struct __align__(16) SplitResult
 	int pad;
 };
 
-/* The split passes and their rounds. */
-constexpr int kSplitMaxRounds = 8;
-constexpr int kSplitMaxBlocks = 1 << 24;    /* blocks of a round split into partition tasks (the task count stays an int) */
+/* The split passes. */
+constexpr int kSplitMaxBlocks = 1 << 24;    /* blocks of a pass split into tasks (the task count stays an int) */
 constexpr int kSplitSerial = -1;            /* firstImp: the block's pass runs whole (OPTION_PCA) */
 constexpr int kSplitNone = 0x7FFFFFFF;      /* firstImp: no improvement yet */
+/* Polls of a warp that waits for a later round's tasks (2 us and more each)
+   before it leaves them to the others: about ten seconds. */
+constexpr int kSplitPolls = 1 << 22;
 
 __host__ __device__ constexpr int SplitIndex(int S)
 {
@@ -115,28 +117,37 @@ __host__ __device__ constexpr int SplitMode(int S)
 	return S == kStepFull2Mode1 ? 1 : (S == kStepFull2Mode3 ? 3 : (S == kStepRot5 ? 5 : (S == kStepRot4 ? 4 : 7)));
 }
 
-/* Rounds of split pass S: one per candidate for the rotation searches,
-   whose choices often improve one after another; three for the partition
-   searches, where a block rarely improves more than twice. */
-__host__ __device__ constexpr int SplitRounds(int S)
+/* Kernel launches of a staged encode: the draft kernel, then per pass its
+   list and its kernel, a split pass's remainder; without /slow the passes that
+   only it reaches are left out. */
+__host__ __device__ constexpr bool StageLaunched(int S, bool slow)
 {
-	return S == kStepRot4 || S == kStepRot5 ? SplitTasks(S) : 3;
+	return slow || (S != kStepFull2Mode1 && S != kStepFull2Mode3 && S != kStepMode6);
 }
 
-/* Kernel launches of one staged encode: the draft kernel, then per pass its
-   list and its kernel, or for a split pass its list, the preparation, a
-   task and a commit kernel per round and the one-warp rest. */
-__host__ __device__ constexpr int StagedLaunches()
+__host__ __device__ constexpr int StagedLaunches(bool slow)
 {
 	int n = 1;
 	for (int S = 0; S < kNumStages; S++)
-		n += SplitIndex(S) >= 0 ? 3 + 2 * SplitRounds(S) : 2;
+		if (StageLaunched(S, slow))
+			n += SplitIndex(S) >= 0 ? 3 : 2;
 	return n;
 }
 
-/* Ints of the zeroed split counters per split pass: [round][list length,
-   task head, kept results, unused], the last row for the one-warp rest. */
-constexpr int kSplitCounterInts = 4 * (kSplitMaxRounds + 1);
+/* The task queue of a split pass (zero before the draft kernel).  The first
+   round's tasks are those of the pass's list, the later rounds' entries are
+   appended to Stages::later; polled together in one 16-byte read. */
+struct __align__(16) SplitQueue
+{
+	int laterHead, laterTail;   /* later tasks taken, later entries published */
+	int finished;               /* blocks that have left the pass */
+	int laterReserve;           /* later entries reserved */
+	int pad0[28];
+	int head;                   /* first-round tasks taken */
+	int kept;                   /* results kept */
+	int restCount, restHead;    /* the one-warp remainder */
+	int pad1[28];
+};
 
 /* Per-launch state of a staged encode (one entry per queue position). */
 struct Stages
@@ -146,14 +157,44 @@ struct Stages
 	int* list;        /* positions of the pass being run, in queue order */
 	int* count;       /* [kNumStages] list lengths */
 	int* counters;    /* [kNumStages + 1] work-queue heads, zero before the draft kernel */
+	int* hist;        /* [kNumStages][256] blocks per bucket of the passes' lists, zero before the draft kernel */
+	int* cursor;      /* [kNumStages][256] positions taken, zero before the draft kernel */
+	int total;        /* positions */
+	int byError;      /* whether the searches' lists go by error (else every list by position) */
 	/* split passes */
-	int* start;       /* per position: the first candidate of the block's next round */
+	int* start;       /* per position: the first candidate of the block's round */
 	int* firstImp;    /* per position: (candidate << 24) | result slot of the round's first improvement */
-	int* splitList[3];   /* the lists of the later rounds (alternately) and of the one-warp remainder */
-	int* split;       /* [5 split passes][kSplitCounterInts] list lengths, task heads, result counts; zero before the draft kernel */
+	int* pending;     /* per position: the round's candidates not done */
+	int* later;       /* the blocks of the later rounds, in the order they were appended */
+	int laterCap;
+	int* rest;        /* the blocks of the one-warp remainder */
+	SplitQueue* split;   /* [5 split passes] */
 	SplitResult* imp;
 	int impCap;
 };
+
+/* Bucket of position k in the list of pass `stage`: 8 per octave of the
+   error, largest first, for the searches (their cost grows with it: the
+   longest start first and no SM waits behind a late hard block), 4 per octave
+   with the opaque blocks last for the refinement of modes 6 and 6Index2 (an
+   opaque block has one p-bit variant and one alpha candidate where another
+   has four and twenty), else by position. */
+__device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, bool opaque)
+{
+	if (!sg.byError || stage < kStepRefineOpaque || stage == kStepFinish)
+		return int((long long)k * 256 / sg.total);
+	const unsigned e = unsigned(max(error, 1));
+	const int msb = 31 - __clz(e);
+	const int b = 255 - min(255, msb * 8 + int((e >> (msb >= 3 ? msb - 3 : 0)) & 7u));
+	return stage == kStepRefine6 ? (opaque ? 128 : 0) + (b >> 1) : b;
+}
+
+/* Records that position k waits for pass n (one thread). */
+__device__ __forceinline__ void Publish(const Stages& sg, int k, int n, int error, bool opaque)
+{
+	sg.next[k] = n;
+	atomicAdd(&sg.hist[n * 256 + StageBucket(sg, n, k, error, opaque)], 1);
+}
 
 __device__ __forceinline__ void SaveRecord(BlockRecord& r, const CellRegs& R, int lane)
 {
@@ -176,10 +217,16 @@ __device__ __forceinline__ void SaveRecord(BlockRecord& r, const CellRegs& R, in
 
 /* Rebuilds a block's state: its pixels and masks, the saved scalars, the
    whole-block area (src/Bc7Core.cpp:1532-1535). */
-__device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const BlockRef& b, const BlockRecord& r, const Params& P,
+__device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const BlockRef& b, const BlockRecord& record, const Params& P,
 	int lane)
 {
 	LoadCell(st, b, R, lane);
+	/* past L1: another SM may have written it within this kernel (split passes) */
+	BlockRecord r;
+	const uint4* from = reinterpret_cast<const uint4*>(&record);
+#pragma unroll
+	for (int i = 0; i < int(sizeof(BlockRecord) / 16); i++)
+		reinterpret_cast<uint4*>(&r)[i] = __ldcg(from + i);
 	R.best[0] = r.best[0];
 	R.best[1] = r.best[1];
 	R.best[2] = r.best[2];
@@ -194,11 +241,52 @@ __device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const B
 	BuildWholeBlock(st, R, P, lane);
 }
 
+/* Shared memory of a warp of stage STAGE: the block state, and the search
+   state as far as the pass uses it (SearchState).  One CTA of the precise
+   mode-2 search took 53 KB with the whole of both, which left 37 KB of L1 for
+   16 warps (18 % hits on the level tables). */
+__host__ __device__ constexpr size_t StageWarpBytes(int stage, bool split)
+{
+	if (stage < kStepRefineOpaque || stage == kStepFinish)
+		return sizeof(WarpState);
+	const bool pca = !split && (stage == kStepFull2Mode1 || stage == kStepFull2Mode3 || stage == kStepMode7);
+	const size_t search = pca ? sizeof(SearchState)
+		: (stage == kStepRefine6 || stage == kStepRefine7 || stage == kStepMode7) ? offsetof(SearchState, table) + sizeof(SearchState::table)
+		: stage == kStepMode6 ? offsetof(SearchState, plane16) + sizeof(SearchState::plane16)
+		: (stage == kStepFull3Mode2 || stage == kStepFull3Mode0) ? offsetof(SearchState, three) + sizeof(SearchState::three)
+		: offsetof(SearchState, three);
+	return kSearchWarpBytes + ((search + 15) & ~size_t(15));
+}
+
+__host__ __device__ constexpr size_t StageSharedBytes(int stage, bool split)
+{
+	return kWarpsPerCta * StageWarpBytes(stage, split);
+}
+
+/* Passes whose blocks a CTA's warps search together, and how many of them (the
+   first of the list): all when there are few, since then the longest search is
+   what the pass takes (a 1024x1024 photo leaves the three-subset search of
+   mode 2 eight blocks, 2.3 ms of one warp each; the mode 7 refinement of an
+   alpha texture's 1200 blocks took 5.4 ms, 0.4 ms of the GPU's warps), else
+   one per CTA of the four-channel searches, whose list begins with the hardest,
+   and none of the three-subset ones, whose teams only share the estimates. */
+__host__ __device__ constexpr bool TeamStage(int S)
+{
+	return S == kStepFull3Mode2 || S == kStepFull3Mode0 || S == kStepRefine6 || S == kStepRefine7 || S == kStepMode6;
+}
+
+__device__ __forceinline__ int TeamBlocks(int S, int n, int ctas)
+{
+	if (S == kStepFull3Mode2 || S == kStepFull3Mode0)
+		return n <= kWarpsPerCta * ctas ? n : 0;
+	return n <= 2 * kWarpsPerCta * ctas ? n : ctas;
+}
+
 /* One stage: passes of the draft chain after the mode 6 fast pass
    (DraftChain), or one pass of the normal / slow chains (NormalPasses). */
 template<int kD, int S>
 __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane,
-	int from = 0)
+	int from, Team& team, TeamState* ts)
 {
 	if constexpr (S == kStepDraftRot)
 	{
@@ -246,20 +334,20 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 			else if constexpr (S == kStepRefine6)
 			{
 				if (R.bestMode == 6)
-					RefineMode6<kD, 6>(st, ss, R, P, T, lane);
+					RefineMode6<kD, 6>(st, ss, R, P, T, team, ts, lane);
 				else
-					RefineMode6<kD, 9>(st, ss, R, P, T, lane);
+					RefineMode6<kD, 9>(st, ss, R, P, T, team, ts, lane);
 			}
 			else
-				RefineMode7<kD>(st, ss, R, P, T, lane);
+				RefineMode7<kD>(st, ss, R, P, T, team, ts, StageWarpBytes(S, false), lane);
 		}
 		R.personalParam = R.bestParam;
 		R.personalMode = R.bestMode;
 	}
 	else if constexpr (S == kStepFull3Mode2)
-		FullThreeSubsets<kD, 2>(st, ss, R, P, T, lane);
+		FullThreeSubsets<kD, 2>(st, ss, R, P, T, lane, team.size, team.rank, StageWarpBytes(S, false));
 	else if constexpr (S == kStepFull3Mode0)
-		FullThreeSubsets<kD, 0>(st, ss, R, P, T, lane);
+		FullThreeSubsets<kD, 0>(st, ss, R, P, T, lane, team.size, team.rank, StageWarpBytes(S, false));
 	else if constexpr (S == kStepFull2Mode1)
 		FullTwoSubsets<kD, 1>(st, ss, R, P, T, lane, from);
 	else if constexpr (S == kStepFull2Mode3)
@@ -271,7 +359,7 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 	else if constexpr (S == kStepMode7)
 		FullMode7<kD>(st, ss, R, P, T, lane, from);
 	else if constexpr (S == kStepMode6)
-		FullMode6<kD>(st, ss, R, P, T, lane);
+		FullMode6<kD>(st, ss, R, P, T, team, ts, lane);
 }
 
 /* The refinement pass of the block's mode, or the pack. */
@@ -389,8 +477,7 @@ __device__ __forceinline__ void FinishBlock(WarpState& st, CellRegs& R, const Pa
    starting block is written at once; every other block saves its record
    for the next stage and waits.  Returns whether the block finished. */
 template<int kD>
-__device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& T, const Params& P, BlockRecord& rec, int& next,
-	int lane)
+__device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& T, const Params& P, const Stages& sg, int k, int lane)
 {
 	CellRegs R;
 	LoadCell(st, b, R, lane);
@@ -409,7 +496,7 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 	{
 		StoreBlock<kD>(b, R, lo, hi, 1.0, 1.0, lane);
 		if (lane == 0)
-			next = kStepNone;
+			sg.next[k] = kStepNone;
 		return true;
 	}
 	BuildWholeBlock(st, R, P, lane);
@@ -463,13 +550,14 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 		R.denoiseStep = 0;
 		R.opaqueAlphaError = 0;
 	}
+	BlockRecord& rec = sg.rec[k];
 	SaveRecord(rec, R, lane);
 	if (lane == 0)
 	{
 		rec.startLo = lo;
 		rec.startHi = hi;
 		rec.water = water;
-		next = n;
+		Publish(sg, k, n, R.errTotal, R.a1.opaque);
 	}
 	__syncwarp();
 	return false;
@@ -478,16 +566,21 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 /* A pass kernel's block: runs pass S (of a split pass, the partitions from
    `from` on) and records the next one. */
 template<int kD, int S>
-__device__ void PassStage(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P, BlockRecord& rec,
-	int& next, int from, int lane)
+__device__ void PassStage(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P, const Stages& sg, int k,
+	int from, Team& team, TeamState* ts, int lane)
 {
 	CellRegs R;
+	BlockRecord& rec = sg.rec[k];
 	RestoreBlock(st, R, b, rec, P, lane);
-	RunStep<kD, S>(st, ss, R, P, T, lane, from);
+	if (TeamStage(S) && team.size > 1)
+		__syncthreads();   /* every warp has read the record before it changes */
+	RunStep<kD, S>(st, ss, R, P, T, lane, from, team, ts);
+	if (team.rank)
+		return;
 	const int n = NextStep(S, R, P);
 	SaveRecord(rec, R, lane);
 	if (lane == 0)
-		next = n;
+		Publish(sg, k, n, R.errTotal, R.a1.opaque);
 	__syncwarp();
 }
 
@@ -504,10 +597,10 @@ __device__ void FinishStage(WarpState& st, const BlockRef& b, const Params& P, c
    finished (its output is written). */
 template<int kD, int STAGE>
 __device__ __forceinline__ bool StageBlock(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P,
-	const Stages& sg, int k, int lane)
+	const Stages& sg, int k, Team& team, TeamState* ts, int lane)
 {
 	if constexpr (STAGE == kStageDraft)
-		return DraftStage<kD>(st, b, T, P, sg.rec[k], sg.next[k], lane);
+		return DraftStage<kD>(st, b, T, P, sg, k, lane);
 	else if constexpr (STAGE == kStepFinish)
 	{
 		FinishStage<kD>(st, b, P, sg.rec[k], lane);
@@ -515,31 +608,9 @@ __device__ __forceinline__ bool StageBlock(WarpState& st, SearchState& ss, const
 	}
 	else
 	{
-		PassStage<kD, STAGE>(st, ss, b, T, P, sg.rec[k], sg.next[k], SplitIndex(STAGE) >= 0 ? sg.start[k] : 0, lane);
+		PassStage<kD, STAGE>(st, ss, b, T, P, sg, k, SplitIndex(STAGE) >= 0 ? sg.start[k] : 0, team, ts, lane);
 		return false;
 	}
-}
-
-/* Shared memory of a warp of stage STAGE: the block state, and the search
-   state as far as the pass uses it (SearchState).  One CTA of the precise
-   mode-2 search took 53 KB with the whole of both, which left 37 KB of L1 for
-   16 warps (18 % hits on the level tables). */
-__host__ __device__ constexpr size_t StageWarpBytes(int stage, bool split)
-{
-	if (stage < kStepRefineOpaque || stage == kStepFinish)
-		return sizeof(WarpState);
-	const bool pca = !split && (stage == kStepFull2Mode1 || stage == kStepFull2Mode3 || stage == kStepMode7);
-	const size_t search = pca ? sizeof(SearchState)
-		: (stage == kStepRefine6 || stage == kStepRefine7 || stage == kStepMode7) ? offsetof(SearchState, table) + sizeof(SearchState::table)
-		: stage == kStepMode6 ? offsetof(SearchState, plane16) + sizeof(SearchState::plane16)
-		: (stage == kStepFull3Mode2 || stage == kStepFull3Mode0) ? offsetof(SearchState, three) + sizeof(SearchState::three)
-		: offsetof(SearchState, three);
-	return kSearchWarpBytes + ((search + 15) & ~size_t(15));
-}
-
-__host__ __device__ constexpr size_t StageSharedBytes(int stage, bool split)
-{
-	return kWarpsPerCta * StageWarpBytes(stage, split);
 }
 
 /* One stage of a staged encode over a list of queue positions (`list`,
@@ -558,12 +629,34 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 	__shared__ LevelTables tables[2];
 	ShareTables(tables, T0, T1);
 	const int n = list ? *count : job.total;
+	__shared__ TeamState ts;
+	/* the first blocks, the hardest, a CTA each (TeamBlocks), the others a
+	   warp each */
+	const int nTeam = TeamStage(STAGE) ? TeamBlocks(STAGE, n, int(gridDim.x)) : 0;
+	Team team{ nTeam > 0 ? kWarpsPerCta : 1, nTeam > 0 ? warp : 0, &ts.exchange, 0 };
 	for (;;)
 	{
 		int i = 0;
-		if (lane == 0)
+		if (team.rank == 0 && lane == 0)
 			i = atomicAdd(head, 1);
-		i = __shfl_sync(kFull, i, 0);
+		if (TeamStage(STAGE) && team.size > 1)
+		{
+			__syncthreads();
+			if (threadIdx.x == 0)
+				ts.task[0] = i;
+			__syncthreads();
+			i = ts.task[0];
+			if (i >= nTeam)
+			{
+				/* every warp for itself from here; warp 0 has a block already */
+				team = SingleWarp();
+				if (warp && lane == 0)
+					i = atomicAdd(head, 1);
+				i = __shfl_sync(kFull, i, 0);
+			}
+		}
+		else
+			i = __shfl_sync(kFull, i, 0);
 		if (i >= n)
 			break;
 		const int k = list ? list[i] : i;
@@ -575,12 +668,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 		if constexpr (kD == kAnyDenoise)
 		{
 			if (d.denoise)
-				finished = StageBlock<1, STAGE>(st, ss, b, tables[1], P, sg, k, lane);
+				finished = StageBlock<1, STAGE>(st, ss, b, tables[1], P, sg, k, team, &ts, lane);
 			else
-				finished = StageBlock<0, STAGE>(st, ss, b, tables[0], P, sg, k, lane);
+				finished = StageBlock<0, STAGE>(st, ss, b, tables[0], P, sg, k, team, &ts, lane);
 		}
 		else
-			finished = StageBlock<kD, STAGE>(st, ss, b, tables[kD], P, sg, k, lane);
+			finished = StageBlock<kD, STAGE>(st, ss, b, tables[kD], P, sg, k, team, &ts, lane);
 		if (finished)
 			BlockFinished(d, lane);
 	}
@@ -590,18 +683,14 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
    searched from the error in its record (the error at the start of the
    round).  An improving candidate before the round's first improvement so
    far keeps its result and lowers the block's firstImp; a candidate after
-   it is not searched (the next round searches it again). */
-template<int kD, int S>
-__device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P,
-	const Stages& sg, int* impCount, int k, int p, int lane)
+   it is not searched (the next round searches it again).  N warps of the CTA
+   run the task together (mode 7: its four). */
+template<int kD, int S, int N>
+__device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* ts, const BlockRef& b, const LevelTables& T, const Params& P,
+	const Stages& sg, SplitQueue& q, int k, int p, int first, int rank, int lane)
 {
 	constexpr int MODE = SplitMode(S);
-	volatile int* first = sg.firstImp + k;
-	/* one read for the whole warp: other warps lower it meanwhile */
-	int firstNow = 0;
-	if (lane == 0)
-		firstNow = *first;
-	if ((__shfl_sync(kFull, firstNow, 0) >> 24) < p)
+	if ((first >> 24) < p)
 		return;
 	CellRegs R;
 	RestoreBlock(st, R, b, sg.rec[k], P, lane);
@@ -635,7 +724,10 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const Block
 		{
 			if (!(0 < E - step) || !(step < E))
 				return;
-			end = Mode7Partition<kD>(st, ss, R, P, T, p, 0, 0, lane);
+			if constexpr (N == 1)
+				end = Mode7Partition<kD>(st, ss, R, P, T, p, 0, 0, lane);
+			else
+				end = Mode7PartitionTeam<kD>(st, ss, *ts, StageWarpBytes(S, true), R, P, T, p, rank, lane);
 		}
 		else
 		{
@@ -647,10 +739,10 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const Block
 		if (R.errTotal == E)
 			return;
 	}
-	if (lane != 0 || (*first >> 24) < p)
+	if (rank != 0 || lane != 0 || (*reinterpret_cast<volatile int*>(sg.firstImp + k) >> 24) < p)
 		return;
 	int slot = 0xFFFFFF;
-	const int at = atomicAdd(impCount, 1);
+	const int at = atomicAdd(&q.kept, 1);
 	if (at < sg.impCap)
 	{
 		SplitResult r;
@@ -663,37 +755,200 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, const Block
 		sg.imp[at] = r;
 		slot = at;
 	}
+	/* the result before the word that leads to it */
+	__threadfence();
 	atomicMin(sg.firstImp + k, (p << 24) | slot);
 }
 
-/* A round of split pass S over the blocks list[i], i < *count (at most
-   kSplitMaxBlocks): tasks (block, candidate p) for p from the block's start
-   candidate, taken through *head block by block, so that the candidates of
-   a block go to as many warps. */
-template<int kD, int S>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, Stages sg, const int* list, const int* count, int* head,
-	int* impCount, LevelTables T0, LevelTables T1)
+/* The end of a block's round of split pass S (one thread, after its last
+   task): the first improving candidate f becomes the block's best and ends
+   the pass, or the block goes on from f + 1 in a later round with the new
+   error; a block without an improvement has finished the pass and gets its
+   next one (NextStep).  Blocks whose result was not kept, and those that
+   must run whole, are left to the one-warp remainder. */
+template<int S>
+__device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, SplitQueue& q, int k)
+{
+	constexpr int MODE = SplitMode(S), NT = SplitTasks(S);
+	const int f = *reinterpret_cast<volatile int*>(sg.firstImp + k);
+	BlockRecord& r = sg.rec[k];
+	int from = -1;
+	bool rest = false;
+	if (f == kSplitSerial)
+	{
+		from = 0;
+		rest = true;
+	}
+	else if (f != kSplitNone)
+	{
+		const int p = f >> 24, slot = f & 0xFFFFFF;
+		if (slot >= sg.impCap)
+		{
+			from = p;   /* its result was not kept: search it again */
+			rest = true;
+		}
+		else
+		{
+			const uint4* e = reinterpret_cast<const uint4*>(sg.imp + slot);
+			SplitResult v;
+			reinterpret_cast<uint4*>(&v)[0] = __ldcg(e);
+			reinterpret_cast<uint4*>(&v)[1] = __ldcg(e + 1);
+			r.errTotal = v.error;
+			r.best[0] = v.best0;
+			if (MODE != 4 && MODE != 5)
+				r.best[1] = v.best1;
+			r.bestParam = v.param;
+			r.bestMode = MODE;
+			if (!v.end && p < NT - 1)
+				from = p + 1;
+		}
+	}
+	if (from >= 0)
+	{
+		sg.start[k] = from;
+		sg.firstImp[k] = kSplitNone;
+		sg.pending[k] = NT - from;
+		const int at = rest ? sg.laterCap : atomicAdd(&q.laterReserve, 1);
+		if (at < sg.laterCap)
+		{
+			sg.later[at] = k;
+			/* published in order: the entries before it are being published by
+			   running warps; should that take seconds, the block (and those
+			   behind it) goes to the remainder */
+			__threadfence();
+			for (int tries = 0; tries < kSplitPolls; tries++)
+			{
+				if (atomicCAS(&q.laterTail, at, at + 1) == at)
+					return;
+				__nanosleep(500);
+			}
+		}
+		sg.rest[atomicAdd(&q.restCount, 1)] = k;
+	}
+	else
+	{
+		const BlockRecord now = r;
+		TexDesc d;
+		BlockRef b;
+		QueuedBlock(job, k, d, b);
+		CellRegs R;
+		R.errTotal = now.errTotal;
+		R.opaqueAlphaError = now.opaqueAlphaError;
+		R.denoiseStep = now.denoiseStep;
+			R.a1.opaque = now.opaque != 0;
+		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.opaque != 0);
+	}
+	__threadfence();
+	atomicAdd(&q.finished, 1);
+}
+
+/* The next task (one thread): of a later round if there is one, else of the
+   first round (n blocks); waits while blocks of either are still running.
+   firstRound: whether the caller has found no end of the first round yet.
+   Returns the task's entry * NT + candidate, the later rounds' entries after
+   the first round's n, or -1. */
+template<int S>
+__device__ __forceinline__ long long SplitTake(const Stages& sg, SplitQueue& q, int n, bool& firstRound)
 {
 	constexpr int NT = SplitTasks(S);
+	for (int polls = 0; polls < kSplitPolls;)
+	{
+		int4 s;
+		asm volatile("ld.volatile.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(s.x), "=r"(s.y), "=r"(s.z), "=r"(s.w) : "l"(&q) : "memory");
+		/* laterHead counts tasks, laterTail entries */
+		if (s.x < s.y * NT)
+		{
+			if (atomicCAS(&q.laterHead, s.x, s.x + 1) == s.x)
+			{
+				__threadfence();   /* the block's record and start after the entry */
+				return (long long)n * NT + s.x;
+			}
+			continue;
+		}
+		if (firstRound)
+		{
+			const int t = atomicAdd(&q.head, 1);
+			if (t < n * NT)
+				return t;
+			firstRound = false;
+		}
+		if (s.z >= n)
+			break;
+		__nanosleep(2000);
+		polls++;
+	}
+	return -1;
+}
+
+/* Warps of a CTA that run a task of split pass S together. */
+__host__ __device__ constexpr int SplitTeam(int S)
+{
+	return S == kStepMode7 ? kWarpsPerCta : 1;
+}
+
+/* Split pass S over the blocks list[i], i < *count (at most kSplitMaxBlocks).
+   The tasks (block, candidate p) are taken block by block, so that the
+   candidates of a block go to as many warps; a block's last task commits the
+   round, and the next round's tasks are taken as soon as it has: the rounds
+   of the hard blocks, whose tasks come first, run beside the other blocks'
+   first round. */
+template<int kD, int S>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, Stages sg, const int* list, const int* count, LevelTables T0,
+	LevelTables T1)
+{
+	constexpr int NT = SplitTasks(S), N = SplitTeam(S);
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
+	__shared__ TeamState team;
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(S, true));
 	SearchState& ss = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&st) + kSearchWarpBytes);
 	__shared__ LevelTables tables[2];
 	ShareTables(tables, T0, T1);
+	SplitQueue& q = sg.split[SplitIndex(S)];
 	const int n = min(*count, kSplitMaxBlocks);
+	const int rank = N > 1 ? warp : 0;
+	bool firstRound = true;
 	for (;;)
 	{
-		int t = 0;
-		if (lane == 0)
-			t = atomicAdd(head, 1);
-		t = __shfl_sync(kFull, t, 0);
-		if (t >= n * NT)
+		int k = -1, p = 0, first = 0;
+		if (rank == 0 && lane == 0)
+		{
+			const long long t = SplitTake<S>(sg, q, n, firstRound);
+			if (t >= 0)
+			{
+				const long long e = t / NT;
+				p = int(t % NT);
+				k = e < n ? list[e] : *reinterpret_cast<volatile int*>(sg.later + (e - n));
+				if (p < *reinterpret_cast<volatile int*>(sg.start + k))
+					p = -1;
+				/* one read for all the task's warps: other warps lower it meanwhile */
+				first = *reinterpret_cast<volatile int*>(sg.firstImp + k);
+			}
+		}
+		if (N > 1)
+		{
+			__syncthreads();   /* the last task's shared state is read */
+			if (threadIdx.x == 0)
+			{
+				team.task[0] = k;
+				team.task[1] = p;
+				team.task[2] = first;
+			}
+			__syncthreads();
+			k = team.task[0];
+			p = team.task[1];
+			first = team.task[2];
+		}
+		else
+		{
+			k = __shfl_sync(kFull, k, 0);
+			p = __shfl_sync(kFull, p, 0);
+			first = __shfl_sync(kFull, first, 0);
+		}
+		if (k < 0)
 			break;
-		const int i = t / NT, p = t % NT;
-		const int k = list[i];
-		if (p < sg.start[k])
+		if (p < 0)
 			continue;
 		TexDesc d;
 		BlockRef b;
@@ -703,196 +958,97 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		{
 			/* OPTION_PCA orders the partitions by their bounds first: the
 			   pass runs whole, in one warp */
-			if (p == 0 && lane == 0)
+			if (rank == 0 && lane == 0)
 				sg.firstImp[k] = kSplitSerial;
 			__syncwarp();
-			continue;
 		}
-		if constexpr (kD == kAnyDenoise)
+		else if constexpr (kD == kAnyDenoise)
 		{
 			if (d.denoise)
-				SplitTask<1, S>(st, ss, b, tables[1], P, sg, impCount, k, p, lane);
+				SplitTask<1, S, N>(st, ss, &team, b, tables[1], P, sg, q, k, p, first, rank, lane);
 			else
-				SplitTask<0, S>(st, ss, b, tables[0], P, sg, impCount, k, p, lane);
+				SplitTask<0, S, N>(st, ss, &team, b, tables[0], P, sg, q, k, p, first, rank, lane);
 		}
 		else
-			SplitTask<kD, S>(st, ss, b, tables[kD], P, sg, impCount, k, p, lane);
-	}
-}
-
-/* Before the first round of a split pass: every block starts at candidate 0
-   with no improvement; blocks past kSplitMaxBlocks (more than the task count
-   can number) go to the one-warp remainder at once. */
-static __global__ void __launch_bounds__(256) KSplitPrepare(Stages sg, const int* list, const int* count, int* restList, int* restCount)
-{
-	const int n = *count;
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-	{
-		const int k = list[i];
-		sg.start[k] = 0;
-		sg.firstImp[k] = kSplitNone;
-		if (i >= kSplitMaxBlocks)
-			restList[atomicAdd(restCount, 1)] = k;
-	}
-}
-
-/* The commit of a round of split pass S, one thread per split block: the
-   first improving candidate f becomes the block's best and ends the pass,
-   or the block goes on from f + 1 in the next round's list (after the last
-   round, in the one-warp remainder's list); a block without an improvement
-   has finished the pass and gets its next one (NextStep). */
-template<int S>
-__global__ void __launch_bounds__(256) KSplitCommit(Job job, Stages sg, const int* list, const int* count, int* nextList,
-	int* nextCount, int* restList, int* restCount, int lastRound)
-{
-	constexpr int MODE = SplitMode(S);
-	const int n = min(*count, kSplitMaxBlocks);
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-	{
-		const int k = list[i];
-		const int f = sg.firstImp[k];
-		BlockRecord& r = sg.rec[k];
-		if (f == kSplitSerial)
+			SplitTask<kD, S, N>(st, ss, &team, b, tables[kD], P, sg, q, k, p, first, rank, lane);
+		/* every warp of a team has read the block's record before its round can
+		   end and change it */
+		if (N > 1)
+			__syncthreads();
+		else
+			__syncwarp();
+		if (rank == 0 && lane == 0)
 		{
-			sg.start[k] = 0;
-			restList[atomicAdd(restCount, 1)] = k;
-			continue;
-		}
-		int from = -1;
-		if (f != kSplitNone)
-		{
-			const int p = f >> 24, slot = f & 0xFFFFFF;
-			if (slot >= sg.impCap)
-				from = p;   /* its result was not kept: search it again */
-			else
+			__threadfence();
+			if (atomicSub(sg.pending + k, 1) == 1)
 			{
-				const SplitResult e = sg.imp[slot];
-				r.errTotal = e.error;
-				r.best[0] = e.best0;
-				if (MODE != 4 && MODE != 5)
-					r.best[1] = e.best1;
-				r.bestParam = e.param;
-				r.bestMode = MODE;
-				if (!e.end && p < SplitTasks(S) - 1)
-					from = p + 1;
+				__threadfence();
+				SplitCommit<S>(job, sg, q, k);
 			}
 		}
-		if (from >= 0)
-		{
-			sg.start[k] = from;
-			sg.firstImp[k] = kSplitNone;
-			if (lastRound)
-				restList[atomicAdd(restCount, 1)] = k;
-			else
-				nextList[atomicAdd(nextCount, 1)] = k;
-			continue;
-		}
-		TexDesc d;
-		BlockRef b;
-		QueuedBlock(job, k, d, b);
-		CellRegs R;
-		R.errTotal = r.errTotal;
-		R.opaqueAlphaError = r.opaqueAlphaError;
-		R.denoiseStep = r.denoiseStep;
-		R.a1.opaque = r.opaque != 0;
-		sg.next[k] = NextStep(S, R, d.P);
+		__syncwarp();
 	}
 }
 
-/* Gathers, in queue order, the positions whose next pass is `stage` into
-   list and their number into *count (one block of 1024 threads, 4096
-   positions per round). */
-static __global__ void __launch_bounds__(1024) KStageList(const int* next, int total, int stage, int* list, int* count)
+/* Gathers the positions whose next pass is `stage` into its list, bucket by
+   bucket (StageBucket), and their number; for a split pass (tasks per block
+   NT > 0) the blocks start at candidate 0, and those past kSplitMaxBlocks
+   (more than the task count can number) go to the remainder at once. */
+static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, int splitIndex, int NT)
 {
-	__shared__ int warpSums[32];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	int base = 0;
-	for (int k0 = 0; k0 < total; k0 += 4096)
+	__shared__ int base[256];
+	const int lane = threadIdx.x & 31;
+	if (threadIdx.x < 32)
 	{
-		const int k = k0 + 4 * int(threadIdx.x);
-		bool on[4];
-		int mine = 0;
-		for (int j = 0; j < 4; j++)
+		/* exclusive scan of the bucket counts: 8 per lane, then the lanes */
+		int c[8], run = 0;
+#pragma unroll
+		for (int j = 0; j < 8; j++)
 		{
-			on[j] = k + j < total && next[k + j] == stage;
-			mine += on[j];
+			c[j] = run;
+			run += sg.hist[stage * 256 + lane * 8 + j];
 		}
-		/* inclusive scan of the per-thread counts over the warp, then the block */
-		int incl = mine;
+		int incl = run;
 		for (int o = 1; o < 32; o <<= 1)
 		{
 			const int v = __shfl_up_sync(kFull, incl, o);
 			if (lane >= o)
 				incl += v;
 		}
-		if (lane == 31)
-			warpSums[warp] = incl;
-		__syncthreads();
-		int before = 0, all = 0;
-		for (int w = 0; w < 32; w++)
-		{
-			const int c = warpSums[w];
-			before += w < warp ? c : 0;
-			all += c;
-		}
-		int at = base + before + incl - mine;
-		for (int j = 0; j < 4; j++)
-			if (on[j])
-				list[at++] = k + j;
-		base += all;
-		__syncthreads();
+#pragma unroll
+		for (int j = 0; j < 8; j++)
+			base[lane * 8 + j] = incl - run + c[j];
+		if (blockIdx.x == 0 && lane == 31)
+			sg.count[stage] = incl;
+		if (lane == 31 && incl == 0)
+			base[0] = -1;
 	}
-	if (threadIdx.x == 0)
-		*count = base;
-}
-
-/* Gathers the positions whose next pass is `stage`, largest error first:
-   a counting sort on 8 buckets per octave of the record's errTotal (one
-   block of 1024 threads).  A search's cost grows with its water, so the
-   longest searches of a pass start first and no SM waits at the end of the
-   pass behind a late hard block; the order inside a bucket is any, and
-   the blocks written are the same either way. */
-static __global__ void __launch_bounds__(1024) KStageListByError(const int* next, const BlockRecord* rec, int total, int stage,
-	int* list, int* count)
-{
-	__shared__ int hist[256];
-	__shared__ int base[256];
-	for (int i = threadIdx.x; i < 256; i += 1024)
-		hist[i] = 0;
 	__syncthreads();
-	auto bucketOf = [&](int k) {
-		const unsigned e = unsigned(max(rec[k].errTotal, 0));
-		if (!e)
-			return 255;
-		const int msb = 31 - __clz(e);
-		const int frac = int((e >> (msb >= 3 ? msb - 3 : 0)) & 7u);
-		return 255 - min(255, msb * 8 + frac);
-	};
-	for (int k = threadIdx.x; k < total; k += 1024)
-		if (next[k] == stage)
-			atomicAdd(&hist[bucketOf(k)], 1);
-	__syncthreads();
-	if (threadIdx.x == 0)
+	if (base[0] < 0)
+		return;
+	for (int k = blockIdx.x * 1024 + threadIdx.x; k < sg.total; k += gridDim.x * 1024)
 	{
-		int run = 0;
-		for (int b = 0; b < 256; b++)
+		if (sg.next[k] != stage)
+			continue;
+		const int b = StageBucket(sg, stage, k, sg.rec[k].errTotal, sg.rec[k].opaque != 0);
+		const int at = base[b] + atomicAdd(&sg.cursor[stage * 256 + b], 1);
+		sg.list[at] = k;
+		if (NT)
 		{
-			base[b] = run;
-			run += hist[b];
+			sg.start[k] = 0;
+			sg.firstImp[k] = kSplitNone;
+			sg.pending[k] = NT;
+			if (at >= kSplitMaxBlocks)
+				sg.rest[atomicAdd(&sg.split[splitIndex].restCount, 1)] = k;
 		}
-		*count = run;
 	}
-	__syncthreads();
-	for (int k = threadIdx.x; k < total; k += 1024)
-		if (next[k] == stage)
-			list[atomicAdd(&base[bucketOf(k)], 1)] = k;
 }
 
 /* Host-side launcher of a staged encode: the draft kernel, then for each
    pass its list and its kernel, then the finish kernel's list and kernel.
    The launches are capturable.  Compiled per kD in encode_*_staged.cu. */
 template<int kD>
-cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, const LevelTables& T0,
+cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, const LevelTables& T0,
 	const LevelTables& T1);
 
 /* Raises the stage kernels' dynamic shared-memory limit (once per process
@@ -901,41 +1057,53 @@ template<int kD>
 cudaError_t StagedEncodeOccupancy(int* ctasPerSm);
 
 /* Bytes of the per-position state of a staged encode of n positions
-   (records, next-pass words, the pass list, the split passes' start
-   partitions, first improvements, round lists and kept results; 256-byte
-   aligned pieces), after kStagedZeroed bytes of counts and queue heads that
-   must be zero before each launch. */
-constexpr size_t kStagedZeroed = 1280;
+   (records, next-pass words, the pass list, the split passes' words, later
+   rounds and kept results; 256-byte aligned pieces), after kStagedZeroed bytes
+   of counts, queues and histograms that must be zero before each launch. */
+constexpr size_t kStagedZeroed = 256 + 5 * sizeof(SplitQueue) + 2 * size_t(kNumStages) * 1024;
+static_assert(kStagedZeroed % 256 == 0 && kNumStages < 32, "the counts and queue heads take 128 bytes each");
 
 constexpr size_t SplitResultCap(int n)
 {
-	return size_t(n) + 256;
+	return 3 * size_t(n) + 1024;
 }
+
+constexpr size_t SplitLaterCap(int n)
+{
+	return n < (1 << 22) - 1024 ? 4 * size_t(n) + 1024 : size_t(1) << 24;   /* its tasks stay an int too */
+}
+
+constexpr size_t StagedAlign(size_t v) { return (v + 255) & ~size_t(255); }
 
 constexpr size_t StagedScratchBytes(int n)
 {
-	return kStagedZeroed + ((size_t(n) * sizeof(BlockRecord) + 255) & ~size_t(255)) + ((size_t(n) * 4 + 255) & ~size_t(255)) * 7 +
+	return kStagedZeroed + StagedAlign(size_t(n) * sizeof(BlockRecord)) + StagedAlign(size_t(n) * 4) * 6 + StagedAlign(SplitLaterCap(n) * 4) +
 		SplitResultCap(n) * sizeof(SplitResult);
 }
 
 /* Splits a staged scratch (256-byte aligned, StagedScratchBytes(n) bytes). */
-inline Stages SplitStaged(uint8_t* p, int n)
+inline Stages SplitStaged(uint8_t* p, int n, bool byError)
 {
 	Stages s;
 	s.count = (int*)p;
 	s.counters = (int*)(p + 128);
-	s.split = (int*)(p + 256);
+	s.split = (SplitQueue*)(p + 256);
+	s.hist = (int*)(p + 256 + 5 * sizeof(SplitQueue));
+	s.cursor = s.hist + kNumStages * 256;
+	s.total = n;
+	s.byError = byError;
 	s.rec = (BlockRecord*)(p + kStagedZeroed);
-	uint8_t* q = p + kStagedZeroed + ((size_t(n) * sizeof(BlockRecord) + 255) & ~size_t(255));
-	const size_t ints = (size_t(n) * 4 + 255) & ~size_t(255);
+	uint8_t* q = p + kStagedZeroed + StagedAlign(size_t(n) * sizeof(BlockRecord));
+	const size_t ints = StagedAlign(size_t(n) * 4);
 	s.next = (int*)q;
 	s.list = (int*)(q + ints);
 	s.start = (int*)(q + 2 * ints);
 	s.firstImp = (int*)(q + 3 * ints);
-	s.splitList[0] = (int*)(q + 4 * ints);
-	s.splitList[1] = (int*)(q + 5 * ints);
-	s.splitList[2] = (int*)(q + 6 * ints);
-	s.imp = (SplitResult*)(q + 7 * ints);
+	s.pending = (int*)(q + 4 * ints);
+	s.rest = (int*)(q + 5 * ints);
+	s.later = (int*)(q + 6 * ints);
+	s.laterCap = int(SplitLaterCap(n));
+	s.imp = (SplitResult*)(q + 6 * ints + StagedAlign(SplitLaterCap(n) * 4));
 	s.impCap = int(SplitResultCap(n));
 	return s;
 }

@@ -209,18 +209,17 @@ struct EncodeVariant
 {
 	cudaError_t (*launch)(int, cudaStream_t, const Job&, const LevelTables&, const LevelTables&);
 	cudaError_t (*occupancy)(int*);
-	cudaError_t (*staged)(int, cudaStream_t, const Job&, const Stages&, const LevelTables&, const LevelTables&);
+	cudaError_t (*staged)(int, cudaStream_t, const Job&, const Stages&, bool, const LevelTables&, const LevelTables&);
 	cudaError_t (*stagedOccupancy)(int*);
 };
 
-constexpr int kNumVariants = 6;
-constexpr int kVariantMixed = 5;   /* batches: kDenoise per texture */
+constexpr int kNumVariants = 5;
+constexpr int kVariantMixed = 4;   /* batches: kDenoise per texture */
 const EncodeVariant kVariants[kNumVariants] = {
 	{ LaunchEncodeKernel<0, false, kShapeCompact>, EncodeKernelOccupancy<0, false, kShapeCompact>, nullptr, nullptr },
 	{ LaunchEncodeKernel<0, true, kShapeOutlined>, EncodeKernelOccupancy<0, true, kShapeOutlined>,
 	  LaunchStagedEncode<0>, StagedEncodeOccupancy<0> },
 	{ LaunchEncodeKernel<1, false, kShapeCompact>, EncodeKernelOccupancy<1, false, kShapeCompact>, nullptr, nullptr },
-	{ LaunchEncodeKernel<1, true, kShapeCompact>, EncodeKernelOccupancy<1, true, kShapeCompact>, nullptr, nullptr },
 	{ LaunchEncodeKernel<1, true, kShapeOutlined>, EncodeKernelOccupancy<1, true, kShapeOutlined>,
 	  LaunchStagedEncode<1>, StagedEncodeOccupancy<1> },
 	{ LaunchEncodeKernel<kAnyDenoise, true, kShapeOutlined>, EncodeKernelOccupancy<kAnyDenoise, true, kShapeOutlined>,
@@ -232,17 +231,11 @@ bool SlotStaged(int slot)
 	return kVariants[slot].staged != nullptr;
 }
 
-/* Picks the instantiation: the compact shape for the stepped default preset
-   (kDenoise 1, refinement without /slow or /data), the outlined one where
-   the full searches dominate (measured on the 1024x1024 and 2048x2048
-   workloads). */
+/* Picks the instantiation by the denoise shift and the passes. */
 int VariantSlot(const nebc7_settings& s)
 {
-	if (!s.doNormal || s.doDraft == 2)
-		return s.denoise ? 2 : 0;
-	if (!s.denoise)
-		return 1;
-	return (s.doSlow || s.linearData) ? 4 : 3;
+	const bool normal = s.doNormal && s.doDraft != 2;
+	return 2 * int(s.denoise != 0) + int(normal);
 }
 
 /* Launch shape of one encode instantiation on one device, looked up once
@@ -414,17 +407,22 @@ size_t LaunchScratchBytes(int nblocks, bool wantSums, const nebc7_settings& s)
 
 /* Launches the encode of `job` with instantiation `slot`: the staged form
    when the slot has one and `staged` (StagedScratchBytes(job.total) bytes,
-   256-byte aligned) is given, else the single kernel. */
-cudaError_t LaunchSlot(int slot, int grid, cudaStream_t stream, const Job& job, const LevelTables& T0, const LevelTables& T1,
-	uint8_t* staged)
+   256-byte aligned) is given, else the single kernel on `grid` CTAs.  slow:
+   whether a texture of the launch asks for the /slow passes. */
+cudaError_t LaunchSlot(int slot, int grid, int ctasPerSm, cudaStream_t stream, const Job& job, bool slow, const LevelTables& T0,
+	const LevelTables& T1, uint8_t* staged)
 {
 	if (staged && kVariants[slot].staged)
 	{
-		const Stages sg = SplitStaged(staged, job.total);
+		const Stages sg = SplitStaged(staged, job.total, slot != kVariantMixed);
 		const cudaError_t e = cudaMemsetAsync(staged, 0, kStagedZeroed, stream);
 		if (e != cudaSuccess)
 			return e;
-		return kVariants[slot].staged(grid, stream, job, sg, T0, T1);
+		/* its passes size their own grids: all resident CTAs at most */
+		const int resident = GridForSlotCap(1 << 30, slot, ctasPerSm);
+		if (resident <= 0)
+			return cudaErrorUnknown;
+		return kVariants[slot].staged(resident, stream, job, sg, slow, T0, T1);
 	}
 	return kVariants[slot].launch(grid, stream, job, T0, T1);
 }
@@ -475,7 +473,7 @@ int LaunchEncode(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long lo
 	}
 	const int slot = VariantSlot(s);
 	uint8_t* staged = SlotStaged(slot) ? scratch + ((EncodeScratchBytes(nblocks, wantSums) + 255) & ~size_t(255)) : nullptr;
-	CK(LaunchSlot(slot, grid, stream, job, *T, *T, staged));
+	CK(LaunchSlot(slot, grid, 0, stream, job, s.doSlow != 0, *T, *T, staged));
 
 	int rc = NEBC7_OK;
 	if (wantSums)
@@ -680,6 +678,7 @@ struct BatchGroup
 	int queueBase;            /* offset of its queue positions in the results */
 	int total;                /* blocks */
 	int grid;
+	bool slow;                /* some texture asks for the /slow passes */
 	long long stagedOff;      /* its staged-encode records in the batch's staged area, or -1 */
 	long long orderOff;       /* its block-order scratch in the batch's order area */
 };
@@ -768,6 +767,7 @@ void BuildSchedule(nebc7_batch* b, int which)
 			g.queueBase = queue;
 			g.total = 0;
 			g.grid = 0;
+			g.slow = false;
 			g.stagedOff = -1;
 			g.orderOff = 0;
 			S.groups.push_back(g);
@@ -789,6 +789,7 @@ void BuildSchedule(nebc7_batch* b, int which)
 		d.P = MakeParams(t.settings);
 		S.table.push_back(d);
 		g.ntex++;
+		g.slow = g.slow || t.settings.doSlow;
 		g.total += d.nblocks;
 		queue += d.nblocks;
 	}
@@ -855,7 +856,7 @@ int EnqueueSchedule(nebc7_batch* b, int which, cudaStream_t st)
 			CK(cudaGetLastError());
 		}
 		job.order = order;
-		CK(LaunchSlot(G.slot, G.grid, gs, job, *b->T[0], *b->T[1],
+		CK(LaunchSlot(G.slot, G.grid, b->ctasPerSm, gs, job, G.slow, *b->T[0], *b->T[1],
 			(b->staged && G.stagedOff >= 0) ? b->stagedArea + G.stagedOff : nullptr));
 	}
 	if (ng > 1)
@@ -1162,10 +1163,13 @@ int LaunchServerBatch(nebc7_server* sv, ServerSlot& slot, std::vector<int64_t>& 
 	/* a batch of heavy requests takes the staged form (one kernel per pass);
 	   a batch of light ones the single kernel, whose blocks and so whose
 	   requests finish as they go */
-	bool heavy = total <= slot.stagedCap;
+	bool heavy = total <= slot.stagedCap, slow = false;
 	for (int64_t id : batch)
+	{
 		heavy = heavy && HeavyRequest(sv->reqs[id]);
-	CK(LaunchSlot(kVariantMixed, grid, st, job, *sv->T[0], *sv->T[1], heavy ? slot.staged : nullptr));
+		slow = slow || sv->reqs[id].settings.doSlow;
+	}
+	CK(LaunchSlot(kVariantMixed, grid, 0, st, job, slow, *sv->T[0], *sv->T[1], heavy ? slot.staged : nullptr));
 	CK(cudaEventRecord(slot.done, st));
 	slot.stage.assign(batch.size(), 0);
 	return NEBC7_OK;
@@ -1705,7 +1709,7 @@ int nebc7_encode_kernels(const nebc7_settings* settings)
 	if (int e = ValidateSettings(settings))
 		return -SetError(e);
 	const int order = OrdersBlocks(*settings) ? 2 : 0;
-	return order + (SlotStaged(VariantSlot(*settings)) ? StagedLaunches() : 1);
+	return order + (SlotStaged(VariantSlot(*settings)) ? StagedLaunches(settings->doSlow != 0) : 1);
 }
 
 int nebc7_init_device(int denoise)
@@ -2019,7 +2023,7 @@ int nebc7_batch_info(const nebc7_batch* b, int* schedule, int* launches, int* bl
 		   first kernel, then a list and a kernel per stage), the sums */
 		int n = 0;
 		for (const BatchGroup& g : b->sched[b->chosen].groups)
-			n += 2 + ((b->staged && g.stagedOff >= 0) ? 1 + 2 * kNumStages : 1) + 1;
+			n += 2 + ((b->staged && g.stagedOff >= 0) ? StagedLaunches(g.slow) : 1) + 1;
 		*launches = n;
 	}
 	if (blocks)
