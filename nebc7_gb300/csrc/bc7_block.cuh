@@ -329,8 +329,16 @@ __device__ inline void DecodeBlock(uint64_t lo, uint64_t hi, int pix, uint8_t ou
    the header in every lane. */
 __device__ inline void DecodeToState(WarpState& st, uint64_t lo, uint64_t hi, Ep best[3], int& param, int& mode, int lane)
 {
-	uint8_t px[4];
-	DecodeBlock(lo, hi, lane & 15, px, best, param, mode);
+	uint8_t px[4] = { 0, 0, 0, 0 };
+	if (lo == 64 && hi == 0)
+	{
+		/* the zero mode 6 block of an encode from scratch */
+		best[0] = best[1] = best[2] = 0;
+		param = 0;
+		mode = 6;
+	}
+	else
+		DecodeBlock(lo, hi, lane & 15, px, best, param, mode);
 	if (lane < 16)
 	{
 		st.dec[lane][0] = px[0];
@@ -383,9 +391,14 @@ __device__ __forceinline__ double SsimRatio(int sasb, int sab, int sasa_sbsb, in
 	return __ddiv_rn(num, den);
 }
 
+/* Double precision is what bounds this: an instruction takes an SM 16 cycles,
+   and the four channels' ratios one after another were most of a draft
+   encode's time.  Lane c computes channel c's, and callers ask for the values
+   only when the launch collects them. */
 __device__ inline void CompareBlocksSSIM(const WarpState& st, const Params& P, int lane, double& alpha, double& color)
 {
-	double r[4];
+	int sasb = 0, vab = 0, sasa_sbsb = 0, vaa = 0;
+#pragma unroll
 	for (int c = 0; c < 4; c++)
 	{
 		unsigned t = 0, s = 0;
@@ -399,15 +412,20 @@ __device__ inline void CompareBlocksSSIM(const WarpState& st, const Params& P, i
 		const unsigned sb = __reduce_add_sync(kFull, s);
 		const unsigned sab = __reduce_add_sync(kFull, t * s);
 		const unsigned saa_sbb = __reduce_add_sync(kFull, t * t + s * s);
-		unsigned vab = sab << 5;
-		unsigned vaa = saa_sbb << 4;
-		unsigned sasb = sa * sb;
-		sasb += sasb;
-		const unsigned sasa_sbsb = sa * sa + sb * sb;
-		vab -= sasb;
-		vaa -= sasa_sbsb;
-		r[c] = SsimRatio(int(sasb), int(vab), int(sasa_sbsb), int(vaa));
+		if ((lane & 3) == c)
+		{
+			const unsigned ab = 2 * (sa * sb), aabb = sa * sa + sb * sb;
+			sasb = int(ab);
+			vab = int((sab << 5) - ab);
+			sasa_sbsb = int(aabb);
+			vaa = int((saa_sbb << 4) - aabb);
+		}
 	}
+	const double mine = SsimRatio(sasb, vab, sasa_sbsb, vaa);
+	double r[4];
+#pragma unroll
+	for (int c = 0; c < 4; c++)
+		r[c] = __shfl_sync(kFull, mine, c);
 	const double ssim = __dadd_rn(__dadd_rn(__dmul_rn(r[1], double(P.wG)), __dmul_rn(r[2], double(P.wR))), __dmul_rn(r[3], double(P.wB)));
 	alpha = r[0];
 	color = __ddiv_rn(ssim, double(P.wColor));
@@ -607,11 +625,10 @@ static __device__ NEBC7_SHARED AreaInfo AreaStats(const WarpState& st, const Cel
 	const bool fast = (R.visible == 0xFFFF) && R.opaque;
 	if (!fast && a.active < a.count)
 		m0[0] = 0;
-	for (int i = 0; i < 16; i++)
+	for (uint32_t rest = vis; rest; rest &= rest - 1)
 	{
-		if (!((vis >> i) & 1))
-			continue;
-		const int v0 = st.px[i][0], v1 = st.px[i][1], v2 = st.px[i][2], v3 = st.px[i][3];
+		const ushort4 px = *reinterpret_cast<const ushort4*>(st.px[__ffs(rest) - 1]);
+		const int v0 = px.x, v1 = px.y, v2 = px.z, v3 = px.w;
 		const int v[4] = { v0, v1, v2, v3 };
 		for (int c = 0; c < 4; c++)
 		{
@@ -776,11 +793,10 @@ __device__ int SubsetErrorMask(const WarpState& st, uint32_t activeMask, Ep ep, 
 	LevelSet<BITS> L;
 	L.Init(ep);
 	int sum = 0;
-	for (int i = 0; i < 16; i++)
+	for (uint32_t rest = activeMask; rest; rest &= rest - 1)
 	{
-		if (!((activeMask >> i) & 1))
-			continue;
-		const int p0 = st.px[i][0], p1 = st.px[i][1], p2 = st.px[i][2], p3 = st.px[i][3];
+		const ushort4 px = *reinterpret_cast<const ushort4*>(st.px[__ffs(rest) - 1]);
+		const int p0 = px.x, p1 = px.y, p2 = px.z, p3 = px.w;
 		int best = 0x7FFFFFFF;
 #pragma unroll
 		for (int k = 0; k < (1 << BITS); k++)
@@ -795,14 +811,43 @@ __device__ int SubsetErrorMask(const WarpState& st, uint32_t activeMask, Ep ep, 
 	return sum;
 }
 
+/* SubsetErrorMask over the whole block for the whole warp: a pixel per lane
+   (with 16 levels, half of them: the other half on the lane 16 further). */
+template<int kD, int BITS>
+__device__ __forceinline__ int BlockErrorWarp(const WarpState& st, uint32_t activeMask, Ep ep, const int w[4], int lane)
+{
+	constexpr int L = BITS == 4 ? 8 : 1 << BITS;
+	const ushort4 px = *reinterpret_cast<const ushort4*>(st.px[lane & 15]);
+	const int p[4] = { px.x, px.y, px.z, px.w };
+	const bool upper = BITS == 4 && lane >= 16;
+	int best = 0x7FFFFFFF;
+#pragma unroll
+	for (int k = 0; k < L; k++)
+	{
+		const int wk = upper ? InterpWeights(BITS)[8 + k] : InterpWeights(BITS)[k];
+		int e = 0;
+#pragma unroll
+		for (int c = 0; c < 4; c++)
+		{
+			const int q = Q<kD>(p[c] - Interp(EpGet(ep, 2 * c), EpGet(ep, 2 * c + 1), wk));
+			e += w[c] * q * q;
+		}
+		best = min(best, e);
+	}
+	if (BITS == 4)
+		best = min(best, __shfl_xor_sync(kFull, best, 16));
+	return int(__reduce_add_sync(kFull, lane < 16 && ((activeMask >> lane) & 1) ? unsigned(best) : 0u));
+}
+
 /* Mode 4/5 error with separate color and alpha-slot indices
    (src/Bc7CoreMode4.cpp:159-839, src/Bc7CoreMode5.cpp:143-401): pixels are
    the Area1 view (transparent pixels with zero data and an alpha-only
    mask); mode 4 visits the visible pixels and adds (16 - active) times the
    alpha error of the lower alpha endpoint, mode 5 visits all 16.
-   `epImg` in image channel order. */
-template<int kD, int CB, int AB, bool MODE4>
-__device__ int RotErrorExact(const WarpState& st, const CellRegs& R, Ep epImg, int rotation, const int w[4])
+   `epImg` in image channel order.  Part `part` of PARTS: every PARTS-th
+   pixel; the error is the parts' sum. */
+template<int kD, int CB, int AB, bool MODE4, int PARTS>
+__device__ int RotErrorExact(const WarpState& st, const CellRegs& R, Ep epImg, int rotation, const int w[4], int part)
 {
 	const int a = RotChannel(rotation);
 	LevelSet<CB> LC;
@@ -810,7 +855,7 @@ __device__ int RotErrorExact(const WarpState& st, const CellRegs& R, Ep epImg, i
 	LC.Init(epImg);
 	LA.Init(epImg);
 	int sum = 0;
-	for (int i = 0; i < 16; i++)
+	for (int i = part; i < 16; i += PARTS)
 	{
 		const bool vis = (R.visible >> i) & 1;
 		if (MODE4 && !vis)
@@ -850,7 +895,7 @@ __device__ int RotErrorExact(const WarpState& st, const CellRegs& R, Ep epImg, i
 		}
 		sum += besta + bestc;
 	}
-	if (MODE4 && R.a1.active < 16)
+	if (MODE4 && R.a1.active < 16 && part == 0)
 	{
 		const int m = min(EpGet(epImg, 0), EpGet(epImg, 1));
 		const int q = Q<kD>(m);

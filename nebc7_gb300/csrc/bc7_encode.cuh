@@ -86,15 +86,15 @@ __device__ __forceinline__ void DraftChain(WarpState& st, CellRegs& R, const Par
 		/* the "Mode6Index2 fast" run: the draft chain reduced to its
 		   first pass (no counterpart in the reference) */
 		if (R.errTotal > step && (kD > 0 || P.denoiseStep > 0))
-			FastMode6<kD, true>(st, R, P, T);
+			FastMode6<kD, true>(st, R, P, T, lane);
 	}
 	else if (R.errTotal > step)
 	{
 		if (kD > 0 || P.denoiseStep > 0)
-			FastMode6<kD, true>(st, R, P, T);
+			FastMode6<kD, true>(st, R, P, T, lane);
 		if (R.errTotal > step)
 		{
-			FastMode6<kD, false>(st, R, P, T);
+			FastMode6<kD, false>(st, R, P, T, lane);
 			if (R.errTotal > step)
 			{
 				FastRot<kD, 4>(st, R, P, lane);
@@ -287,7 +287,8 @@ __device__ void EncodeBlockAt(WarpState& st, SearchState* ss, const BlockRef& b,
 			lo = savedLo;
 			hi = savedHi;
 		}
-		CompareBlocksSSIM(st, P, lane, qa, qc);
+		if (b.result)
+			CompareBlocksSSIM(st, P, lane, qa, qc);
 	}
 
 	if (lane == 0)

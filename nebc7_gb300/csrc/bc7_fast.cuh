@@ -309,31 +309,33 @@ __device__ NEBC7_ONCE void FastMode7(WarpState& st, CellRegs& R, const Params& P
 template<int kD, int MODE>
 __device__ NEBC7_ONCE void FastRot(WarpState& st, CellRegs& R, const Params& P, int lane)
 {
-	constexpr int NR = MODE == 4 ? 8 : 4;
+	constexpr int NR = MODE == 4 ? 8 : 4, PARTS = 32 / NR;
 	const int step = R.denoiseStep;
 	const int w[4] = { P.wA, P.wG, P.wR, P.wB };
-	Ep mine = 0;
-	if (lane < NR)
+	/* lane = choice + NR * part of the pixels */
+	const int choice = lane & (NR - 1), part = lane / NR;
+	const int rotation = MODE == 4 ? c_rot4[choice] : c_rot5[choice];
+	Ep mine;
+	int e;
+	if (MODE == 4)
 	{
-		const int rotation = MODE == 4 ? c_rot4[lane] : c_rot5[lane];
-		int e;
-		if (MODE == 4)
-		{
-			mine = QuantMode4(R.a1.bounds, rotation);
-			const Ep img = EpSwapRot(mine, rotation);
-			if (rotation & 4)
-				e = RotErrorExact<kD, 3, 2, true>(st, R, img, rotation, w);
-			else
-				e = RotErrorExact<kD, 2, 3, true>(st, R, img, rotation, w);
-		}
+		mine = QuantMode4(R.a1.bounds, rotation);
+		const Ep img = EpSwapRot(mine, rotation);
+		if (rotation & 4)
+			e = RotErrorExact<kD, 3, 2, true, PARTS>(st, R, img, rotation, w, part);
 		else
-		{
-			mine = QuantMode5(R.a1.bounds, rotation);
-			const Ep img = EpSwapRot(mine, rotation);
-			e = RotErrorExact<kD, 2, 2, false>(st, R, img, rotation, w);
-		}
-		st.scan[lane] = step + e;
+			e = RotErrorExact<kD, 2, 3, true, PARTS>(st, R, img, rotation, w, part);
 	}
+	else
+	{
+		mine = QuantMode5(R.a1.bounds, rotation);
+		const Ep img = EpSwapRot(mine, rotation);
+		e = RotErrorExact<kD, 2, 2, false, PARTS>(st, R, img, rotation, w, part);
+	}
+	for (int o = NR; o < 32; o <<= 1)
+		e += __shfl_xor_sync(kFull, e, o);
+	if (lane < NR)
+		st.scan[lane] = step + e;
 	__syncwarp();
 	int T = R.errTotal;
 	const int won = AcceptScan(st, NR, T, step, step);
@@ -349,16 +351,16 @@ __device__ NEBC7_ONCE void FastRot(WarpState& st, CellRegs& R, const Params& P, 
 
 /* Modes 6 and 6Index2: one candidate. */
 template<int kD, bool INDEX2>
-__device__ NEBC7_ONCE void FastMode6(WarpState& st, CellRegs& R, const Params& P, const LevelTables& T)
+__device__ NEBC7_ONCE void FastMode6(WarpState& st, CellRegs& R, const Params& P, const LevelTables& T, int lane)
 {
 	const int step = R.denoiseStep;
 	const int w[4] = { P.wA, P.wG, P.wR, P.wB };
 	const Ep ep = QuantMode6(R.a1.bounds);
 	int E = step;
 	if (INDEX2)
-		E += TransparentError2(T, P, 16, R.a1.active, int(ep & 0xFFFF)) + SubsetErrorMask<kD, 2>(st, R.visible, ep, w);
+		E += TransparentError2(T, P, 16, R.a1.active, int(ep & 0xFFFF)) + BlockErrorWarp<kD, 2>(st, R.visible, ep, w, lane);
 	else
-		E += TransparentError4(T, P, 16, R.a1.active, int(ep & 0xFFFF)) + SubsetErrorMask<kD, 4>(st, R.visible, ep, w);
+		E += TransparentError4(T, P, 16, R.a1.active, int(ep & 0xFFFF)) + BlockErrorWarp<kD, 4>(st, R.visible, ep, w, lane);
 	if (E < R.errTotal)
 	{
 		R.errTotal = E - step;

@@ -467,7 +467,8 @@ __device__ __forceinline__ void FinishBlock(WarpState& st, CellRegs& R, const Pa
 		hi = startHi;
 	}
 	double qa = 1.0, qc = 1.0;
-	CompareBlocksSSIM(st, P, lane, qa, qc);
+	if (b.result)
+		CompareBlocksSSIM(st, P, lane, qa, qc);
 	StoreBlock<kD>(b, R, lo, hi, qa, qc, lane);
 }
 
@@ -525,17 +526,17 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 			/* the "Mode6Index2 fast" run: the draft chain reduced to its
 			   first pass (no counterpart in the reference) */
 			if (R.errTotal > step && (kD > 0 || P.denoiseStep > 0))
-				FastMode6<kD, true>(st, R, P, T);
+				FastMode6<kD, true>(st, R, P, T, lane);
 		}
 		else
 		{
 			if (R.errTotal > step)
 			{
 				if (kD > 0 || P.denoiseStep > 0)
-					FastMode6<kD, true>(st, R, P, T);
+					FastMode6<kD, true>(st, R, P, T, lane);
 				if (R.errTotal > step)
 				{
-					FastMode6<kD, false>(st, R, P, T);
+					FastMode6<kD, false>(st, R, P, T, lane);
 					if (R.errTotal > step)
 						n = kStepDraftRot;
 				}
