@@ -12,24 +12,125 @@
 
 namespace nebc7 {
 
-/* Edge replication of a w x h BGRA image to the padded pw x ph texture:
-   columns past w repeat column w - 1, rows past h repeat row h - 1. */
-__global__ void KPadTexture(const uint8_t* src, long long srcStride, int w, int h, uint8_t* dst, long long dstStride, int pw,
-	int ph)
+/* Four pixels of a row; by 16-byte reads and writes when the buffers allow
+   them (WIDE), else by 4-byte ones. */
+template<bool WIDE>
+__device__ __forceinline__ uint4 LoadRow(const uint8_t* p)
 {
-	const int x = blockIdx.x * blockDim.x + threadIdx.x;
-	const int y = blockIdx.y;
-	if (x >= pw || y >= ph)
-		return;
-	const int sx = x < w ? x : w - 1;
-	const int sy = y < h ? y : h - 1;
-	*reinterpret_cast<uint32_t*>(dst + y * dstStride + x * 4) =
-		*reinterpret_cast<const uint32_t*>(src + sy * srcStride + sx * 4);
+	if (WIDE)
+		return *reinterpret_cast<const uint4*>(p);
+	const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
+	return make_uint4(q[0], q[1], q[2], q[3]);
 }
 
-/* Alpha mask with an outline: bytes A, G, R, B of a pixel are 0xFF, and G,
+template<bool WIDE>
+__device__ __forceinline__ void StoreRow(uint8_t* p, uint4 v)
+{
+	if (WIDE)
+	{
+		*reinterpret_cast<uint4*>(p) = v;
+		return;
+	}
+	uint32_t* q = reinterpret_cast<uint32_t*>(p);
+	q[0] = v.x;
+	q[1] = v.y;
+	q[2] = v.z;
+	q[3] = v.w;
+}
+
+/* Edge replication of a w x h BGRA image to the padded pw x ph texture:
+   columns past w repeat column w - 1, rows past h repeat row h - 1.  MASK: also
+   the alpha mask with an outline: bytes A, G, R, B of a pixel are 0xFF, and G,
    R, B are 0xFF only if some pixel of the (2 radius + 1)^2 window around it
-   (clipped to the texture) has non-zero alpha.  radius < 0: all 0xFF. */
+   (clipped to the texture) has non-zero alpha; 0 <= radius <= kOutlineRadius.
+   A CTA makes 256 x kPadRows pixels, four a thread, and reads each source
+   pixel once, with the window's border; a row of 32 pixels' alpha is one word,
+   the window the OR of 2 radius + 1 rows and a few shifts.  Memory bound; the
+   window test per pixel read every pixel up to nine times more, from memory. */
+constexpr int kPadRows = 16;
+constexpr int kOutlineRadius = 31;
+
+/* Shared bytes of a mask tile: a nibble byte per four pixels, ten words a
+   row (eight and one to each side), the outlined words. */
+constexpr size_t PadSharedBytes(int radius)
+{
+	return size_t(kPadRows + 2 * radius) * (80 + 40) + kPadRows * 32;
+}
+
+template<bool MASK, bool WIDE>
+__global__ void __launch_bounds__(256) KPadTexture(const uint8_t* src, long long srcStride, int w, int h, uint8_t* dst, long long dstStride, int pw,
+	int ph, int radius, uint8_t* mask)
+{
+	extern __shared__ __align__(16) uint8_t padTile[];
+	const int x0 = blockIdx.x * 256, y0 = blockIdx.y * kPadRows;
+	const int border = MASK ? radius : 0, rows = kPadRows + 2 * border;
+	constexpr int side = MASK ? 8 : 0, quads = 64 + 2 * side;   /* of four pixels; `side` to each side for the border */
+	uint8_t* const nibbles = padTile;
+	uint32_t* const words = reinterpret_cast<uint32_t*>(padTile + rows * 80);
+	uint32_t* const outlined = words + rows * 10;
+	for (int i = threadIdx.x; i < rows * quads; i += 256)
+	{
+		const int row = i / quads, q = i - row * quads - side;
+		const int x = x0 + 4 * q, y = y0 + row - border;
+		uint4 v = make_uint4(0, 0, 0, 0);
+		if (x >= 0 && x < pw && y >= 0 && y < ph)
+		{
+			const uint8_t* p = src + (long long)min(y, h - 1) * srcStride;
+			v.x = *reinterpret_cast<const uint32_t*>(p + (long long)min(x, w - 1) * 4);
+			v.y = *reinterpret_cast<const uint32_t*>(p + (long long)min(x + 1, w - 1) * 4);
+			v.z = *reinterpret_cast<const uint32_t*>(p + (long long)min(x + 2, w - 1) * 4);
+			v.w = *reinterpret_cast<const uint32_t*>(p + (long long)min(x + 3, w - 1) * 4);
+			if (!MASK || (q >= 0 && q < 64 && row >= border && row < border + kPadRows))
+				StoreRow<WIDE>(dst + y * dstStride + (long long)x * 4, v);
+		}
+		if (MASK)
+			nibbles[i] = uint8_t(int((v.x >> 24) != 0) | int((v.y >> 24) != 0) << 1 | int((v.z >> 24) != 0) << 2 | int((v.w >> 24) != 0) << 3);
+	}
+	if (!MASK)
+		return;
+	__syncthreads();
+	for (int i = threadIdx.x; i < rows * 10; i += 256)
+	{
+		const uint2 n = reinterpret_cast<const uint2*>(nibbles)[i];
+		auto pack = [](uint32_t v) { return (v & 0xF) | ((v >> 4) & 0xF0) | ((v >> 8) & 0xF00) | ((v >> 12) & 0xF000); };
+		words[i] = pack(n.x) | (pack(n.y) << 16);
+	}
+	__syncthreads();
+	if (threadIdx.x < kPadRows * 8)
+	{
+		const uint32_t* p = words + (threadIdx.x >> 3) * 10 + 1 + (threadIdx.x & 7);
+		uint32_t a = 0, m = 0, b = 0;
+		for (int r = 0; r <= 2 * border; r++, p += 10)
+		{
+			a |= p[-1];
+			m |= p[0];
+			b |= p[1];
+		}
+		/* smeared by 0 .. radius pixels to each side */
+		uint64_t left = (uint64_t(m) << 32) | a, right = (uint64_t(b) << 32) | m;
+		for (int done = 0; done < border;)
+		{
+			const int step = min(done + 1, border - done);
+			left |= left << step;
+			right |= right >> step;
+			done += step;
+		}
+		outlined[threadIdx.x] = uint32_t(left >> 32) | uint32_t(right);
+	}
+	__syncthreads();
+	for (int i = threadIdx.x; i < kPadRows * 64; i += 256)
+	{
+		const int row = i >> 6, q = i & 63;
+		const int x = x0 + 4 * q, y = y0 + row;
+		if (x >= pw || y >= ph)
+			continue;
+		const uint32_t n = outlined[row * 8 + (q >> 3)] >> ((q & 7) * 4);
+		auto pixel = [&](int j) { return (n >> j) & 1 ? 0xFFFFFFFFu : 0x000000FFu; };
+		StoreRow<WIDE>(mask + y * dstStride + (long long)x * 4, make_uint4(pixel(0), pixel(1), pixel(2), pixel(3)));
+	}
+}
+
+/* The mask alone, for any radius; radius < 0: all 0xFF. */
 __global__ void KOutlineMask(const uint8_t* tex, long long stride, int pw, int ph, int radius, uint8_t* mask)
 {
 	const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -55,35 +156,40 @@ __global__ void KOutlineMask(const uint8_t* tex, long long stride, int pw, int p
 /* Glitch map: a block whose decoded pixels differ from the source by at
    least the threshold in some masked channel (A 16, G 12, R 16, B 20;
    16 each with linear weights) keeps its source pixels, any other block is
-   cleared.  One thread per pixel; the block's verdict by warp vote over its
-   16 pixels (a warp holds two blocks side by side). */
-__global__ void KBadBlocks(const uint8_t* src, const uint8_t* dec, const uint8_t* mask, long long stride, int w, int h, int linear,
+   cleared.  A thread takes a row of a block; a warp eight blocks side by side
+   (128 contiguous bytes of each of their four rows), the block's verdict by
+   vote over its four lanes.  Memory bound: three images in, one out. */
+template<bool WIDE>
+__global__ void __launch_bounds__(256) KBadBlocks(const uint8_t* src, const uint8_t* dec, const uint8_t* mask, long long stride, int w, int h, int linear,
 	uint8_t* out)
 {
-	const int bx = blockIdx.x * 2 + (threadIdx.x >> 4);
+	const int lane = threadIdx.x & 31;
+	const int bx = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8 + (lane & 7);
 	const int by = blockIdx.y;
-	const int i = threadIdx.x & 15;
-	const bool in = bx * 4 < w && by * 4 < h;
-	const long long off = (long long)(by * 4 + (i >> 2)) * stride + (bx * 4 + (i & 3)) * 4;
+	const bool in = bx * 4 < w;
+	const long long off = (long long)(by * 4 + (lane >> 3)) * stride + (long long)bx * 16;
 	bool bad = false;
-	uint32_t s = 0;
+	uint4 s = make_uint4(0, 0, 0, 0);
 	if (in)
 	{
-		s = *reinterpret_cast<const uint32_t*>(src + off);
-		const uint32_t d = *reinterpret_cast<const uint32_t*>(dec + off);
-		const uint32_t m = mask ? *reinterpret_cast<const uint32_t*>(mask + off) : 0xFFFFFFFFu;
-		/* BGRA bytes; mask bytes are A, G, R, B */
+		s = LoadRow<WIDE>(src + off);
+		const uint4 d = LoadRow<WIDE>(dec + off);
+		uint4 m = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+		if (mask)
+			m = LoadRow<WIDE>(mask + off);
 		const int thrB = linear ? 16 : 20, thrG = linear ? 16 : 12, thrR = 16, thrA = 16;
-		const int chB = abs(int(s & 0xFF) - int(d & 0xFF)) & int(m >> 24);
-		const int chG = abs(int((s >> 8) & 0xFF) - int((d >> 8) & 0xFF)) & int((m >> 8) & 0xFF);
-		const int chR = abs(int((s >> 16) & 0xFF) - int((d >> 16) & 0xFF)) & int((m >> 16) & 0xFF);
-		const int chA = abs(int(s >> 24) - int(d >> 24)) & int(m & 0xFF);
-		bad = chB >= thrB || chG >= thrG || chR >= thrR || chA >= thrA;
+		auto glitch = [&](uint32_t s, uint32_t d, uint32_t m) {
+			/* BGRA bytes; mask bytes are A, G, R, B */
+			const uint32_t a = __vabsdiffu4(s, d);
+			const int chB = int(a & 0xFF) & int(m >> 24), chG = int((a >> 8) & 0xFF) & int((m >> 8) & 0xFF);
+			const int chR = int((a >> 16) & 0xFF) & int((m >> 16) & 0xFF), chA = int(a >> 24) & int(m & 0xFF);
+			return chB >= thrB || chG >= thrG || chR >= thrR || chA >= thrA;
+		};
+		bad = glitch(s.x, d.x, m.x) || glitch(s.y, d.y, m.y) || glitch(s.z, d.z, m.z) || glitch(s.w, d.w, m.w);
 	}
 	const unsigned votes = __ballot_sync(0xFFFFFFFFu, bad);
-	const bool blockBad = (votes >> (threadIdx.x & 16)) & 0xFFFF;
 	if (in)
-		*reinterpret_cast<uint32_t*>(out + off) = blockBad ? s : 0u;
+		StoreRow<WIDE>(out + off, ((votes >> (lane & 7)) & 0x01010101u) ? s : make_uint4(0, 0, 0, 0));
 }
 
 /* Partition map: every block keeps its mode and partition (or rotation)

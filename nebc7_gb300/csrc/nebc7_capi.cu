@@ -1653,8 +1653,8 @@ int nebc7_decode_device(const uint8_t* d_blocks, uint8_t* d_bgra, long long stri
 	if (w <= 0 || h <= 0 || (w & 3) || (h & 3) || stride < (long long)w * 4 || (stride & 3) || ((uintptr_t)d_blocks & 15))
 		return SetError(NEBC7_EINVAL);
 	const long long nb = (long long)(w / 4) * (h / 4);
-	const long long threads = nb * 16;
-	KDecode<<<unsigned((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_blocks, d_bgra, stride, w / 4, int(nb));
+	const bool wide = !(((uintptr_t)d_bgra | (uintptr_t)stride) & 15);
+	KDecode<<<unsigned((nb + 127) / 128), 128, 0, (cudaStream_t)stream>>>(d_blocks, d_bgra, stride, w / 4, int(nb), wide);
 	CK(cudaGetLastError());
 	return NEBC7_OK;
 }
@@ -2208,14 +2208,19 @@ int nebc7_prepare_device(const uint8_t* d_src, long long src_stride, int w, int 
 	if (std::max(pw, ph) > 16384)
 		return SetError(NEBC7_ETOOBIG);
 	const cudaStream_t st = (cudaStream_t)stream;
-	const dim3 grid((pw + 255) / 256, ph);
-	KPadTexture<<<grid, 256, 0, st>>>(d_src, src_stride, w, h, d_padded, (long long)pw * 4, pw, ph);
-	CK(cudaGetLastError());
-	if (d_mask)
+	const dim3 tiles((pw + 255) / 256, (ph + kPadRows - 1) / kPadRows);
+	const bool wide = !(((uintptr_t)d_padded | (uintptr_t)d_mask) & 15);
+	if (d_mask && radius >= 0 && radius <= kOutlineRadius)
+		(wide ? KPadTexture<true, true> : KPadTexture<true, false>)<<<tiles, 256, PadSharedBytes(radius), st>>>(d_src, src_stride, w, h, d_padded,
+			(long long)pw * 4, pw, ph, radius, d_mask);
+	else
 	{
-		KOutlineMask<<<grid, 256, 0, st>>>(d_padded, (long long)pw * 4, pw, ph, radius, d_mask);
-		CK(cudaGetLastError());
+		(wide ? KPadTexture<false, true> : KPadTexture<false, false>)<<<tiles, 256, 0, st>>>(d_src, src_stride, w, h, d_padded,
+			(long long)pw * 4, pw, ph, 0, nullptr);
+		if (d_mask)
+			KOutlineMask<<<dim3((pw + 255) / 256, ph), 256, 0, st>>>(d_padded, (long long)pw * 4, pw, ph, radius, d_mask);
 	}
+	CK(cudaGetLastError());
 	return NEBC7_OK;
 }
 
@@ -2225,8 +2230,9 @@ int nebc7_bad_blocks_device(const uint8_t* d_src, const uint8_t* d_decoded, cons
 	if (!d_src || !d_decoded || !d_out || w <= 0 || h <= 0 || (w & 3) || (h & 3) || stride < (long long)w * 4 || (stride & 3) ||
 		((uintptr_t)d_src & 3) || ((uintptr_t)d_decoded & 3) || ((uintptr_t)d_mask & 3) || ((uintptr_t)d_out & 3))
 		return SetError(NEBC7_EINVAL);
-	const dim3 grid((w / 4 + 1) / 2, h / 4);
-	KBadBlocks<<<grid, 32, 0, (cudaStream_t)stream>>>(d_src, d_decoded, d_mask, stride, w, h, linear, d_out);
+	const bool wide = !(((uintptr_t)d_src | (uintptr_t)d_decoded | (uintptr_t)d_mask | (uintptr_t)d_out | (uintptr_t)stride) & 15);
+	const dim3 grid((w / 4 + 63) / 64, h / 4);
+	(wide ? KBadBlocks<true> : KBadBlocks<false>)<<<grid, 256, 0, (cudaStream_t)stream>>>(d_src, d_decoded, d_mask, stride, w, h, linear, d_out);
 	CK(cudaGetLastError());
 	return NEBC7_OK;
 }
