@@ -37,6 +37,15 @@ constexpr int kFar = 0x3FFFFFFF;
    padding, so that the pixels of a column lie in different banks. */
 constexpr int kTableRow = 21;
 
+/* The partitions of a three-subset search that its estimates leave. */
+struct __align__(16) ThreeEstimates
+{
+	int2 order[64];      /* (estimate, partition) */
+	int lines[64][2];    /* per partition, estimates of subsets 2 and 3 */
+	int est[64][3][3];   /* per partition, subset, channel (G, R, B) estimates */
+	int count;
+};
+
 /* Per-warp search state.  The staged kernels reserve only the bytes up to the
    last member their pass uses (SearchBytes), so that more of the SM's memory
    is L1. */
@@ -50,13 +59,7 @@ struct __align__(16) SearchState
 	int2 lists[4][4][32];    /* [p-bit variant][channel][entry] = (error, color) */
 	union
 	{
-		struct
-		{
-			int2 order[64];      /* (estimate, partition) */
-			int lines[64][2];    /* per partition, estimates of subsets 2 and 3 */
-			int est[64][3][3];   /* per partition, subset, channel (G, R, B) estimates */
-			int count;
-		} three;                 /* the three-subset searches */
+		ThreeEstimates three;         /* the three-subset searches */
 		int4 table[16 * kTableRow];   /* four channels, 2-bit indices: R's terms, [pixel][candidate] */
 		int plane16[3][256];          /* four channels, 4-bit indices: planes of 16 levels */
 	};
@@ -396,6 +399,44 @@ struct PlaneLanes
 /* Three channels with one index (src/Bc7CoreMode0.cpp:242-415; modes 4, 5) */
 /* ---------------------------------------------------------------------- */
 
+/* What the warps of a team share of one combination search: the smallest
+   error found so far with its place in the search's order (error << 32 |
+   variant, four list indices; three channels use the last three), and the next unit of each variant. */
+struct TeamSearch
+{
+	unsigned long long key;
+	int next[4];
+};
+
+/* Place of a combination in the search's order. */
+__device__ __forceinline__ unsigned SearchPlace(int v, int i0, int i1, int i2, int i3)
+{
+	return unsigned(((((v << 5 | i0) << 5 | i1) << 5 | i2) << 5) | i3);
+}
+
+/* What a team shares of a block's search. */
+struct TeamState
+{
+	TeamSearch search;
+	TeamExchange exchange;
+	int bound[2][4];       /* [subset][channel] estimates */
+	int valid;             /* variants whose lists leave room */
+	int task[3];           /* the CTA's task: queue position, candidate, first improvement */
+};
+
+/* Starts a team's search from `water`; the last one's outcome is read. */
+__device__ __forceinline__ void StartTeamSearch(TeamState& ts, int water)
+{
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		ts.search.key = (unsigned long long)(unsigned(water)) << 32;
+		ts.search.next[0] = ts.search.next[1] = ts.search.next[2] = ts.search.next[3] = 0;
+		ts.valid = 0;
+	}
+	__syncthreads();
+}
+
 /* One channel's sorted candidate list in a search: its pixels' channel, its
    weight, and the list. */
 struct SearchChannel
@@ -421,9 +462,12 @@ struct Found3
    their alpha of 0 (x is then the alpha channel). */
 template<int kD, int IB>
 __device__ NEBC7_SHARED Found3 SearchThree(const Area& ar, int np, SearchChannel X, SearchChannel Y, SearchChannel Z, int hidden,
-	int water, int4* planes, int lane)
+	int water, int4* planes, const Team& team, TeamState* ts, int lane)
 {
 	Found3 f{ water, 0, 0, 0, 0 };
+	const bool shared = team.size > 1;
+	if (shared)
+		StartTeamSearch(*ts, water);
 	if (X.minErr + Y.minErr + Z.minErr >= water)
 		return f;
 	const int2 ly = lane < Y.n ? Y.list[lane] : make_int2(kFar, 0);
@@ -438,8 +482,26 @@ __device__ NEBC7_SHARED Found3 SearchThree(const Area& ar, int np, SearchChannel
 	pl.Pixels(ar, X.c, xx);
 	pl.Pixels(ar, Y.c, xy);
 	const int none[Lanes::N] = {};
-	for (int ix = 0; ix < X.n; ix++)
+	/* the error that a combination at (ix, iy) has to be below (SearchFour2) */
+	auto refresh = [&](int ix, int iy) {
+		if (shared)
+		{
+			const unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&ts->search.key);
+			water = int(k >> 32) + int(unsigned(k) > SearchPlace(0, 0, ix, iy, 31));
+		}
+	};
+	for (int ix = 0;; ix++)
 	{
+		if (shared)
+		{
+			int u = 0;
+			if (lane == 0)
+				u = atomicAdd(&ts->search.next[0], 1);
+			ix = __shfl_sync(kFull, u, 0);
+		}
+		if (ix >= X.n)
+			break;
+		refresh(ix, 0);
 		const int2 lx = X.list[ix];
 		if (lx.x + Y.minErr + Z.minErr >= water)
 			break;
@@ -472,6 +534,7 @@ __device__ NEBC7_SHARED Found3 SearchThree(const Area& ar, int np, SearchChannel
 			if (!first)
 			{
 				iy = __ffs(open) - 1;
+				refresh(ix, iy);
 				const int eXY = __shfl_sync(kFull, errXY, iy);
 				y = make_int2(__shfl_sync(kFull, ly.x, iy), __shfl_sync(kFull, ly.y, iy));
 				eval = lz.x + eXY < water && errXZ - 1 + y.x < water;
@@ -502,13 +565,30 @@ __device__ NEBC7_SHARED Found3 SearchThree(const Area& ar, int np, SearchChannel
 			const int low = __reduce_min_sync(kFull, err);
 			if (low < water)
 			{
+				const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
 				water = low;
-				f.taken = 1;
-				f.x = lx.y;
-				f.y = y.y;
-				f.z = __shfl_sync(kFull, lz.y, __ffs(__ballot_sync(kFull, err == low)) - 1);
+				if (!shared)
+				{
+					f.taken = 1;
+					f.x = lx.y;
+					f.y = y.y;
+					f.z = __shfl_sync(kFull, lz.y, j);
+				}
+				else if (lane == 0)
+					atomicMin(&ts->search.key, (unsigned long long)(unsigned(low)) << 32 | SearchPlace(0, 0, ix, iy, j));
 			}
 		}
+	}
+	if (shared)
+	{
+		__syncthreads();
+		const unsigned long long k = ts->search.key;
+		const unsigned place = unsigned(k);
+		water = int(k >> 32);
+		f.taken = water < f.water;
+		f.x = X.list[(place >> 10) & 31].y;
+		f.y = Y.list[(place >> 5) & 31].y;
+		f.z = Z.list[place & 31].y;
 	}
 	f.water = water;
 	return f;
@@ -561,16 +641,15 @@ __device__ __forceinline__ int ChannelWeight(const Params& P, int c)
    estB: lower bounds of the later channels' errors. */
 template<int kD>
 __device__ NEBC7_PASS bool InitLevels3(SearchState& ss, int v, const Area& ar, const Params& P, const Spec3& sp, bool pbit, int water,
-	int estR, int estB, int lane)
+	int estR, int estB, Team& team, int lane)
 {
-	Team one = SingleWarp();
 	int used = 0;
 #pragma unroll 1
 	for (int c = 1; c < 4; c++)
 	{
 		const int rest = c == 1 ? estR + estB : (c == 2 ? estB : 0);
 		const ChanList cl = ChannelLevels<kD, false>(ss.lists[v][c - 1], ar, c, ChannelWeight(P, c), water - used - rest, sp.bits,
-			pbit ? VariantPbits(v) : -1, false, sp.table, sp.byDiff, 32, ss.values, one, lane);
+			pbit ? VariantPbits(v) : -1, false, sp.table, sp.byDiff, 32, ss.values, team, lane);
 		if (lane == 0)
 			ss.chan[v][c - 1] = cl;
 		used += cl.minErr;
@@ -585,13 +664,13 @@ __device__ NEBC7_PASS bool InitLevels3(SearchState& ss, int v, const Area& ar, c
    the same water, then the variants are searched in order. */
 template<int kD, int MODE>
 __device__ NEBC7_PASS int SearchSubset3(SearchState& ss, const Area& ar, const Params& P, const Spec3& sp, int water, int estR, int estB,
-	Ep& best, bool& any, int lane)
+	Ep& best, bool& any, Team& team, TeamState* ts, int lane)
 {
 	constexpr int IB = (MODE == 0 || MODE == 1) ? 3 : 2;
 	int valid = 0;
 #pragma unroll 1
 	for (int v = 0; v < sp.variants; v++)
-		valid |= int(InitLevels3<kD>(ss, v, ar, P, sp, MODE != 2, water, estR, estB, lane)) << v;
+		valid |= int(InitLevels3<kD>(ss, v, ar, P, sp, MODE != 2, water, estR, estB, team, lane)) << v;
 	any = valid != 0;
 #pragma unroll 1
 	for (int v = 0; v < sp.variants; v++)
@@ -600,7 +679,7 @@ __device__ NEBC7_PASS int SearchSubset3(SearchState& ss, const Area& ar, const P
 			continue;
 		auto channel = [&](int c, int w) { return SearchChannel{ c, w, ss.lists[v][c - 1], ss.chan[v][c - 1].count, ss.chan[v][c - 1].minErr }; };
 		const Found3 f = SearchThree<kD, IB>(ar, ar.info.active, channel(1, P.wG), channel(2, P.wR), channel(3, P.wB), 0, water,
-			ss.plane, lane);
+			ss.plane, team, ts, lane);
 		water = f.water;
 		if (f.taken)
 			best = EpSetCh(Ep2(1, f.x, 2, f.y), 3, f.z);
@@ -623,7 +702,8 @@ __device__ NEBC7_PASS void BuildSubset(WarpState& st, const CellRegs& R, const P
 
 /* ModeN::CompressBlock for modes 0-3 (src/Bc7CoreMode0.cpp:417-498). */
 template<int kD, int MODE>
-__device__ NEBC7_PASS void RefineOpaque(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void RefineOpaque(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team,
+	TeamState* ts, int lane)
 {
 	constexpr int NS = (MODE == 0 || MODE == 2) ? 3 : 2;
 	constexpr int IB = (MODE == 0 || MODE == 1) ? 3 : 2;
@@ -642,7 +722,7 @@ __device__ NEBC7_PASS void RefineOpaque(WarpState& st, SearchState& ss, CellRegs
 			if (water)
 			{
 				bool any;
-				const int w2 = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, 0, 0, b, any, lane);
+				const int w2 = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, 0, 0, b, any, team, ts, lane);
 				if (any)
 				{
 					water = w2;
@@ -753,6 +833,7 @@ __device__ __forceinline__ bool ThreeSubsetsPartition(WarpState& st, SearchState
 {
 	Ep mc0 = 0, mc1 = 0, mc2 = 0;
 	int error = R.opaqueAlphaError;
+	Team one = SingleWarp();
 #pragma unroll 1
 	for (int s = 0; s < 3; s++)
 	{
@@ -761,7 +842,7 @@ __device__ __forceinline__ bool ThreeSubsetsPartition(WarpState& st, SearchState
 		BuildSubset<kD>(st, R, P, st.sub[0], 3, p, s, true, lane);
 		bool any;
 		Ep b = 0;
-		const int r = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, ss.three.est[p][s][1], ss.three.est[p][s][2], b, any, lane);
+		const int r = SearchSubset3<kD, MODE>(ss, st.sub[0], P, sp, water, ss.three.est[p][s][1], ss.three.est[p][s][2], b, any, one, nullptr, lane);
 		if (!any || !(r < water))
 			return false;
 		error += r;
@@ -781,26 +862,22 @@ __device__ __forceinline__ bool ThreeSubsetsPartition(WarpState& st, SearchState
 	return error <= R.opaqueAlphaError;
 }
 
-/* Full searches of modes 0 and 2 (src/Bc7CoreMode0.cpp:532-642,
-   src/Bc7CoreMode2.cpp:456-566).  With size > 1 the CTA's warps take every
-   size-th partition's estimates (all from the block's error, whatever the
-   order) into the first warp's state, `stateStride` bytes before each next,
-   and the first warp searches. */
+/* The estimates of a full search of modes 0 and 2 (the first loop of
+   src/Bc7CoreMode0.cpp:532-642, src/Bc7CoreMode2.cpp:456-566), sorted, in
+   ss.three of the team's first warp.  A team's warps take every size-th
+   partition (all estimates are from the block's error, whatever the order);
+   their states are `stateStride` bytes apart. */
 template<int kD, int MODE>
-__device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane,
-	int size = 1, int rank = 0, size_t stateStride = 0)
+__device__ __forceinline__ void ThreeSubsetsEstimates(WarpState& st, SearchState& ss, const CellRegs& R, const Params& P, const Spec3& sp,
+	const Team& team, size_t stateStride, int lane)
 {
 	constexpr int NP = MODE == 0 ? 16 : 64;
-	const Spec3 sp = GetSpec3(MODE, T);
-	SearchState& s0 = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&ss) - rank * stateStride);
-	if (rank == 0 && lane == 0)
+	SearchState& s0 = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&ss) - team.rank * stateStride);
+	if (team.rank == 0 && lane == 0)
 		s0.three.count = 0;
-	if (size > 1)
-		__syncthreads();
-	else
-		__syncwarp();
+	team.Sync();
 #pragma unroll 1
-	for (int p = rank; p < NP; p += size)
+	for (int p = team.rank; p < NP; p += team.size)
 	{
 		if (R.personalMode == MODE && R.personalParam == p)
 			continue;
@@ -808,16 +885,18 @@ __device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, Cell
 		if (ThreeSubsetsEstimate<kD, MODE>(st, ss, s0, R, P, sp, p, total, lane) && lane == 0)
 			s0.three.order[atomicAdd(&s0.three.count, 1)] = make_int2(total, p);
 	}
-	if (size > 1)
-	{
-		__syncthreads();
-		if (rank)
-			return;
-	}
-	else
-		__syncwarp();
+	team.Sync();
+	if (team.rank == 0)
+		StableSortOrder(ss.three.order, ss.three.count, lane);
+}
+
+/* Full searches of modes 0 and 2. */
+template<int kD, int MODE>
+__device__ NEBC7_PASS void FullThreeSubsets(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+{
+	const Spec3 sp = GetSpec3(MODE, T);
+	ThreeSubsetsEstimates<kD, MODE>(st, ss, R, P, sp, SingleWarp(), 0, lane);
 	const int count = ss.three.count;
-	StableSortOrder(ss.three.order, count, lane);
 #pragma unroll 1
 	for (int i = 0; i < count; i++)
 	{
@@ -849,6 +928,7 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 		if (!((s == 0 ? line0 : line1) < water))
 			return false;
 	}
+	Team one = SingleWarp();
 	Ep mc0 = 0, mc1 = 0;
 	int error = 0;
 #pragma unroll 1
@@ -857,7 +937,7 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 		const int water = room - (s == 0 ? line1 : error);
 		bool any;
 		Ep b = 0;
-		const int r = SearchSubset3<kD, MODE>(ss, st.sub[s], P, sp, water, ss.bound[s][1], ss.bound[s][2], b, any, lane);
+		const int r = SearchSubset3<kD, MODE>(ss, st.sub[s], P, sp, water, ss.bound[s][1], ss.bound[s][2], b, any, one, nullptr, lane);
 		if (!any || !(r < water))
 			return false;
 		error += r;
@@ -961,21 +1041,6 @@ __device__ __forceinline__ int TableError(const int4* plane, const int4* table, 
 			break;
 	}
 	return sum;
-}
-
-/* What the warps of a team share of one four-channel search: the smallest
-   error found so far with its place in the search's order (error << 32 |
-   variant, four list indices), and the next unit of each variant. */
-struct TeamSearch
-{
-	unsigned long long key;
-	int next[4];
-};
-
-/* Place of a combination in the search's order. */
-__device__ __forceinline__ unsigned SearchPlace(int v, int i0, int i1, int i2, int i3)
-{
-	return unsigned(((((v << 5 | i0) << 5 | i1) << 5 | i2) << 5) | i3);
 }
 
 /* The four-channel combination search with 2-bit indices (modes 7 and
@@ -1267,29 +1332,6 @@ __device__ NEBC7_SHARED Found SearchFour(SearchState& ss, const SearchState& fro
 	else
 		return SearchFour2<kD>(ss, from.chan[slot], from.lists[slot], v, ar, ai.count, ai.active, ai.opaque, w, alphaTable, best, water, team,
 			lane);
-}
-
-/* What a team shares of a block's search. */
-struct TeamState
-{
-	TeamSearch search;
-	TeamExchange exchange;
-	int bound[2][4];       /* [subset][channel] estimates */
-	int valid;             /* variants whose lists leave room */
-	int task[3];           /* the CTA's task: queue position, candidate, first improvement */
-};
-
-/* Starts a team's search from `water`; the last one's outcome is read. */
-__device__ __forceinline__ void StartTeamSearch(TeamState& ts, int water)
-{
-	__syncthreads();
-	if (threadIdx.x == 0)
-	{
-		ts.search.key = (unsigned long long)(unsigned(water)) << 32;
-		ts.search.next[0] = ts.search.next[1] = ts.search.next[2] = ts.search.next[3] = 0;
-		ts.valid = 0;
-	}
-	__syncthreads();
 }
 
 /* The endpoints of a team's outcome in the lists it was found in. */
@@ -1775,7 +1817,7 @@ __device__ __noinline__ int TryVariantsRot(const Area& ar, const AreaInfo& ai, c
    src/Bc7CoreMode5.cpp:628-686) + TryVariants. */
 template<int kD, int MODE>
 __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, const CellRegs& R, const Params& P, const LevelTables& T,
-	Ep& mcStorage, int water, int rotation, int lane)
+	Ep& mcStorage, int water, int rotation, Team& team, TeamState* ts, int lane)
 {
 	const Area& ar = st.area1;
 	const AreaInfo& ai = ar.info;
@@ -1797,7 +1839,6 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		ctab = T.d2v8;
 		atab = T.d2v8;
 	}
-	Team one = SingleWarp();
 	int used = 0;
 #pragma unroll 1
 	for (int c = 0; c < 4; c++)
@@ -1809,7 +1850,7 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		else if (c == a)
 			cl = ChannelLevelsSingle<kD>(ss.lists[0][c], ar, c, w, water - used, abits, c != 0, atab, ss.values, lane);
 		else
-			cl = ChannelLevels<kD, false>(ss.lists[0][c], ar, c, w, water - used, cbits, -1, c != 0, ctab, true, 32, ss.values, one, lane);
+			cl = ChannelLevels<kD, false>(ss.lists[0][c], ar, c, w, water - used, cbits, -1, c != 0, ctab, true, 32, ss.values, team, lane);
 		if (lane == 0)
 			ss.chan[0][c] = cl;
 		used += cl.minErr;
@@ -1837,9 +1878,9 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		const int hidden = a != 0 ? 16 - ai.active : 0;
 		Found3 f;
 		if (idx32)
-			f = SearchThree<kD, 3>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, lane);
+			f = SearchThree<kD, 3>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, team, ts, lane);
 		else
-			f = SearchThree<kD, 2>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, lane);
+			f = SearchThree<kD, 2>(ar, ai.active, channel(x), channel(y), channel(z), hidden, water - slot, ss.plane, team, ts, lane);
 		if (f.taken)
 			mcStorage = EpSwapRot(EpSetCh(EpSetCh(Ep2(x, f.x, y, f.y), z, f.z), a, ss.lists[0][a][0].y), rot);
 		return f.water + slot;
@@ -1852,7 +1893,8 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 }
 
 template<int kD>
-__device__ NEBC7_PASS void RefineMode4(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void RefineMode4(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team, TeamState* ts,
+	int lane)
 {
 	/* src/Bc7CoreMode4.cpp:1795-1822 */
 	int rotation = R.bestParam;
@@ -1860,7 +1902,7 @@ __device__ NEBC7_PASS void RefineMode4(WarpState& st, SearchState& ss, CellRegs&
 	for (int i = 0; i < 2; i++, rotation ^= 4)
 	{
 		Ep mc = 0;
-		const int error = CompressRotSubset<kD, 4>(st, ss, R, P, T, mc, R.errTotal, rotation, lane);
+		const int error = CompressRotSubset<kD, 4>(st, ss, R, P, T, mc, R.errTotal, rotation, team, ts, lane);
 		if (R.errTotal > error)
 		{
 			R.errTotal = error;
@@ -1873,11 +1915,12 @@ __device__ NEBC7_PASS void RefineMode4(WarpState& st, SearchState& ss, CellRegs&
 }
 
 template<int kD>
-__device__ NEBC7_PASS void RefineMode5(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane)
+__device__ NEBC7_PASS void RefineMode5(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, Team& team, TeamState* ts,
+	int lane)
 {
 	/* src/Bc7CoreMode5.cpp:890-911 */
 	Ep mc = 0;
-	const int error = CompressRotSubset<kD, 5>(st, ss, R, P, T, mc, R.errTotal, R.bestParam, lane);
+	const int error = CompressRotSubset<kD, 5>(st, ss, R, P, T, mc, R.errTotal, R.bestParam, team, ts, lane);
 	if (R.errTotal > error)
 	{
 		R.errTotal = error;
@@ -1893,6 +1936,7 @@ __device__ NEBC7_PASS void FullRot(WarpState& st, SearchState& ss, CellRegs& R, 
 	   search may resume at choice `from` */
 	const int step = R.denoiseStep;
 	constexpr int NR = MODE == 4 ? 8 : 4;
+	Team one = SingleWarp();
 #pragma unroll 1
 	for (int ri = from; ri < NR; ri++)
 	{
@@ -1904,7 +1948,7 @@ __device__ NEBC7_PASS void FullRot(WarpState& st, SearchState& ss, CellRegs& R, 
 		Ep mc = 0;
 		int error = step;
 		if (error < R.errTotal)
-			error += CompressRotSubset<kD, MODE>(st, ss, R, P, T, mc, R.errTotal - error, rotation, lane);
+			error += CompressRotSubset<kD, MODE>(st, ss, R, P, T, mc, R.errTotal - error, rotation, one, nullptr, lane);
 		if (R.errTotal > error)
 		{
 			R.errTotal = error - step;
@@ -1930,12 +1974,12 @@ __device__ void NormalPasses(WarpState& st, SearchState& ss, CellRegs& R, const 
 
 	switch (R.bestMode)
 	{
-	case 0: if (R.errTotal > OA) RefineOpaque<kD, 0>(st, ss, R, P, T, lane); break;
-	case 1: if (R.errTotal > OA) RefineOpaque<kD, 1>(st, ss, R, P, T, lane); break;
-	case 2: if (R.errTotal > OA) RefineOpaque<kD, 2>(st, ss, R, P, T, lane); break;
-	case 3: if (R.errTotal > OA) RefineOpaque<kD, 3>(st, ss, R, P, T, lane); break;
-	case 4: if (R.errTotal > 0) RefineMode4<kD>(st, ss, R, P, T, lane); break;
-	case 5: if (R.errTotal > 0) RefineMode5<kD>(st, ss, R, P, T, lane); break;
+	case 0: if (R.errTotal > OA) RefineOpaque<kD, 0>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 1: if (R.errTotal > OA) RefineOpaque<kD, 1>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 2: if (R.errTotal > OA) RefineOpaque<kD, 2>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 3: if (R.errTotal > OA) RefineOpaque<kD, 3>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 4: if (R.errTotal > 0) RefineMode4<kD>(st, ss, R, P, T, one, nullptr, lane); break;
+	case 5: if (R.errTotal > 0) RefineMode5<kD>(st, ss, R, P, T, one, nullptr, lane); break;
 	case 6: if (R.errTotal > 0) RefineMode6<kD, 6>(st, ss, R, P, T, one, nullptr, lane); break;
 	case 7: if (R.errTotal > 0) RefineMode7<kD>(st, ss, R, P, T, one, nullptr, 0, lane); break;
 	case 9: if (R.errTotal > 0) RefineMode6<kD, 9>(st, ss, R, P, T, one, nullptr, lane); break;

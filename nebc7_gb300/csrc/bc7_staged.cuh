@@ -47,14 +47,8 @@ namespace nebc7 {
    chain, then the normal and slow chains; kStepFinish packs. */
 enum StageStep
 {
-	kStepDraftRot = 0,     /* fast passes of modes 4 and 5 */
-	kStepDraftMode7,       /* fast pass of mode 7 */
-	kStepDraftOpaque31,    /* fast passes of the opaque modes 3 and 1 */
-	kStepDraftOpaque20,    /* fast passes of the opaque modes 2 and 0 */
-	kStepRefineOpaque,     /* refinement of modes 0-3 */
-	kStepRefineRot,        /* of modes 4 and 5 */
-	kStepRefine6,          /* of modes 6 and 6Index2 */
-	kStepRefine7,          /* of mode 7 */
+	kStepDraftRest = 0,    /* fast passes of modes 4, 5, 7 and the opaque modes 3, 1, 2, 0 */
+	kStepRefine,
 	kStepFull3Mode2,
 	kStepFull3Mode0,
 	kStepFull2Mode1,
@@ -70,6 +64,27 @@ enum StageStep
 constexpr int kStageDraft = -1;
 constexpr int kStepNone = -1;   /* finished in the first kernel (an exact starting block) */
 
+/* The kinds of refinement, in the order of their list: few blocks with long
+   searches first. */
+enum RefineKind
+{
+	kRefine7 = 0,
+	kRefine6,        /* modes 6 and 6Index2 of blocks with alpha */
+	kRefineOpaque,   /* modes 0-3 */
+	kRefineRot,      /* modes 4 and 5 */
+	kRefine6Opaque,  /* modes 6 and 6Index2 of opaque blocks: one p-bit variant, one alpha candidate */
+};
+
+__device__ __forceinline__ int RefineKindOf(int mode, bool opaque)
+{
+	return mode < 4 ? kRefineOpaque : (mode < 6 ? kRefineRot : (mode == 7 ? kRefine7 : (opaque ? kRefine6Opaque : kRefine6)));
+}
+
+/* Buckets of the refinement's list per kind; the first ones, modes 6, 6Index2
+   and 7 of blocks with alpha, can search long. */
+constexpr int kRefineBuckets = 51;
+constexpr int kRefineHeavy = 2 * kRefineBuckets;
+
 /* A block's Cell scalars between pass kernels. */
 struct __align__(16) BlockRecord
 {
@@ -79,7 +94,8 @@ struct __align__(16) BlockRecord
 	int errTotal, personalParam, personalMode, denoiseStep;
 	int water;                   /* the error at the start of the draft chain */
 	int opaque;                  /* the whole-block area's opaque flag */
-	int pad[2];
+	int handed;                  /* 1 + its slot of handed estimates, or 0 */
+	int pad;
 };
 
 /* An improving candidate of a split pass: its endpoints, error and
@@ -88,9 +104,9 @@ struct __align__(16) BlockRecord
    src/Bc7CoreMode4.cpp:1852-1853). */
 struct __align__(16) SplitResult
 {
-	Ep best0, best1;
+	Ep best0, best1, best2;
 	int error, end, param;
-	int pad;
+	int pad[3];
 };
 
 /* The split passes. */
@@ -103,18 +119,36 @@ constexpr int kSplitPolls = 1 << 22;
 
 __host__ __device__ constexpr int SplitIndex(int S)
 {
-	return S == kStepFull2Mode1 ? 0 : (S == kStepFull2Mode3 ? 1 : (S == kStepRot5 ? 2 : (S == kStepRot4 ? 3 : (S == kStepMode7 ? 4 : -1))));
+	return S == kStepFull2Mode1 ? 0 : (S == kStepFull2Mode3 ? 1 : (S == kStepRot5 ? 2 : (S == kStepRot4 ? 3 : (S == kStepMode7 ? 4 :
+		(S == kStepFull3Mode2 ? 5 : (S == kStepFull3Mode0 ? 6 : -1))))));
 }
+
+constexpr int kSplitPasses = 7;
+
+/* The three-subset passes estimate first, a warp or a team per block, and hand
+   a block to the tasks when more than kInlineCandidates partitions are left:
+   a photo's hardest blocks searched 30 and more one after another, 7 ms in
+   one warp with the rest of the GPU idle, where most blocks have one to
+   four. */
+__host__ __device__ constexpr bool ThreeSubsetStep(int S)
+{
+	return S == kStepFull3Mode2 || S == kStepFull3Mode0;
+}
+
+constexpr int kInlineCandidates = 6;
+constexpr int kHandOverBlocks = 8192;   /* a longer list fills the GPU as it is (precise 1024x1024, 65536 blocks: 40.1 ms inline, 45.6 handed over) */
+constexpr int kHandedBlocks = 2048;   /* blocks whose estimates a pass can hand over; the others finish inline */
 
 /* Candidates (tasks) per block of split pass S, and its mode. */
 __host__ __device__ constexpr int SplitTasks(int S)
 {
-	return S == kStepRot4 ? 8 : (S == kStepRot5 ? 4 : 64);
+	return S == kStepRot4 ? 8 : (S == kStepRot5 ? 4 : (S == kStepFull3Mode0 ? 16 : 64));
 }
 
 __host__ __device__ constexpr int SplitMode(int S)
 {
-	return S == kStepFull2Mode1 ? 1 : (S == kStepFull2Mode3 ? 3 : (S == kStepRot5 ? 5 : (S == kStepRot4 ? 4 : 7)));
+	return S == kStepFull2Mode1 ? 1 : (S == kStepFull2Mode3 ? 3 : (S == kStepRot5 ? 5 : (S == kStepRot4 ? 4 : (S == kStepMode7 ? 7 :
+		(S == kStepFull3Mode2 ? 2 : 0)))));
 }
 
 /* Kernel launches of a staged encode: the draft kernel, then per pass its
@@ -130,7 +164,7 @@ __host__ __device__ constexpr int StagedLaunches(bool slow)
 	int n = 1;
 	for (int S = 0; S < kNumStages; S++)
 		if (StageLaunched(S, slow))
-			n += SplitIndex(S) >= 0 ? 3 : 2;
+			n += ThreeSubsetStep(S) ? 4 : (SplitIndex(S) >= 0 ? 3 : 2);
 	return n;
 }
 
@@ -146,7 +180,8 @@ struct __align__(16) SplitQueue
 	int head;                   /* first-round tasks taken */
 	int kept;                   /* results kept */
 	int restCount, restHead;    /* the one-warp remainder */
-	int pad1[28];
+	int handedCount;            /* blocks handed over (three-subset passes) */
+	int pad1[27];
 };
 
 /* Per-launch state of a staged encode (one entry per queue position). */
@@ -155,7 +190,7 @@ struct Stages
 	BlockRecord* rec;
 	int* next;        /* the pass a position waits for, kStepFinish, or kStepNone */
 	int* list;        /* positions of the pass being run, in queue order */
-	int* count;       /* [kNumStages] list lengths */
+	int* count;       /* [kNumStages] list lengths, then the number of blocks of the refinement's heavy buckets */
 	int* counters;    /* [kNumStages + 1] work-queue heads, zero before the draft kernel */
 	int* hist;        /* [kNumStages][256] blocks per bucket of the passes' lists, zero before the draft kernel */
 	int* cursor;      /* [kNumStages][256] positions taken, zero before the draft kernel */
@@ -168,32 +203,39 @@ struct Stages
 	int* later;       /* the blocks of the later rounds, in the order they were appended */
 	int laterCap;
 	int* rest;        /* the blocks of the one-warp remainder */
-	SplitQueue* split;   /* [5 split passes] */
+	SplitQueue* split;   /* [kSplitPasses] */
+	int* handed;      /* the blocks handed over by a three-subset pass, */
+	ThreeEstimates* estimates;   /* and their estimates, by slot */
+	int handedCap;
 	SplitResult* imp;
 	int impCap;
 };
 
 /* Bucket of position k in the list of pass `stage`: 8 per octave of the
    error, largest first, for the searches (their cost grows with it: the
-   longest start first and no SM waits behind a late hard block), 4 per octave
-   with the opaque blocks last for the refinement of modes 6 and 6Index2 (an
-   opaque block has one p-bit variant and one alpha candidate where another
-   has four and twenty), else by position. */
-__device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, bool opaque)
+   longest start first and no SM waits behind a late hard block), for the
+   refinement by kind and 1.6 per octave within it (so that the warps of an SM
+   run the same code), else by position. */
+__device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, int mode, bool opaque)
 {
-	if (!sg.byError || stage < kStepRefineOpaque || stage == kStepFinish)
+	if (!sg.byError || stage < kStepRefine || stage == kStepFinish)
 		return int((long long)k * 256 / sg.total);
 	const unsigned e = unsigned(max(error, 1));
 	const int msb = 31 - __clz(e);
 	const int b = 255 - min(255, msb * 8 + int((e >> (msb >= 3 ? msb - 3 : 0)) & 7u));
-	return stage == kStepRefine6 ? (opaque ? 128 : 0) + (b >> 1) : b;
+	if (stage == kStepRefine)
+	{
+		const int kind = RefineKindOf(mode, opaque);
+		return kind <= kRefine6 ? b * kRefineHeavy >> 8 : kRefineBuckets * kind + (b * kRefineBuckets >> 8);
+	}
+	return b;
 }
 
 /* Records that position k waits for pass n (one thread). */
-__device__ __forceinline__ void Publish(const Stages& sg, int k, int n, int error, bool opaque)
+__device__ __forceinline__ void Publish(const Stages& sg, int k, int n, int error, int mode, bool opaque)
 {
 	sg.next[k] = n;
-	atomicAdd(&sg.hist[n * 256 + StageBucket(sg, n, k, error, opaque)], 1);
+	atomicAdd(&sg.hist[n * 256 + StageBucket(sg, n, k, error, mode, opaque)], 1);
 }
 
 __device__ __forceinline__ void SaveRecord(BlockRecord& r, const CellRegs& R, int lane)
@@ -247,13 +289,13 @@ __device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const B
    16 warps (18 % hits on the level tables). */
 __host__ __device__ constexpr size_t StageWarpBytes(int stage, bool split)
 {
-	if (stage < kStepRefineOpaque || stage == kStepFinish)
+	if (stage < kStepRefine || stage == kStepFinish)
 		return sizeof(WarpState);
 	const bool pca = !split && (stage == kStepFull2Mode1 || stage == kStepFull2Mode3 || stage == kStepMode7);
 	const size_t search = pca ? sizeof(SearchState)
-		: (stage == kStepRefine6 || stage == kStepRefine7 || stage == kStepMode7) ? offsetof(SearchState, table) + sizeof(SearchState::table)
+		: (stage == kStepRefine || stage == kStepMode7) ? offsetof(SearchState, table) + sizeof(SearchState::table)
 		: stage == kStepMode6 ? offsetof(SearchState, plane16) + sizeof(SearchState::plane16)
-		: (stage == kStepFull3Mode2 || stage == kStepFull3Mode0) ? offsetof(SearchState, three) + sizeof(SearchState::three)
+		: ThreeSubsetStep(stage) ? offsetof(SearchState, three) + sizeof(SearchState::three)
 		: offsetof(SearchState, three);
 	return kSearchWarpBytes + ((search + 15) & ~size_t(15));
 }
@@ -263,91 +305,122 @@ __host__ __device__ constexpr size_t StageSharedBytes(int stage, bool split)
 	return kWarpsPerCta * StageWarpBytes(stage, split);
 }
 
-/* Passes whose blocks a CTA's warps search together, and how many of them (the
-   first of the list): all when there are few, since then the longest search is
-   what the pass takes (a 1024x1024 photo leaves the three-subset search of
-   mode 2 eight blocks, 2.3 ms of one warp each; the mode 7 refinement of an
-   alpha texture's 1200 blocks took 5.4 ms, 0.4 ms of the GPU's warps), else
-   one per CTA of the four-channel searches, whose list begins with the hardest,
-   and none of the three-subset ones, whose teams only share the estimates. */
+/* Passes whose blocks a CTA's warps search together when there are few
+   (TeamBlocks): then the longest search is what the pass takes (a 1024x1024
+   photo leaves the three-subset search of mode 2 eight blocks, 2.3 ms of one
+   warp each; the mode 7 refinement of an alpha texture's 1200 blocks took
+   5.4 ms, 0.4 ms of the GPU's warps).  Of a long refinement list the first two
+   blocks per CTA, which the list's order makes the ones with long searches, and
+   up to 16 per CTA of those with alpha (modes 6, 6Index2, 7): on a 1118x1105
+   alpha texture one mode 6 block took a warp 33 ms, and the 56065 blocks'
+   refinement 34.0 ms with 2 per CTA, 15.8 ms with 16. */
 __host__ __device__ constexpr bool TeamStage(int S)
 {
-	return S == kStepFull3Mode2 || S == kStepFull3Mode0 || S == kStepRefine6 || S == kStepRefine7 || S == kStepMode6;
+	return ThreeSubsetStep(S) || S == kStepRefine || S == kStepMode6;
 }
 
-__device__ __forceinline__ int TeamBlocks(int S, int n, int ctas)
+__device__ __forceinline__ int TeamBlocks(int S, int n, int heavy, int ctas)
 {
-	if (S == kStepFull3Mode2 || S == kStepFull3Mode0)
-		return n <= kWarpsPerCta * ctas ? n : 0;
-	return n <= 2 * kWarpsPerCta * ctas ? n : ctas;
+	if (n <= (ThreeSubsetStep(S) ? 1 : 2) * kWarpsPerCta * ctas)
+		return n;
+	return S == kStepRefine ? max(min(heavy, 16 * ctas), min(n, 2 * ctas)) : 0;
 }
 
-/* One stage: passes of the draft chain after the mode 6 fast pass
+/* The refinement of a block's mode (ModeN::CompressBlock), one function per
+   kind: each has registers and code of its own (inlined into one kernel body
+   the kinds spilled and outgrew the instruction cache, 30 -> 38 ms on an alpha
+   texture; one kernel per kind waits for the longest search of each).  The
+   warp's state, the tables and the team's exchange come as shared-memory
+   addresses, so that the accesses stay shared ones. */
+template<int kD, int KIND>
+__device__ __noinline__ void RefineOne(CellRegs& shared, unsigned stAt, unsigned tablesAt, unsigned tsAt, int size, int rank, int lane)
+{
+	WarpState& st = *static_cast<WarpState*>(__cvta_shared_to_generic(stAt));
+	SearchState& ss = *static_cast<SearchState*>(__cvta_shared_to_generic(stAt + kSearchWarpBytes));
+	const LevelTables& T = *static_cast<const LevelTables*>(__cvta_shared_to_generic(tablesAt));
+	TeamState* ts = static_cast<TeamState*>(__cvta_shared_to_generic(tsAt));
+	const Params& P = st.P;
+	CellRegs R = shared;
+	Team team{ size, rank, &ts->exchange, 0 };
+	if constexpr (KIND == kRefineOpaque)
+	{
+		switch (R.bestMode)
+		{
+		case 0: RefineOpaque<kD, 0>(st, ss, R, P, T, team, ts, lane); break;
+		case 1: RefineOpaque<kD, 1>(st, ss, R, P, T, team, ts, lane); break;
+		case 2: RefineOpaque<kD, 2>(st, ss, R, P, T, team, ts, lane); break;
+		default: RefineOpaque<kD, 3>(st, ss, R, P, T, team, ts, lane); break;
+		}
+	}
+	else if constexpr (KIND == kRefineRot)
+	{
+		if (R.bestMode == 4)
+			RefineMode4<kD>(st, ss, R, P, T, team, ts, lane);
+		else
+			RefineMode5<kD>(st, ss, R, P, T, team, ts, lane);
+	}
+	else if constexpr (KIND == kRefine6)
+	{
+		if (R.bestMode == 6)
+			RefineMode6<kD, 6>(st, ss, R, P, T, team, ts, lane);
+		else
+			RefineMode6<kD, 9>(st, ss, R, P, T, team, ts, lane);
+	}
+	else
+		RefineMode7<kD>(st, ss, R, P, T, team, ts, StageWarpBytes(kStepRefine, false), lane);
+	shared = R;
+}
+
+/* One stage: the passes of the draft chain after the mode 6 fast pass
    (DraftChain), or one pass of the normal / slow chains (NormalPasses). */
 template<int kD, int S>
 __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T, int lane,
 	int from, Team& team, TeamState* ts)
 {
-	if constexpr (S == kStepDraftRot)
+	if constexpr (S == kStepDraftRest)
 	{
-		/* entered with errTotal > step (src/Bc7Core.cpp:1558-1566) */
+		/* entered with errTotal > step (src/Bc7Core.cpp:1558-1597) */
+		const int step = R.denoiseStep, gate = R.opaqueAlphaError + step;
 		FastRot<kD, 4>(st, R, P, lane);
-		if (R.errTotal > R.denoiseStep)
-			FastRot<kD, 5>(st, R, P, lane);
-	}
-	else if constexpr (S == kStepDraftMode7)
-		FastMode7<kD>(st, R, P, T, lane);
-	else if constexpr (S == kStepDraftOpaque31)
-	{
-		/* entered with errTotal > OA + step (src/Bc7Core.cpp:1577-1585) */
-		FastOpaque<kD, 3>(st, R, P, lane);
-		if (R.errTotal > R.opaqueAlphaError + R.denoiseStep)
-			FastOpaque<kD, 1>(st, R, P, lane);
-	}
-	else if constexpr (S == kStepDraftOpaque20)
-	{
-		FastOpaque<kD, 2>(st, R, P, lane);
-		if (R.errTotal > R.opaqueAlphaError + R.denoiseStep)
-			FastOpaque<kD, 0>(st, R, P, lane);
-	}
-	else if constexpr (S >= kStepRefineOpaque && S <= kStepRefine7)
-	{
-		if (R.errTotal > (S == kStepRefineOpaque ? R.opaqueAlphaError : 0))
+		if (R.errTotal > step)
 		{
-			if constexpr (S == kStepRefineOpaque)
+			FastRot<kD, 5>(st, R, P, lane);
+			if (R.errTotal > step)
+				FastMode7<kD>(st, R, P, T, lane);
+		}
+		if (int(int16_t(R.a1.minmax[0])) > 255 - 16 && R.errTotal > gate)
+		{
+			FastOpaque<kD, 3>(st, R, P, lane);
+			if (R.errTotal > gate)
 			{
-				switch (R.bestMode)
+				FastOpaque<kD, 1>(st, R, P, lane);
+				if (R.errTotal > gate)
 				{
-				case 0: RefineOpaque<kD, 0>(st, ss, R, P, T, lane); break;
-				case 1: RefineOpaque<kD, 1>(st, ss, R, P, T, lane); break;
-				case 2: RefineOpaque<kD, 2>(st, ss, R, P, T, lane); break;
-				default: RefineOpaque<kD, 3>(st, ss, R, P, T, lane); break;
+					FastOpaque<kD, 2>(st, R, P, lane);
+					if (R.errTotal > gate)
+						FastOpaque<kD, 0>(st, R, P, lane);
 				}
 			}
-			else if constexpr (S == kStepRefineRot)
+		}
+	}
+	else if constexpr (S == kStepRefine)
+	{
+		if (R.errTotal > (R.bestMode < 4 ? R.opaqueAlphaError : 0))
+		{
+			const unsigned stAt = unsigned(__cvta_generic_to_shared(&st));
+			const unsigned tablesAt = unsigned(__cvta_generic_to_shared(&T));
+			const unsigned tsAt = unsigned(__cvta_generic_to_shared(ts));
+			switch (RefineKindOf(R.bestMode, false))
 			{
-				if (R.bestMode == 4)
-					RefineMode4<kD>(st, ss, R, P, T, lane);
-				else
-					RefineMode5<kD>(st, ss, R, P, T, lane);
+			case kRefine7: RefineOne<kD, kRefine7>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
+			case kRefineOpaque: RefineOne<kD, kRefineOpaque>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
+			case kRefineRot: RefineOne<kD, kRefineRot>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
+			default: RefineOne<kD, kRefine6>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
 			}
-			else if constexpr (S == kStepRefine6)
-			{
-				if (R.bestMode == 6)
-					RefineMode6<kD, 6>(st, ss, R, P, T, team, ts, lane);
-				else
-					RefineMode6<kD, 9>(st, ss, R, P, T, team, ts, lane);
-			}
-			else
-				RefineMode7<kD>(st, ss, R, P, T, team, ts, StageWarpBytes(S, false), lane);
 		}
 		R.personalParam = R.bestParam;
 		R.personalMode = R.bestMode;
 	}
-	else if constexpr (S == kStepFull3Mode2)
-		FullThreeSubsets<kD, 2>(st, ss, R, P, T, lane, team.size, team.rank, StageWarpBytes(S, false));
-	else if constexpr (S == kStepFull3Mode0)
-		FullThreeSubsets<kD, 0>(st, ss, R, P, T, lane, team.size, team.rank, StageWarpBytes(S, false));
 	else if constexpr (S == kStepFull2Mode1)
 		FullTwoSubsets<kD, 1>(st, ss, R, P, T, lane, from);
 	else if constexpr (S == kStepFull2Mode3)
@@ -362,47 +435,24 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 		FullMode6<kD>(st, ss, R, P, T, team, ts, lane);
 }
 
-/* The refinement pass of the block's mode, or the pack. */
-__device__ __forceinline__ int AfterDraft(const CellRegs& R, const Params& P)
+__device__ __forceinline__ int AfterDraft(const Params& P)
 {
-	if (!P.doNormal || P.doDraft == 2)
-		return kStepFinish;
-	return R.bestMode < 4 ? kStepRefineOpaque : (R.bestMode < 6 ? kStepRefineRot : (R.bestMode == 7 ? kStepRefine7 : kStepRefine6));
+	return (P.doNormal && P.doDraft != 2) ? kStepRefine : kStepFinish;
 }
 
-/* The draft chain's opaque passes run for blocks whose alpha stays above
-   239 (src/Bc7Core.cpp:1577), after the transparent chain however far it
-   went; then the normal passes, or the pack. */
-__device__ __forceinline__ int AfterTransparentChain(const CellRegs& R, const Params& P)
-{
-	if (int(int16_t(R.a1.minmax[0])) > 255 - 16 && R.errTotal > R.opaqueAlphaError + R.denoiseStep)
-		return kStepDraftOpaque31;
-	return AfterDraft(R, P);
-}
-
-/* The pass after S: the nesting of the draft chain (src/Bc7Core.cpp:
-   1546-1597, DraftChain) and of the normal and slow chains in NormalPasses
-   (src/Bc7Core.cpp:1677-1745), whose conditions are tested when each pass
-   is reached. */
+/* The pass after S: the nesting of the normal and slow chains in
+   NormalPasses (src/Bc7Core.cpp:1677-1745), whose conditions are tested when
+   each pass is reached. */
 __device__ __forceinline__ int NextStep(int S, const CellRegs& R, const Params& P)
 {
 	const int OA = R.opaqueAlphaError, step = R.denoiseStep, e = R.errTotal;
-	switch (S)
-	{
-	case kStepDraftRot: return e > step ? kStepDraftMode7 : AfterTransparentChain(R, P);
-	case kStepDraftMode7: return AfterTransparentChain(R, P);
-	case kStepDraftOpaque31: return e > OA + step ? kStepDraftOpaque20 : AfterDraft(R, P);
-	case kStepDraftOpaque20: return AfterDraft(R, P);
-	default: break;
-	}
+	if (S == kStepDraftRest)
+		return AfterDraft(P);
 	if (R.a1.opaque)
 	{
 		switch (S)
 		{
-		case kStepRefineOpaque:
-		case kStepRefineRot:
-		case kStepRefine6:
-		case kStepRefine7: return e > OA + step ? kStepFull3Mode2 : kStepFinish;
+		case kStepRefine: return e > OA + step ? kStepFull3Mode2 : kStepFinish;
 		case kStepFull3Mode2: return e > OA + step ? kStepFull3Mode0 : kStepFinish;
 		case kStepFull3Mode0: return (P.doSlow && e > OA + step) ? kStepFull2Mode1 : kStepFinish;
 		case kStepFull2Mode1: return e > OA + step ? kStepFull2Mode3 : kStepFinish;
@@ -415,10 +465,7 @@ __device__ __forceinline__ int NextStep(int S, const CellRegs& R, const Params& 
 	}
 	switch (S)
 	{
-	case kStepRefineOpaque:
-	case kStepRefineRot:
-	case kStepRefine6:
-	case kStepRefine7: return e > step ? kStepRot5 : kStepFinish;
+	case kStepRefine: return e > step ? kStepRot5 : kStepFinish;
 	case kStepRot5: return e > step ? kStepRot4 : kStepFinish;
 	case kStepRot4: return e > step ? kStepMode7 : kStepFinish;
 	case kStepMode7: return (P.doSlow && e > step) ? kStepMode6 : kStepFinish;
@@ -535,14 +582,9 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 				if (kD > 0 || P.denoiseStep > 0)
 					FastMode6<kD, true>(st, R, P, T, lane);
 				if (R.errTotal > step)
-				{
 					FastMode6<kD, false>(st, R, P, T, lane);
-					if (R.errTotal > step)
-						n = kStepDraftRot;
-				}
 			}
-			if (n != kStepDraftRot)
-				n = AfterTransparentChain(R, P);
+			n = R.errTotal > step ? int(kStepDraftRest) : AfterDraft(P);
 		}
 	}
 	else
@@ -555,12 +597,84 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 	SaveRecord(rec, R, lane);
 	if (lane == 0)
 	{
+		rec.handed = 0;
 		rec.startLo = lo;
 		rec.startHi = hi;
 		rec.water = water;
-		Publish(sg, k, n, R.errTotal, R.a1.opaque);
+		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque);
 	}
 	__syncwarp();
+	return false;
+}
+
+/* FullThreeSubsets of the block at position k: the estimates, then the search
+   in the (team's first) warp, or its hand-over to the tasks of KEncodeSplit
+   (returns true).  A block that was handed and comes back (a result that was
+   not kept) goes on from candidate `from` with its estimates. */
+template<int kD, int S>
+__device__ __forceinline__ bool ThreeSubsetsStage(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T,
+	const Stages& sg, int k, int from, bool hand, const Team& team, int lane)
+{
+	constexpr int MODE = SplitMode(S);
+	const Spec3 sp = GetSpec3(MODE, T);
+	BlockRecord& rec = sg.rec[k];
+	const int handed = __ldcg(&rec.handed);
+	const bool resume = handed != 0;
+	if (resume)
+	{
+		if (team.rank)
+			return false;
+		const int* src = reinterpret_cast<const int*>(sg.estimates + (handed - 1));
+		for (int i = lane; i < int(sizeof(ThreeEstimates) / 4); i += 32)
+			reinterpret_cast<int*>(&ss.three)[i] = __ldcg(src + i);
+		__syncwarp();
+		if (lane == 0)
+			rec.handed = 0;
+	}
+	else
+	{
+		ThreeSubsetsEstimates<kD, MODE>(st, ss, R, P, sp, team, StageWarpBytes(S, false), lane);
+		if (team.rank)
+			return false;
+		/* sorted: the first ones are below the error */
+		int left = 0;
+		for (int i = lane; i < ss.three.count; i += 32)
+			left += ss.three.order[i].x < R.errTotal;
+		left = int(__reduce_add_sync(kFull, unsigned(left)));
+		if (hand && left > kInlineCandidates)
+		{
+			SplitQueue& q = sg.split[SplitIndex(S)];
+			int slot = 0;
+			if (lane == 0)
+				slot = atomicAdd(&q.handedCount, 1);
+			slot = __shfl_sync(kFull, slot, 0);
+			if (slot < sg.handedCap)
+			{
+				int* dst = reinterpret_cast<int*>(sg.estimates + slot);
+				for (int i = lane; i < int(sizeof(ThreeEstimates) / 4); i += 32)
+					dst[i] = reinterpret_cast<const int*>(&ss.three)[i];
+				if (lane == 0)
+				{
+					rec.handed = slot + 1;
+					sg.handed[slot] = k;
+					sg.start[k] = 0;
+					sg.firstImp[k] = kSplitNone;
+					sg.pending[k] = SplitTasks(S);
+				}
+				__syncwarp();
+				return true;
+			}
+		}
+		from = 0;
+	}
+	const int count = ss.three.count;
+#pragma unroll 1
+	for (int i = from; i < count; i++)
+	{
+		const int2 o = ss.three.order[i];
+		if (o.x < R.errTotal && ThreeSubsetsPartition<kD, MODE>(st, ss, R, P, sp, o.y, lane))
+			break;
+	}
 	return false;
 }
 
@@ -568,20 +682,26 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
    `from` on) and records the next one. */
 template<int kD, int S>
 __device__ void PassStage(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P, const Stages& sg, int k,
-	int from, Team& team, TeamState* ts, int lane)
+	int from, bool hand, Team& team, TeamState* ts, int lane)
 {
 	CellRegs R;
 	BlockRecord& rec = sg.rec[k];
 	RestoreBlock(st, R, b, rec, P, lane);
 	if (TeamStage(S) && team.size > 1)
 		__syncthreads();   /* every warp has read the record before it changes */
-	RunStep<kD, S>(st, ss, R, P, T, lane, from, team, ts);
+	if constexpr (ThreeSubsetStep(S))
+	{
+		if (ThreeSubsetsStage<kD, S>(st, ss, R, P, T, sg, k, from, hand, team, lane))
+			return;   /* handed to the tasks */
+	}
+	else
+		RunStep<kD, S>(st, ss, R, P, T, lane, from, team, ts);
 	if (team.rank)
 		return;
 	const int n = NextStep(S, R, P);
 	SaveRecord(rec, R, lane);
 	if (lane == 0)
-		Publish(sg, k, n, R.errTotal, R.a1.opaque);
+		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque);
 	__syncwarp();
 }
 
@@ -598,7 +718,7 @@ __device__ void FinishStage(WarpState& st, const BlockRef& b, const Params& P, c
    finished (its output is written). */
 template<int kD, int STAGE>
 __device__ __forceinline__ bool StageBlock(WarpState& st, SearchState& ss, const BlockRef& b, const LevelTables& T, const Params& P,
-	const Stages& sg, int k, Team& team, TeamState* ts, int lane)
+	const Stages& sg, int k, bool hand, Team& team, TeamState* ts, int lane)
 {
 	if constexpr (STAGE == kStageDraft)
 		return DraftStage<kD>(st, b, T, P, sg, k, lane);
@@ -609,7 +729,7 @@ __device__ __forceinline__ bool StageBlock(WarpState& st, SearchState& ss, const
 	}
 	else
 	{
-		PassStage<kD, STAGE>(st, ss, b, T, P, sg, k, SplitIndex(STAGE) >= 0 ? sg.start[k] : 0, team, ts, lane);
+		PassStage<kD, STAGE>(st, ss, b, T, P, sg, k, SplitIndex(STAGE) >= 0 ? sg.start[k] : 0, hand, team, ts, lane);
 		return false;
 	}
 }
@@ -631,9 +751,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 	ShareTables(tables, T0, T1);
 	const int n = list ? *count : job.total;
 	__shared__ TeamState ts;
-	/* the first blocks, the hardest, a CTA each (TeamBlocks), the others a
-	   warp each */
-	const int nTeam = TeamStage(STAGE) ? TeamBlocks(STAGE, n, int(gridDim.x)) : 0;
+	/* the first blocks of a list a CTA each (TeamBlocks), the others a warp each */
+	const int nTeam = TeamStage(STAGE) ? TeamBlocks(STAGE, n, sg.count[kNumStages], int(gridDim.x)) : 0;
 	Team team{ nTeam > 0 ? kWarpsPerCta : 1, nTeam > 0 ? warp : 0, &ts.exchange, 0 };
 	for (;;)
 	{
@@ -649,7 +768,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 			i = ts.task[0];
 			if (i >= nTeam)
 			{
-				/* every warp for itself from here; warp 0 has a block already */
+				/* every warp for itself from here; the first has a block already */
 				team = SingleWarp();
 				if (warp && lane == 0)
 					i = atomicAdd(head, 1);
@@ -669,12 +788,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 		if constexpr (kD == kAnyDenoise)
 		{
 			if (d.denoise)
-				finished = StageBlock<1, STAGE>(st, ss, b, tables[1], P, sg, k, team, &ts, lane);
+				finished = StageBlock<1, STAGE>(st, ss, b, tables[1], P, sg, k, n <= kHandOverBlocks, team, &ts, lane);
 			else
-				finished = StageBlock<0, STAGE>(st, ss, b, tables[0], P, sg, k, team, &ts, lane);
+				finished = StageBlock<0, STAGE>(st, ss, b, tables[0], P, sg, k, n <= kHandOverBlocks, team, &ts, lane);
 		}
 		else
-			finished = StageBlock<kD, STAGE>(st, ss, b, tables[kD], P, sg, k, team, &ts, lane);
+			finished = StageBlock<kD, STAGE>(st, ss, b, tables[kD], P, sg, k, n <= kHandOverBlocks, team, &ts, lane);
 		if (finished)
 			BlockFinished(d, lane);
 	}
@@ -698,6 +817,7 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 	const int E = R.errTotal, step = R.denoiseStep;
 	bool end;
 	int param = p;
+	Team one = SingleWarp();
 	/* the conditions of the candidate loops (FullTwoSubsets, FullMode7, FullRot) */
 	if constexpr (MODE == 4 || MODE == 5)
 	{
@@ -709,13 +829,32 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 		Ep mc = 0;
 		int error = step;
 		if (error < E)
-			error += CompressRotSubset<kD, MODE>(st, ss, R, P, T, mc, E - error, rotation, lane);
+			error += CompressRotSubset<kD, MODE>(st, ss, R, P, T, mc, E - error, rotation, one, nullptr, lane);
 		if (!(E > error))
 			return;
 		R.errTotal = error - step;
 		R.best[0] = mc;
 		end = error <= step;
 		param = rotation;
+	}
+	else if constexpr (MODE == 0 || MODE == 2)
+	{
+		/* candidate p of the sorted estimates */
+		const ThreeEstimates& from = sg.estimates[__ldcg(&sg.rec[k].handed) - 1];
+		if (p >= __ldcg(&from.count))
+			return;
+		const int2 o = __ldcg(&from.order[p]);
+		if (!(o.x < E))
+			return;
+		param = o.y;
+		if (lane < 9)
+			(&ss.three.est[param][0][0])[lane] = __ldcg(&from.est[param][0][0] + lane);
+		else if (lane < 11)
+			ss.three.lines[param][lane - 9] = __ldcg(&from.lines[param][lane - 9]);
+		__syncwarp();
+		end = ThreeSubsetsPartition<kD, MODE>(st, ss, R, P, GetSpec3(MODE, T), param, lane);
+		if (R.errTotal == E)
+			return;
 	}
 	else
 	{
@@ -749,10 +888,11 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 		SplitResult r;
 		r.best0 = R.best[0];
 		r.best1 = R.best[1];
+		r.best2 = R.best[2];
 		r.error = R.errTotal;
 		r.end = end;
 		r.param = param;
-		r.pad = 0;
+		r.pad[0] = r.pad[1] = r.pad[2] = 0;
 		sg.imp[at] = r;
 		slot = at;
 	}
@@ -792,12 +932,15 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
 		{
 			const uint4* e = reinterpret_cast<const uint4*>(sg.imp + slot);
 			SplitResult v;
-			reinterpret_cast<uint4*>(&v)[0] = __ldcg(e);
-			reinterpret_cast<uint4*>(&v)[1] = __ldcg(e + 1);
+#pragma unroll
+			for (int i = 0; i < int(sizeof(SplitResult) / 16); i++)
+				reinterpret_cast<uint4*>(&v)[i] = __ldcg(e + i);
 			r.errTotal = v.error;
 			r.best[0] = v.best0;
 			if (MODE != 4 && MODE != 5)
 				r.best[1] = v.best1;
+			if (MODE == 0 || MODE == 2)
+				r.best[2] = v.best2;
 			r.bestParam = v.param;
 			r.bestMode = MODE;
 			if (!v.end && p < NT - 1)
@@ -837,7 +980,8 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
 		R.opaqueAlphaError = now.opaqueAlphaError;
 		R.denoiseStep = now.denoiseStep;
 			R.a1.opaque = now.opaque != 0;
-		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.opaque != 0);
+		r.handed = 0;
+		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.bestMode, now.opaque != 0);
 	}
 	__threadfence();
 	atomicAdd(&q.finished, 1);
@@ -907,8 +1051,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 	__shared__ LevelTables tables[2];
 	ShareTables(tables, T0, T1);
 	SplitQueue& q = sg.split[SplitIndex(S)];
-	const int n = min(*count, kSplitMaxBlocks);
-	const int rank = N > 1 ? warp : 0;
+	const int n = min(*count, ThreeSubsetStep(S) ? sg.handedCap : kSplitMaxBlocks);
+	const int rank = N > 1 ? warp : 0;   /* within the task's warps */
 	bool firstRound = true;
 	for (;;)
 	{
@@ -955,7 +1099,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		BlockRef b;
 		QueuedBlock(job, k, d, b);
 		const Params& P = SharedParams(st, d, lane);
-		if (P.pca && SplitMode(S) != 4 && SplitMode(S) != 5)
+		if (P.pca && (SplitMode(S) & 1) && SplitMode(S) != 5)
 		{
 			/* OPTION_PCA orders the partitions by their bounds first: the
 			   pass runs whole, in one warp */
@@ -1021,6 +1165,8 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 			base[lane * 8 + j] = incl - run + c[j];
 		if (blockIdx.x == 0 && lane == 31)
 			sg.count[stage] = incl;
+		if (stage == kStepRefine && blockIdx.x == 0 && lane == kRefineHeavy / 8)
+			sg.count[kNumStages] = base[kRefineHeavy];
 		if (lane == 31 && incl == 0)
 			base[0] = -1;
 	}
@@ -1031,7 +1177,7 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 	{
 		if (sg.next[k] != stage)
 			continue;
-		const int b = StageBucket(sg, stage, k, sg.rec[k].errTotal, sg.rec[k].opaque != 0);
+		const int b = StageBucket(sg, stage, k, sg.rec[k].errTotal, sg.rec[k].bestMode, sg.rec[k].opaque != 0);
 		const int at = base[b] + atomicAdd(&sg.cursor[stage * 256 + b], 1);
 		sg.list[at] = k;
 		if (NT)
@@ -1061,7 +1207,7 @@ cudaError_t StagedEncodeOccupancy(int* ctasPerSm);
    (records, next-pass words, the pass list, the split passes' words, later
    rounds and kept results; 256-byte aligned pieces), after kStagedZeroed bytes
    of counts, queues and histograms that must be zero before each launch. */
-constexpr size_t kStagedZeroed = 256 + 5 * sizeof(SplitQueue) + 2 * size_t(kNumStages) * 1024;
+constexpr size_t kStagedZeroed = 256 + kSplitPasses * sizeof(SplitQueue) + 2 * size_t(kNumStages) * 1024;
 static_assert(kStagedZeroed % 256 == 0 && kNumStages < 32, "the counts and queue heads take 128 bytes each");
 
 constexpr size_t SplitResultCap(int n)
@@ -1074,12 +1220,17 @@ constexpr size_t SplitLaterCap(int n)
 	return n < (1 << 22) - 1024 ? 4 * size_t(n) + 1024 : size_t(1) << 24;   /* its tasks stay an int too */
 }
 
+constexpr size_t HandedCap(int n)
+{
+	return n < kHandedBlocks ? n : kHandedBlocks;
+}
+
 constexpr size_t StagedAlign(size_t v) { return (v + 255) & ~size_t(255); }
 
 constexpr size_t StagedScratchBytes(int n)
 {
 	return kStagedZeroed + StagedAlign(size_t(n) * sizeof(BlockRecord)) + StagedAlign(size_t(n) * 4) * 6 + StagedAlign(SplitLaterCap(n) * 4) +
-		SplitResultCap(n) * sizeof(SplitResult);
+		StagedAlign(SplitResultCap(n) * sizeof(SplitResult)) + StagedAlign(HandedCap(n) * 4) + HandedCap(n) * sizeof(ThreeEstimates);
 }
 
 /* Splits a staged scratch (256-byte aligned, StagedScratchBytes(n) bytes). */
@@ -1089,7 +1240,7 @@ inline Stages SplitStaged(uint8_t* p, int n, bool byError)
 	s.count = (int*)p;
 	s.counters = (int*)(p + 128);
 	s.split = (SplitQueue*)(p + 256);
-	s.hist = (int*)(p + 256 + 5 * sizeof(SplitQueue));
+	s.hist = (int*)(p + 256 + kSplitPasses * sizeof(SplitQueue));
 	s.cursor = s.hist + kNumStages * 256;
 	s.total = n;
 	s.byError = byError;
@@ -1106,6 +1257,10 @@ inline Stages SplitStaged(uint8_t* p, int n, bool byError)
 	s.laterCap = int(SplitLaterCap(n));
 	s.imp = (SplitResult*)(q + 6 * ints + StagedAlign(SplitLaterCap(n) * 4));
 	s.impCap = int(SplitResultCap(n));
+	uint8_t* h = (uint8_t*)s.imp + StagedAlign(SplitResultCap(n) * sizeof(SplitResult));
+	s.handed = (int*)h;
+	s.estimates = (ThreeEstimates*)(h + StagedAlign(HandedCap(n) * 4));
+	s.handedCap = int(HandedCap(n));
 	return s;
 }
 

@@ -16,30 +16,36 @@ inline int StageGrid(int grid, long long tasks, int warps)
 	return ctas < grid ? int(ctas) : grid;
 }
 
-/* The list of pass STAGE and its kernel; a split pass's blocks that must run
-   whole (OPTION_PCA, results not kept) follow in one warp each, from their
-   start candidates. */
+/* The list of pass STAGE and its kernels: of a split pass the tasks, of a
+   three-subset pass its estimates and the tasks of the blocks they hand over;
+   then a split pass's blocks that must run whole (OPTION_PCA, results not
+   kept), in one warp each from their start candidates. */
 template<int kD, int STAGE>
 cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Stages& sg, const LevelTables& T0, const LevelTables& T1)
 {
 	constexpr int split = SplitIndex(STAGE);
+	constexpr bool three = ThreeSubsetStep(STAGE);
 	if (STAGE != kStageDraft)
 	{
 		const int ctas = (job.total + 1023) / 1024;
-		KStageList<<<ctas < 152 ? ctas : 152, 1024, 0, stream>>>(sg, STAGE, split, split >= 0 ? SplitTasks(STAGE) : 0);
+		KStageList<<<ctas < 152 ? ctas : 152, 1024, 0, stream>>>(sg, STAGE, split, split >= 0 && !three ? SplitTasks(STAGE) : 0);
+	}
+	const int stageGrid = StageGrid(grid, job.total, TeamStage(STAGE) ? kWarpsPerCta : 1);
+	if constexpr (split < 0 || three)
+	{
+		const bool all = STAGE == kStageDraft;
+		KEncodeStage<kD, STAGE><<<stageGrid, kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, all ? nullptr : sg.list,
+			all ? nullptr : sg.count + STAGE, sg.counters + (STAGE + 1), T0, T1);
 	}
 	if constexpr (split >= 0)
 	{
 		/* a small texture's tasks fill more SMs than its blocks */
-		KEncodeSplit<kD, STAGE><<<StageGrid(grid, (long long)job.total * SplitTasks(STAGE), SplitTeam(STAGE)), kWarpsPerCta * 32, StageSharedBytes(STAGE, true), stream>>>(job, sg, sg.list, sg.count + STAGE, T0, T1);
-		KEncodeStage<kD, STAGE><<<StageGrid(grid, job.total, TeamStage(STAGE) ? kWarpsPerCta : 1), kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, sg.rest,
+		const int blocks = three ? sg.handedCap : job.total;
+		KEncodeSplit<kD, STAGE><<<StageGrid(grid, (long long)blocks * SplitTasks(STAGE), SplitTeam(STAGE)), kWarpsPerCta * 32,
+			StageSharedBytes(STAGE, true), stream>>>(job, sg, three ? sg.handed : sg.list, three ? &sg.split[split].handedCount : sg.count + STAGE,
+			T0, T1);
+		KEncodeStage<kD, STAGE><<<stageGrid, kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, sg.rest,
 			&sg.split[split].restCount, &sg.split[split].restHead, T0, T1);
-	}
-	else
-	{
-		const bool all = STAGE == kStageDraft;
-		KEncodeStage<kD, STAGE><<<StageGrid(grid, job.total, TeamStage(STAGE) ? kWarpsPerCta : 1), kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, all ? nullptr : sg.list,
-			all ? nullptr : sg.count + STAGE, sg.counters + (STAGE + 1), T0, T1);
 	}
 	return cudaGetLastError();
 }
