@@ -384,6 +384,28 @@ struct PlaneLanes
 		}
 	}
 
+	__device__ __forceinline__ void Load(int (&e)[N], const int4* plane, int lane) const
+	{
+		const int* p = reinterpret_cast<const int*>(plane);
+#pragma unroll
+		for (int m = 0; m < N; m++)
+			e[m] = (32 / L) * m < np ? p[lane + 32 * m] : 0;
+	}
+
+	__device__ __forceinline__ void Store2(int4* plane, const int (&e)[N], int4* plane2, const int (&f)[N], int lane) const
+	{
+		int* p = reinterpret_cast<int*>(plane);
+		int* q = reinterpret_cast<int*>(plane2);
+#pragma unroll
+		for (int m = 0; m < N; m++)
+			if ((32 / L) * m < np)
+			{
+				p[lane + 32 * m] = e[m];
+				q[lane + 32 * m] = f[m];
+			}
+		__syncwarp();
+	}
+
 	__device__ __forceinline__ void Store(int4* plane, const int (&e)[N], int lane) const
 	{
 		int* p = reinterpret_cast<int*>(plane);
@@ -1064,7 +1086,11 @@ __device__ __forceinline__ int TableError(const int4* plane, const int4* table, 
  * w q^2 per pixel and level do not depend on the outer loops, so B's are kept
  * in the lane's registers (lane = candidate) and R's in a shared-memory
  * table, and a pixel costs one broadcast read of the plane and four fused
- * add-minimum steps instead of four differences, squares and products. */
+ * add-minimum steps instead of four differences, squares and products.  Two
+ * G candidates at a time share a pass over R's table, and an alpha
+ * candidate's R and G sums one over its plane: the sums are chains of shared
+ * loads, and two in flight hide each other's latency (mode 7 pass of a
+ * 1118x1105 alpha texture: 47.2 -> 45.1 ms). */
 template<int kD>
 __device__ __forceinline__ Found SearchFour2(SearchState& ss, const ChanList (&chan)[4], const int2 (*lists)[32], int v, const Area& ar, int count,
 	int np, bool opq, Weights w, const uint8_t* alphaTable, Ep best, int water, TeamSearch* team, int lane)
@@ -1138,17 +1164,23 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, const ChanList (&c
 		int errAR = l2.x + e0, errAG = l1.x + e0;
 		if (!opq)
 		{
-			const int sumR = TableError(pA, ss.table, at, np, lane < n2 ? water - ea - min1 - min3 : kNoLimit);
-			errAR = lane < n2 ? sumR + ea : kFar;
-			int sum = 0;
-			const int limit = lane < n1 ? water - ea - min2 - min3 : kNoLimit;
-			for (int i = 0; i < np; i++)
+			/* both in one pass over the plane */
+			const int limitR = lane < n2 ? water - ea - min1 - min3 : kNoLimit, limitG = lane < n1 ? water - ea - min2 - min3 : kNoLimit;
+			int sumR = 0, sumG = 0;
+			for (int i = 0; i < np; i += 2)
 			{
-				sum += RowMin(pA[i], LevelTerms<kD>(int(ar.px[i][1]), l1.y, w.g));
-				if (!__any_sync(kFull, sum < limit))
+#pragma unroll
+				for (int j = i; j < i + 2; j++)
+				{
+					const int4 row = pA[j];
+					sumR += RowMin(row, ss.table[j * kTableRow + at]);
+					sumG += j < np ? RowMin(row, LevelTerms<kD>(int(ar.px[j][1]), l1.y, w.g)) : 0;
+				}
+				if (!__any_sync(kFull, sumR < limitR || sumG < limitG))
 					break;
 			}
-			errAG = lane < n1 ? sum + ea : kFar;
+			errAR = lane < n2 ? sumR + ea : kFar;
+			errAG = lane < n1 ? sumG + ea : kFar;
 		}
 		const bool mine = stripes == 1 || (lane & 3) == unit;
 		int i1 = 0;
@@ -1158,50 +1190,82 @@ __device__ __forceinline__ Found SearchFour2(SearchState& ss, const ChanList (&c
 			const unsigned open1 = __ballot_sync(kFull, lane >= i1 && mine && l1.x + e0 + min2 + min3 < water && errAG + min2 + min3 < water);
 			if (!open1)
 				break;
-			i1 = __ffs(open1) - 1;
-			refresh(i0, i1);
-			const int place1 = i1;
-			const int eAG = __shfl_sync(kFull, errAG, i1);
-			const int2 g = make_int2(__shfl_sync(kFull, l1.x, i1), __shfl_sync(kFull, l1.y, i1));
-			i1++;
-			const bool openR = l2.x + eAG + min3 < water && errAR + g.x + min3 < water;
-			if (!__any_sync(kFull, openR))
-				continue;
-			pl.Add(gg, ga, xg, g.y, w.g);
-			pl.Store(pAG, gg, lane);
-			const int sumR = TableError(pAG, ss.table, at, np, openR ? water - ea - min3 : kNoLimit);
-			const int errAGR = openR ? sumR + ea : kFar;
-			unsigned open2 = __ballot_sync(kFull, errAGR + min3 < water);
-			if (!open2)
-				continue;
-			const bool openB = l3.x + eAG + min2 < water;
-			const int sumB = termsB.Error(pAG, np, w.b, openB ? water - ea - min2 : kNoLimit);
-			const int errAGB = openB ? sumB + ea : kFar;
-			while (open2)
+			/* two of them at a time: a pass over R's table serves both */
+			const int first = __ffs(open1) - 1, more = int(open1 & (open1 - 1));
+			const int second = more ? __ffs(more) - 1 : first;
+			i1 = second + 1;
+			refresh(i0, first);
+			const int colG[2] = { __shfl_sync(kFull, l1.y, first), __shfl_sync(kFull, l1.y, second) };
+			int errAGR[2];
 			{
-				const int i2 = __ffs(open2) - 1;
-				open2 &= open2 - 1;
-				const int e2 = __shfl_sync(kFull, errAGR, i2);
-				const int2 r = make_int2(__shfl_sync(kFull, l2.x, i2), __shfl_sync(kFull, l2.y, i2));
-				const bool eval = l3.x + e2 < water && errAGB + r.x < water;
-				if (!__any_sync(kFull, eval))
+				const int eAG0 = __shfl_sync(kFull, errAG, first), eAG1 = __shfl_sync(kFull, errAG, second);
+				const int eG0 = __shfl_sync(kFull, l1.x, first), eG1 = __shfl_sync(kFull, l1.x, second);
+				const bool openR0 = l2.x + eAG0 + min3 < water && errAR + eG0 + min3 < water;
+				const bool openR1 = more && l2.x + eAG1 + min3 < water && errAR + eG1 + min3 < water;
+				if (!__any_sync(kFull, openR0 || openR1))
 					continue;
-				const int* t = reinterpret_cast<const int*>(ss.table) + (pl.row * kTableRow + i2) * 4 + (lane & 3);
-				gr[0] = pl.row < np ? gg[0] + t[0] : 0;
-				gr[1] = pl.row + 8 < np ? gg[1] + t[8 * kTableRow * 4] : 0;
-				pl.Store(pAGR, gr, lane);
-				const int sum = termsB.Error(pAGR, np, w.b, eval ? water - ea : kNoLimit);
-				const int err = eval ? sum + ea : kFar;
-				/* the first lane of the smallest error below the water */
-				const int low = __reduce_min_sync(kFull, err);
-				if (low < water)
+				pl.Add(gg, ga, xg, colG[0], w.g);
+				pl.Add(gr, ga, xg, colG[1], w.g);
+				pl.Store2(pAG, gg, pAG + 32, gr, lane);
+				const int limit0 = openR0 ? water - ea - min3 : kNoLimit, limit1 = openR1 ? water - ea - min3 : kNoLimit;
+				int sum0 = 0, sum1 = 0;
+				for (int i = 0; i < np; i += 2)
 				{
-					const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
-					water = low;
-					if (!team)
-						best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, g.y), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
-					else if (lane == 0)
-						atomicMin(&team->key, (unsigned long long)(unsigned(low)) << 32 | SearchPlace(v, i0, place1, i2, j));
+#pragma unroll
+					for (int j = i; j < i + 2; j++)
+					{
+						const int4 t = ss.table[j * kTableRow + at];
+						sum0 += RowMin(pAG[j], t);
+						sum1 += RowMin(pAG[j + 32], t);
+					}
+					if (!__any_sync(kFull, sum0 < limit0 || sum1 < limit1))
+						break;
+				}
+				errAGR[0] = openR0 ? sum0 + ea : kFar;
+				errAGR[1] = openR1 ? sum1 + ea : kFar;
+			}
+#pragma unroll 1
+			for (int h = 0; h < 2; h++)
+			{
+				const int place1 = h ? second : first;
+				const int errR = h ? errAGR[1] : errAGR[0];
+				if (h)
+					refresh(i0, place1);
+				unsigned open2 = __ballot_sync(kFull, errR + min3 < water);
+				if (!open2)
+					continue;
+				const int4* const plane = pAG + 32 * h;
+				const int eAG = __shfl_sync(kFull, errAG, place1);
+				const bool openB = l3.x + eAG + min2 < water;
+				const int sumB = termsB.Error(plane, np, w.b, openB ? water - ea - min2 : kNoLimit);
+				const int errAGB = openB ? sumB + ea : kFar;
+				pl.Load(gg, plane, lane);
+				while (open2)
+				{
+					const int i2 = __ffs(open2) - 1;
+					open2 &= open2 - 1;
+					const int e2 = __shfl_sync(kFull, errR, i2);
+					const int2 r = make_int2(__shfl_sync(kFull, l2.x, i2), __shfl_sync(kFull, l2.y, i2));
+					const bool eval = l3.x + e2 < water && errAGB + r.x < water;
+					if (!__any_sync(kFull, eval))
+						continue;
+					const int* t = reinterpret_cast<const int*>(ss.table) + (pl.row * kTableRow + i2) * 4 + (lane & 3);
+					gr[0] = pl.row < np ? gg[0] + t[0] : 0;
+					gr[1] = pl.row + 8 < np ? gg[1] + t[8 * kTableRow * 4] : 0;
+					pl.Store(pAGR, gr, lane);
+					const int sum = termsB.Error(pAGR, np, w.b, eval ? water - ea : kNoLimit);
+					const int err = eval ? sum + ea : kFar;
+					/* the first lane of the smallest error below the water */
+					const int low = __reduce_min_sync(kFull, err);
+					if (low < water)
+					{
+						const int j = __ffs(__ballot_sync(kFull, err == low)) - 1;
+						water = low;
+						if (!team)
+							best = EpSetCh(EpSetCh(Ep2(0, a.y, 1, h ? colG[1] : colG[0]), 2, r.y), 3, __shfl_sync(kFull, l3.y, j));
+						else if (lane == 0)
+							atomicMin(&team->key, (unsigned long long)(unsigned(low)) << 32 | SearchPlace(v, i0, place1, i2, j));
+					}
 				}
 			}
 		}
