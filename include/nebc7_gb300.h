@@ -312,12 +312,12 @@ typedef struct nebc7_server_counters
    arrival order while the arena has room, and starts a batch of admitted
    requests on every free stream, so requests that arrive while others run
    join the device as soon as a stream and memory free up.  A batch is the
-   oldest admitted request and later ones of its kind: heavy presets (the
-   precise preset, /slow, /data) run as one staged launch (a kernel per
-   pass), light ones as one persistent launch with presets mixed, the
-   cheapest requests dealt first; each request of a light batch returns
-   (its blocks copied back) as soon as its own blocks are done, while the
-   rest of the launch still runs.  Besides the arena, every stream holds the
+   oldest admitted request and later ones of its kind: presets that run the
+   full searches on most blocks (the precise preset, /slow, /data) and the
+   other refining ones each as a staged launch (a kernel per pass), draft-only
+   ones as one persistent launch, the cheapest requests dealt first; each
+   request of a draft-only batch returns (its blocks copied back) as soon as
+   its own blocks are done, while the rest of the launch still runs.  Besides the arena, every stream holds the
    staged form's per-block state (its record, pass lists, split-pass rounds
    and kept results): 156 bytes per block for up to min(4194304,
    hbm_budget / 104) blocks. */

@@ -95,7 +95,7 @@ struct __align__(16) BlockRecord
 	int water;                   /* the error at the start of the draft chain */
 	int opaque;                  /* the whole-block area's opaque flag */
 	int handed;                  /* 1 + its slot of handed estimates, or 0 */
-	int pad;
+	int denoise;                 /* which of the two code paths (kD) it takes */
 };
 
 /* An improving candidate of a split pass: its endpoints, error and
@@ -195,7 +195,7 @@ struct Stages
 	int* hist;        /* [kNumStages][256] blocks per bucket of the passes' lists, zero before the draft kernel */
 	int* cursor;      /* [kNumStages][256] positions taken, zero before the draft kernel */
 	int total;        /* positions */
-	int byError;      /* whether the searches' lists go by error (else every list by position) */
+	int mixed;        /* whether blocks of both denoise forms are in the launch */
 	/* split passes */
 	int* start;       /* per position: the first candidate of the block's round */
 	int* firstImp;    /* per position: (candidate << 24) | result slot of the round's first improvement */
@@ -213,29 +213,39 @@ struct Stages
 
 /* Bucket of position k in the list of pass `stage`: 8 per octave of the
    error, largest first, for the searches (their cost grows with it: the
-   longest start first and no SM waits behind a late hard block), for the
-   refinement by kind and 1.6 per octave within it (so that the warps of an SM
-   run the same code), else by position. */
-__device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, int mode, bool opaque)
+   longest start first and no SM waits behind a late hard block), 4 per octave
+   and denoised blocks first in a mixed launch (the two forms are different
+   code), for the refinement by kind and 1.6 per octave within it (so that the
+   warps of an SM run the same code), else by position. */
+__device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, int mode, bool opaque, int denoise)
 {
-	if (!sg.byError || stage < kStepRefine || stage == kStepFinish)
+	if (stage < kStepRefine || stage == kStepFinish)
 		return int((long long)k * 256 / sg.total);
 	const unsigned e = unsigned(max(error, 1));
 	const int msb = 31 - __clz(e);
 	const int b = 255 - min(255, msb * 8 + int((e >> (msb >= 3 ? msb - 3 : 0)) & 7u));
+	const int kind = RefineKindOf(mode, opaque);
+	/* the buckets of the block's kind, and in a mixed launch the half of its
+	   denoise form */
+	int from = 0, width = 256;
 	if (stage == kStepRefine)
 	{
-		const int kind = RefineKindOf(mode, opaque);
-		return kind <= kRefine6 ? b * kRefineHeavy >> 8 : kRefineBuckets * kind + (b * kRefineBuckets >> 8);
+		width = kind <= kRefine6 ? kRefineHeavy : kRefineBuckets;
+		from = kind <= kRefine6 ? 0 : kRefineBuckets * kind;
 	}
-	return b;
+	if (sg.mixed)
+	{
+		width >>= 1;
+		from += denoise ? 0 : width;
+	}
+	return from + (b * width >> 8);
 }
 
 /* Records that position k waits for pass n (one thread). */
-__device__ __forceinline__ void Publish(const Stages& sg, int k, int n, int error, int mode, bool opaque)
+__device__ __forceinline__ void Publish(const Stages& sg, int k, int n, int error, int mode, bool opaque, int denoise)
 {
 	sg.next[k] = n;
-	atomicAdd(&sg.hist[n * 256 + StageBucket(sg, n, k, error, mode, opaque)], 1);
+	atomicAdd(&sg.hist[n * 256 + StageBucket(sg, n, k, error, mode, opaque, denoise)], 1);
 }
 
 __device__ __forceinline__ void SaveRecord(BlockRecord& r, const CellRegs& R, int lane)
@@ -598,10 +608,11 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 	if (lane == 0)
 	{
 		rec.handed = 0;
+		rec.denoise = kD;
 		rec.startLo = lo;
 		rec.startHi = hi;
 		rec.water = water;
-		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque);
+		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque, kD);
 	}
 	__syncwarp();
 	return false;
@@ -701,7 +712,7 @@ __device__ void PassStage(WarpState& st, SearchState& ss, const BlockRef& b, con
 	const int n = NextStep(S, R, P);
 	SaveRecord(rec, R, lane);
 	if (lane == 0)
-		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque);
+		Publish(sg, k, n, R.errTotal, R.bestMode, R.a1.opaque, kD);
 	__syncwarp();
 }
 
@@ -981,7 +992,7 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
 		R.denoiseStep = now.denoiseStep;
 			R.a1.opaque = now.opaque != 0;
 		r.handed = 0;
-		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.bestMode, now.opaque != 0);
+		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.bestMode, now.opaque != 0, now.denoise);
 	}
 	__threadfence();
 	atomicAdd(&q.finished, 1);
@@ -1177,7 +1188,7 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 	{
 		if (sg.next[k] != stage)
 			continue;
-		const int b = StageBucket(sg, stage, k, sg.rec[k].errTotal, sg.rec[k].bestMode, sg.rec[k].opaque != 0);
+		const int b = StageBucket(sg, stage, k, sg.rec[k].errTotal, sg.rec[k].bestMode, sg.rec[k].opaque != 0, sg.rec[k].denoise);
 		const int at = base[b] + atomicAdd(&sg.cursor[stage * 256 + b], 1);
 		sg.list[at] = k;
 		if (NT)
@@ -1234,7 +1245,7 @@ constexpr size_t StagedScratchBytes(int n)
 }
 
 /* Splits a staged scratch (256-byte aligned, StagedScratchBytes(n) bytes). */
-inline Stages SplitStaged(uint8_t* p, int n, bool byError)
+inline Stages SplitStaged(uint8_t* p, int n, bool mixed)
 {
 	Stages s;
 	s.count = (int*)p;
@@ -1243,7 +1254,7 @@ inline Stages SplitStaged(uint8_t* p, int n, bool byError)
 	s.hist = (int*)(p + 256 + kSplitPasses * sizeof(SplitQueue));
 	s.cursor = s.hist + kNumStages * 256;
 	s.total = n;
-	s.byError = byError;
+	s.mixed = mixed;
 	s.rec = (BlockRecord*)(p + kStagedZeroed);
 	uint8_t* q = p + kStagedZeroed + StagedAlign(size_t(n) * sizeof(BlockRecord));
 	const size_t ints = StagedAlign(size_t(n) * 4);

@@ -414,7 +414,7 @@ cudaError_t LaunchSlot(int slot, int grid, int ctasPerSm, cudaStream_t stream, c
 {
 	if (staged && kVariants[slot].staged)
 	{
-		const Stages sg = SplitStaged(staged, job.total, slot != kVariantMixed);
+		const Stages sg = SplitStaged(staged, job.total, slot == kVariantMixed);
 		const cudaError_t e = cudaMemsetAsync(staged, 0, kStagedZeroed, stream);
 		if (e != cudaSuccess)
 			return e;
@@ -1085,11 +1085,23 @@ namespace {
 constexpr size_t kServerBlockBytes = 64 + 16 + sizeof(BlockResult);
 constexpr int kServerStagedBlocks = 1 << 22;
 
-/* A request whose preset runs the full searches on most blocks (the
-   precise preset, /slow, /data). */
-bool HeavyRequest(const ServerRequest& r)
+/* The requests that share a launch: draft-only ones, the refining presets,
+   and those that run the full searches on most blocks (the precise preset,
+   /slow, /data).  The latter two take the staged form: the hard blocks of the
+   default preset's alpha textures keep a persistent launch waiting on a few
+   warps (24 mixed requests of 64 to 512 pixels a side: 244 ms with the default
+   preset's in one persistent launch with the draft ones, 115 ms). */
+enum RequestKind
 {
-	return BlockCost(r.settings) >= 400.0;
+	kRequestDraft,
+	kRequestRefined,
+	kRequestHeavy,
+};
+
+RequestKind KindOf(const ServerRequest& r)
+{
+	const double cost = BlockCost(r.settings);
+	return cost <= 1.0 ? kRequestDraft : (cost < 400.0 ? kRequestRefined : kRequestHeavy);
 }
 
 size_t RequestBytes(const ServerRequest& r)
@@ -1157,19 +1169,23 @@ int LaunchServerBatch(nebc7_server* sv, ServerSlot& slot, std::vector<int64_t>& 
 	job.status = slot.dCounter + 1;
 	job.order = nullptr;
 	job.single = slot.hTable[0];
-	const int grid = GridForSlot(total, kVariantMixed);
-	if (grid <= 0)
-		return SetError(NEBC7_ECUDA);
-	/* a batch of heavy requests takes the staged form (one kernel per pass);
-	   a batch of light ones the single kernel, whose blocks and so whose
-	   requests finish as they go */
-	bool heavy = total <= slot.stagedCap, slow = false;
+	/* draft-only requests take the single kernel, whose blocks and so whose
+	   requests finish as they go; the others the staged form (one kernel per
+	   pass) */
+	bool staged = total <= slot.stagedCap, slow = false;
+	int variant = VariantSlot(sv->reqs[batch[0]].settings);
 	for (int64_t id : batch)
 	{
-		heavy = heavy && HeavyRequest(sv->reqs[id]);
-		slow = slow || sv->reqs[id].settings.doSlow;
+		const nebc7_settings& s = sv->reqs[id].settings;
+		staged = staged && KindOf(sv->reqs[id]) != kRequestDraft;
+		slow = slow || s.doSlow;
+		if (VariantSlot(s) != variant)
+			variant = kVariantMixed;
 	}
-	CK(LaunchSlot(kVariantMixed, grid, 0, st, job, slow, *sv->T[0], *sv->T[1], heavy ? slot.staged : nullptr));
+	const int grid = GridForSlot(total, variant);
+	if (grid <= 0)
+		return SetError(NEBC7_ECUDA);
+	CK(LaunchSlot(variant, grid, 0, st, job, slow, *sv->T[0], *sv->T[1], staged ? slot.staged : nullptr));
 	CK(cudaEventRecord(slot.done, st));
 	slot.stage.assign(batch.size(), 0);
 	return NEBC7_OK;
@@ -1298,16 +1314,16 @@ void ServerLoop(nebc7_server* sv)
 			if (slot.busy || sv->admitted.empty())
 				continue;
 			/* the oldest admitted request and, in arrival order, others of its
-			   kind (heavy or light presets) up to max_batch requests and, for
-			   heavy ones, the staged records' capacity */
+			   kind up to max_batch requests and, for staged ones, the staged
+			   records' capacity */
 			std::vector<int64_t> batch;
-			const bool heavy = HeavyRequest(sv->reqs[sv->admitted.front()]);
+			const RequestKind kind = KindOf(sv->reqs[sv->admitted.front()]);
 			long long blocks = 0;
 			for (auto it = sv->admitted.begin(); it != sv->admitted.end() && int(batch.size()) < sv->cfg.max_batch;)
 			{
 				const ServerRequest& r = sv->reqs[*it];
 				const long long nb = (long long)(r.w / 4) * (r.h / 4);
-				if (HeavyRequest(r) != heavy || (!batch.empty() && heavy && blocks + nb > slot.stagedCap))
+				if (KindOf(r) != kind || (!batch.empty() && kind != kRequestDraft && blocks + nb > slot.stagedCap))
 				{
 					++it;
 					continue;
