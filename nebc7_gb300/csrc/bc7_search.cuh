@@ -823,6 +823,138 @@ __device__ __forceinline__ void StableSortOrder(int2* order, int n, int lane)
 	__syncwarp();
 }
 
+/* ---------------------------------------------------------------------- */
+/* A bound of every endpoint pair at once                                  */
+/* ---------------------------------------------------------------------- */
+
+/* The channels of a bound: their weights' roots (zero outside), the sum and
+   the least of the weights. */
+struct LineWeights
+{
+	float root[4], sum;
+	int least;
+};
+
+__device__ __forceinline__ LineWeights LineWeightsOf(const Params& P, unsigned channels)
+{
+	LineWeights lw;
+	lw.sum = 0.0f;
+	lw.least = 0x7FFFFFFF;
+#pragma unroll
+	for (int c = 0; c < 4; c++)
+	{
+		const int w = (channels >> c) & 1 ? ChannelWeight(P, c) : 0;
+		lw.root[c] = sqrtf(float(w));
+		lw.sum += float(w);
+		if ((channels >> c) & 1)
+			lw.least = min(lw.least, w);
+	}
+	return lw;
+}
+
+/* Sums of pixels' values and products (the upper triangle) over the channels
+   FIRST..3. */
+template<int FIRST>
+struct Moments
+{
+	int n, sum[4], xy[4][4];
+};
+
+/* A lower bound of the error of the pixels of `mo` in one subset, whatever its
+   endpoints and indices: the levels of a subset lie on a line of color space
+   but for their rounding, and no line comes closer to the pixels than their
+   principal axis.
+ *
+ * With weighted channels (x_c sqrt(w_c)) the squared distances to the best line
+ * sum to trace - l, l the largest eigenvalue of the scatter matrix M, and
+ * l^4 <= |M^4| (Frobenius).  An interpolated level is at most 1/2 from the
+ * line in each channel, and 2 |d >> 1| at most 1 from |d| (kD 1), so the root
+ * of the error falls short of the root of that sum by at most
+ * (1/2 or 3/2) sqrt(n sum(w)); with kD 0 a difference past 127 counts as 127,
+ * and such a candidate's error is at least 127^2 of the least weight.  The
+ * moments are exact (n sum(x y) < 2^24); the factors next to 1 cover the float
+ * arithmetic on them, about 1e-6.
+ *
+ * It ends most partitions of mode 7 before their scans (1118x1105 alpha texture,
+ * default: 45.1 -> 13.4 ms of the pass; 1700x940: 1013 -> 173 ms of the call),
+ * a quarter of the time of mode 1's.  The three-subset and rotation searches go
+ * without: their blocks' errors are near the rounding slack, and the bound cost
+ * more than it saved (precise 1024x1024 photo 40.1 -> 47.6 ms). */
+template<int kD, int FIRST>
+__device__ __forceinline__ int LineBoundOf(const Moments<FIRST>& mo, const LineWeights& lw)
+{
+	const float n = float(mo.n);
+	float m[4][4], trace = 0.0f;
+#pragma unroll
+	for (int c = FIRST; c < 4; c++)
+#pragma unroll
+		for (int d = c; d < 4; d++)
+		{
+			m[c][d] = m[d][c] = float(mo.n * mo.xy[c][d] - mo.sum[c] * mo.sum[d]) * (lw.root[c] * lw.root[d]);
+			if (c == d)
+				trace += m[c][c];
+		}
+	if (mo.n < 3 || !(trace > 0.0f))
+		return 0;   /* two pixels lie on a line */
+	const float scale = 1.0f / trace;
+#pragma unroll
+	for (int c = FIRST; c < 4; c++)
+#pragma unroll
+		for (int d = FIRST; d < 4; d++)
+			m[c][d] *= scale;
+	float norm = 0.0f;
+#pragma unroll
+	for (int step = 0; step < 2; step++)
+	{
+		float q[4][4];
+		norm = 0.0f;
+#pragma unroll
+		for (int c = FIRST; c < 4; c++)
+#pragma unroll
+			for (int d = c; d < 4; d++)
+			{
+				float t = 0.0f;
+#pragma unroll
+				for (int k = FIRST; k < 4; k++)
+					t += m[c][k] * m[k][d];
+				q[c][d] = q[d][c] = t;
+				norm += c == d ? t * t : 2.0f * t * t;
+			}
+#pragma unroll
+		for (int c = FIRST; c < 4; c++)
+#pragma unroll
+			for (int d = FIRST; d < 4; d++)
+				m[c][d] = q[c][d];
+	}
+	/* |M^4| = sqrt(norm); its fourth root, of a trace of 1 */
+	const float top = sqrtf(sqrtf(sqrtf(norm))) * 1.00001f + 0.00001f;
+	const float off = trace / n * fmaxf(1.0f - top, 0.0f) * 0.99999f;
+	const float root = fmaxf(sqrtf(off) - (kD ? 1.5f : 0.5f) * 1.00001f * sqrtf(n * lw.sum), 0.0f);
+	const int b = int(fminf(root * root * (kD ? 0.25f : 1.0f) * 0.9999f, 1.0e9f));
+	return kD ? b : min(b, lw.least * 127 * 127);
+}
+
+/* LineBoundOf for the first np pixels of an area.  Warp-collective. */
+template<int kD, int FIRST>
+__device__ __forceinline__ int LineBound(const Area& ar, int np, const LineWeights& lw, int lane)
+{
+	Moments<FIRST> mo;
+	mo.n = np;
+	int x[4];
+#pragma unroll
+	for (int c = FIRST; c < 4; c++)
+	{
+		x[c] = lane < np ? int(ar.px[lane][c]) : 0;
+		mo.sum[c] = int(__reduce_add_sync(kFull, unsigned(x[c])));
+	}
+#pragma unroll
+	for (int c = FIRST; c < 4; c++)
+#pragma unroll
+		for (int d = c; d < 4; d++)
+			mo.xy[c][d] = int(__reduce_add_sync(kFull, unsigned(x[c] * x[d])));
+	return LineBoundOf<kD, FIRST>(mo, lw);
+}
+
 /* The estimates of partition p of a full search of modes 0 and 2 (the first
    loop of src/Bc7CoreMode0.cpp:532-642): its subsets' estimates to out.three,
    and whether they leave room below the error. */
@@ -937,10 +1069,20 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 	int line0, int line1, int lane)
 {
 	const int room = R.errTotal - R.denoiseStep - R.opaqueAlphaError;
+	const LineWeights lw = LineWeightsOf(P, 14);
+	int low[2] = { 0, 0 };
 #pragma unroll 1
 	for (int s = 0; s < 2; s++)
 	{
 		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		low[0] = low[1];
+		low[1] = LineBound<kD, 1>(st.sub[s], st.sub[s].info.active, lw, lane);
+	}
+	if (low[0] + low[1] >= room)
+		return false;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
 		const int water = room - line1 - (s == 0 ? 0 : line0);
 		const int line = EstimateLevels3<kD>(ss, st.sub[s], P, sp, water, ss.bound[s], lane);
 		if (s == 0)
@@ -950,6 +1092,8 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 		if (!((s == 0 ? line0 : line1) < water))
 			return false;
 	}
+	if (max(line0, low[0]) + max(line1, low[1]) >= room)
+		return false;
 	Team one = SingleWarp();
 	Ep mc0 = 0, mc1 = 0;
 	int error = 0;
@@ -963,6 +1107,8 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 		if (!any || !(r < water))
 			return false;
 		error += r;
+		if (s == 0 && error + low[1] >= room)
+			return false;
 		if (s == 0)
 			mc0 = b;
 		else
@@ -1558,7 +1704,7 @@ __device__ NEBC7_PASS void FullMode6(WarpState& st, SearchState& ss, CellRegs& R
 	const int step = R.denoiseStep;
 	/* EstimateBest (src/Bc7CoreMode6.cpp:1383-1396): 0 without OPTION_PCA */
 	const int line = P.pca ? PcaBound<kD>(st.area1, R.a1, P, R.a1.opaque ? 3 : 4, lane) : 0;
-	if (line < R.errTotal - step)
+	if (line < R.errTotal - step && LineBound<kD, 0>(st.area1, st.area1.info.active, LineWeightsOf(P, 15), lane) < R.errTotal - step)
 	{
 		Ep mc = 0;
 		const int error = CompressSubsetSingle<kD, 6>(ss, st.area1, P, T, mc, R.errTotal - step, team, ts, lane);
@@ -1652,10 +1798,20 @@ __device__ __forceinline__ bool Mode7Partition(WarpState& st, SearchState& ss, C
 	int p, int line0, int line1, int lane)
 {
 	const int room = R.errTotal - R.denoiseStep;
+	const LineWeights lw = LineWeightsOf(P, 15);
+	int low[2] = { 0, 0 };
 #pragma unroll 1
 	for (int s = 0; s < 2; s++)
 	{
 		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		low[0] = low[1];
+		low[1] = LineBound<kD, 0>(st.sub[s], st.sub[s].info.active, lw, lane);
+	}
+	if (low[0] + low[1] >= room)
+		return false;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
 		const int water = room - line1 - (s == 0 ? 0 : line0);
 		const int line = EstimateLevels7<kD>(ss, st.sub[s], P, T, water, ss.bound[s], lane);
 		if (s == 0)
@@ -1705,12 +1861,23 @@ __device__ __forceinline__ bool Mode7PartitionTeam(WarpState& st, SearchState& s
 {
 	Team team{ 4, rank, &ts.exchange, 0 };
 	const int room = R.errTotal - R.denoiseStep;
-	int line1 = 0, used = 0;
+	const LineWeights lw = LineWeightsOf(P, 15);
+	int line1 = 0, used = 0, low[2];
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		const int b = LineBound<kD, 0>(st.sub[s], st.sub[s].info.active, lw, lane);
+		low[1] = b;
+		if (s == 0)
+			low[0] = b;
+	}
+	if (low[0] + low[1] >= room)
+		return false;
 #pragma unroll 1
 	for (int s = 0; s < 2; s++)
 	{
 		const Area& ar = st.sub[s];
-		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
 		const int water = room - used;
 		int l = 0;
 		if (ar.info.active && (rank || !ar.info.opaque) && water > 0)
@@ -1726,6 +1893,8 @@ __device__ __forceinline__ bool Mode7PartitionTeam(WarpState& st, SearchState& s
 			return false;
 		used += error;
 		line1 = error;
+		if (s == 0 ? max(error, low[0]) + low[1] >= room : max(used - error, low[0]) + max(error, low[1]) >= room)
+			return false;
 	}
 	Ep mc0 = 0, mc1 = 0;
 	int error = 0;
@@ -1739,6 +1908,8 @@ __device__ __forceinline__ bool Mode7PartitionTeam(WarpState& st, SearchState& s
 		if (!any || !(r < water))
 			return false;
 		error += r;
+		if (s == 0 && error + low[1] >= room)
+			return false;
 		if (s == 0)
 			mc0 = b;
 		else
@@ -1903,6 +2074,16 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 		ctab = T.d2v8;
 		atab = T.d2v8;
 	}
+	/* With every visible pixel's masks full the bounds are lower bounds (the
+	   slot channel's list error is its exact error, and a hidden pixel counts
+	   with its alpha of 0 alone): the three channels that share the colour
+	   index are searched by SearchThree, the slot channel's one candidate a
+	   constant.  Other masks can make a bound exceed the error, and the
+	   reference's order of tests decides: TryVariantsRot. */
+	bool full = true;
+	if (lane < ai.active)
+		full = (ar.mk[lane][0] & ar.mk[lane][1] & ar.mk[lane][2] & ar.mk[lane][3]) == 0xFFFF;
+	full = __all_sync(kFull, full);
 	int used = 0;
 #pragma unroll 1
 	for (int c = 0; c < 4; c++)
@@ -1923,16 +2104,7 @@ __device__ NEBC7_PASS int CompressRotSubset(WarpState& st, SearchState& ss, cons
 	}
 	__syncwarp();
 	const int rot = rotation & 3;
-	/* With every visible pixel's masks full the bounds are lower bounds (the
-	   slot channel's list error is its exact error, and a hidden pixel counts
-	   with its alpha of 0 alone): the three channels that share the colour
-	   index are searched by SearchThree, the slot channel's one candidate a
-	   constant.  Other masks can make a bound exceed the error, and the
-	   reference's order of tests decides: TryVariantsRot. */
-	bool full = true;
-	if (lane < ai.active)
-		full = (ar.mk[lane][0] & ar.mk[lane][1] & ar.mk[lane][2] & ar.mk[lane][3]) == 0xFFFF;
-	if (__all_sync(kFull, full))
+	if (full)
 	{
 		const int x = a == 0 ? 1 : 0, y = a <= 1 ? 2 : 1, z = a == 3 ? 2 : 3;
 		auto channel = [&](int c) {

@@ -1,0 +1,46 @@
+"""Partitions passed over by the principal-axis bound of their subsets, where
+it lies closest to the error: the pixels of each half on a line of the four
+channels, with noise from none to the rounding slack and past it, and values at
+the ends of the scale, whose differences the undenoised error caps.  Against
+the CPU oracle port; blocks and integer error sums are bit-exact."""
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from nebc7_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def blocks(kind, n, seed):
+    rng = synth.SplitMix64(seed)
+    if kind == "extremes":
+        px = rng.below(2, n * 64).reshape(n, 16, 4) * 255
+        px[::3] = np.where(rng.below(8, px[::3].size).reshape(px[::3].shape) == 0, 128, px[::3])
+    else:
+        ends = rng.below(256, n * 16).reshape(n, 2, 2, 4)
+        half = np.arange(16) % 4 // 2                       # left and right columns
+        t = (np.arange(16) * 5 % 16)[None, :, None] / 15.0
+        a, b = ends[:, 0][:, half], ends[:, 1][:, half]
+        amp = np.array([0, 1, 4, 24])[np.arange(n) % 4][:, None, None]
+        noise = rng.below(1 << 16, n * 64).reshape(n, 16, 4) % (2 * amp + 1) - amp
+        px = np.clip(np.rint(a + (b - a) * t) + noise, 0, 255)
+    return px.reshape(n, 64).astype(np.uint8), np.full((n, 64), 255, np.uint8)
+
+
+@pytest.mark.parametrize("kind,n", [("lines", 32), ("extremes", 9)])
+@pytest.mark.parametrize("denoise,step,slow", [(1, 9, 0), (1, 9, 1), (0, 0, 1)])
+def test_bounded_partitions_match_oracle(native, port, kind, n, denoise, step, slow):
+    from nebc7_gb300._native import Settings
+    c, m = blocks(kind, n, 300 + n)
+    st = Settings(denoise, step, 1, 1, slow, 0)
+    a, b = np.zeros((n, 16), np.uint8), np.zeros((n, 16), np.uint8)
+    e1, _ = port.compress_blocks(c, m, a, denoise, step, 1, 1, slow, 0, threads=16)
+    e2 = np.zeros(2, np.int64)
+    assert native.nebc7_encode_blocks_host(c.ctypes.data, m.ctypes.data, b.ctypes.data, n, ctypes.byref(st), e2.ctypes.data,
+                                           None) == 0
+    bad = np.nonzero((a != b).any(1))[0]
+    assert len(bad) == 0, f"{len(bad)} blocks differ, first {bad[:8].tolist()}"
+    assert e1.tolist() == e2.tolist()
