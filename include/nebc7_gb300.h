@@ -130,6 +130,13 @@ int nebc7_encode_device(uint8_t* d_dst, const uint8_t* d_bgra, const uint8_t* d_
 int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long stride, int w, int h,
 	const nebc7_settings* settings, int64_t* errs, double* ssim);
 
+/* As nebc7_encode_host for an unpadded host image (w x h pixels, `stride`
+   bytes a row, at most 16384 a side once padded): it is padded and, with
+   radius >= 0, masked on the device as nebc7_prepare_device does (-1: no
+   mask).  dst holds the padded texture's blocks. */
+int nebc7_encode_image_host(uint8_t* dst, const uint8_t* bgra, long long stride, int w, int h, int radius,
+	const nebc7_settings* settings, int64_t* errs, double* ssim);
+
 /* Independent blocks: cells / masks hold 64 bytes per block (4 rows of 4
    pixels), io 16 bytes per block (starting block in, result out).  Host
    buffers. */

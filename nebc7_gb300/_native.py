@@ -156,6 +156,7 @@ SIGNATURES = {
     "nebc7_set_preset": (I, [I, I]),
     "nebc7_last_error": (I, []),
     "nebc7_encode_device": (I, [VP, VP, VP, LL, I, I, ctypes.POINTER(Settings), VP, VP, VP]),
+    "nebc7_encode_image_host": (I, [VP, VP, LL, I, I, I, ctypes.POINTER(Settings), VP, VP]),
     "nebc7_encode_host": (I, [VP, VP, VP, LL, I, I, ctypes.POINTER(Settings), VP, VP]),
     "nebc7_encode_blocks_host": (I, [VP, VP, VP, I, ctypes.POINTER(Settings), VP, VP]),
     "nebc7_decode_device": (I, [VP, VP, LL, I, I, VP]),

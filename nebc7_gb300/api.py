@@ -125,6 +125,17 @@ class Bc7Core:
                                           _ptr(err), _ptr(ssim)), "process_texture")
         return EncodeStats(int(err[0]), int(err[1]), float(ssim[0]), float(ssim[1]))
 
+    def process_image(self, dst: np.ndarray, img_bgra: np.ndarray, radius: int) -> EncodeStats:
+        """process_texture of an unpadded C-contiguous BGRA image, padded and
+        (radius >= 0) masked on the device (src/Bc7Compress.cpp:33-105, 397-426)."""
+        h, w = img_bgra.shape[:2]
+        err = np.zeros(2, np.int64)
+        ssim = np.zeros(2, np.float64)
+        s = self.settings()
+        check(self._lib.nebc7_encode_image_host(_ptr(dst), _ptr(img_bgra), w * 4, w, h, radius, ctypes.byref(s),
+                                                _ptr(err), _ptr(ssim)), "process_image")
+        return EncodeStats(int(err[0]), int(err[1]), float(ssim[0]), float(ssim[1]))
+
 
 def padded_size(w: int, h: int) -> tuple[int, int]:
     """src/Bc7Compress.cpp:397-398: at least 4, rounded up to a multiple of 4."""
@@ -215,13 +226,22 @@ def encode_image(img_bgra: np.ndarray, flags: str = "", preset: Preset = DEFAULT
                  start: np.ndarray | None = None) -> EncodedImage:
     """The CLI's encode path on an in-memory BGRA image (top-down rows)."""
     o = parse_flags(flags)
-    padded = pad_texture(np.ascontiguousarray(img_bgra, dtype=np.uint8))
-    ph, pw = padded.shape[:2]
-    mask = outline_mask(padded, o["radius"]) if o["mask"] else None
+    img = np.ascontiguousarray(img_bgra, dtype=np.uint8)
+    # the device pads and masks; numpy took 14 of 53 ms for a 1118x1105 image
+    on_device = img.ndim == 3 and img.shape[2] == 4 and min(img.shape) > 0 and max(padded_size(*img.shape[:2])) <= 16384
+    if on_device:
+        pw, ph = padded_size(img.shape[1], img.shape[0])
+    else:
+        padded = pad_texture(img)
+        ph, pw = padded.shape[:2]
+        mask = outline_mask(padded, o["radius"]) if o["mask"] else None
     core = Bc7Core(preset)
     core.init_tables(o["draft"], o["normal"], o["slow"], o["linear"])
     blocks = np.zeros(((ph // 4) * (pw // 4), 16), np.uint8) if start is None else np.array(start, np.uint8)
-    stats = core.process_texture(blocks, padded, mask, pw, ph)
+    if on_device:
+        stats = core.process_image(blocks, img, o["radius"] if o["mask"] else -1)
+    else:
+        stats = core.process_texture(blocks, padded, mask, pw, ph)
     return EncodedImage(blocks, pw, ph, stats)
 
 

@@ -1586,13 +1586,42 @@ int nebc7_encode_device(uint8_t* d_dst, const uint8_t* d_bgra, const uint8_t* d_
 	return LaunchEncode(d_dst, d_bgra, d_mask, stride, w / 4, int(nb), *settings, errs, ssim, (cudaStream_t)stream);
 }
 
-int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long stride, int w, int h,
+namespace {
+
+/* Pads the image and, with a mask, outlines it (nebc7_prepare_device, checked
+   arguments). */
+int PrepareTexture(const uint8_t* d_src, long long src_stride, int w, int h, uint8_t* d_padded, uint8_t* d_mask, int radius, cudaStream_t st)
+{
+	const int pw = (std::max(4, w) + 3) & ~3, ph = (std::max(4, h) + 3) & ~3;
+	const dim3 tiles((pw + 255) / 256, (ph + kPadRows - 1) / kPadRows);
+	const bool wide = !(((uintptr_t)d_padded | (uintptr_t)d_mask) & 15);
+	if (d_mask && radius >= 0 && radius <= kOutlineRadius)
+		(wide ? KPadTexture<true, true> : KPadTexture<true, false>)<<<tiles, 256, PadSharedBytes(radius), st>>>(d_src, src_stride, w, h, d_padded,
+			(long long)pw * 4, pw, ph, radius, d_mask);
+	else
+	{
+		(wide ? KPadTexture<false, true> : KPadTexture<false, false>)<<<tiles, 256, 0, st>>>(d_src, src_stride, w, h, d_padded,
+			(long long)pw * 4, pw, ph, 0, nullptr);
+		if (d_mask)
+			KOutlineMask<<<dim3((pw + 255) / 256, ph), 256, 0, st>>>(d_padded, (long long)pw * 4, pw, ph, radius, d_mask);
+	}
+	CK(cudaGetLastError());
+	return NEBC7_OK;
+}
+
+/* An unpadded host image, padded and masked on the device: its size and the
+   outline radius of its mask (-1: no mask). */
+struct RawImage
+{
+	int w, h, radius;
+};
+
+/* Encodes a host texture of padded size w x h from scratch or from dst's
+   blocks: `bgra` and `mask` padded, or `bgra` the image `raw` describes. */
+int EncodeHost(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long stride, int w, int h, const RawImage* raw,
 	const nebc7_settings* settings, int64_t* errs, double* ssim)
 {
-	if (int e = ValidateSettings(settings))
-		return SetError(e);
-	if (w <= 0 || h <= 0 || (w & 3) || (h & 3) || stride < (long long)w * 4)
-		return SetError(NEBC7_EINVAL);
+	const bool outline = raw && raw->radius >= 0;
 	const size_t nb = size_t(w / 4) * (h / 4);
 	const size_t img = size_t(w) * 4 * h;
 	if (nb > size_t(0x7FFFFFFF))
@@ -1604,7 +1633,8 @@ int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, lo
 		return SetError(NEBC7_ECUDA);
 	const size_t offImg = Align256(nb * 16);
 	const size_t offMask = offImg + Align256(img);
-	const size_t offScratch = offMask + (mask ? Align256(img) : 0);
+	const size_t offRaw = offMask + (mask || outline ? Align256(img) : 0);
+	const size_t offScratch = offRaw + (raw ? Align256(size_t(raw->w) * 4 * raw->h) : 0);
 	if (!ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, *settings)))
 	{
 		ReleaseSlot(slot);
@@ -1613,9 +1643,19 @@ int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, lo
 	cudaStream_t st = slot->stream;
 	uint8_t* dd = slot->buf;
 	uint8_t* db = slot->buf + offImg;
-	uint8_t* dm = mask ? slot->buf + offMask : nullptr;
+	uint8_t* dm = mask || outline ? slot->buf + offMask : nullptr;
 	int rc = NEBC7_OK;
-	if (cudaMemcpy2DAsync(db, size_t(w) * 4, bgra, size_t(stride), size_t(w) * 4, size_t(h), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+	if (raw)
+	{
+		const size_t row = size_t(raw->w) * 4;
+		uint8_t* dr = slot->buf + offRaw;
+		if (cudaMemcpy2DAsync(dr, row, bgra, size_t(stride), row, size_t(raw->h), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+			cudaMemcpyAsync(dd, dst, nb * 16, cudaMemcpyHostToDevice, st) != cudaSuccess)
+			rc = SetError(NEBC7_ECUDA);
+		else
+			rc = PrepareTexture(dr, (long long)row, raw->w, raw->h, db, dm, raw->radius, st);
+	}
+	else if (cudaMemcpy2DAsync(db, size_t(w) * 4, bgra, size_t(stride), size_t(w) * 4, size_t(h), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 		(mask && cudaMemcpy2DAsync(dm, size_t(w) * 4, mask, size_t(stride), size_t(w) * 4, size_t(h), cudaMemcpyHostToDevice, st) != cudaSuccess) ||
 		cudaMemcpyAsync(dd, dst, nb * 16, cudaMemcpyHostToDevice, st) != cudaSuccess)
 		rc = SetError(NEBC7_ECUDA);
@@ -1643,6 +1683,32 @@ int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, lo
 		cudaStreamSynchronize(st);
 	ReleaseSlot(slot);
 	return rc;
+}
+
+} // namespace
+
+int nebc7_encode_host(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long stride, int w, int h,
+	const nebc7_settings* settings, int64_t* errs, double* ssim)
+{
+	if (int e = ValidateSettings(settings))
+		return SetError(e);
+	if (w <= 0 || h <= 0 || (w & 3) || (h & 3) || stride < (long long)w * 4)
+		return SetError(NEBC7_EINVAL);
+	return EncodeHost(dst, bgra, mask, stride, w, h, nullptr, settings, errs, ssim);
+}
+
+int nebc7_encode_image_host(uint8_t* dst, const uint8_t* bgra, long long stride, int w, int h, int radius,
+	const nebc7_settings* settings, int64_t* errs, double* ssim)
+{
+	if (int e = ValidateSettings(settings))
+		return SetError(e);
+	if (w <= 0 || h <= 0 || stride < (long long)w * 4 || radius < -1)
+		return SetError(NEBC7_EINVAL);
+	const int pw = (std::max(4, w) + 3) & ~3, ph = (std::max(4, h) + 3) & ~3;
+	if (std::max(pw, ph) > 16384)
+		return SetError(NEBC7_ETOOBIG);
+	const RawImage raw{ w, h, radius };
+	return EncodeHost(dst, bgra, nullptr, stride, pw, ph, &raw, settings, errs, ssim);
 }
 
 int nebc7_encode_blocks_host(const uint8_t* cells, const uint8_t* masks, uint8_t* io, int n,
@@ -2223,21 +2289,7 @@ int nebc7_prepare_device(const uint8_t* d_src, long long src_stride, int w, int 
 	const int pw = (std::max(4, w) + 3) & ~3, ph = (std::max(4, h) + 3) & ~3;
 	if (std::max(pw, ph) > 16384)
 		return SetError(NEBC7_ETOOBIG);
-	const cudaStream_t st = (cudaStream_t)stream;
-	const dim3 tiles((pw + 255) / 256, (ph + kPadRows - 1) / kPadRows);
-	const bool wide = !(((uintptr_t)d_padded | (uintptr_t)d_mask) & 15);
-	if (d_mask && radius >= 0 && radius <= kOutlineRadius)
-		(wide ? KPadTexture<true, true> : KPadTexture<true, false>)<<<tiles, 256, PadSharedBytes(radius), st>>>(d_src, src_stride, w, h, d_padded,
-			(long long)pw * 4, pw, ph, radius, d_mask);
-	else
-	{
-		(wide ? KPadTexture<false, true> : KPadTexture<false, false>)<<<tiles, 256, 0, st>>>(d_src, src_stride, w, h, d_padded,
-			(long long)pw * 4, pw, ph, 0, nullptr);
-		if (d_mask)
-			KOutlineMask<<<dim3((pw + 255) / 256, ph), 256, 0, st>>>(d_padded, (long long)pw * 4, pw, ph, radius, d_mask);
-	}
-	CK(cudaGetLastError());
-	return NEBC7_OK;
+	return PrepareTexture(d_src, src_stride, w, h, d_padded, d_mask, radius, (cudaStream_t)stream);
 }
 
 int nebc7_bad_blocks_device(const uint8_t* d_src, const uint8_t* d_decoded, const uint8_t* d_mask, long long stride, int w, int h,
