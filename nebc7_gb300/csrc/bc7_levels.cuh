@@ -215,27 +215,32 @@ struct ValueGroup
 	}
 };
 
+/* The rest of a lane's error sum after its first group of four values (`s`),
+   given up after a group once no lane's sum is at most `limit`.  Returns
+   whether some lane's is.  Warp-collective. */
+template<bool SQUARED>
+__device__ __forceinline__ bool CandidateRest(const uint8_t* row, const int2* values, int n, bool on, int limit, int& s)
+{
+	for (int u = 4;; u += 4)
+	{
+		if (!__any_sync(kFull, on && s <= limit))
+			return false;
+		if (u >= n)
+			return true;
+		ValueGroup g;
+		g.Load(values + u);
+		s += int(g.Sum<SQUARED>(row));
+	}
+}
+
 /* Error sum of a lane's candidate (`row`: its place in the table, the values'
-   offsets go from there), given up after a group of four values once no
-   lane's sum is at most `limit`.  Returns whether some lane's is.
-   Warp-collective. */
+   offsets go from there), given up as CandidateRest. */
 template<bool SQUARED>
 __device__ __forceinline__ bool CandidateSum(const uint8_t* row, const ValueGroup& first, const int2* values, int n, bool on, int limit,
 	int& sum)
 {
-	unsigned s = first.Sum<SQUARED>(row);
-	for (int u = 4;; u += 4)
-	{
-		if (!__any_sync(kFull, on && int(s) <= limit))
-			return false;
-		if (u >= n)
-			break;
-		ValueGroup g;
-		g.Load(values + u);
-		s += g.Sum<SQUARED>(row);
-	}
-	sum = int(s);
-	return true;
+	sum = int(first.Sum<SQUARED>(row));
+	return CandidateRest<SQUARED>(row, values, n, on, limit, sum);
 }
 
 /* Sets node 0 (a zero-error candidate) of a list. */
@@ -310,8 +315,9 @@ __device__ __forceinline__ int ValueStride(int shift, bool byDiff)
 
 /* LevelsBuffer and LevelsBufferHalf: writes up to maxSize nodes (err, color).
  *
- * What bounds it: instruction issue, about 1200 candidates a scan in the
- * default preset.  Every row of the window has the same candidates (low
+ * What bounds it: the latency of the table reads (256 KB, mostly in L2), about
+ * 1200 candidates a scan in the default preset and 4000 in an alpha block's
+ * mode 6; two batches are in flight at a time.  Every row of the window has the same candidates (low
  * endpoints up to the window's, rounded up as the reference's 16-wide chunks
  * do), so rows and columns are taken as one sequence of candidates in
  * ascending order, 32 a batch with every lane in use, and a batch ends after
@@ -373,34 +379,54 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	unsigned thr = 0xFFFFFFFFu;
 	int row = start / rowLen, col = start - row * rowLen;
 	int iH = win.HL + (pvar ? pH : 0);   /* the batch's first row */
-	while (iH < win.HH)
-	{
-		const int myH = iH + row * step;
-		const bool on = myH < win.HH;
-		const int cc = on ? (myH << shift) + col * step + (pvar ? pL : 0) : 0;
-		int s;
-		if (CandidateSum<HALF>(table + CandidateBase(cc, shift, byDiff), first, values, n, on, limit, s))
-		{
-			const unsigned key = (unsigned(s) << 16) | unsigned(cc);
-			const unsigned want = __ballot_sync(kFull, on && s <= limit && key < thr);
-			if (want)
-			{
-				list = MergeTop(list, key, want, lane, maxSize);
-				thr = __shfl_sync(kFull, list, maxSize - 1);
-				limit = min(limit, int(thr >> 16));
-				/* maxSize zero-error candidates found: later ones (larger c)
-				   cannot enter */
-				if (thr < 0x10000u)
-					break;
-			}
-		}
-		/* the next candidates; row stays relative to the batch's first */
+	/* the next candidates; row stays relative to the batch's first */
+	auto advance = [&]() {
 		row += stepRows;
 		col += stepCols;
 		if (col >= rowLen)
 		{
 			col -= rowLen;
 			row++;
+		}
+	};
+	while (iH < win.HH)
+	{
+		/* two batches at a time */
+		int cc[2];
+		bool on[2];
+#pragma unroll
+		for (int h = 0; h < 2; h++)
+		{
+			const int myH = iH + row * step;
+			on[h] = myH < win.HH;
+			cc[h] = on[h] ? (myH << shift) + col * step + (pvar ? pL : 0) : 0;
+			advance();
+		}
+		const uint8_t* const place[2] = { table + CandidateBase(cc[0], shift, byDiff), table + CandidateBase(cc[1], shift, byDiff) };
+		const unsigned s0 = first.Sum<HALF>(place[0]), s1 = first.Sum<HALF>(place[1]);
+		if (__any_sync(kFull, (on[0] && int(s0) <= limit) || (on[1] && int(s1) <= limit)))
+		{
+#pragma unroll 1
+			for (int h = 0; h < 2; h++)
+			{
+				const bool mine = h ? on[1] : on[0];
+				int s = int(h ? s1 : s0);
+				if (CandidateRest<HALF>(h ? place[1] : place[0], values, n, mine, limit, s))
+				{
+					const unsigned key = (unsigned(s) << 16) | unsigned(h ? cc[1] : cc[0]);
+					const unsigned want = __ballot_sync(kFull, mine && s <= limit && key < thr);
+					if (want)
+					{
+						list = MergeTop(list, key, want, lane, maxSize);
+						thr = __shfl_sync(kFull, list, maxSize - 1);
+						limit = min(limit, int(thr >> 16));
+					}
+				}
+			}
+			/* maxSize zero-error candidates found: later ones (larger c)
+			   cannot enter */
+			if (thr < 0x10000u)
+				break;
 		}
 		const int ahead = __shfl_sync(kFull, row, 0);
 		iH += ahead * step;

@@ -68,22 +68,26 @@ constexpr int kStepNone = -1;   /* finished in the first kernel (an exact starti
    searches first. */
 enum RefineKind
 {
-	kRefine7 = 0,
-	kRefine6,        /* modes 6 and 6Index2 of blocks with alpha */
+	kRefine6 = 0,    /* mode 6 of blocks with alpha */
+	kRefine7,
+	kRefine6Index2,  /* of blocks with alpha */
 	kRefineOpaque,   /* modes 0-3 */
 	kRefineRot,      /* modes 4 and 5 */
-	kRefine6Opaque,  /* modes 6 and 6Index2 of opaque blocks: one p-bit variant, one alpha candidate */
+	kRefineEasy,     /* modes 6 and 6Index2 of opaque blocks: one p-bit variant, one alpha candidate */
+	kRefineKinds
 };
 
 __device__ __forceinline__ int RefineKindOf(int mode, bool opaque)
 {
-	return mode < 4 ? kRefineOpaque : (mode < 6 ? kRefineRot : (mode == 7 ? kRefine7 : (opaque ? kRefine6Opaque : kRefine6)));
+	if (mode < 6)
+		return mode < 4 ? kRefineOpaque : kRefineRot;
+	return mode == 7 ? kRefine7 : (opaque ? kRefineEasy : (mode == 6 ? kRefine6 : kRefine6Index2));
 }
 
 /* Buckets of the refinement's list per kind; the first ones, modes 6, 6Index2
    and 7 of blocks with alpha, can search long. */
-constexpr int kRefineBuckets = 51;
-constexpr int kRefineHeavy = 2 * kRefineBuckets;
+constexpr int kRefineBuckets = 256 / kRefineKinds;
+constexpr int kRefineHeavy = kRefineOpaque * kRefineBuckets;
 
 /* A block's Cell scalars between pass kernels. */
 struct __align__(16) BlockRecord
@@ -215,7 +219,7 @@ struct Stages
    error, largest first, for the searches (their cost grows with it: the
    longest start first and no SM waits behind a late hard block), 4 per octave
    and denoised blocks first in a mixed launch (the two forms are different
-   code), for the refinement by kind and 1.6 per octave within it (so that the
+   code), for the refinement by kind and 1.3 per octave within it (so that the
    warps of an SM run the same code), else by position. */
 __device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, int error, int mode, bool opaque, int denoise)
 {
@@ -230,8 +234,8 @@ __device__ __forceinline__ int StageBucket(const Stages& sg, int stage, int k, i
 	int from = 0, width = 256;
 	if (stage == kStepRefine)
 	{
-		width = kind <= kRefine6 ? kRefineHeavy : kRefineBuckets;
-		from = kind <= kRefine6 ? 0 : kRefineBuckets * kind;
+		width = kRefineBuckets;
+		from = kRefineBuckets * kind;
 	}
 	if (sg.mixed)
 	{
@@ -420,13 +424,14 @@ __device__ __forceinline__ void RunStep(WarpState& st, SearchState& ss, CellRegs
 			const unsigned stAt = unsigned(__cvta_generic_to_shared(&st));
 			const unsigned tablesAt = unsigned(__cvta_generic_to_shared(&T));
 			const unsigned tsAt = unsigned(__cvta_generic_to_shared(ts));
-			switch (RefineKindOf(R.bestMode, false))
-			{
-			case kRefine7: RefineOne<kD, kRefine7>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
-			case kRefineOpaque: RefineOne<kD, kRefineOpaque>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
-			case kRefineRot: RefineOne<kD, kRefineRot>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
-			default: RefineOne<kD, kRefine6>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane); break;
-			}
+			if (R.bestMode < 4)
+				RefineOne<kD, kRefineOpaque>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane);
+			else if (R.bestMode < 6)
+				RefineOne<kD, kRefineRot>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane);
+			else if (R.bestMode == 7)
+				RefineOne<kD, kRefine7>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane);
+			else
+				RefineOne<kD, kRefine6>(R, stAt, tablesAt, tsAt, team.size, team.rank, lane);
 		}
 		R.personalParam = R.bestParam;
 		R.personalMode = R.bestMode;
