@@ -443,7 +443,8 @@ struct TeamState
 	TeamExchange exchange;
 	int bound[2][4];       /* [subset][channel] estimates */
 	int valid;             /* variants whose lists leave room */
-	int task[3];           /* the CTA's task: queue position, candidate, first improvement */
+	int task[4];           /* the CTA's tasks: queue position, first candidate, first improvement, how many */
+	int open[4];           /* which of them are open */
 };
 
 /* Starts a team's search from `water`; the last one's outcome is read. */
@@ -1845,6 +1846,21 @@ __device__ __forceinline__ bool Mode7Partition(WarpState& st, SearchState& ss, C
 	R.bestParam = p;
 	R.bestMode = 7;
 	return error <= 0;
+}
+
+/* Whether the line bounds of partition p's subsets leave room for mode 7. */
+template<int kD>
+__device__ __forceinline__ bool Mode7Open(WarpState& st, const CellRegs& R, const Params& P, int p, int lane)
+{
+	const LineWeights lw = LineWeightsOf(P, 15);
+	int low = 0;
+#pragma unroll 1
+	for (int s = 0; s < 2; s++)
+	{
+		BuildSubset<kD>(st, R, P, st.sub[s], 2, p, s, true, lane);
+		low += LineBound<kD, 0>(st.sub[s], st.sub[s].info.active, lw, lane);
+	}
+	return low < R.errTotal - R.denoiseStep;
 }
 
 /* Mode7Partition by the CTA's four warps: the four channels' estimates, the

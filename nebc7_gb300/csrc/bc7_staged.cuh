@@ -917,6 +917,20 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 	atomicMin(sg.firstImp + k, (p << 24) | slot);
 }
 
+/* Whether candidate p of the block at position k can improve on the error at
+   the start of the round, as far as the line bound tells (mode 7). */
+template<int kD, int S>
+__device__ NEBC7_PASS bool SplitOpen(WarpState& st, const BlockRef& b, const Params& P, const Stages& sg, int k, int p, int lane)
+{
+	if constexpr (SplitMode(S) == 7)
+	{
+		CellRegs R;
+		RestoreBlock(st, R, b, sg.rec[k], P, lane);
+		return !(R.personalMode == 7 && R.personalParam == p) && Mode7Open<kD>(st, R, P, p, lane);
+	}
+	return true;
+}
+
 /* The end of a block's round of split pass S (one thread, after its last
    task): the first improving candidate f becomes the block's best and ends
    the pass, or the block goes on from f + 1 in a later round with the new
@@ -1009,7 +1023,7 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
    Returns the task's entry * NT + candidate, the later rounds' entries after
    the first round's n, or -1. */
 template<int S>
-__device__ __forceinline__ long long SplitTake(const Stages& sg, SplitQueue& q, int n, bool& firstRound)
+__device__ __forceinline__ long long SplitTake(const Stages& sg, SplitQueue& q, int n, bool& firstRound, int grab = 1)
 {
 	constexpr int NT = SplitTasks(S);
 	for (int polls = 0; polls < kSplitPolls;)
@@ -1028,7 +1042,8 @@ __device__ __forceinline__ long long SplitTake(const Stages& sg, SplitQueue& q, 
 		}
 		if (firstRound)
 		{
-			const int t = atomicAdd(&q.head, 1);
+			/* `grab` first-round tasks from here (NT is a multiple of it) */
+			const int t = atomicAdd(&q.head, grab);
 			if (t < n * NT)
 				return t;
 			firstRound = false;
@@ -1047,6 +1062,12 @@ __host__ __device__ constexpr int SplitTeam(int S)
 	return S == kStepMode7 ? kWarpsPerCta : 1;
 }
 
+/* From this many blocks on, a team takes four mode 7 candidates at a time, whose
+   bounds its warps compute beside each other: three of four candidates end
+   there (1118x1105 alpha texture, 3455 blocks: 13.5 -> 11.4 ms).  A shorter list
+   would leave CTAs without a task while others search four in turn. */
+constexpr int kGrabBlocks = 1024;
+
 /* Split pass S over the blocks list[i], i < *count (at most kSplitMaxBlocks).
    The tasks (block, candidate p) are taken block by block, so that the
    candidates of a block go to as many warps; a block's last task commits the
@@ -1059,7 +1080,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 {
 	constexpr int NT = SplitTasks(S), N = SplitTeam(S);
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
-	__shared__ TeamState team;
+	__shared__ TeamState ts;
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(S, true));
@@ -1069,37 +1090,46 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 	SplitQueue& q = sg.split[SplitIndex(S)];
 	const int n = min(*count, ThreeSubsetStep(S) ? sg.handedCap : kSplitMaxBlocks);
 	const int rank = N > 1 ? warp : 0;   /* within the task's warps */
+	const int grab = N > 1 && n >= kGrabBlocks ? N : 1;
 	bool firstRound = true;
+	/* task t: the block's position k and candidate p (-1 if the round starts
+	   after it), and the first improvement so far */
+	auto task = [&](long long t, int& k, int& p, int& first) {
+		const long long e = t / NT;
+		p = int(t % NT);
+		k = e < n ? list[e] : *reinterpret_cast<volatile int*>(sg.later + (e - n));
+		if (p < *reinterpret_cast<volatile int*>(sg.start + k))
+			p = -1;
+		first = *reinterpret_cast<volatile int*>(sg.firstImp + k);
+	};
 	for (;;)
 	{
-		int k = -1, p = 0, first = 0;
+		int k = -1, p = 0, first = 0, count = 1;
 		if (rank == 0 && lane == 0)
 		{
-			const long long t = SplitTake<S>(sg, q, n, firstRound);
+			const long long t = SplitTake<S>(sg, q, n, firstRound, grab);
 			if (t >= 0)
-			{
-				const long long e = t / NT;
-				p = int(t % NT);
-				k = e < n ? list[e] : *reinterpret_cast<volatile int*>(sg.later + (e - n));
-				if (p < *reinterpret_cast<volatile int*>(sg.start + k))
-					p = -1;
-				/* one read for all the task's warps: other warps lower it meanwhile */
-				first = *reinterpret_cast<volatile int*>(sg.firstImp + k);
-			}
+				task(t, k, p, first);
+			if (N > 1)
+				count = grab > 1 && t >= 0 && t < (long long)n * NT ? grab : 1;
 		}
 		if (N > 1)
 		{
 			__syncthreads();   /* the last task's shared state is read */
 			if (threadIdx.x == 0)
 			{
-				team.task[0] = k;
-				team.task[1] = p;
-				team.task[2] = first;
+				/* one read of the first improvement for all the task's warps:
+				   other warps lower it meanwhile */
+				ts.task[0] = k;
+				ts.task[1] = p;
+				ts.task[2] = first;
+				ts.task[3] = count;
 			}
 			__syncthreads();
-			k = team.task[0];
-			p = team.task[1];
-			first = team.task[2];
+			k = ts.task[0];
+			p = ts.task[1];
+			first = ts.task[2];
+			count = ts.task[3];
 		}
 		else
 		{
@@ -1109,7 +1139,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		}
 		if (k < 0)
 			break;
-		if (p < 0)
+		if (p < 0 && count == 1)
 			continue;
 		TexDesc d;
 		BlockRef b;
@@ -1121,27 +1151,60 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 			   pass runs whole, in one warp */
 			if (rank == 0 && lane == 0)
 				sg.firstImp[k] = kSplitSerial;
+			first = kSplitSerial;
 			__syncwarp();
 		}
-		else if constexpr (kD == kAnyDenoise)
+		/* of several tasks (of one block, from candidate p on), each warp
+		   looks whether one is open */
+		unsigned open = 1;
+		if (N > 1 && count > 1)
 		{
-			if (d.denoise)
-				SplitTask<1, S, N>(st, ss, &team, b, tables[1], P, sg, q, k, p, first, rank, lane);
-			else
-				SplitTask<0, S, N>(st, ss, &team, b, tables[0], P, sg, q, k, p, first, rank, lane);
-		}
-		else
-			SplitTask<kD, S, N>(st, ss, &team, b, tables[kD], P, sg, q, k, p, first, rank, lane);
-		/* every warp of a team has read the block's record before its round can
-		   end and change it */
-		if (N > 1)
+			bool mine = false;
+			if ((first >> 24) >= p + warp)
+			{
+				if constexpr (kD == kAnyDenoise)
+				{
+					if (d.denoise)
+						mine = SplitOpen<1, S>(st, b, P, sg, k, p + warp, lane);
+					else
+						mine = SplitOpen<0, S>(st, b, P, sg, k, p + warp, lane);
+				}
+				else
+					mine = SplitOpen<kD, S>(st, b, P, sg, k, p + warp, lane);
+			}
+			if (lane == 0)
+				ts.open[warp] = mine;
 			__syncthreads();
-		else
-			__syncwarp();
+			open = 0;
+			for (int j = 0; j < N; j++)
+				open |= unsigned(ts.open[j]) << j;
+		}
+		else if (first == kSplitSerial)
+			open = 0;
+		while (open)
+		{
+			const int at = p + __ffs(open) - 1;
+			open &= open - 1;
+			if constexpr (kD == kAnyDenoise)
+			{
+				if (d.denoise)
+					SplitTask<1, S, N>(st, ss, &ts, b, tables[1], P, sg, q, k, at, first, rank, lane);
+				else
+					SplitTask<0, S, N>(st, ss, &ts, b, tables[0], P, sg, q, k, at, first, rank, lane);
+			}
+			else
+				SplitTask<kD, S, N>(st, ss, &ts, b, tables[kD], P, sg, q, k, at, first, rank, lane);
+			/* every warp of a team has read the block's record before its round
+			   can end and change it, and the task's shared state */
+			if (N > 1)
+				__syncthreads();
+			else
+				__syncwarp();
+		}
 		if (rank == 0 && lane == 0)
 		{
 			__threadfence();
-			if (atomicSub(sg.pending + k, 1) == 1)
+			if (atomicSub(sg.pending + k, count) == count)
 			{
 				__threadfence();
 				SplitCommit<S>(job, sg, q, k);

@@ -44,3 +44,28 @@ def test_bounded_partitions_match_oracle(native, port, kind, n, denoise, step, s
     bad = np.nonzero((a != b).any(1))[0]
     assert len(bad) == 0, f"{len(bad)} blocks differ, first {bad[:8].tolist()}"
     assert e1.tolist() == e2.tolist()
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1030])
+def test_long_lists_equal_short_ones(native, n):
+    """A list of 1024 blocks or more takes its mode 7 candidates four at a time,
+    a shorter one singly: the blocks of one call equal those of calls of a third."""
+    from nebc7_gb300._native import Settings
+    rng = synth.SplitMix64(n)
+    c = (96 + rng.below(64, n * 64)).reshape(n, 64).astype(np.uint8)
+    m = np.full((n, 64), 255, np.uint8)
+    st = Settings(1, 9, 1, 1, 0, 0)
+
+    def encode(lo, hi):
+        out = np.zeros((hi - lo, 16), np.uint8)
+        cc, mm = np.ascontiguousarray(c[lo:hi]), np.ascontiguousarray(m[lo:hi])
+        e = np.zeros(2, np.int64)
+        assert native.nebc7_encode_blocks_host(cc.ctypes.data, mm.ctypes.data, out.ctypes.data, hi - lo, ctypes.byref(st),
+                                               e.ctypes.data, None) == 0
+        return out, e
+
+    whole, errors = encode(0, n)
+    cuts = [0, n // 3, 2 * n // 3, n]
+    parts = [encode(a, b) for a, b in zip(cuts, cuts[1:])]
+    assert (whole == np.concatenate([p[0] for p in parts])).all()
+    assert (errors == sum(p[1] for p in parts)).all()
