@@ -409,30 +409,14 @@ constexpr size_t EncodeSharedBytes()
 	return kWarpsPerCta * (sizeof(WarpState) + (NORMAL ? sizeof(SearchState) : 0));
 }
 
-/* Code shapes of the refining kernel.  Compact: every routine inlined (the
-   fastest for the default preset, whose time goes to one refinement).
-   Outlined: the routines the full searches call from many places kept out
-   of line (NEBC7_SHARED) and registers bounded for 4 CTAs per SM (the
-   fastest for the precise preset, /slow and /data, whose time goes to the
-   full searches).  The translation unit of an instantiation chooses
-   NEBC7_SHARED to match. */
-constexpr int kShapeCompact = 0;
-constexpr int kShapeOutlined = 1;
-
-/* Resident CTAs per SM the compact refining kernel is compiled for (bounds
-   its registers per thread; the draft-only kernels and the outlined shape
-   are compiled for 4). */
-#ifndef NEBC7_COMPACT_MIN_CTAS
-#define NEBC7_COMPACT_MIN_CTAS 1
-#endif
-
 /* Persistent encode kernel over a launch's textures.  NORMAL compiles the
    refinement / full-search passes (run for textures whose preset asks for
    them); only that instantiation reserves the per-warp search state in
-   shared memory.  kD: the kDenoise of every texture, or kAnyDenoise. */
-template<int kD, bool NORMAL, int SHAPE>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, (SHAPE == kShapeOutlined || !NORMAL) ? 4 : NEBC7_COMPACT_MIN_CTAS)
-	KEncode(Job job, LevelTables T0, LevelTables T1)
+   shared memory, and keeps the routines the full searches call from many places
+   out of line (NEBC7_PASS, NEBC7_SHARED, set by its translation unit).  kD: the
+   kDenoise of every texture, or kAnyDenoise. */
+template<int kD, bool NORMAL>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncode(Job job, LevelTables T0, LevelTables T1)
 {
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
 	const int lane = threadIdx.x & 31;
@@ -456,10 +440,10 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, (SHAPE == kShapeOutlined ||
 /* Host-side launchers of KEncode.  Each instantiation is compiled in a
    translation unit of its own (encode_d<kD>_<passes>.cu), so they build in
    parallel; the C ABI layer only sees these declarations. */
-template<int kD, bool NORMAL, int SHAPE>
+template<int kD, bool NORMAL>
 cudaError_t LaunchEncodeKernel(int grid, cudaStream_t stream, const Job& job, const LevelTables& T0, const LevelTables& T1);
 
-template<int kD, bool NORMAL, int SHAPE>
+template<int kD, bool NORMAL>
 cudaError_t EncodeKernelOccupancy(int* ctasPerSm);
 
 } // namespace nebc7

@@ -1,5 +1,5 @@
-/* Staged encode kernels: kDenoise read per texture (mixed batches);
-   one kernel per pass, the pass-level routines out of line. */
+/* Staged encode kernels: kDenoise read per texture (mixed batches); one kernel
+   per pass, everything but the refinement's kinds inlined. */
 #define NEBC7_PASS __forceinline__
 #define NEBC7_SHARED __forceinline__
 #define NEBC7_ONCE __noinline__

@@ -1,5 +1,6 @@
-/* Staged encode kernels: differences halved (kDenoise 1: /slow and /data);
-   one kernel per pass, the pass-level routines out of line. */
+/* Staged encode kernels: differences halved (kDenoise 1: the default preset,
+   /slow and /data); one kernel per pass, everything but the refinement's kinds
+   inlined. */
 #define NEBC7_PASS __forceinline__
 #define NEBC7_SHARED __forceinline__
 #define NEBC7_ONCE __noinline__

@@ -201,10 +201,11 @@ int ValidateSettings(const nebc7_settings* s)
 	return NEBC7_OK;
 }
 
-/* The encode instantiations: denoise shift x passes x code shape.  The
-   outlined ones also have a staged form (bc7_staged.cuh: one kernel per
-   pass), used where the launch has room for its per-block records; the
-   single kernel serves the allocation-free entry and the request loop. */
+/* The encode instantiations: denoise shift x passes.  The refining ones also
+   have a staged form (bc7_staged.cuh: one kernel per pass), used where the
+   launch has room for its per-block records; their single kernel serves the
+   allocation-free entry, batches whose plan asks for it and server batches
+   larger than a stream's records. */
 struct EncodeVariant
 {
 	cudaError_t (*launch)(int, cudaStream_t, const Job&, const LevelTables&, const LevelTables&);
@@ -216,13 +217,13 @@ struct EncodeVariant
 constexpr int kNumVariants = 5;
 constexpr int kVariantMixed = 4;   /* batches: kDenoise per texture */
 const EncodeVariant kVariants[kNumVariants] = {
-	{ LaunchEncodeKernel<0, false, kShapeCompact>, EncodeKernelOccupancy<0, false, kShapeCompact>, nullptr, nullptr },
-	{ LaunchEncodeKernel<0, true, kShapeOutlined>, EncodeKernelOccupancy<0, true, kShapeOutlined>,
+	{ LaunchEncodeKernel<0, false>, EncodeKernelOccupancy<0, false>, nullptr, nullptr },
+	{ LaunchEncodeKernel<0, true>, EncodeKernelOccupancy<0, true>,
 	  LaunchStagedEncode<0>, StagedEncodeOccupancy<0> },
-	{ LaunchEncodeKernel<1, false, kShapeCompact>, EncodeKernelOccupancy<1, false, kShapeCompact>, nullptr, nullptr },
-	{ LaunchEncodeKernel<1, true, kShapeOutlined>, EncodeKernelOccupancy<1, true, kShapeOutlined>,
+	{ LaunchEncodeKernel<1, false>, EncodeKernelOccupancy<1, false>, nullptr, nullptr },
+	{ LaunchEncodeKernel<1, true>, EncodeKernelOccupancy<1, true>,
 	  LaunchStagedEncode<1>, StagedEncodeOccupancy<1> },
-	{ LaunchEncodeKernel<kAnyDenoise, true, kShapeOutlined>, EncodeKernelOccupancy<kAnyDenoise, true, kShapeOutlined>,
+	{ LaunchEncodeKernel<kAnyDenoise, true>, EncodeKernelOccupancy<kAnyDenoise, true>,
 	  LaunchStagedEncode<kAnyDenoise>, StagedEncodeOccupancy<kAnyDenoise> },
 };
 
