@@ -315,13 +315,15 @@ __device__ __forceinline__ int ValueStride(int shift, bool byDiff)
 
 /* LevelsBuffer and LevelsBufferHalf: writes up to maxSize nodes (err, color).
  *
- * What bounds it: the latency of the table reads (256 KB, mostly in L2), about
- * 1200 candidates a scan in the default preset and 4000 in an alpha block's
- * mode 6; two batches are in flight at a time.  Every row of the window has the same candidates (low
- * endpoints up to the window's, rounded up as the reference's 16-wide chunks
- * do), so rows and columns are taken as one sequence of candidates in
- * ascending order, 32 a batch with every lane in use, and a batch ends after
- * the four values that reject most unless a lane can still enter the list. */
+ * What bounds it: the latency of the table reads (256 KB, mostly in L2) and the
+ * chains behind them, about 1200 candidates a scan in the default preset and
+ * 4000 in an alpha block's mode 6; so two batches are in flight at a time
+ * (64x64 icon 0.76 -> 0.73 ms, refinement of a 1024x1024 photo, precise, 8.6 ->
+ * 8.2).  Every row of the window has the same candidates (low endpoints up to
+ * the window's, rounded up as the reference's 16-wide chunks do), so rows and
+ * columns are taken as one sequence of candidates in ascending order, 32 a
+ * batch with every lane in use, and a batch ends after the four values that
+ * reject most unless a lane can still enter the list. */
 template<int kD, bool HALF>
 __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
 	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, Team& team, int lane)

@@ -1,41 +1,47 @@
 /*
- * BC7 block encoder for sm_103a -- the staged encode of the presets whose
- * time goes to the full searches (precise, /slow, /data, mixed batches).
+ * BC7 block encoder for sm_103a -- the staged encode of every refining preset
+ * (default, precise, /slow, /data, mixed batches).
  *
  * The per-block pipeline of src/Bc7Core.cpp:1516-1823 runs as a sequence of
  * persistent kernels instead of one: the start of the draft chain (the
  * starting block, the Mode6Index2 and mode 6 fast passes), the rest of the
- * draft chain in four kernels, one kernel per refinement / full-search pass
- * of the normal and slow chains (src/Bc7Core.cpp:1604-1745), then the final
- * pack, self-check and quality sums.  Every kernel holds the code of one or
- * two passes, so the warps of an SM run the same few kilobytes of
- * instructions; in a single kernel whose warps
- * sit in different passes the instruction working set outgrows the
- * instruction cache and most issue slots are lost to instruction fetch.
+ * draft chain, the refinement, one or two kernels per full-search pass of the
+ * normal and slow chains (src/Bc7Core.cpp:1604-1745), then the final pack,
+ * self-check and quality sums.  The warps of an SM so run the same few
+ * kilobytes of instructions; in a single kernel whose warps sit in different
+ * passes the instruction working set outgrows the instruction cache and most
+ * issue slots are lost to instruction fetch.  And a pass can hand its hard
+ * blocks to several warps: a 1000x516 alpha texture of the default preset took
+ * 424 ms in one kernel, a single block most of them, and takes 32 ms so.
  *
  * Between kernels a block's state (the reference's Cell scalars: best
  * endpoints, mode, partition, errors, stepping values, the starting block)
  * is kept in a BlockRecord per queue position; the pixel data and the
- * whole-block area are rebuilt from the texture when a pass starts.  Each
- * pass kernel runs the blocks whose next pass it is, gathered by
- * KStageList (queue order) or KStageListByError (largest error first).
+ * whole-block area are rebuilt from the texture when a pass starts.  A block
+ * that ends a pass counts itself into a bucket of its next one (Publish,
+ * StageBucket), and KStageList gathers each pass's blocks bucket by bucket.
  * The passes, their order and their entry conditions are those of
  * NormalPasses, so the blocks are the same bits as the single-kernel
  * encode's.
  *
- * The full searches of modes 1, 3 and 7 (64 two-subset partitions each)
- * and of modes 4 and 5 (8 and 4 rotation / index-size choices) are split
- * passes: a few hard blocks take most of their time, and one warp per block
- * would leave the GPU waiting for them.  A split pass runs in rounds.  In a
- * round every candidate (partition or rotation) of every block in the
- * round's list is a task of its own, taken by any warp, searched from the
- * block's error at the start of the round.  The candidates before a block's
- * first improving candidate f searched from that error, as the reference's
- * loop does, so their verdicts stand; f's result is the reference's too.
- * The round's commit applies f and ends the pass, or the block continues
- * in the next round from candidate f + 1 with the new error.  Improvements
- * are rare, so most blocks finish in the first round; blocks still
- * searching after SplitRounds(S) rounds finish their pass in one warp each.
+ * The searches of a few hard blocks take most of a pass, and one warp per
+ * block would leave the GPU waiting for them.  So
+ * - the refinement, the three-subset searches and the full mode 6 search run
+ *   their few or first blocks with a CTA's four warps each (TeamBlocks);
+ * - the full searches of modes 1, 3 and 7 (64 two-subset partitions each) and of
+ *   modes 4 and 5 (8 and 4 rotation / index-size choices) are split passes, and
+ *   so are the partitions that the estimates of modes 2 and 0 leave of a block
+ *   (ThreeSubsetsStage).
+ * A split pass runs in rounds.  In a round every candidate (partition or
+ * rotation) of a block is a task of its own, searched from the block's error at
+ * the start of the round.  The candidates before the block's first improving
+ * candidate f searched from that error, as the reference's loop does, so their
+ * verdicts stand; f's result is the reference's too.  The block's last task
+ * commits the round: it applies f and ends the pass, or appends the block's
+ * next round, from candidate f + 1 with the new error, to the queue that the
+ * running warps take tasks from.  Improvements are rare, so most blocks finish
+ * in the first round.  Blocks whose result was not kept, or that must run whole
+ * (OPTION_PCA), finish the pass in one warp each.
  */
 #pragma once
 

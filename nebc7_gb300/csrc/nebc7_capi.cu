@@ -398,12 +398,21 @@ cudaError_t EnqueueBlockOrder(const uint8_t* bgra, long long stride, int blocksW
 	return cudaGetLastError();
 }
 
+/* The most blocks of a staged launch, whose lists are indexed with ints past
+   their ends: 42 GB of records.  The single kernel takes more. */
+constexpr int kStagedMaxBlocks = 1 << 28;
+
+bool TakesStaged(const nebc7_settings& s, int nblocks)
+{
+	return SlotStaged(VariantSlot(s)) && nblocks <= kStagedMaxBlocks;
+}
+
 /* Scratch of one encode launch: the staged form adds its per-block records
    after the EncodeScratchBytes pieces. */
-size_t LaunchScratchBytes(int nblocks, bool wantSums, const nebc7_settings& s)
+size_t LaunchScratchBytes(int nblocks, bool wantSums, bool staged)
 {
 	const size_t base = (EncodeScratchBytes(nblocks, wantSums) + 255) & ~size_t(255);
-	return SlotStaged(VariantSlot(s)) ? base + StagedScratchBytes(nblocks) : base;
+	return staged ? base + StagedScratchBytes(nblocks) : base;
 }
 
 /* Launches the encode of `job` with instantiation `slot`: the staged form
@@ -429,10 +438,11 @@ cudaError_t LaunchSlot(int slot, int grid, int ctasPerSm, cudaStream_t stream, c
 }
 
 /* Enqueues one encode.  `scratchIn` (LaunchScratchBytes bytes, 256-byte
-   aligned) is used when given, otherwise the scratch is taken from the
-   stream-ordered allocator. */
+   aligned, for the staged form if `stagedIn`) is used when given, otherwise the
+   scratch is taken from the stream-ordered allocator; without room for the
+   staged form's records the single kernel encodes. */
 int LaunchEncode(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long stride, int blocksW, int nblocks,
-	const nebc7_settings& s, int64_t* errs, double* ssim, cudaStream_t stream, uint8_t* scratchIn = nullptr)
+	const nebc7_settings& s, int64_t* errs, double* ssim, cudaStream_t stream, uint8_t* scratchIn = nullptr, bool stagedIn = false)
 {
 	if (nblocks <= 0)
 	{
@@ -450,8 +460,15 @@ int LaunchEncode(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long lo
 
 	const bool wantSums = errs || ssim;
 	uint8_t* scratch = scratchIn;
-	if (!scratch && cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, s), stream) != cudaSuccess)
-		return SetError(NEBC7_ENOMEM);
+	bool useStaged = scratch ? stagedIn : TakesStaged(s, nblocks);
+	if (!scratch && cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, useStaged), stream) != cudaSuccess)
+	{
+		cudaGetLastError();
+		const bool retry = useStaged;
+		useStaged = false;
+		if (!retry || cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, false), stream) != cudaSuccess)
+			return SetError(NEBC7_ENOMEM);
+	}
 	const EncodeScratch e = SplitScratch(scratch, nblocks, wantSums);
 	int* status = e.status;
 	long long* sums = e.sums;
@@ -473,7 +490,7 @@ int LaunchEncode(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long lo
 		return SetError(NEBC7_ECUDA);
 	}
 	const int slot = VariantSlot(s);
-	uint8_t* staged = SlotStaged(slot) ? scratch + ((EncodeScratchBytes(nblocks, wantSums) + 255) & ~size_t(255)) : nullptr;
+	uint8_t* staged = useStaged ? scratch + ((EncodeScratchBytes(nblocks, wantSums) + 255) & ~size_t(255)) : nullptr;
 	CK(LaunchSlot(slot, grid, 0, stream, job, s.doSlow != 0, *T, *T, staged));
 
 	int rc = NEBC7_OK;
@@ -801,7 +818,7 @@ void BuildSchedule(nebc7_batch* b, int which)
 		g.orderOff = ooff;
 		ooff += (long long)OrderScratchBytes(g.total);
 		g.stagedOff = -1;
-		if (SlotStaged(g.slot) && g.total > 0)
+		if (SlotStaged(g.slot) && g.total > 0 && g.total <= kStagedMaxBlocks)
 		{
 			g.stagedOff = off;
 			off += (long long)((StagedScratchBytes(g.total) + 255) & ~size_t(255));
@@ -1636,7 +1653,15 @@ int EncodeHost(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long
 	const size_t offMask = offImg + Align256(img);
 	const size_t offRaw = offMask + (mask || outline ? Align256(img) : 0);
 	const size_t offScratch = offRaw + (raw ? Align256(size_t(raw->w) * 4 * raw->h) : 0);
-	if (!ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, *settings)))
+	bool staged = TakesStaged(*settings, int(nb));
+	bool room = ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, staged));
+	if (!room && staged)
+	{
+		cudaGetLastError();
+		staged = false;
+		room = ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, false));
+	}
+	if (!room)
 	{
 		ReleaseSlot(slot);
 		return SetError(NEBC7_ENOMEM);
@@ -1663,7 +1688,7 @@ int EncodeHost(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long
 	int64_t e[2];
 	double q[2];
 	if (rc == NEBC7_OK)
-		rc = LaunchEncode(dd, db, dm, (long long)w * 4, w / 4, int(nb), *settings, e, q, st, slot->buf + offScratch);
+		rc = LaunchEncode(dd, db, dm, (long long)w * 4, w / 4, int(nb), *settings, e, q, st, slot->buf + offScratch, staged);
 	if (rc == NEBC7_OK && (cudaMemcpyAsync(dst, dd, nb * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
 		cudaStreamSynchronize(st) != cudaSuccess))
 		rc = SetError(NEBC7_ECUDA);
