@@ -159,11 +159,10 @@ def issue_roofline(prof, kernel_ms, sm_mhz, n_sms):
     clock sampled during the timed region.  The instructions per launch come
     from the committed ncu capture of the same workload and the same CUDA
     sources (None when the capture is of another build, or without a clock
-    sample).  kernel_ms is the CUDA-event time of the encode call: KEncode
-    plus, for the refining presets, the two block-order kernels in front of
-    it (KBlockBuckets, KBlockOrder; about 13 us of a 5.5 ms call); for a
-    staged encode every pass kernel, and the capture's instruction count is
-    the sum over the same launches."""
+    sample).  kernel_ms is the CUDA-event time of the encode call: KEncode for
+    the draft-only presets, the two block-order kernels and every pass kernel
+    of the staged encode for the refining ones; the capture's instruction count
+    is the sum over the same launches."""
     prof = current_capture(prof)
     if not prof or not prof.get("warp_inst_per_launch") or not sm_mhz or not kernel_ms or kernel_ms <= 0:
         return None
@@ -496,8 +495,8 @@ def run_ours(args, rank, world, local):
                                  "of the encode call (ncu, same CUDA sources) over the issue peak; work: the "
                                  "reference's algorithmic int ops over the integer-lane peak; hbm: algorithmic "
                                  "input/output bytes, of measured peak. kernel_ms covers the encode call: "
-                                 "KBlockBuckets + KBlockOrder + KEncode for the single-kernel presets, every "
-                                 "pass kernel of the staged encode for precise, /slow and /data"})
+                                 "KEncode for the draft-only presets; KBlockBuckets, KBlockOrder and every pass "
+                                 "kernel of the staged encode for the refining ones"})
         cpu = {"value": cpu_value, "unit": "Mpx/s", "cores": cores, "kind": "port", "sample": sample,
                "reference_simd_equiv": simd_equivalent(args.workload, cpu_value)}
         line = {
