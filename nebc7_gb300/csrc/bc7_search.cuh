@@ -1093,7 +1093,9 @@ __device__ __forceinline__ bool TwoSubsetsPartition(WarpState& st, SearchState& 
 		if (!((s == 0 ? line0 : line1) < water))
 			return false;
 	}
-	if (max(line0, low[0]) + max(line1, low[1]) >= room)
+	/* OPTION_PCA's bounds may exceed the errors: then only the reference's
+	   own tests use them */
+	if (!P.pca && max(line0, low[0]) + max(line1, low[1]) >= room)
 		return false;
 	Team one = SingleWarp();
 	Ep mc0 = 0, mc1 = 0;

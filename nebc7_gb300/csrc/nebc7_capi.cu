@@ -666,9 +666,9 @@ int CoreWeightColor()
 
 namespace {
 
-/* Relative cost of one block by preset (measured block throughput on the
-   1024x1024 and 2048x2048 workloads: draft 1, default 11, precise 400,
-   /slow 480, /data 7200); orders a batch's queue longest first. */
+/* Cost class of one block by preset (the single kernels' block throughput on
+   photos and normal maps: draft 1, default 11, precise 400, /slow 480, /data
+   7200); orders a batch's queue longest first. */
 double BlockCost(const nebc7_settings& s)
 {
 	if (!s.doNormal || s.doDraft == 2)

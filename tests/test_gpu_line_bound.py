@@ -69,3 +69,26 @@ def test_long_lists_equal_short_ones(native, n):
     parts = [encode(a, b) for a, b in zip(cuts, cuts[1:])]
     assert (whole == np.concatenate([p[0] for p in parts])).all()
     assert (errors == sum(p[1] for p in parts)).all()
+
+
+@pytest.mark.parametrize("denoise,step", [(1, 9), (0, 0)])
+def test_bounds_beside_option_pca(native, port, denoise, step):
+    """OPTION_PCA's own bounds may exceed the errors, so a line bound may only
+    end a partition by itself, not together with one of them."""
+    from nebc7_gb300._native import Settings
+    n = 24
+    c, m = blocks("lines", n, 911)
+    c.reshape(n, 16, 4)[..., 3] = 255
+    a, b = np.zeros((n, 16), np.uint8), np.zeros((n, 16), np.uint8)
+    assert native.nebc7_set_pca(1) == 0
+    port.lib.nebc7_oracle_set_pca(1)
+    try:
+        e1, _ = port.compress_blocks(c, m, a, denoise, step, 1, 1, 1, 0, threads=16)
+        e2 = np.zeros(2, np.int64)
+        st = Settings(denoise, step, 1, 1, 1, 0)
+        assert native.nebc7_encode_blocks_host(c.ctypes.data, m.ctypes.data, b.ctypes.data, n, ctypes.byref(st), e2.ctypes.data,
+                                               None) == 0
+    finally:
+        native.nebc7_set_pca(0)
+        port.lib.nebc7_oracle_set_pca(0)
+    assert (a == b).all() and e1.tolist() == e2.tolist()
