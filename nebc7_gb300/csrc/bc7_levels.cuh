@@ -449,7 +449,8 @@ __device__ __forceinline__ ChanList ChannelLevelsScan(int2* nodes, const Area& a
 	return res;
 }
 
-/* Out-of-line copy of the scan for its many call sites. */
+/* The scan as its call sites take it (NEBC7_SHARED: out of line in the single
+   kernels). */
 template<int kD, bool HALF>
 __device__ NEBC7_SHARED ChanList ChannelLevels(int2* nodes, const Area& ar, int offset, int weight, int water, int bits, int pbits,
 	bool transparent, const uint8_t* table, bool byDiff, int maxSize, int2* values, Team& team, int lane)

@@ -8,13 +8,14 @@
  * one whose error is strictly below the running best ("water"), skipping
  * combinations by comparing bounds (a sorted channel error plus the other
  * channels' minima, or a memoised error over a subset of channels) with the
- * water.  The warp keeps the outer loops uniform and in order, computes the
- * memoised subset-of-channel errors for a whole loop level at once (lane =
- * list entry, early exit at the water in force when the level starts, which
- * decides every later comparison the same way), evaluates the innermost
- * channel's candidates in parallel and then replays the innermost loop's
- * acceptances in order (ReplayInner), so that the result matches the
- * sequential search even where masked pixels make a bound exceed the error.
+ * water.  Where those bounds are lower bounds of the error, the search ends
+ * with the first combination, in its order, of the smallest error below the
+ * water; SearchThree, SearchFour2 and SearchFour4 compute that, one warp or a
+ * CTA's four.  Where masked pixels can make a bound exceed the error (modes 4
+ * and 5), TryVariantsRot keeps the reference's order of tests: the outer loops
+ * uniform and in order, the memoised errors of a loop level at once (lane =
+ * list entry), the innermost channel's candidates in parallel and their
+ * acceptances replayed in order.
  */
 #pragma once
 
@@ -1533,8 +1534,8 @@ __device__ __forceinline__ Found SearchFour4(SearchState& ss, int v, const Area&
 	return Found{ water, best };
 }
 
-/* Out-of-line copy for modes 6 and 7; the Mode6Index2 refinement (the
-   common case of the default preset) inlines the body. */
+/* The search of index width IB over the lists of slot `slot`: with 4-bit indices
+   those of `ss`, with 2-bit ones those of `from` (a team's other warp's). */
 template<int kD, int IB>
 __device__ NEBC7_SHARED Found SearchFour(SearchState& ss, const SearchState& from, int slot, int v, const Area& ar, Weights w, const uint8_t* alphaTable,
 	Ep best, int water, TeamSearch* team, int lane)
