@@ -123,6 +123,11 @@ struct __align__(16) SplitResult
 constexpr int kSplitMaxBlocks = 1 << 24;    /* blocks of a pass split into tasks (the task count stays an int) */
 constexpr int kSplitSerial = -1;            /* firstImp: the block's pass runs whole (OPTION_PCA) */
 constexpr int kSplitNone = 0x7FFFFFFF;      /* firstImp: no improvement yet */
+/* firstImp otherwise: the candidate above the slot of its kept result, or above
+   kSplitNoSlot if there was no room for it.  Every slot is below that mark
+   (SplitResultCap). */
+constexpr int kSplitSlotBits = 24;
+constexpr int kSplitNoSlot = (1 << kSplitSlotBits) - 1;
 /* Polls of a warp that waits for a later round's tasks (2 us and more each)
    before it leaves them to the others: about ten seconds. */
 constexpr int kSplitPolls = 1 << 22;
@@ -134,6 +139,7 @@ __host__ __device__ constexpr int SplitIndex(int S)
 }
 
 constexpr int kSplitPasses = 7;
+constexpr int kSplitMaxTasks = 64;   /* candidates of a block at most */
 
 /* The three-subset passes estimate first, a warp or a team per block, and hand
    a block to the tasks when more than kInlineCandidates partitions are left:
@@ -208,7 +214,7 @@ struct Stages
 	int mixed;        /* whether blocks of both denoise forms are in the launch */
 	/* split passes */
 	int* start;       /* per position: the first candidate of the block's round */
-	int* firstImp;    /* per position: (candidate << 24) | result slot of the round's first improvement */
+	int* firstImp;    /* per position: (candidate << kSplitSlotBits) | result slot of the round's first improvement */
 	int* pending;     /* per position: the round's candidates not done */
 	int* later;       /* the blocks of the later rounds, in the order they were appended */
 	int laterCap;
@@ -832,7 +838,7 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 	const Stages& sg, SplitQueue& q, int k, int p, int first, int rank, int lane)
 {
 	constexpr int MODE = SplitMode(S);
-	if ((first >> 24) < p)
+	if ((first >> kSplitSlotBits) < p)
 		return;
 	CellRegs R;
 	RestoreBlock(st, R, b, sg.rec[k], P, lane);
@@ -901,9 +907,9 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 		if (R.errTotal == E)
 			return;
 	}
-	if (rank != 0 || lane != 0 || (*reinterpret_cast<volatile int*>(sg.firstImp + k) >> 24) < p)
+	if (rank != 0 || lane != 0 || (*reinterpret_cast<volatile int*>(sg.firstImp + k) >> kSplitSlotBits) < p)
 		return;
-	int slot = 0xFFFFFF;
+	int slot = kSplitNoSlot;
 	const int at = atomicAdd(&q.kept, 1);
 	if (at < sg.impCap)
 	{
@@ -920,7 +926,7 @@ __device__ NEBC7_PASS void SplitTask(WarpState& st, SearchState& ss, TeamState* 
 	}
 	/* the result before the word that leads to it */
 	__threadfence();
-	atomicMin(sg.firstImp + k, (p << 24) | slot);
+	atomicMin(sg.firstImp + k, (p << kSplitSlotBits) | slot);
 }
 
 /* Whether candidate p of the block at position k can improve on the error at
@@ -958,7 +964,7 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
 	}
 	else if (f != kSplitNone)
 	{
-		const int p = f >> 24, slot = f & 0xFFFFFF;
+		const int p = f >> kSplitSlotBits, slot = f & kSplitNoSlot;
 		if (slot >= sg.impCap)
 		{
 			from = p;   /* its result was not kept: search it again */
@@ -1166,7 +1172,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 		if (N > 1 && count > 1)
 		{
 			bool mine = false;
-			if ((first >> 24) >= p + warp)
+			if ((first >> kSplitSlotBits) >= p + warp)
 			{
 				if constexpr (kD == kAnyDenoise)
 				{
@@ -1295,10 +1301,17 @@ cudaError_t StagedEncodeOccupancy(int* ctasPerSm);
 constexpr size_t kStagedZeroed = 256 + kSplitPasses * sizeof(SplitQueue) + 2 * size_t(kNumStages) * 1024;
 static_assert(kStagedZeroed % 256 == 0 && kNumStages < 32, "the counts and queue heads take 128 bytes each");
 
+/* Results a pass keeps.  A slot has to fit its field of a firstImp word, below
+   the mark: with more room than that, results past 2^24 ran into the
+   candidate's bits and another block's was taken for them.  What finds no slot
+   is searched again by the remainder. */
 constexpr size_t SplitResultCap(int n)
 {
-	return 3 * size_t(n) + 1024;
+	return 3 * size_t(n) + 1024 < size_t(kSplitNoSlot) ? 3 * size_t(n) + 1024 : size_t(kSplitNoSlot);
 }
+
+static_assert(SplitResultCap(0x7FFFFFFF) == size_t(kSplitNoSlot) && kSplitMaxTasks << kSplitSlotBits <= kSplitNone,
+	"candidates and slots fit a firstImp word");
 
 constexpr size_t SplitLaterCap(int n)
 {
