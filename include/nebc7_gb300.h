@@ -162,6 +162,13 @@ int nebc7_decode_blocks_host(const uint8_t* blocks, uint8_t* bgra, int n);
    build of the reference (they are tested against the CPU restatement). */
 int nebc7_set_pca(int on);
 
+/* Limits, for the staged encodes that the calling thread enqueues from here on,
+   how many improving results a pass keeps, how many blocks go on in a later
+   round, and how many blocks' estimates are handed to other warps (negative: no
+   limit but the state's size).  What finds no room is searched by one warp, so
+   the blocks are the same; the tests reach that path so. */
+int nebc7_limit_staged_rooms(int results, int later, int handed);
+
 /* The steps of an encode with these settings as its pass structure counts
    them (the block order's two, then one, or for the full-search presets a
    list and a step per pass and two per round of a split pass): a fixed

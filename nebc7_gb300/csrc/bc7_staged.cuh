@@ -284,8 +284,9 @@ __device__ __forceinline__ void SaveRecord(BlockRecord& r, const CellRegs& R, in
 }
 
 /* Rebuilds a block's state: its pixels and masks, the saved scalars, the
-   whole-block area (src/Bc7Core.cpp:1532-1535). */
-__device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const BlockRef& b, const BlockRecord& record, const Params& P,
+   whole-block area (src/Bc7Core.cpp:1532-1535).  Returns the record's
+   `handed`. */
+__device__ __forceinline__ int RestoreBlock(WarpState& st, CellRegs& R, const BlockRef& b, const BlockRecord& record, const Params& P,
 	int lane)
 {
 	LoadCell(st, b, R, lane);
@@ -307,6 +308,7 @@ __device__ __forceinline__ void RestoreBlock(WarpState& st, CellRegs& R, const B
 	R.personalMode = r.personalMode;
 	R.denoiseStep = r.denoiseStep;
 	BuildWholeBlock(st, R, P, lane);
+	return r.handed;
 }
 
 /* Shared memory of a warp of stage STAGE: the block state, and the search
@@ -638,17 +640,17 @@ __device__ bool DraftStage(WarpState& st, const BlockRef& b, const LevelTables& 
 /* FullThreeSubsets of the block at position k: the estimates, then the search
    in the (team's first) warp, or its hand-over to the tasks of KEncodeSplit
    (returns true).  A block that was handed and comes back (a result that was
-   not kept) goes on from candidate `from` with its estimates. */
+   not kept) goes on from candidate `from` with its estimates; `handed` is its
+   record's, as every warp of the team read it before the first one clears it
+   here: warps that disagree would part at the estimates' barriers. */
 template<int kD, int S>
 __device__ __forceinline__ bool ThreeSubsetsStage(WarpState& st, SearchState& ss, CellRegs& R, const Params& P, const LevelTables& T,
-	const Stages& sg, int k, int from, bool hand, const Team& team, int lane)
+	const Stages& sg, int k, int handed, int from, bool hand, const Team& team, int lane)
 {
 	constexpr int MODE = SplitMode(S);
 	const Spec3 sp = GetSpec3(MODE, T);
 	BlockRecord& rec = sg.rec[k];
-	const int handed = __ldcg(&rec.handed);
-	const bool resume = handed != 0;
-	if (resume)
+	if (handed)
 	{
 		if (team.rank)
 			return false;
@@ -714,12 +716,12 @@ __device__ void PassStage(WarpState& st, SearchState& ss, const BlockRef& b, con
 {
 	CellRegs R;
 	BlockRecord& rec = sg.rec[k];
-	RestoreBlock(st, R, b, rec, P, lane);
+	const int handed = RestoreBlock(st, R, b, rec, P, lane);
 	if (TeamStage(S) && team.size > 1)
 		__syncthreads();   /* every warp has read the record before it changes */
 	if constexpr (ThreeSubsetStep(S))
 	{
-		if (ThreeSubsetsStage<kD, S>(st, ss, R, P, T, sg, k, from, hand, team, lane))
+		if (ThreeSubsetsStage<kD, S>(st, ss, R, P, T, sg, k, handed, from, hand, team, lane))
 			return;   /* handed to the tasks */
 	}
 	else

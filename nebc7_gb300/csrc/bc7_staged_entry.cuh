@@ -8,12 +8,12 @@
 
 namespace nebc7 {
 
-/* CTAs for `tasks` tasks of `warps` warps each, at most `grid` (the resident
-   ones). */
+/* CTAs for `tasks` tasks of `warps` warps each, at least one and at most `grid`
+   (the resident ones). */
 inline int StageGrid(int grid, long long tasks, int warps)
 {
 	const long long ctas = (tasks * warps + kWarpsPerCta - 1) / kWarpsPerCta;
-	return ctas < grid ? int(ctas) : grid;
+	return ctas < 1 ? 1 : (ctas < grid ? int(ctas) : grid);
 }
 
 /* The list of pass STAGE and its kernels: of a split pass the tasks, of a

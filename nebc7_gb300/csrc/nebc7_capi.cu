@@ -415,6 +415,26 @@ size_t LaunchScratchBytes(int nblocks, bool wantSums, bool staged)
 	return staged ? base + StagedScratchBytes(nblocks) : base;
 }
 
+/* The calling thread's rooms of the staged form (nebc7_limit_staged_rooms);
+   negative: as its scratch has them. */
+struct StagedLimits
+{
+	int results = -1, later = -1, handed = -1;
+
+	void Apply(Stages& sg) const
+	{
+		auto lower = [](int& cap, int limit) {
+			if (limit >= 0 && limit < cap)
+				cap = limit;
+		};
+		lower(sg.impCap, results);
+		lower(sg.laterCap, later);
+		lower(sg.handedCap, handed);
+	}
+};
+
+thread_local StagedLimits tStagedLimits;
+
 /* Launches the encode of `job` with instantiation `slot`: the staged form
    when the slot has one and `staged` (StagedScratchBytes(job.total) bytes,
    256-byte aligned) is given, else the single kernel on `grid` CTAs.  slow:
@@ -424,7 +444,8 @@ cudaError_t LaunchSlot(int slot, int grid, int ctasPerSm, cudaStream_t stream, c
 {
 	if (staged && kVariants[slot].staged)
 	{
-		const Stages sg = SplitStaged(staged, job.total, slot == kVariantMixed);
+		Stages sg = SplitStaged(staged, job.total, slot == kVariantMixed);
+		tStagedLimits.Apply(sg);
 		const cudaError_t e = cudaMemsetAsync(staged, 0, kStagedZeroed, stream);
 		if (e != cudaSuccess)
 			return e;
@@ -1796,6 +1817,14 @@ int nebc7_set_pca(int on)
 	if (on != 0 && on != 1)
 		return SetError(NEBC7_EINVAL);
 	gPca.store(on);
+	return NEBC7_OK;
+}
+
+int nebc7_limit_staged_rooms(int results, int later, int handed)
+{
+	tStagedLimits.results = results;
+	tStagedLimits.later = later;
+	tStagedLimits.handed = handed;
 	return NEBC7_OK;
 }
 
