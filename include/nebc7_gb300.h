@@ -162,6 +162,13 @@ int nebc7_decode_blocks_host(const uint8_t* blocks, uint8_t* bgra, int n);
    build of the reference (they are tested against the CPU restatement). */
 int nebc7_set_pca(int on);
 
+/* Limits the records of the staged form, 280 bytes per block and up to 7 MB,
+   for the encodes, batches and servers that the calling thread makes from here
+   on (negative: no limit but the device's free memory).  A launch without room
+   for them runs the single kernel, a server's streams hold those of fewer blocks;
+   the blocks are the same. */
+int nebc7_limit_staged_records(long long bytes);
+
 /* Limits, for the staged encodes that the calling thread enqueues from here on,
    how many improving results a pass keeps, how many blocks go on in a later
    round, and how many blocks' estimates are handed to other warps (negative: no
@@ -331,10 +338,12 @@ typedef struct nebc7_server_counters
    other refining ones each as a staged launch (a kernel per pass), draft-only
    ones as one persistent launch, the cheapest requests dealt first; each
    request of a draft-only batch returns (its blocks copied back) as soon as
-   its own blocks are done, while the rest of the launch still runs.  Besides the arena, every stream holds the
-   staged form's per-block state (its record, pass lists, split-pass rounds
-   and kept results): 156 bytes per block for up to min(4194304,
-   hbm_budget / 104) blocks. */
+   its own blocks are done, while the rest of the launch still runs.  Besides
+   the arena, every stream holds the staged form's per-block state (its record,
+   pass lists, split-pass rounds and kept results): 280 bytes per block, and up
+   to 7 MB, for up to min(4194304, hbm_budget / 104 + 1) blocks, or half as many
+   as often as it takes where that is not free.  A request of more blocks runs
+   the single kernel. */
 int nebc7_server_create(const nebc7_server_config* cfg, nebc7_server** out);
 
 /* Queues one texture (host buffers; pinned memory lets the copies run

@@ -165,6 +165,7 @@ SIGNATURES = {
     "nebc7_encode_launches": (I, [ctypes.POINTER(Settings)]),
     "nebc7_encode_kernels": (I, [ctypes.POINTER(Settings)]),
     "nebc7_set_pca": (I, [I]),
+    "nebc7_limit_staged_records": (I, [LL]),
     "nebc7_limit_staged_rooms": (I, [I, I, I]),
     "nebc7_table_read": (I, [I, I, VP, LL, ctypes.POINTER(LL)]),
     "nebc7_launch_shape": (I, [VP, VP, VP]),

@@ -399,7 +399,7 @@ cudaError_t EnqueueBlockOrder(const uint8_t* bgra, long long stride, int blocksW
 }
 
 /* The most blocks of a staged launch, whose lists are indexed with ints past
-   their ends: 42 GB of records.  The single kernel takes more. */
+   their ends: 33 GB of records.  The single kernel takes more. */
 constexpr int kStagedMaxBlocks = 1 << 28;
 
 bool TakesStaged(const nebc7_settings& s, int nblocks)
@@ -415,11 +415,16 @@ size_t LaunchScratchBytes(int nblocks, bool wantSums, bool staged)
 	return staged ? base + StagedScratchBytes(nblocks) : base;
 }
 
-/* The calling thread's rooms of the staged form (nebc7_limit_staged_rooms);
-   negative: as its scratch has them. */
+/* The calling thread's limits of the staged form: the bytes of a launch's
+   records (nebc7_limit_staged_records) and its rooms
+   (nebc7_limit_staged_rooms); negative: none but the device's memory, and as its
+   scratch has them. */
 struct StagedLimits
 {
+	long long records = -1;
 	int results = -1, later = -1, handed = -1;
+
+	bool Allow(size_t bytes) const { return records < 0 || bytes <= size_t(records); }
 
 	void Apply(Stages& sg) const
 	{
@@ -434,6 +439,22 @@ struct StagedLimits
 };
 
 thread_local StagedLimits tStagedLimits;
+
+/* Device memory for staged records, or an error that leaves none behind:
+   callers then do without the staged form. */
+cudaError_t StagedMalloc(uint8_t** p, size_t bytes)
+{
+	*p = nullptr;
+	if (!tStagedLimits.Allow(bytes))
+		return cudaErrorMemoryAllocation;
+	const cudaError_t e = cudaMalloc((void**)p, bytes);
+	if (e != cudaSuccess)
+	{
+		*p = nullptr;
+		cudaGetLastError();
+	}
+	return e;
+}
 
 /* Launches the encode of `job` with instantiation `slot`: the staged form
    when the slot has one and `staged` (StagedScratchBytes(job.total) bytes,
@@ -482,12 +503,16 @@ int LaunchEncode(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long lo
 	const bool wantSums = errs || ssim;
 	uint8_t* scratch = scratchIn;
 	bool useStaged = scratch ? stagedIn : TakesStaged(s, nblocks);
-	if (!scratch && cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, useStaged), stream) != cudaSuccess)
+	auto allocate = [&](bool staged) {
+		return (!staged || tStagedLimits.Allow(StagedScratchBytes(nblocks))) &&
+			cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, staged), stream) == cudaSuccess;
+	};
+	if (!scratch && !allocate(useStaged))
 	{
 		cudaGetLastError();
 		const bool retry = useStaged;
 		useStaged = false;
-		if (!retry || cudaMallocAsync((void**)&scratch, LaunchScratchBytes(nblocks, wantSums, false), stream) != cudaSuccess)
+		if (!retry || !allocate(false))
 			return SetError(NEBC7_ENOMEM);
 	}
 	const EncodeScratch e = SplitScratch(scratch, nblocks, wantSums);
@@ -847,6 +872,25 @@ void BuildSchedule(nebc7_batch* b, int which)
 	}
 	S.stagedBytes = size_t(off);
 	S.orderBytes = size_t(ooff);
+}
+
+/* The staged records of both schedules, which share one area; without room for
+   the larger schedule's its groups run the single kernel, then the other's. */
+void AllocateBatchRecords(nebc7_batch* b)
+{
+	for (;;)
+	{
+		const size_t bytes = std::max(b->sched[0].stagedBytes, b->sched[1].stagedBytes);
+		if (!bytes || StagedMalloc(&b->stagedArea, bytes) == cudaSuccess)
+			return;
+		for (BatchSchedule& S : b->sched)
+			if (S.stagedBytes == bytes)
+			{
+				S.stagedBytes = 0;
+				for (BatchGroup& g : S.groups)
+					g.stagedOff = -1;
+			}
+	}
 }
 
 /* Enqueues schedule `which` on stream st (capturable): clears the outputs
@@ -1211,7 +1255,7 @@ int LaunchServerBatch(nebc7_server* sv, ServerSlot& slot, std::vector<int64_t>& 
 	/* draft-only requests take the single kernel, whose blocks and so whose
 	   requests finish as they go; the others the staged form (one kernel per
 	   pass) */
-	bool staged = total <= slot.stagedCap, slow = false;
+	bool staged = slot.staged && total <= slot.stagedCap, slow = false;
 	int variant = VariantSlot(sv->reqs[batch[0]].settings);
 	for (int64_t id : batch)
 	{
@@ -1354,7 +1398,7 @@ void ServerLoop(nebc7_server* sv)
 				continue;
 			/* the oldest admitted request and, in arrival order, others of its
 			   kind up to max_batch requests and, for staged ones, the staged
-			   records' capacity */
+			   records' capacity if the slot has any */
 			std::vector<int64_t> batch;
 			const RequestKind kind = KindOf(sv->reqs[sv->admitted.front()]);
 			long long blocks = 0;
@@ -1362,7 +1406,7 @@ void ServerLoop(nebc7_server* sv)
 			{
 				const ServerRequest& r = sv->reqs[*it];
 				const long long nb = (long long)(r.w / 4) * (r.h / 4);
-				if (KindOf(r) != kind || (!batch.empty() && kind != kRequestDraft && blocks + nb > slot.stagedCap))
+				if (KindOf(r) != kind || (!batch.empty() && kind != kRequestDraft && slot.staged && blocks + nb > slot.stagedCap))
 				{
 					++it;
 					continue;
@@ -1675,7 +1719,8 @@ int EncodeHost(uint8_t* dst, const uint8_t* bgra, const uint8_t* mask, long long
 	const size_t offRaw = offMask + (mask || outline ? Align256(img) : 0);
 	const size_t offScratch = offRaw + (raw ? Align256(size_t(raw->w) * 4 * raw->h) : 0);
 	bool staged = TakesStaged(*settings, int(nb));
-	bool room = ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, staged));
+	bool room = (!staged || tStagedLimits.Allow(StagedScratchBytes(int(nb)))) &&
+		ReserveSlot(slot, offScratch + LaunchScratchBytes(int(nb), true, staged));
 	if (!room && staged)
 	{
 		cudaGetLastError();
@@ -1820,6 +1865,12 @@ int nebc7_set_pca(int on)
 	return NEBC7_OK;
 }
 
+int nebc7_limit_staged_records(long long bytes)
+{
+	tStagedLimits.records = bytes;
+	return NEBC7_OK;
+}
+
 int nebc7_limit_staged_rooms(int results, int later, int handed)
 {
 	tStagedLimits.results = results;
@@ -1912,11 +1963,8 @@ int nebc7_batch_create(const nebc7_texture* textures, int n, int flags, nebc7_ba
 		const size_t offRes = 256 + ((sizeof(int) * 2 * ng + 255) & ~size_t(255));
 		const size_t offErr = offRes + ((size_t(total) * sizeof(BlockResult) + 255) & ~size_t(255));
 		const size_t bytes = offErr + size_t(n) * 4 * sizeof(long long);
-		const size_t stagedBytes = std::max(b->sched[0].stagedBytes, b->sched[1].stagedBytes);
 		const size_t orderBytes = std::max(b->sched[0].orderBytes, b->sched[1].orderBytes);
-		if (cudaMalloc((void**)&b->dmem, bytes) != cudaSuccess ||
-			(stagedBytes && cudaMalloc((void**)&b->stagedArea, stagedBytes) != cudaSuccess) ||
-			cudaMalloc((void**)&b->orderArea, orderBytes) != cudaSuccess)
+		if (cudaMalloc((void**)&b->dmem, bytes) != cudaSuccess || cudaMalloc((void**)&b->orderArea, orderBytes) != cudaSuccess)
 			rc = SetError(NEBC7_ENOMEM);
 		else
 		{
@@ -1936,6 +1984,8 @@ int nebc7_batch_create(const nebc7_texture* textures, int n, int flags, nebc7_ba
 			if (rc == NEBC7_OK && cudaMemcpy(S.dTable, S.table.data(), sizeof(TexDesc) * S.table.size(), cudaMemcpyHostToDevice) != cudaSuccess)
 				rc = SetError(NEBC7_ECUDA);
 		}
+		if (rc == NEBC7_OK)
+			AllocateBatchRecords(b);
 		if (rc == NEBC7_OK && cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking) != cudaSuccess)
 			rc = SetError(NEBC7_ECUDA);
 		for (size_t i = 0; i < ng && rc == NEBC7_OK; i++)
@@ -1960,8 +2010,9 @@ int nebc7_batch_create(const nebc7_texture* textures, int n, int flags, nebc7_ba
 		FreeBatch(b);
 		return rc;
 	}
-	/* without tuning: one launch per preset group when the batch mixes presets */
-	b->chosen = b->sched[1].groups.size() > 1 ? 1 : 0;
+	/* without tuning: one launch per preset group when the batch mixes presets,
+	   or when only those have their records */
+	b->chosen = b->sched[1].groups.size() > 1 || b->sched[0].stagedBytes < b->sched[1].stagedBytes ? 1 : 0;
 	*out = b;
 	return NEBC7_OK;
 }
@@ -2216,11 +2267,17 @@ int nebc7_server_create(const nebc7_server_config* cfg, nebc7_server** out)
 			cudaMalloc((void**)&slot.dSums, sizeof(long long) * 4 * cap) != cudaSuccess ||
 			cudaMalloc((void**)&slot.dCounter, 256) != cudaSuccess)
 			rc = SetError(NEBC7_ENOMEM);
-		/* the staged form's records: a launch holds at most one block per
-		   kServerBlockBytes of the arena */
+	}
+	/* the staged form's records, after all that a server cannot do without: a
+	   launch holds at most one block per kServerBlockBytes of the arena; where
+	   so much is not free, half as often as it takes */
+	for (ServerSlot& slot : sv->slots)
+	{
+		if (rc != NEBC7_OK)
+			break;
 		slot.stagedCap = int(std::min<size_t>(kServerStagedBlocks, cfg->hbm_budget / kServerBlockBytes + 1));
-		if (rc == NEBC7_OK && cudaMalloc((void**)&slot.staged, StagedScratchBytes(slot.stagedCap)) != cudaSuccess)
-			rc = SetError(NEBC7_ENOMEM);
+		while (slot.stagedCap > 0 && StagedMalloc(&slot.staged, StagedScratchBytes(slot.stagedCap)) != cudaSuccess)
+			slot.stagedCap /= 2;
 	}
 	/* size the mixed kernel's launch before any request arrives */
 	if (rc == NEBC7_OK && GridForSlot(1, kVariantMixed) <= 0)
