@@ -391,7 +391,7 @@ int nebc7_partition_map_device(const uint8_t* d_blocks, uint8_t* d_out, int nblo
    key "T=u" (bottom-up rows) instead of "T=d". */
 int nebc7_ktx_header(int w, int h, int flip, uint8_t* out);
 
-/* Persistent-grid sizing of the encode kernel of the default preset
+/* Persistent-grid sizing of the single encode kernel of the default preset
    (kDenoise 1 with the refinement passes): CTAs per SM and warps per CTA. */
 int nebc7_launch_shape(int* ctas_per_sm, int* warps_per_cta, int* sm_count);
 

@@ -409,14 +409,20 @@ constexpr size_t EncodeSharedBytes()
 	return kWarpsPerCta * (sizeof(WarpState) + (NORMAL ? sizeof(SearchState) : 0));
 }
 
+/* Resident CTAs per SM that the single kernel is compiled for (bounds its
+   registers per thread); set by its translation unit. */
+#ifndef NEBC7_SINGLE_CTAS
+#define NEBC7_SINGLE_CTAS 4
+#endif
+
 /* Persistent encode kernel over a launch's textures.  NORMAL compiles the
    refinement / full-search passes (run for textures whose preset asks for
    them); only that instantiation reserves the per-warp search state in
-   shared memory, and keeps the routines the full searches call from many places
-   out of line (NEBC7_PASS, NEBC7_SHARED, set by its translation unit).  kD: the
-   kDenoise of every texture, or kAnyDenoise. */
+   shared memory.  Its translation unit says which routines stay out of line
+   (NEBC7_PASS, NEBC7_SHARED).  kD: the kDenoise of every texture, or
+   kAnyDenoise. */
 template<int kD, bool NORMAL>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncode(Job job, LevelTables T0, LevelTables T1)
+__global__ void __launch_bounds__(kWarpsPerCta * 32, NEBC7_SINGLE_CTAS) KEncode(Job job, LevelTables T0, LevelTables T1)
 {
 	extern __shared__ __align__(16) unsigned char encodeSmem[];
 	const int lane = threadIdx.x & 31;

@@ -239,66 +239,58 @@ int VariantSlot(const nebc7_settings& s)
 	return 2 * int(s.denoise != 0) + int(normal);
 }
 
-/* Launch shape of one encode instantiation on one device, looked up once
-   (with the device current): this also raises the kernel's dynamic
-   shared-memory limit, so it runs before the first launch on the device. */
+/* Launch shapes of the encode instantiations on one device, each looked up once
+   (with the device current): this also raises the kernels' dynamic
+   shared-memory limits, so it runs before the first launch on the device. */
 struct LaunchShape
 {
 	int sms = 0;
-	int perSm[kNumVariants] = {};
+	int perSm[kNumVariants] = {};        /* of the single kernel */
+	int stagedPerSm[kNumVariants] = {};  /* of the staged form's kernels */
 };
 
 std::mutex gShapeMutex;
 LaunchShape gShapes[kMaxDevices];
 
-/* Grid of a persistent launch of `slot` over nblocks blocks: one CTA per
-   kWarpsPerCta blocks up to the resident CTAs of every SM, or up to
-   ctasPerSm per SM when that is given (> 0) and smaller. */
-int GridForSlotCap(int nblocks, int slot, int ctasPerSm);
-
-int GridForSlot(int nblocks, int slot)
-{
-	return GridForSlotCap(nblocks, slot, 0);
-}
-
-int GridForSlotCap(int nblocks, int slot, int ctasPerSm)
+/* Resident CTAs of `slot`, of its single kernel or its staged form: of every
+   SM, or up to ctasPerSm per SM when that is given (> 0) and smaller.  0 on
+   failure. */
+int ResidentCtas(int slot, bool staged, int ctasPerSm)
 {
 	int dev = 0;
 	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
 		return 0;
-	int sms, perSm;
+	std::lock_guard<std::mutex> lock(gShapeMutex);
+	LaunchShape& L = gShapes[dev];
+	if (!L.sms)
 	{
-		std::lock_guard<std::mutex> lock(gShapeMutex);
-		LaunchShape& L = gShapes[dev];
-		if (!L.sms)
-		{
-			cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev);
-			if (L.sms <= 0)
-				L.sms = 1;
-		}
-		if (!L.perSm[slot])
-		{
-			int n = 0;
-			if (kVariants[slot].occupancy(&n) != cudaSuccess)
-				return 0;
-			if (kVariants[slot].stagedOccupancy)
-			{
-				/* prepares the stage kernels too; the grid fits both forms */
-				int m = 0;
-				if (kVariants[slot].stagedOccupancy(&m) != cudaSuccess)
-					return 0;
-				n = std::min(n, m);
-			}
-			L.perSm[slot] = n > 0 ? n : 1;
-		}
-		sms = L.sms;
-		perSm = L.perSm[slot];
+		cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev);
+		if (L.sms <= 0)
+			L.sms = 1;
 	}
-	if (ctasPerSm > 0 && ctasPerSm < perSm)
-		perSm = ctasPerSm;
-	const int ctasNeeded = (nblocks + kWarpsPerCta - 1) / kWarpsPerCta;
-	const int g = sms * perSm;
-	return ctasNeeded < g ? ctasNeeded : g;
+	if (!L.perSm[slot])
+	{
+		int n = 0, m = 0;
+		if (kVariants[slot].occupancy(&n) != cudaSuccess ||
+			(kVariants[slot].stagedOccupancy && kVariants[slot].stagedOccupancy(&m) != cudaSuccess))
+			return 0;
+		L.perSm[slot] = std::max(n, 1);
+		L.stagedPerSm[slot] = std::max(m, 1);
+	}
+	const int perSm = staged ? L.stagedPerSm[slot] : L.perSm[slot];
+	return L.sms * (ctasPerSm > 0 ? std::min(ctasPerSm, perSm) : perSm);
+}
+
+/* Grid of a persistent launch of `slot`'s single kernel over nblocks blocks: one
+   CTA per kWarpsPerCta blocks up to the resident ones. */
+int GridForSlotCap(int nblocks, int slot, int ctasPerSm)
+{
+	return std::min((nblocks + kWarpsPerCta - 1) / kWarpsPerCta, ResidentCtas(slot, false, ctasPerSm));
+}
+
+int GridForSlot(int nblocks, int slot)
+{
+	return GridForSlotCap(nblocks, slot, 0);
 }
 
 int GridFor(int nblocks, const nebc7_settings& s)
@@ -471,7 +463,7 @@ cudaError_t LaunchSlot(int slot, int grid, int ctasPerSm, cudaStream_t stream, c
 		if (e != cudaSuccess)
 			return e;
 		/* its passes size their own grids: all resident CTAs at most */
-		const int resident = GridForSlotCap(1 << 30, slot, ctasPerSm);
+		const int resident = ResidentCtas(slot, true, ctasPerSm);
 		if (resident <= 0)
 			return cudaErrorUnknown;
 		return kVariants[slot].staged(resident, stream, job, sg, slow, T0, T1);
