@@ -184,7 +184,9 @@ int nebc7_limit_staged_rooms(int results, int later, int handed);
 int nebc7_encode_launches(const nebc7_settings* settings);
 
 /* How many kernels an encode with these settings launches, not counting the
-   sums' reduction; a negative error code for invalid settings. */
+   sums' reduction; a negative error code for invalid settings.  A refining encode
+   of no more blocks than the device holds warps (2432 on 152 SMs) launches two
+   less, those of the block order. */
 int nebc7_encode_kernels(const nebc7_settings* settings);
 
 /* Builds the level tables of `denoise` on the current device ahead of use. */

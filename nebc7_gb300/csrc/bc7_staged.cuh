@@ -200,6 +200,17 @@ struct __align__(16) SplitQueue
 	int pad1[27];
 };
 
+/* Waits for the kernels before this one in its stream.  Every kernel of the
+   staged form starts with this and is launched as the programmatic dependent of
+   the one before it, so that its launch overlaps that one's end; a pass without
+   blocks then returns at once.  Of the chain's 24 to 32 kernels most find nothing
+   to do in an easy texture: 64x64 of one colour 371 -> 310 us a call, a 64x64
+   photo 724 -> 650, loose cells 287 -> 216. */
+__device__ __forceinline__ void WaitForLaunch()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 /* Per-launch state of a staged encode (one entry per queue position). */
 struct Stages
 {
@@ -778,9 +789,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeStage(Job job, St
 	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(STAGE, false));
 	SearchState& ss = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&st) + kSearchWarpBytes);
 	__shared__ LevelTables tables[2];
-	ShareTables(tables, T0, T1);
-	const int n = list ? *count : job.total;
 	__shared__ TeamState ts;
+	WaitForLaunch();
+	const int n = list ? *count : job.total;
+	if (n == 0)
+		return;
+	ShareTables(tables, T0, T1);
 	/* the first blocks of a list a CTA each (TeamBlocks), the others a warp each */
 	const int nTeam = TeamStage(STAGE) ? TeamBlocks(STAGE, n, sg.count[kNumStages], int(gridDim.x)) : 0;
 	Team team{ nTeam > 0 ? kWarpsPerCta : 1, nTeam > 0 ? warp : 0, &ts.exchange, 0 };
@@ -1100,9 +1114,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32, 4) KEncodeSplit(Job job, St
 	WarpState& st = *reinterpret_cast<WarpState*>(encodeSmem + warp * StageWarpBytes(S, true));
 	SearchState& ss = *reinterpret_cast<SearchState*>(reinterpret_cast<unsigned char*>(&st) + kSearchWarpBytes);
 	__shared__ LevelTables tables[2];
-	ShareTables(tables, T0, T1);
 	SplitQueue& q = sg.split[SplitIndex(S)];
+	WaitForLaunch();
 	const int n = min(*count, ThreeSubsetStep(S) ? sg.handedCap : kSplitMaxBlocks);
+	if (n == 0)
+		return;
+	ShareTables(tables, T0, T1);
 	const int rank = N > 1 ? warp : 0;   /* within the task's warps */
 	const int grab = N > 1 && n >= kGrabBlocks ? N : 1;
 	bool firstRound = true;
@@ -1236,6 +1253,7 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 {
 	__shared__ int base[256];
 	const int lane = threadIdx.x & 31;
+	WaitForLaunch();
 	if (threadIdx.x < 32)
 	{
 		/* exclusive scan of the bucket counts: 8 per lane, then the lanes */

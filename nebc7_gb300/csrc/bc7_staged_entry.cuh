@@ -16,6 +16,24 @@ inline int StageGrid(int grid, long long tasks, int warps)
 	return ctas < 1 ? 1 : (ctas < grid ? int(ctas) : grid);
 }
 
+/* Launches a kernel of the staged form as the programmatic dependent of the one
+   before it (WaitForLaunch). */
+template<class... P, class... A>
+cudaError_t LaunchChained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const A&... args)
+{
+	cudaLaunchAttribute chained = {};
+	chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	chained.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t config = {};
+	config.gridDim = dim3(grid);
+	config.blockDim = dim3(threads);
+	config.dynamicSmemBytes = smem;
+	config.stream = stream;
+	config.attrs = &chained;
+	config.numAttrs = 1;
+	return cudaLaunchKernelEx(&config, kernel, P(args)...);
+}
+
 /* The list of pass STAGE and its kernels: of a split pass the tasks, of a
    three-subset pass its estimates and the tasks of the blocks they hand over;
    then a split pass's blocks that must run whole (OPTION_PCA, results not
@@ -23,31 +41,34 @@ inline int StageGrid(int grid, long long tasks, int warps)
 template<int kD, int STAGE>
 cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Stages& sg, const LevelTables& T0, const LevelTables& T1)
 {
-	constexpr int split = SplitIndex(STAGE);
-	constexpr bool three = ThreeSubsetStep(STAGE);
-	if (STAGE != kStageDraft)
+	constexpr int split = SplitIndex(STAGE), threads = kWarpsPerCta * 32;
+	constexpr bool three = ThreeSubsetStep(STAGE), draft = STAGE == kStageDraft;
+	cudaError_t e = cudaSuccess;
+	if (!draft)
 	{
 		const int ctas = (job.total + 1023) / 1024;
-		KStageList<<<ctas < 152 ? ctas : 152, 1024, 0, stream>>>(sg, STAGE, split, split >= 0 && !three ? SplitTasks(STAGE) : 0);
+		e = LaunchChained(KStageList, ctas < 152 ? ctas : 152, 1024, 0, stream, sg, STAGE, split, split >= 0 && !three ? SplitTasks(STAGE) : 0);
 	}
 	const int stageGrid = StageGrid(grid, job.total, TeamStage(STAGE) ? kWarpsPerCta : 1);
 	if constexpr (split < 0 || three)
 	{
-		const bool all = STAGE == kStageDraft;
-		KEncodeStage<kD, STAGE><<<stageGrid, kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, all ? nullptr : sg.list,
-			all ? nullptr : sg.count + STAGE, sg.counters + (STAGE + 1), T0, T1);
+		if (e == cudaSuccess)
+			e = LaunchChained(KEncodeStage<kD, STAGE>, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg,
+				draft ? nullptr : sg.list, draft ? nullptr : sg.count + STAGE, sg.counters + (STAGE + 1), T0, T1);
 	}
 	if constexpr (split >= 0)
 	{
 		/* a small texture's tasks fill more SMs than its blocks */
 		const int blocks = three ? sg.handedCap : job.total;
-		KEncodeSplit<kD, STAGE><<<StageGrid(grid, (long long)blocks * SplitTasks(STAGE), SplitTeam(STAGE)), kWarpsPerCta * 32,
-			StageSharedBytes(STAGE, true), stream>>>(job, sg, three ? sg.handed : sg.list, three ? &sg.split[split].handedCount : sg.count + STAGE,
-			T0, T1);
-		KEncodeStage<kD, STAGE><<<stageGrid, kWarpsPerCta * 32, StageSharedBytes(STAGE, false), stream>>>(job, sg, sg.rest,
-			&sg.split[split].restCount, &sg.split[split].restHead, T0, T1);
+		if (e == cudaSuccess)
+			e = LaunchChained(KEncodeSplit<kD, STAGE>, StageGrid(grid, (long long)blocks * SplitTasks(STAGE), SplitTeam(STAGE)), threads,
+				StageSharedBytes(STAGE, true), stream, job, sg, three ? sg.handed : sg.list,
+				three ? &sg.split[split].handedCount : sg.count + STAGE, T0, T1);
+		if (e == cudaSuccess)
+			e = LaunchChained(KEncodeStage<kD, STAGE>, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg, sg.rest,
+				&sg.split[split].restCount, &sg.split[split].restHead, T0, T1);
 	}
-	return cudaGetLastError();
+	return e;
 }
 
 /* The passes from STAGE on. */
