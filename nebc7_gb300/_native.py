@@ -213,6 +213,9 @@ def load(path: Path | None = None) -> ctypes.CDLL:
         return lib
 
 
+ENOMEM = 3   # NEBC7_ENOMEM
+
+
 class NativeError(RuntimeError):
     CODES = {
         1: "invalid argument",

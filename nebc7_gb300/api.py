@@ -227,6 +227,7 @@ def encode_image(img_bgra: np.ndarray, flags: str = "", preset: Preset = DEFAULT
     """The CLI's encode path on an in-memory BGRA image (top-down rows)."""
     o = parse_flags(flags)
     img = np.ascontiguousarray(img_bgra, dtype=np.uint8)
+    radius = o["radius"] if o["mask"] else -1
     # the device pads and masks; numpy took 14 of 53 ms for a 1118x1105 image
     on_device = img.ndim == 3 and img.shape[2] == 4 and min(img.shape) > 0 and max(padded_size(*img.shape[:2])) <= 16384
     if on_device:
@@ -234,13 +235,20 @@ def encode_image(img_bgra: np.ndarray, flags: str = "", preset: Preset = DEFAULT
     else:
         padded = pad_texture(img)
         ph, pw = padded.shape[:2]
-        mask = outline_mask(padded, o["radius"]) if o["mask"] else None
     core = Bc7Core(preset)
     core.init_tables(o["draft"], o["normal"], o["slow"], o["linear"])
     blocks = np.zeros(((ph // 4) * (pw // 4), 16), np.uint8) if start is None else np.array(start, np.uint8)
+    stats = None
     if on_device:
-        stats = core.process_image(blocks, img, o["radius"] if o["mask"] else -1)
-    else:
+        try:
+            stats = core.process_image(blocks, img, radius)
+        except NativeError as e:
+            if e.code != _native.ENOMEM:
+                raise
+            # without device memory for the unpadded image too
+            padded = pad_texture(img)
+    if stats is None:
+        mask = outline_mask(padded, radius) if radius >= 0 else None
         stats = core.process_texture(blocks, padded, mask, pw, ph)
     return EncodedImage(blocks, pw, ph, stats)
 
