@@ -127,8 +127,14 @@ class Bc7Core:
 
     def process_image(self, dst: np.ndarray, img_bgra: np.ndarray, radius: int) -> EncodeStats:
         """process_texture of an unpadded C-contiguous BGRA image, padded and
-        (radius >= 0) masked on the device (src/Bc7Compress.cpp:33-105, 397-426)."""
+        (radius >= 0) masked on the device (src/Bc7Compress.cpp:33-105, 397-426);
+        dst (uint8) holds the padded texture's blocks, at least."""
+        if img_bgra.dtype != np.uint8 or img_bgra.ndim != 3 or img_bgra.shape[2] != 4 or not img_bgra.flags.c_contiguous:
+            raise ValueError("the image must be a C-contiguous uint8 array [h, w, 4]")
         h, w = img_bgra.shape[:2]
+        pw, ph = padded_size(w, h)
+        if dst.dtype != np.uint8 or not dst.flags.c_contiguous or not dst.flags.writeable or dst.size < pw * ph:
+            raise ValueError(f"expected {pw * ph // 16} blocks of a {pw}x{ph} texture in a C-contiguous uint8 array")
         err = np.zeros(2, np.int64)
         ssim = np.zeros(2, np.float64)
         s = self.settings()
@@ -237,7 +243,7 @@ def encode_image(img_bgra: np.ndarray, flags: str = "", preset: Preset = DEFAULT
         ph, pw = padded.shape[:2]
     core = Bc7Core(preset)
     core.init_tables(o["draft"], o["normal"], o["slow"], o["linear"])
-    blocks = np.zeros(((ph // 4) * (pw // 4), 16), np.uint8) if start is None else np.array(start, np.uint8)
+    blocks = np.zeros(((ph // 4) * (pw // 4), 16), np.uint8) if start is None else np.array(start, np.uint8, order="C")
     stats = None
     if on_device:
         try:

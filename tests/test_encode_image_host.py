@@ -56,3 +56,40 @@ def test_other_errors_are_raised(library):
     with pytest.raises(nb.NativeError) as e:
         nb.encode_image(np.zeros((4, 4, 4), np.uint8))
     assert e.value.code == 2 and "nebc7_encode_host" not in lib.calls
+
+
+IMAGE = np.zeros((13, 8, 4), np.uint8)
+BLOCKS = np.zeros((8, 16), np.uint8)     # of the 8x16 padded texture
+
+
+def read_only(a):
+    a = a.copy()
+    a.flags.writeable = False
+    return a
+
+
+@pytest.mark.parametrize("dst,img", [
+    (BLOCKS, IMAGE[:, ::2]), (BLOCKS, IMAGE.astype(np.int32)), (BLOCKS, np.zeros((13, 8, 3), np.uint8)),
+    (BLOCKS, np.zeros((13, 8), np.uint8)), (BLOCKS, np.asfortranarray(IMAGE)), (BLOCKS[:7], IMAGE), (BLOCKS[::2], IMAGE),
+    (BLOCKS.astype(np.uint16), IMAGE), (read_only(BLOCKS), IMAGE)])
+def test_process_image_refuses_what_it_cannot_pass_on(library, dst, img):
+    """The library reads and writes through bare pointers."""
+    lib = library()
+    with pytest.raises(ValueError):
+        nb.Bc7Core().process_image(dst, img, 1)
+    assert lib.calls == []
+
+
+def test_process_image_takes_whole_images(library):
+    lib = library()
+    for dst in (BLOCKS.copy(), np.zeros(200, np.uint8)):
+        nb.Bc7Core().process_image(dst, IMAGE, -1)
+    assert lib.calls == ["nebc7_encode_image_host"] * 2
+
+
+def test_starting_blocks_short_of_the_texture_are_refused(library):
+    lib = library()
+    with pytest.raises(ValueError):
+        nb.encode_image(IMAGE, start=BLOCKS[:5])
+    nb.encode_image(IMAGE, start=np.asfortranarray(BLOCKS))
+    assert lib.calls[-1] == "nebc7_encode_image_host"
