@@ -176,11 +176,11 @@ int nebc7_limit_staged_records(long long bytes);
    the blocks are the same; the tests reach that path so. */
 int nebc7_limit_staged_rooms(int results, int later, int handed);
 
-/* The steps of an encode with these settings as its pass structure counts
-   them (the block order's two, then one, or for the full-search presets a
-   list and a step per pass and two per round of a split pass): a fixed
-   number per preset.  The kernels that run them, which is what is launched,
-   are nebc7_encode_kernels'.  A negative error code for invalid settings. */
+/* Deprecated: a constant per preset, kept for existing callers (1 for the
+   draft-only presets, 3 for the default one, 78 for the others).  It counted the
+   steps of an earlier pass structure and says nothing about what is launched
+   now: that is nebc7_encode_kernels.  A negative error code for invalid
+   settings. */
 int nebc7_encode_launches(const nebc7_settings* settings);
 
 /* How many kernels an encode with these settings launches, not counting the

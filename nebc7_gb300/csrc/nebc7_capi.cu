@@ -1881,11 +1881,7 @@ int nebc7_encode_launches(const nebc7_settings* settings)
 		return -SetError(e);
 	if (!OrdersBlocks(*settings))
 		return 1;
-	if (settings->denoise && !settings->doSlow && !settings->linearData)
-		return 3;
-	/* 14 passes after the first: a list and a kernel each, and for the five
-	   split ones a preparation, a remainder and two steps per round */
-	return 2 + 1 + 2 * (14 - 5) + (3 + 2 * 3) * 3 + (3 + 2 * 4) + (3 + 2 * 8);
+	return settings->denoise && !settings->doSlow && !settings->linearData ? 3 : 78;
 }
 
 int nebc7_encode_kernels(const nebc7_settings* settings)
