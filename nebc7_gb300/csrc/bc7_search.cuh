@@ -1197,24 +1197,6 @@ __device__ NEBC7_PASS void FullTwoSubsets(WarpState& st, SearchState& ss, CellRe
 /* Modes 6, 6Index2, 7: four channels with the transparent-alpha term       */
 /* ---------------------------------------------------------------------- */
 
-/* Error of every lane's candidate over a plane of np pixels (rows up to the
-   next multiple of four are zero): terms from the candidate table's column
-   `at`.  Ends once no lane is below its limit, so a lane's value is exact
-   whenever it is below it.  Warp-collective: every lane calls it. */
-__device__ __forceinline__ int TableError(const int4* plane, const int4* table, int at, int np, int limit)
-{
-	int sum = 0;
-	for (int i = 0; i < np; i += 4)
-	{
-#pragma unroll
-		for (int j = 0; j < 4; j++)
-			sum += RowMin(plane[i + j], table[(i + j) * kTableRow + at]);
-		if (!__any_sync(kFull, sum < limit))
-			break;
-	}
-	return sum;
-}
-
 /* The four-channel combination search with 2-bit indices (modes 7 and
    6Index2; src/Bc7CoreMode6.cpp:1163-1331) over the lists of variant v.
  *
@@ -1872,8 +1854,8 @@ __device__ __forceinline__ bool Mode7Open(WarpState& st, const CellRegs& R, cons
    The estimates take the subset's whole water where the reference takes what
    the earlier channels leave: an estimate below that rest is the same (a
    candidate below it lies in both windows), and one that is not ends the
-   subset either way.  A hard partition of an alpha block takes 2 ms in a
-   team where one warp took 8. */
+   subset either way.  A hard partition of an alpha block takes a team 2 to
+   4 ms, a warp alone three to four times as long. */
 template<int kD>
 __device__ __forceinline__ bool Mode7PartitionTeam(WarpState& st, SearchState& ss, TeamState& ts, size_t stateStride, CellRegs& R, const Params& P,
 	const LevelTables& T, int p, int rank, int lane)

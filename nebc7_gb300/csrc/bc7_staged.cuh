@@ -152,7 +152,12 @@ __host__ __device__ constexpr bool ThreeSubsetStep(int S)
 }
 
 constexpr int kInlineCandidates = 6;
-constexpr int kHandOverBlocks = 8192;   /* a longer list fills the GPU as it is (precise 1024x1024, 65536 blocks: 40.1 ms inline, 45.6 handed over) */
+/* A longer list fills the GPU as it is.  Precise photos handed over and inline:
+   64x64 1.98 and 3.82 ms, 256x256 9.73 and 10.25, 320x320 12.0 and 11.5, 512x512
+   23.3 and 19.7, 1024x1024 44.8 and 39.6; /data normal maps 256x256 (short lists)
+   2.15 and 5.28, 512x512 4.21 and 8.00: from 5000 blocks to this line the
+   precise preset loses 5 %, beyond it handing over would lose more. */
+constexpr int kHandOverBlocks = 8192;
 constexpr int kHandedBlocks = 2048;   /* blocks whose estimates a pass can hand over; the others finish inline */
 
 /* Candidates (tasks) per block of split pass S, and its mode. */
@@ -1037,7 +1042,7 @@ __device__ __forceinline__ void SplitCommit(const Job& job, const Stages& sg, Sp
 		R.errTotal = now.errTotal;
 		R.opaqueAlphaError = now.opaqueAlphaError;
 		R.denoiseStep = now.denoiseStep;
-			R.a1.opaque = now.opaque != 0;
+		R.a1.opaque = now.opaque != 0;
 		r.handed = 0;
 		Publish(sg, k, NextStep(S, R, d.P), now.errTotal, now.bestMode, now.opaque != 0, now.denoise);
 	}
@@ -1093,7 +1098,10 @@ __host__ __device__ constexpr int SplitTeam(int S)
 /* From this many blocks on, a team takes four mode 7 candidates at a time, whose
    bounds its warps compute beside each other: three of four candidates end
    there (1118x1105 alpha texture, 3455 blocks: 13.5 -> 11.4 ms).  A shorter list
-   would leave CTAs without a task while others search four in turn. */
+   would leave CTAs without a task while others search four in turn.  Whole
+   encodes of alpha textures one and four at a time: 64x64 5.5 and 5.9 ms, 256x256
+   13.8 and 15.2, 512x512 21.7 and 20.4, 1024x1024 32.9 and 31.3; /slow 256x256
+   15.6 and 17.0, 512x512 24.1 and 22.6. */
 constexpr int kGrabBlocks = 1024;
 
 /* Split pass S over the blocks list[i], i < *count (at most kSplitMaxBlocks).
@@ -1274,6 +1282,7 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 #pragma unroll
 		for (int j = 0; j < 8; j++)
 			base[lane * 8 + j] = incl - run + c[j];
+		__syncwarp();   /* the first lane's entries before the mark of an empty list */
 		if (blockIdx.x == 0 && lane == 31)
 			sg.count[stage] = incl;
 		if (stage == kStepRefine && blockIdx.x == 0 && lane == kRefineHeavy / 8)

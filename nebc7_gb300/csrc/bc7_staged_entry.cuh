@@ -122,7 +122,8 @@ cudaError_t StagedEncodeOccupancy(int* ctasPerSm)
 	const cudaError_t e = PrepareStagesFrom<kD, kStageDraft>();
 	if (e != cudaSuccess)
 		return e;
-	/* every stage kernel has the refining kernel's shared memory and bounds */
+	/* every stage kernel is compiled for four CTAs per SM, and the 7.6 to 53 KB
+	   of shared memory that one takes leave room for them */
 	return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctasPerSm, KEncodeStage<kD, kStepFull3Mode2>, kWarpsPerCta * 32,
 		StageSharedBytes(kStepFull3Mode2, false));
 }
