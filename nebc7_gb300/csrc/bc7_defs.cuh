@@ -95,7 +95,7 @@ struct LevelTables
 	const uint16_t* c3v7s; /* [256][128]     */
 	const uint16_t* c3v5;  /* [256][32]      */
 	const uint8_t* d4h;    /* [511][256] nibbles, by differences (HalfAt) */
-	const uint8_t* d2h;    /* [511][256] nibbles, by differences (HalfAt) */
+	const uint8_t* d2h;    /* [511][256] nibbles, by differences (HalfAt); the encode reads h2s, built from it */
 	const uint8_t* d3v8;   /* [511][512] bytes of 3-bit indices, by differences (DiffAt) */
 	const uint8_t* h4s;    /* [511][512] squares of the d4h entries, a byte each, by differences (DiffAt) */
 	const uint8_t* h2s;    /* [511][512] squares of the d2h entries */
