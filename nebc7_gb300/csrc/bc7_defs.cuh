@@ -15,18 +15,18 @@ namespace nebc7 {
 /* Marks the routines that many passes call (candidate lists, estimates,
    combination searches, subset statistics).  Out of line, a kernel with all
    passes holds one copy of each; the staged kernels, with one pass each, and the
-   default preset's single kernel inline them. */
+   draft-only ones inline them. */
 #ifndef NEBC7_SHARED
 #define NEBC7_SHARED __noinline__
 #endif
 
 /* Marks the pass-level routines of the refinement and full searches (one
    refinement, one full search of a mode, a subset search, an estimate
-   pass).  The single kernels of the precise preset and of mixed launches define
-   it __noinline__: with the passes inlined into the kernel body its code
-   outgrows the instruction cache, and warps that sit in different passes stall on
-   instruction fetch.  The kernels that inline NEBC7_SHARED inline it too; empty
-   by default (the compiler decides). */
+   pass).  The single refining kernels define it __noinline__: with the passes
+   inlined into the kernel body its code outgrows the instruction cache, warps
+   that sit in different passes stall on instruction fetch, and the thread's stack
+   grows with it.  The staged kernels inline it; empty by default (the compiler
+   decides). */
 #ifndef NEBC7_PASS
 #define NEBC7_PASS
 #endif
