@@ -162,7 +162,7 @@ int nebc7_decode_blocks_host(const uint8_t* blocks, uint8_t* bgra, int n);
    build of the reference (they are tested against the CPU restatement). */
 int nebc7_set_pca(int on);
 
-/* Limits the records of the staged form, 280 bytes per block and up to 7 MB,
+/* Limits the records of the staged form, at most 172 bytes per block and 14 MB,
    for the encodes, batches and servers that the calling thread makes from here
    on (negative: no limit but the device's free memory).  A launch without room
    for them runs the single kernel, a server's streams hold those of fewer blocks;
@@ -342,9 +342,9 @@ typedef struct nebc7_server_counters
    request of a draft-only batch returns (its blocks copied back) as soon as
    its own blocks are done, while the rest of the launch still runs.  Besides
    the arena, every stream holds the staged form's per-block state (its record,
-   pass lists, split-pass rounds and kept results): 280 bytes per block, and up
-   to 7 MB, for up to min(4194304, hbm_budget / 104 + 1) blocks, or half as many
-   as often as it takes where that is not free.  A request of more blocks runs
+   pass lists, split-pass rounds and kept results): at most 172 bytes per block
+   and 14 MB, for up to min(4194304, hbm_budget / 104 + 1) blocks, or half as
+   many as often as it takes where that is not free.  A request of more blocks runs
    the single kernel. */
 int nebc7_server_create(const nebc7_server_config* cfg, nebc7_server** out);
 

@@ -1330,21 +1330,35 @@ cudaError_t StagedEncodeOccupancy(int* ctasPerSm);
 constexpr size_t kStagedZeroed = 256 + kSplitPasses * sizeof(SplitQueue) + 2 * size_t(kNumStages) * 1024;
 static_assert(kStagedZeroed % 256 == 0 && kNumStages < 32, "the counts and queue heads take 128 bytes each");
 
-/* Results a pass keeps.  A slot has to fit its field of a firstImp word, below
-   the mark: with more room than that, results past 2^24 ran into the
-   candidate's bits and another block's was taken for them.  What finds no slot
-   is searched again by the remainder. */
+/* Spare entries past one a block in the rooms of a large launch: all that the
+   blocks a pass hands over can ask for. */
+constexpr size_t kSplitSpare = size_t(kHandedBlocks) * kSplitMaxTasks;
+
+constexpr size_t LeastOf(size_t a, size_t b, size_t c)
+{
+	return a < b ? (a < c ? a : c) : (b < c ? b : c);
+}
+
+/* Results a pass keeps: three a block of a small launch, one of a large one
+   (noise and two-colour blocks keep up to 0.65 a block in a pass of modes 1, 3, 4
+   or 5, photos and alpha textures 0.005; the blocks handed over by modes 2 and 0
+   up to 4 each).  A slot has to fit its field of a firstImp word, below the mark:
+   with more room than that, results past 2^24 ran into the candidate's bits and
+   another block's was taken for them.  What finds no slot is searched again by
+   the remainder. */
 constexpr size_t SplitResultCap(int n)
 {
-	return 3 * size_t(n) + 1024 < size_t(kSplitNoSlot) ? 3 * size_t(n) + 1024 : size_t(kSplitNoSlot);
+	return LeastOf(3 * size_t(n) + 1024, size_t(n) + kSplitSpare, size_t(kSplitNoSlot));
 }
 
 static_assert(SplitResultCap(0x7FFFFFFF) == size_t(kSplitNoSlot) && kSplitMaxTasks << kSplitSlotBits <= kSplitNone,
 	"candidates and slots fit a firstImp word");
 
+/* Entries of a pass's later rounds (up to 0.45 a block in those textures); their
+   tasks stay an int. */
 constexpr size_t SplitLaterCap(int n)
 {
-	return n < (1 << 22) - 1024 ? 4 * size_t(n) + 1024 : size_t(1) << 24;   /* its tasks stay an int too */
+	return LeastOf(4 * size_t(n) + 1024, size_t(n) + kSplitSpare, size_t(1) << 24);
 }
 
 constexpr size_t HandedCap(int n)

@@ -25,7 +25,7 @@ int main(int argc, char** argv)
 }
 """
 
-SIZES = [1, 1000, 1 << 20, 5_591_000, 5_592_000, 1 << 23, 1 << 24, 1 << 28]
+SIZES = [1, 1000, 43_000, 65_536, 1 << 20, 5_591_000, 5_592_000, 1 << 23, 1 << 24, 1 << 28]
 
 
 @pytest.fixture(scope="module")
@@ -43,8 +43,17 @@ def test_kept_results_fit_their_field(rooms, n):
     """A kept result's slot shares a 32-bit word with its candidate (up to 63):
     24 bits, all ones for "not kept"."""
     results = rooms[n][0]
-    assert results == min(3 * n + 1024, 0xFFFFFF)
+    assert results == min(3 * n + 1024, n + 2 ** 17, 0xFFFFFF)
     for slot in (0, results - 1):
         word = (63 << 24) | slot
         assert (word >> 24, word & 0xFFFFFF) == (63, slot) and slot != 0xFFFFFF and word < 0x7FFFFFFF
     assert rooms[n][3] >= n * (96 + 6 * 4) + results * rooms[n][4]
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_state_bytes(rooms, n):
+    """The bound the header gives, and later rounds whose tasks (64 a block) an
+    int can number."""
+    results, later, handed, total, _ = rooms[n]
+    assert total <= 172 * n + 14_000_000
+    assert handed == min(n, 2048) and later >= min(n, 1 << 24) and later * 64 <= 2 ** 30
