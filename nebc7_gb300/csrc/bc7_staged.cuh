@@ -206,8 +206,8 @@ struct __align__(16) SplitQueue
 };
 
 /* Waits for the kernels before this one in its stream.  Every kernel of the
-   staged form starts with this and is launched as the programmatic dependent of
-   the one before it, so that its launch overlaps that one's end; a pass without
+   staged form starts with this and can be launched as the programmatic dependent
+   of the one before it, so that its launch overlaps that one's end; a pass without
    blocks then returns at once.  Of the chain's 24 to 32 kernels most find nothing
    to do in an easy texture: 64x64 of one colour 371 -> 310 us a call, a 64x64
    photo 724 -> 650, loose cells 287 -> 216. */
@@ -1312,11 +1312,11 @@ static __global__ void __launch_bounds__(1024) KStageList(Stages sg, int stage, 
 }
 
 /* Host-side launcher of a staged encode: the draft kernel, then for each
-   pass its list and its kernel, then the finish kernel's list and kernel.
-   The launches are capturable.  Compiled per kD in encode_*_staged.cu. */
+   pass its list and its kernel, then the finish kernel's list and kernel; chain:
+   as programmatic dependents (WaitForLaunch).  The launches are capturable.  Compiled per kD in encode_*_staged.cu. */
 template<int kD>
-cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, const LevelTables& T0,
-	const LevelTables& T1);
+cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, bool chain,
+	const LevelTables& T0, const LevelTables& T1);
 
 /* Raises the stage kernels' dynamic shared-memory limit (once per process
    and device, before the first launch) and reports CTAs per SM. */

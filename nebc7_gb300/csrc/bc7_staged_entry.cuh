@@ -16,10 +16,10 @@ inline int StageGrid(int grid, long long tasks, int warps)
 	return ctas < 1 ? 1 : (ctas < grid ? int(ctas) : grid);
 }
 
-/* Launches a kernel of the staged form as the programmatic dependent of the one
-   before it (WaitForLaunch). */
+/* Launches a kernel of the staged form; chain: as the programmatic dependent
+   of the one before it (WaitForLaunch). */
 template<class... P, class... A>
-cudaError_t LaunchChained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const A&... args)
+cudaError_t LaunchChained(void (*kernel)(P...), bool chain, int grid, int threads, size_t smem, cudaStream_t stream, const A&... args)
 {
 	cudaLaunchAttribute chained = {};
 	chained.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -30,7 +30,7 @@ cudaError_t LaunchChained(void (*kernel)(P...), int grid, int threads, size_t sm
 	config.dynamicSmemBytes = smem;
 	config.stream = stream;
 	config.attrs = &chained;
-	config.numAttrs = 1;
+	config.numAttrs = chain ? 1 : 0;
 	return cudaLaunchKernelEx(&config, kernel, P(args)...);
 }
 
@@ -39,7 +39,8 @@ cudaError_t LaunchChained(void (*kernel)(P...), int grid, int threads, size_t sm
    then a split pass's blocks that must run whole (OPTION_PCA, results not
    kept), in one warp each from their start candidates. */
 template<int kD, int STAGE>
-cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Stages& sg, const LevelTables& T0, const LevelTables& T1)
+cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool chain, const LevelTables& T0,
+	const LevelTables& T1)
 {
 	constexpr int split = SplitIndex(STAGE), threads = kWarpsPerCta * 32;
 	constexpr bool three = ThreeSubsetStep(STAGE), draft = STAGE == kStageDraft;
@@ -47,13 +48,13 @@ cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Sta
 	if (!draft)
 	{
 		const int ctas = (job.total + 1023) / 1024;
-		e = LaunchChained(KStageList, ctas < 152 ? ctas : 152, 1024, 0, stream, sg, STAGE, split, split >= 0 && !three ? SplitTasks(STAGE) : 0);
+		e = LaunchChained(KStageList, chain, ctas < 152 ? ctas : 152, 1024, 0, stream, sg, STAGE, split, split >= 0 && !three ? SplitTasks(STAGE) : 0);
 	}
 	const int stageGrid = StageGrid(grid, job.total, TeamStage(STAGE) ? kWarpsPerCta : 1);
 	if constexpr (split < 0 || three)
 	{
 		if (e == cudaSuccess)
-			e = LaunchChained(KEncodeStage<kD, STAGE>, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg,
+			e = LaunchChained(KEncodeStage<kD, STAGE>, chain, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg,
 				draft ? nullptr : sg.list, draft ? nullptr : sg.count + STAGE, sg.counters + (STAGE + 1), T0, T1);
 	}
 	if constexpr (split >= 0)
@@ -61,11 +62,11 @@ cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Sta
 		/* a small texture's tasks fill more SMs than its blocks */
 		const int blocks = three ? sg.handedCap : job.total;
 		if (e == cudaSuccess)
-			e = LaunchChained(KEncodeSplit<kD, STAGE>, StageGrid(grid, (long long)blocks * SplitTasks(STAGE), SplitTeam(STAGE)), threads,
+			e = LaunchChained(KEncodeSplit<kD, STAGE>, chain, StageGrid(grid, (long long)blocks * SplitTasks(STAGE), SplitTeam(STAGE)), threads,
 				StageSharedBytes(STAGE, true), stream, job, sg, three ? sg.handed : sg.list,
 				three ? &sg.split[split].handedCount : sg.count + STAGE, T0, T1);
 		if (e == cudaSuccess)
-			e = LaunchChained(KEncodeStage<kD, STAGE>, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg, sg.rest,
+			e = LaunchChained(KEncodeStage<kD, STAGE>, chain, stageGrid, threads, StageSharedBytes(STAGE, false), stream, job, sg, sg.rest,
 				&sg.split[split].restCount, &sg.split[split].restHead, T0, T1);
 	}
 	return e;
@@ -73,24 +74,24 @@ cudaError_t LaunchStage(int grid, cudaStream_t stream, const Job& job, const Sta
 
 /* The passes from STAGE on. */
 template<int kD, int STAGE>
-cudaError_t LaunchStagesFrom(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, const LevelTables& T0,
-	const LevelTables& T1)
+cudaError_t LaunchStagesFrom(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, bool chain,
+	const LevelTables& T0, const LevelTables& T1)
 {
 	if constexpr (STAGE < kNumStages)
 	{
 		if (StageLaunched(STAGE, slow))
-			if (const cudaError_t e = LaunchStage<kD, STAGE>(grid, stream, job, sg, T0, T1))
+			if (const cudaError_t e = LaunchStage<kD, STAGE>(grid, stream, job, sg, chain, T0, T1))
 				return e;
-		return LaunchStagesFrom<kD, STAGE + 1>(grid, stream, job, sg, slow, T0, T1);
+		return LaunchStagesFrom<kD, STAGE + 1>(grid, stream, job, sg, slow, chain, T0, T1);
 	}
 	return cudaSuccess;
 }
 
 template<int kD>
-cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, const LevelTables& T0,
-	const LevelTables& T1)
+cudaError_t LaunchStagedEncode(int grid, cudaStream_t stream, const Job& job, const Stages& sg, bool slow, bool chain,
+	const LevelTables& T0, const LevelTables& T1)
 {
-	return LaunchStagesFrom<kD, kStageDraft>(grid, stream, job, sg, slow, T0, T1);
+	return LaunchStagesFrom<kD, kStageDraft>(grid, stream, job, sg, slow, chain, T0, T1);
 }
 
 template<int kD, int STAGE>
@@ -131,6 +132,6 @@ cudaError_t StagedEncodeOccupancy(int* ctasPerSm)
 } // namespace nebc7
 
 #define NEBC7_INSTANTIATE_STAGED(KD) \
-	template cudaError_t nebc7::LaunchStagedEncode<KD>(int, cudaStream_t, const nebc7::Job&, const nebc7::Stages&, bool, \
+	template cudaError_t nebc7::LaunchStagedEncode<KD>(int, cudaStream_t, const nebc7::Job&, const nebc7::Stages&, bool, bool, \
 		const nebc7::LevelTables&, const nebc7::LevelTables&); \
 	template cudaError_t nebc7::StagedEncodeOccupancy<KD>(int*);
